@@ -26,6 +26,7 @@ SOURCES = [
     "capi.cu",
     "vm_vector.cu",
     "mm_tcgen05.cu",
+    "mm_tile.cu",
     "attn_tcgen05.cu",
 ]
 

@@ -206,6 +206,113 @@ __device__ __forceinline__ void run_epilogue(const MmParam &P, const EpiPos &pos
   }
 }
 
+__device__ __forceinline__ float load_bias(const MmParam &P, uint32_t col) {
+  if (P.bias_dtype == T_F32) return __ldg(reinterpret_cast<const float *>(P.bias_ptr) + col);
+  const unsigned short raw = __ldg(reinterpret_cast<const unsigned short *>(P.bias_ptr) + col);
+  if (P.bias_dtype == T_BF16) return __uint_as_float(static_cast<uint32_t>(raw) << 16);
+  return __half2float(__ushort_as_half(raw));
+}
+
+// tile index -> (batch, m block, n block), grouped along M so that the A panel of a group stays in L2 while
+// the group sweeps over N
+__device__ __forceinline__ void tile_coords(uint32_t t, uint32_t mblocks, uint32_t nblocks, uint32_t kGroupM, uint32_t &bz,
+                                            uint32_t &mb, uint32_t &nb) {
+  const uint32_t per_batch = mblocks * nblocks;
+  bz = t / per_batch;
+  t -= bz * per_batch;
+  const uint32_t group_tiles = kGroupM * nblocks;
+  const uint32_t g = t / group_tiles;
+  const uint32_t first_m = g * kGroupM;
+  const uint32_t gm = min(kGroupM, mblocks - first_m);
+  const uint32_t in_group = t - g * group_tiles;
+  mb = first_m + in_group % gm;
+  nb = in_group / gm;
+}
+
+// Bias of column `col` as fp32 (0 without a bias or past the last column).
+__device__ __forceinline__ float bias_at(const MmParam &P, uint32_t col) {
+  return P.bias_ptr != 0 && col < P.N ? load_bias(P, col) : 0.0f;
+}
+// Adds sixteen columns' bias from shared memory (staged as fp32 while the product was being made: read from global memory
+// here, each strip waited for its own loads).
+__device__ __forceinline__ void add_bias_staged(uint32_t saddr, uint32_t (&r)[16]) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    float4 b;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "r"(saddr + 16u * g));
+    r[4 * g + 0] = f2u(u2f(r[4 * g + 0]) + b.x);
+    r[4 * g + 1] = f2u(u2f(r[4 * g + 1]) + b.y);
+    r[4 * g + 2] = f2u(u2f(r[4 * g + 2]) + b.z);
+    r[4 * g + 3] = f2u(u2f(r[4 * g + 3]) + b.w);
+  }
+}
+
+// Sixteen fp32 values in the operand type, packed two at a time (hardware round to nearest even, NaN kept).
+__device__ __forceinline__ void pack_strip(uint32_t dtype, const uint32_t (&v)[16], uint32_t (&pk)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (dtype == T_BF16) {
+      pk[i] = pack_bf16x2(u2f(v[2 * i]), u2f(v[2 * i + 1]));
+    } else {
+      const __half2 h = __floats2half2_rn(u2f(v[2 * i]), u2f(v[2 * i + 1]));
+      pk[i] = *reinterpret_cast<const uint32_t *>(&h);
+    }
+  }
+}
+
+// Rounding to the operand type and the post-fusion program for one 16-column strip of one row (bias already added).
+// When the whole program is a store in the operand type (plain or gated), the sixteen 16-bit results come back in `pk` and
+// the slot of their tensor is returned: the caller stores them through shared memory, so that rows of any alignment leave
+// as contiguous runs.  Any other program is stored from here and 0xffffffff is returned.
+__device__ __forceinline__ uint32_t finish_strip(const MmParam &P, const EpiPos &pos, uint32_t (&r)[16], uint32_t (&pk)[8]) {
+  pack_strip(P.in_dtype, r, pk);   // the product in the operand type
+  if (P.fast_store_slot != 0xffffffffu && P.tensor[P.fast_store_slot].dtype == P.in_dtype) return P.fast_store_slot;
+  // back to the 32-bit register form of the rounded product
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (P.in_dtype == T_BF16) {
+      r[2 * i] = pk[i] << 16;
+      r[2 * i + 1] = pk[i] & 0xffff0000u;
+    } else {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&pk[i]));
+      r[2 * i] = __float_as_uint(f.x);
+      r[2 * i + 1] = __float_as_uint(f.y);
+    }
+  }
+  if (P.gate_slot != 0xffffffffu) {
+    // y = x / (c2 + exp(c1 * (x + c0 * x^3))): each step rounded on its own, as the interpreter's words are
+    const float c0 = __uint_as_float(P.gate_c[0]), c1 = __uint_as_float(P.gate_c[1]), c2 = __uint_as_float(P.gate_c[2]);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float x = __uint_as_float(r[i]);
+      float a = __fmul_rn(x, x);
+      a = __fmul_rn(a, x);
+      a = __fmul_rn(a, c0);
+      a = __fadd_rn(a, x);
+      a = __fmul_rn(a, c1);
+      a = fast_exp(a);
+      a = __fadd_rn(a, c2);
+      r[i] = f2u(fast_div(x, a));
+    }
+    pack_strip(P.in_dtype, r, pk);
+    return P.gate_slot;
+  }
+  if (pos.valid == 0) return 0xffffffffu;
+  if (P.fast_store_slot != 0xffffffffu && pos.valid == 16u) {
+    // one store of the product widened to fp32 (a partial product that another launch finishes)
+    const EpiTensor &t = P.tensor[P.fast_store_slot];
+    uint8_t *dst = reinterpret_cast<uint8_t *>(t.ptr) + (epi_offset(t, pos) << 2);
+    if (t.dtype == T_F32 && (reinterpret_cast<uint64_t>(dst) & 15u) == 0) {
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+        *reinterpret_cast<uint4 *>(dst + 16 * g) = make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+      return 0xffffffffu;
+    }
+  }
+  run_epilogue(P, pos, r);
+  return 0xffffffffu;
+}
+
 }  // namespace
 }  // namespace dvmb
 

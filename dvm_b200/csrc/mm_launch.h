@@ -2,6 +2,8 @@
 #ifndef DVM_B200_MM_LAUNCH_H_
 #define DVM_B200_MM_LAUNCH_H_
 
+#include <cuda.h>
+
 #include <cstdint>
 
 #include "isa.h"
@@ -55,9 +57,21 @@ struct MmParam {
 
 // Enqueue the MatMul.  Returns 0, a cudaError_t (> 0), or a negative code for an unsupported shape.
 int LaunchMatMul(const MmParam &p, void *stream);
-// True when the tcgen05 path can take this problem (TMA alignment rules); otherwise LaunchMatMul runs the
-// general SIMT kernel.
-bool MatMulUsesTensorCores(const MmParam &p);
+// True when the copy engine cannot address an operand (rows of `inner` 16-bit elements, batch slices of `slice`): base, row
+// pitch or slice not a multiple of 16 bytes.  Its tiles are then loaded by the tile kernel's work warps.
+bool MmOperandNeedsGather(uint64_t ptr, uint64_t inner, uint64_t slice, uint32_t batches);
+inline bool MmGatherA(const MmParam &p) {
+  return MmOperandNeedsGather(p.a_ptr, p.a_mmajor ? p.M : p.K, static_cast<uint64_t>(p.M) * p.K, p.a_batches);
+}
+inline bool MmGatherB(const MmParam &p) {
+  return MmOperandNeedsGather(p.b_ptr, p.b_kmajor ? p.K : p.N, static_cast<uint64_t>(p.N) * p.K, p.b_batches);
+}
+inline bool MmNeedsGather(const MmParam &p) { return MmGatherA(p) || MmGatherB(p); }
+// The tile kernel (mm_tile.cu): 128 x bn tiles (bn 64 or 128), K cut into `split` (1, 2, 4, 8) parts.
+int LaunchMmTile(const MmParam &p, uint32_t bn, uint32_t split, void *stream);
+unsigned int ReadMmTileStatus();
+// 3-d tensor map over a [batches, rows, inner] 16-bit operand: boxes of box_rows rows of 64 elements, 128-byte swizzle.
+int EncodeMmOperand(CUtensorMap *map, uint64_t ptr, uint64_t inner, uint64_t rows, uint64_t batches, uint32_t box_rows);
 unsigned int ReadMatMulStatus();
 
 // Fused attention  O[b,h] = softmax(scale * Q[b,h] K[b,h]^T) V[b,h]  (non-causal), bf16 or fp16 operands,

@@ -7,22 +7,24 @@
 // MatMul at all (src/system.cc:290-294).  Semantics kept: fp16/bf16 operands, fp32 accumulation, optional bias
 // added in fp32, result rounded to the operand dtype, then the fused vector ops.
 //
-// One CTA = one 128 x 256 tile of C at a time (persistent over tiles, grouped along M for L2 reuse):
-//   warp 0     TMA producer: A [128 x 64] and B [256 x 64] per stage (64 x 64 boxes when the operand is stored
+// Two CTAs of a cluster = one 256 x 256 tile of C at a time (persistent over tiles, grouped along M for L2 reuse):
+//   warp 0     TMA producer: A [128 x 64] and half of B [128 x 64] per stage (64 x 64 boxes when the operand is stored
 //              with the contraction axis outermost)
 //   warp 1     MMA issuer: four tcgen05.mma (K = 16) per stage into one of two TMEM accumulators
-//   warps 2-5  epilogue: tcgen05.ld 16 columns at a time, bias, rounding, post-fusion program, stores
+//   warps 2-9  epilogue: tcgen05.ld 16 columns at a time, bias, rounding, post-fusion program; 16-bit results leave as
+//              runs of 128 bytes per row through shared memory
 // Every mbarrier wait is bounded; on expiry a status word is set and the kernel runs to its end.
 //
-// Problems the copy engine cannot address (row pitch or base not 16-byte aligned) run on a plain SIMT kernel
-// with the same epilogue.
+// Problems that do not fill the machine with such tiles, and problems the copy engine cannot address (row pitch or base
+// not 16-byte aligned), run as smaller tiles (mm_tile.cu).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cstddef>
 #include <cstdint>
-#include <cstdio>
 #include <cstdlib>
 #include <cstring>
 
@@ -36,185 +38,60 @@ __device__ WaitStatus g_mm_status = {0u, 0u};
 
 namespace {
 
-// Tile geometry.  One CTA owns 128 rows x 256 columns of C at a time.  In the paired form (CTAS = 2) the two CTAs
-// of a cluster share one MMA of 256 x 256: each stages its own 128 rows of A and one half (128 columns) of B, so
-// a CTA moves 32 KB per k-block instead of 48 KB.
+// Tile geometry.  The two CTAs of a cluster share one MMA of 256 x 256: each stages its own 128 rows of A and one half
+// (128 columns) of B, i.e. 32 KB per k-block.
 constexpr uint32_t BM = 128, BN = 256, BK = 64;
 constexpr uint32_t kABytes = BM * BK * 2;   // 16 KB
 constexpr uint32_t kEpiWarps = 8;
+constexpr uint32_t kEpiCols = BN / (kEpiWarps / 4);   // columns of the tile a warp drains
 constexpr uint32_t kThreads = 64 + 32 * kEpiWarps;
 constexpr uint32_t kTmemCols = 512;   // two 256-column fp32 accumulators
-// shared memory: [0, 1024) barriers + tmem pointer, then the stages (1024-byte aligned for the 128B swizzle)
-constexpr uint32_t kSmemHeader = 1024;
-template <int CTAS>
-struct Geo {
-  static constexpr uint32_t kBBytes = (BN / CTAS) * BK * 2;
-  static constexpr uint32_t kStageBytes = kABytes + kBBytes;
-  static constexpr uint32_t kStages = CTAS == 1 ? 4 : 6;
-  static constexpr uint32_t kSmemBytes = kSmemHeader + kStages * kStageBytes + 1024;
-};
+// shared memory: [0, 1024) barriers + tmem pointer, the bias of each epilogue warp's columns as fp32, then the stages
+// (1024-byte aligned for the 128B swizzle)
+constexpr uint32_t kBiasOff = 1024;
+constexpr uint32_t kSmemHeader = kBiasOff + kEpiWarps * kEpiCols * 4;
+constexpr uint32_t kBBytes = (BN / 2) * BK * 2;
+constexpr uint32_t kStageBytes = kABytes + kBBytes;
+constexpr uint32_t kStages = 5;
+// Results of 64 columns at a time, per epilogue warp: 32 rows of 128 bytes.  Stored from the registers of the thread that owns
+// the row, every 16-byte store was a write request of its own, and a tile's epilogue took 14 600 cycles against 5 100 for
+// ten k-blocks of MMAs; worth more than the sixth operand stage that the 32 KB would hold.
+constexpr uint32_t kOutBytes = 32 * 128;
+constexpr uint32_t kSmemBytes = kSmemHeader + kStages * kStageBytes + kEpiWarps * kOutBytes + 1024;
 
 struct MmMaps {
   CUtensorMap a, b;
 };
 
-__device__ __forceinline__ float load_bias(const MmParam &P, uint32_t col) {
-  if (P.bias_dtype == T_F32) return __ldg(reinterpret_cast<const float *>(P.bias_ptr) + col);
-  const unsigned short raw = __ldg(reinterpret_cast<const unsigned short *>(P.bias_ptr) + col);
-  if (P.bias_dtype == T_BF16) return __uint_as_float(static_cast<uint32_t>(raw) << 16);
-  return __half2float(__ushort_as_half(raw));
+// 32 rows of 64 staged columns (128 bytes, 16-byte piece p of row r at p ^ (r & 7)) to the result tensor.
+__device__ __forceinline__ void copy_out(const MmParam &P, uint32_t slot, uint32_t b0, uint32_t b1, uint32_t row0, uint32_t col0,
+                                         uint32_t saddr, uint32_t lane) {
+  const EpiTensor &t = P.tensor[slot];
+  unsigned short *const out = reinterpret_cast<unsigned short *>(t.ptr) + ((int64_t)b0 * t.sb0 + (int64_t)b1 * t.sb1 + (int64_t)row0 * t.sm + col0);
+  if (((reinterpret_cast<uint64_t>(out) | (uint64_t)(t.sm * 2)) & 15u) == 0 && col0 + 64u <= P.N) {
+    const uint32_t piece = lane & 7u;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+      const uint32_t row = 4 * i + (lane >> 3);
+      uint4 q;
+      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "r"(saddr + row * 128u + ((piece ^ (row & 7u)) << 4)));
+      if (row0 + row < P.M) *reinterpret_cast<uint4 *>(out + (int64_t)row * t.sm + piece * 8u) = q;
+    }
+    return;
+  }
+  // a ragged edge, or rows at any even address: one element per lane
+#pragma unroll 1
+  for (uint32_t row = 0; row < 32 && row0 + row < P.M; ++row)
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+      const uint32_t col = h * 32u + lane;
+      unsigned short v;
+      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(saddr + row * 128u + (((col >> 3) ^ (row & 7u)) << 4) + (col & 7u) * 2u));
+      if (col0 + col < P.N) out[(int64_t)row * t.sm + col] = v;
+    }
 }
 
-__device__ __forceinline__ float round_operand_type(uint32_t dtype, float v) {
-  return dtype == T_BF16 ? round_bf16(v) : round_f16(v);
-}
-
-// tile index -> (batch, m block, n block), grouped along M so that the A panel of a group stays in L2 while
-// the group sweeps over N
-__device__ __forceinline__ void tile_coords(uint32_t t, uint32_t mblocks, uint32_t nblocks, uint32_t kGroupM, uint32_t &bz,
-                                            uint32_t &mb, uint32_t &nb) {
-  const uint32_t per_batch = mblocks * nblocks;
-  bz = t / per_batch;
-  t -= bz * per_batch;
-  const uint32_t group_tiles = kGroupM * nblocks;
-  const uint32_t g = t / group_tiles;
-  const uint32_t first_m = g * kGroupM;
-  const uint32_t gm = min(kGroupM, mblocks - first_m);
-  const uint32_t in_group = t - g * group_tiles;
-  mb = first_m + in_group % gm;
-  nb = in_group / gm;
-}
-
-// Bias, rounding to the operand type and the post-fusion program for one 16-column strip of one row.
-__device__ __forceinline__ void finish_strip(const MmParam &P, const EpiPos &pos, uint32_t (&r)[16]) {
-  const bool whole = pos.valid == 16u;
-  if (P.bias_ptr != 0) {
-    const uint32_t bsh = P.bias_dtype == T_F32 ? 2u : 1u;
-    if (whole && ((P.bias_ptr + ((uint64_t)pos.col << bsh)) & 15u) == 0) {
-      // sixteen bias values as 16-byte loads
-      if (bsh == 2u) {
-        const uint4 *bp = reinterpret_cast<const uint4 *>(P.bias_ptr) + (pos.col >> 2);
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const uint4 b = __ldg(bp + g);
-          r[4 * g + 0] = __float_as_uint(__uint_as_float(r[4 * g + 0]) + __uint_as_float(b.x));
-          r[4 * g + 1] = __float_as_uint(__uint_as_float(r[4 * g + 1]) + __uint_as_float(b.y));
-          r[4 * g + 2] = __float_as_uint(__uint_as_float(r[4 * g + 2]) + __uint_as_float(b.z));
-          r[4 * g + 3] = __float_as_uint(__uint_as_float(r[4 * g + 3]) + __uint_as_float(b.w));
-        }
-      } else {
-        const uint4 *bp = reinterpret_cast<const uint4 *>(P.bias_ptr) + (pos.col >> 3);
-        const uint4 b0 = __ldg(bp), b1 = __ldg(bp + 1);
-        const uint32_t w[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float lo, hi;
-          if (P.bias_dtype == T_BF16) {
-            lo = __uint_as_float(w[i] << 16);
-            hi = __uint_as_float(w[i] & 0xffff0000u);
-          } else {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[i]));
-            lo = f.x;
-            hi = f.y;
-          }
-          r[2 * i] = __float_as_uint(__uint_as_float(r[2 * i]) + lo);
-          r[2 * i + 1] = __float_as_uint(__uint_as_float(r[2 * i + 1]) + hi);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if ((uint32_t)i < pos.valid) r[i] = __float_as_uint(__uint_as_float(r[i]) + load_bias(P, pos.col + i));
-    }
-  }
-  // The product in the operand type: packed two at a time (hardware round to nearest even, NaN kept).
-  uint32_t pk[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (P.in_dtype == T_BF16) {
-      pk[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-    } else {
-      const __half2 h = __floats2half2_rn(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-      pk[i] = *reinterpret_cast<const uint32_t *>(&h);
-    }
-  }
-  if (P.fast_store_slot != 0xffffffffu && whole) {
-    // the whole post-fusion program is one store of the product: write it without interpreting
-    const EpiTensor &t = P.tensor[P.fast_store_slot];
-    const size_t off = epi_offset(t, pos);
-    if (t.dtype == P.in_dtype) {
-      uint8_t *dst = reinterpret_cast<uint8_t *>(t.ptr) + (off << 1);
-      if ((reinterpret_cast<uint64_t>(dst) & 15u) == 0) {
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        *reinterpret_cast<uint4 *>(dst + 16) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-        return;
-      }
-    }
-  }
-  // back to the 32-bit register form of the rounded product
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (P.in_dtype == T_BF16) {
-      r[2 * i] = pk[i] << 16;
-      r[2 * i + 1] = pk[i] & 0xffff0000u;
-    } else {
-      const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&pk[i]));
-      r[2 * i] = __float_as_uint(f.x);
-      r[2 * i + 1] = __float_as_uint(f.y);
-    }
-  }
-  if (P.gate_slot != 0xffffffffu && whole) {
-    // y = x / (c2 + exp(c1 * (x + c0 * x^3))): each step rounded on its own, as the interpreter's words are
-    const EpiTensor &t = P.tensor[P.gate_slot];
-    uint8_t *dst = reinterpret_cast<uint8_t *>(t.ptr) + (epi_offset(t, pos) << 1);
-    if ((reinterpret_cast<uint64_t>(dst) & 15u) == 0) {
-      const float c0 = __uint_as_float(P.gate_c[0]), c1 = __uint_as_float(P.gate_c[1]), c2 = __uint_as_float(P.gate_c[2]);
-      float y[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float x = __uint_as_float(r[i]);
-        float a = __fmul_rn(x, x);
-        a = __fmul_rn(a, x);
-        a = __fmul_rn(a, c0);
-        a = __fadd_rn(a, x);
-        a = __fmul_rn(a, c1);
-        a = fast_exp(a);
-        a = __fadd_rn(a, c2);
-        y[i] = fast_div(x, a);
-      }
-      uint32_t o[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (P.in_dtype == T_BF16) {
-          o[i] = pack_bf16x2(y[2 * i], y[2 * i + 1]);
-        } else {
-          const __half2 h = __floats2half2_rn(y[2 * i], y[2 * i + 1]);
-          o[i] = *reinterpret_cast<const uint32_t *>(&h);
-        }
-      }
-      *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
-      *reinterpret_cast<uint4 *>(dst + 16) = make_uint4(o[4], o[5], o[6], o[7]);
-      return;
-    }
-  }
-  if (P.fast_store_slot != 0xffffffffu && whole) {
-    const EpiTensor &t = P.tensor[P.fast_store_slot];
-    if (t.dtype == T_F32) {
-      uint8_t *dst = reinterpret_cast<uint8_t *>(t.ptr) + (epi_offset(t, pos) << 2);
-      if ((reinterpret_cast<uint64_t>(dst) & 15u) == 0) {
-#pragma unroll
-        for (int g = 0; g < 4; ++g)
-          *reinterpret_cast<uint4 *>(dst + 16 * g) = make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
-        return;
-      }
-    }
-  }
-  run_epilogue(P, pos, r);
-}
-
-template <int CTAS>
-__device__ __forceinline__ void mm_body(const MmParam &P, const MmMaps &maps, const uint32_t epoch) {
-  using G = Geo<CTAS>;
+__device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, const uint32_t epoch) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // 1024-byte alignment of the stage area (required by the 128-byte swizzle pattern)
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -225,85 +102,68 @@ __device__ __forceinline__ void mm_body(const MmParam &P, const MmMaps &maps, co
   const uint32_t stages = base + kSmemHeader;
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t rank = CTAS == 2 ? cluster_ctarank() : 0u;   // position inside the CTA pair
-  const uint32_t unit = blockIdx.x / CTAS, num_units = gridDim.x / CTAS;
-  const uint32_t mblocks = (P.M + BM * CTAS - 1) / (BM * CTAS), nblocks = (P.N + BN - 1) / BN;
+  const uint32_t rank = cluster_ctarank();   // position inside the CTA pair
+  const uint32_t unit = blockIdx.x / 2, num_units = gridDim.x / 2;
+  const uint32_t mblocks = (P.M + BM * 2 - 1) / (BM * 2), nblocks = (P.N + BN - 1) / BN;
   const uint32_t batch = P.batch0 * P.batch1;
   const uint32_t num_tiles = mblocks * nblocks * batch;
   const uint32_t kblocks = (P.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
-    for (uint32_t s = 0; s < G::kStages; ++s) {
+    for (uint32_t s = 0; s < kStages; ++s) {
       mbar_init(bar_full + 8 * s, 1);
       mbar_init(bar_empty + 8 * s, 1);
     }
     for (uint32_t a = 0; a < 2; ++a) {
       mbar_init(bar_tfull + 8 * a, 1);
-      mbar_init(bar_tempty + 8 * a, kEpiWarps * CTAS);   // one arrival per epilogue warp of the pair
+      mbar_init(bar_tempty + 8 * a, kEpiWarps * 2);   // one arrival per epilogue warp of the pair
     }
     fence_barrier_init();
   }
   if (warp == 1) {
-    if (CTAS == 2) {
-      tmem_alloc_pair(base + 192, kTmemCols);
-      tmem_relinquish_pair();
-    } else {
-      tmem_alloc(base + 192, kTmemCols);
-      tmem_relinquish();
-    }
+    tmem_alloc_pair(base + 192, kTmemCols);
+    tmem_relinquish_pair();
   }
   tcgen05_before_sync();
-  if (CTAS == 2) {
-    cluster_sync_all();   // the peer's barriers are initialised before anything signals them
-  } else {
-    __syncthreads();
-  }
+  cluster_sync_all();   // the peer's barriers are initialised before anything signals them
   tcgen05_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
+  // (The two issuing loops run under elect.sync: inside a plain `lane == 0` branch every MMA took about 100 cycles to
+  // issue and every TMA load 150-280 - operands moved to uniform registers one by one - and a k-block 560-630 cycles
+  // whatever the tile, against 512 of tensor work.)
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
+      const bool a_m = P.a_mmajor != 0, b_k = P.b_kmajor != 0;
       uint32_t stage = 0, parity = 1;
       for (uint32_t t = unit; t < num_tiles; t += num_units) {
         uint32_t bz, mb, nb;
         tile_coords(t, mblocks, nblocks, P.group_m, bz, mb, nb);
         const uint32_t b0 = bz / P.batch1, b1 = bz - b0 * P.batch1;
         const int za = (int)(b0 * P.a_mul0 + b1 * P.a_mul1), zb = (int)(b0 * P.b_mul0 + b1 * P.b_mul1);
-        const int row0 = (int)((mb * CTAS + rank) * BM);
-        const int col0 = (int)(nb * BN + rank * (BN / CTAS));
-        for (uint32_t kb = 0; kb < kblocks; ++kb) {
+        const int row0 = (int)((mb * 2 + rank) * BM);
+        const int col0 = (int)(nb * BN + rank * (BN / 2));
+        int k = 0;
+        for (uint32_t kb = 0; kb < kblocks; ++kb, k += (int)BK) {
           mbar_wait(bar_empty + 8 * stage, parity, 1, &g_mm_status, epoch);
-          const uint32_t sa = stages + stage * G::kStageBytes, sb = sa + kABytes;
+          const uint32_t sa = stages + stage * kStageBytes, sb = sa + kABytes;
           // the pair's first CTA counts the bytes of both CTAs on its barrier
-          uint32_t full = bar_full + 8 * stage;
-          if (CTAS == 2) {
-            if (rank == 0) mbar_expect_tx(full, 2 * G::kStageBytes);
-            full = map_to_cta(full, 0);
-          } else {
-            mbar_expect_tx(full, G::kStageBytes);
-          }
-          auto load = [&](uint32_t dst, const CUtensorMap *map, int x, int y, int z) {
-            if (CTAS == 2) {
-              tma_load_3d_pair(dst, map, full, x, y, z);
-            } else {
-              tma_load_3d(dst, map, full, x, y, z);
-            }
-          };
-          if (!P.a_mmajor) {
-            load(sa, &maps.a, (int)(kb * BK), row0, za);
+          if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 2 * kStageBytes);
+          const uint32_t full = map_to_cta(bar_full + 8 * stage, 0);
+          if (!a_m) {
+            tma_load_3d_pair(sa, &maps.a, full, k, row0, za);
           } else {
 #pragma unroll
-            for (uint32_t j = 0; j < BM / 64; ++j) load(sa + j * (64 * BK * 2), &maps.a, row0 + (int)(j * 64), (int)(kb * BK), za);
+            for (uint32_t j = 0; j < BM / 64; ++j) tma_load_3d_pair(sa + j * (64 * BK * 2), &maps.a, full, row0 + (int)(j * 64), k, za);
           }
-          if (P.b_kmajor) {
-            load(sb, &maps.b, (int)(kb * BK), col0, zb);
+          if (b_k) {
+            tma_load_3d_pair(sb, &maps.b, full, k, col0, zb);
           } else {
 #pragma unroll
-            for (uint32_t j = 0; j < BN / CTAS / 64; ++j)
-              load(sb + j * (64 * BK * 2), &maps.b, col0 + (int)(j * 64), (int)(kb * BK), zb);
+            for (uint32_t j = 0; j < BN / 2 / 64; ++j) tma_load_3d_pair(sb + j * (64 * BK * 2), &maps.b, full, col0 + (int)(j * 64), k, zb);
           }
-          if (++stage == G::kStages) {
+          if (++stage == kStages) {
             stage = 0;
             parity ^= 1u;
           }
@@ -312,12 +172,16 @@ __device__ __forceinline__ void mm_body(const MmParam &P, const MmMaps &maps, co
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (the pair's first CTA only) ------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       // instruction descriptor: D fp32 (bit 4), A/B format (bits 7, 10: 1 = bf16), A / B stored with the
       // contraction axis outermost (bits 15 / 16), N >> 3 at bit 17, M >> 4 at bit 24
       const uint32_t fmt = P.in_dtype == T_BF16 ? 1u : 0u;
       const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((P.a_mmajor ? 1u : 0u) << 15) |
-                             ((P.b_kmajor ? 0u : 1u) << 16) | ((BN >> 3) << 17) | (((BM * CTAS) >> 4) << 24);
+                             ((P.b_kmajor ? 0u : 1u) << 16) | ((BN >> 3) << 17) | (((BM * 2) >> 4) << 24);
+      // (descriptors of stage 0; a stage or a K = 16 step further is an addition to their address fields)
+      const uint64_t da0 = P.a_mmajor ? make_smem_desc(stages, 64 * BK * 2, 1024) : make_smem_desc(stages, 0, 1024);
+      const uint64_t db0 = P.b_kmajor ? make_smem_desc(stages + kABytes, 0, 1024) : make_smem_desc(stages + kABytes, 64 * BK * 2, 1024);
+      const uint64_t step_a = P.a_mmajor ? 2048 >> 4 : 32 >> 4, step_b = P.b_kmajor ? 32 >> 4 : 2048 >> 4;
       uint32_t stage = 0, parity = 0, acc = 0, acc_parity = 1;
       for (uint32_t t = unit; t < num_tiles; t += num_units) {
         mbar_wait(bar_tempty + 8 * acc, acc_parity, 2, &g_mm_status, epoch);
@@ -325,35 +189,17 @@ __device__ __forceinline__ void mm_body(const MmParam &P, const MmMaps &maps, co
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (uint32_t kb = 0; kb < kblocks; ++kb) {
           mbar_wait(bar_full + 8 * stage, parity, 3, &g_mm_status, epoch);
-          tcgen05_after_sync();
-          const uint32_t sa = stages + stage * G::kStageBytes, sb = sa + kABytes;
+          const uint64_t da = da0 + stage * (kStageBytes >> 4), db = db0 + stage * (kStageBytes >> 4);
 #pragma unroll
-          for (uint32_t kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = P.a_mmajor ? make_smem_desc(sa + kk * 2048, 64 * BK * 2, 1024) : make_smem_desc(sa + kk * 32, 0, 1024);
-            const uint64_t db = P.b_kmajor ? make_smem_desc(sb + kk * 32, 0, 1024) : make_smem_desc(sb + kk * 2048, 64 * BK * 2, 1024);
-            if (CTAS == 2) {
-              umma_f16_pair(d_tmem, da, db, idesc, (kb | kk) != 0 ? 1u : 0u);
-            } else {
-              umma_f16_cta1(d_tmem, da, db, idesc, (kb | kk) != 0 ? 1u : 0u);
-            }
-          }
-          // the stage is free (in both CTAs) once these MMAs have read it
-          if (CTAS == 2) {
-            umma_commit_pair(bar_empty + 8 * stage, 3);
-          } else {
-            umma_commit_cta1(bar_empty + 8 * stage);
-          }
-          if (++stage == G::kStages) {
+          for (uint32_t kk = 0; kk < BK / 16; ++kk)
+            umma_f16_pair(d_tmem, da + kk * step_a, db + kk * step_b, idesc, (kb | kk) != 0 ? 1u : 0u);
+          umma_commit_pair(bar_empty + 8 * stage, 3);   // the stage is free (in both CTAs) once these MMAs have read it
+          if (++stage == kStages) {
             stage = 0;
             parity ^= 1u;
           }
         }
-        // accumulator complete
-        if (CTAS == 2) {
-          umma_commit_pair(bar_tfull + 8 * acc, 3);
-        } else {
-          umma_commit_cta1(bar_tfull + 8 * acc);
-        }
+        umma_commit_pair(bar_tfull + 8 * acc, 3);   // accumulator complete
         if (++acc == 2) {
           acc = 0;
           acc_parity ^= 1u;
@@ -364,35 +210,71 @@ __device__ __forceinline__ void mm_body(const MmParam &P, const MmMaps &maps, co
     // ------------------------------ epilogue warps ------------------------------
     const uint32_t ew = warp - 2;
     const uint32_t quarter = warp & 3u;          // TMEM lane quarter this warp may read
-    const uint32_t col_half = ew >> 2;           // which 128 columns of the tile
+    const uint32_t col0 = (ew >> 2) * kEpiCols;  // the columns of the tile this warp drains
     const uint32_t row_in_tile = quarter * 32 + lane;
+    const uint32_t out_saddr = stages + kStages * kStageBytes + ew * kOutBytes;
+    // (the program is one store in the operand type: its results go out through shared memory)
+    uint32_t staged_slot = P.gate_slot;
+    if (staged_slot == 0xffffffffu && P.fast_store_slot != 0xffffffffu && P.tensor[P.fast_store_slot].dtype == P.in_dtype)
+      staged_slot = P.fast_store_slot;
+    const uint32_t bias_saddr = base + kBiasOff + ew * (kEpiCols * 4u);
     uint32_t acc = 0, acc_parity = 0;
     for (uint32_t t = unit; t < num_tiles; t += num_units) {
       uint32_t bz, mb, nb;
       tile_coords(t, mblocks, nblocks, P.group_m, bz, mb, nb);
+      if (P.bias_ptr != 0) {
+        __syncwarp();   // (the warp has read the previous tile's)
+#pragma unroll
+        for (uint32_t c = lane; c < kEpiCols; c += 32) {
+          const float b = bias_at(P, nb * BN + col0 + c);
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_saddr + 4u * c), "f"(b) : "memory");
+        }
+        __syncwarp();
+      }
       mbar_wait(bar_tfull + 8 * acc, acc_parity, 4, &g_mm_status, epoch);
       tcgen05_after_sync();
       EpiPos pos;
       pos.b0 = bz / P.batch1;
       pos.b1 = bz - pos.b0 * P.batch1;
-      pos.row = (mb * CTAS + rank) * BM + row_in_tile;
-      const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * BN + col_half * (BN / 2);
-      for (uint32_t c0 = 0; c0 < BN / 2; c0 += 16) {
-        uint32_t r[16];
-        tmem_ld_32x32b_x16(taddr + c0, r);   // every lane of the warp takes part, valid row or not
-        pos.col = nb * BN + col_half * (BN / 2) + c0;
-        if (pos.row >= P.M || pos.col >= P.N) continue;
-        pos.valid = min(16u, P.N - pos.col);
-        finish_strip(P, pos, r);
+      pos.row = (mb * 2 + rank) * BM + row_in_tile;
+      const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * BN + col0;
+      // (one strip per trip and no unrolling: eight copies of the strip code did not fit the instruction cache and made
+      // the epilogue of a CTA's first tile 4 us longer)
+      uint32_t next[16];
+      tmem_ld_32x32b_x16_nowait(taddr, next);
+#pragma unroll 1
+      for (uint32_t c = 0; c < kEpiCols; c += 16) {
+        uint32_t r[16], pk[8];
+        tmem_ld_wait16(next);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) r[i] = next[i];
+        if (c + 16 < kEpiCols) tmem_ld_32x32b_x16_nowait(taddr + c + 16, next);   // on its way while this strip is worked on
+        pos.col = nb * BN + col0 + c;
+        uint32_t slot = 0xffffffffu;
+        if (pos.col < P.N) {   // (rows past the matrix take part: their results are not copied out)
+          pos.valid = pos.row < P.M ? min(16u, P.N - pos.col) : 0u;
+          if (P.bias_ptr != 0) add_bias_staged(bias_saddr + c * 4u, r);
+          slot = finish_strip(P, pos, r, pk);
+        }
+        if (staged_slot == 0xffffffffu) continue;
+        // row `lane`, 16-byte pieces 2 (c / 16 % 4) and the next, each at piece ^ (row & 7)
+        if (slot != 0xffffffffu) {
+          const uint32_t piece = (c >> 3) & 7u, row_saddr = out_saddr + lane * 128u;
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + ((piece ^ (lane & 7u)) << 4)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + (((piece + 1u) ^ (lane & 7u)) << 4)), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
+        }
+        if ((c & 48u) == 48u) {
+          __syncwarp();
+          const uint32_t first_col = nb * BN + col0 + (c & ~63u), first_row = (mb * 2 + rank) * BM + quarter * 32u;
+          copy_out(P, staged_slot, pos.b0, pos.b1, first_row, first_col, out_saddr, lane);
+          __syncwarp();
+        }
       }
+      tmem_ld_wait16(next);
       tcgen05_before_sync();
       __syncwarp();
       if (lane == 0) {
-        if (CTAS == 2) {
-          mbar_arrive_cluster(map_to_cta(bar_tempty + 8 * acc, 0));
-        } else {
-          mbar_arrive(bar_tempty + 8 * acc);
-        }
+        mbar_arrive_cluster(map_to_cta(bar_tempty + 8 * acc, 0));
       }
       if (++acc == 2) {
         acc = 0;
@@ -400,74 +282,20 @@ __device__ __forceinline__ void mm_body(const MmParam &P, const MmMaps &maps, co
       }
     }
   }
+  __syncwarp();
   tcgen05_before_sync();
-  if (CTAS == 2) {
-    cluster_sync_all();   // neither CTA leaves while the other may still read its shared memory or signal it
-  } else {
-    __syncthreads();
-  }
+  cluster_sync_all();   // neither CTA leaves while the other may still read its shared memory or signal it
   if (warp == 1) {
     tcgen05_after_sync();
-    if (CTAS == 2) {
-      tmem_dealloc_pair(tmem_base, kTmemCols);
-    } else {
-      tmem_dealloc(tmem_base, kTmemCols);
-    }
+    tmem_dealloc_pair(tmem_base, kTmemCols);
   }
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(kThreads, 1) dvm_b200_mm_tcgen05(const __grid_constant__ MmParam P,
-                                                                   const __grid_constant__ MmMaps maps,
-                                                                   const uint32_t epoch) {
-  mm_body<1>(P, maps, epoch);
-}
-
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   dvm_b200_mm_tcgen05_pair(const __grid_constant__ MmParam P, const __grid_constant__ MmMaps maps, const uint32_t epoch) {
-  mm_body<2>(P, maps, epoch);
-}
-
-// General SIMT MatMul for problems the copy engine cannot address: one thread per 16-column strip of a row,
-// fp32 accumulation in order of k.  Correct for every shape and alignment; not a performance path.
-__global__ void __launch_bounds__(128) dvm_b200_mm_simt(const __grid_constant__ MmParam P) {
-  const uint32_t strips = (P.N + 15u) / 16u;
-  const uint64_t total = (uint64_t)P.batch0 * P.batch1 * P.M * strips;
-  for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t strip = (uint32_t)(idx % strips);
-    const uint64_t rest = idx / strips;
-    EpiPos pos;
-    pos.row = (uint32_t)(rest % P.M);
-    const uint32_t bz = (uint32_t)(rest / P.M);
-    pos.b0 = bz / P.batch1;
-    pos.b1 = bz - pos.b0 * P.batch1;
-    pos.col = strip * 16u;
-    pos.valid = min(16u, P.N - pos.col);
-    const size_t za = (size_t)(pos.b0 * P.a_mul0 + pos.b1 * P.a_mul1) * P.M * P.K;
-    const size_t zb = (size_t)(pos.b0 * P.b_mul0 + pos.b1 * P.b_mul1) * P.N * P.K;
-    const unsigned short *A = reinterpret_cast<const unsigned short *>(P.a_ptr) + za;
-    const unsigned short *B = reinterpret_cast<const unsigned short *>(P.b_ptr) + zb;
-    float accv[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) accv[i] = 0.0f;
-    for (uint32_t k = 0; k < P.K; ++k) {
-      const unsigned short ar = P.a_mmajor ? A[(size_t)k * P.M + pos.row] : A[(size_t)pos.row * P.K + k];
-      const float a = u2f(widen(P.in_dtype, ar));
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        if ((uint32_t)i < pos.valid) {
-          const uint32_t c = pos.col + i;
-          const unsigned short br = P.b_kmajor ? B[(size_t)c * P.K + k] : B[(size_t)k * P.N + c];
-          accv[i] = fmaf(a, u2f(widen(P.in_dtype, br)), accv[i]);
-        }
-      }
-    }
-    uint32_t r[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) r[i] = f2u(accv[i]);
-    finish_strip(P, pos, r);
-  }
+  pair_body(P, maps, epoch);
 }
 
 namespace {
@@ -484,8 +312,10 @@ PFN_cuTensorMapEncodeTiled GetEncode() {
   return fn;
 }
 
+}  // namespace
+
 // 3-d map over a [batches, rows, inner] row-major operand: box = [1, box_rows, 64 elements], 128-byte swizzle
-int EncodeOperand(CUtensorMap *map, uint64_t ptr, uint64_t inner, uint64_t rows, uint64_t batches, uint32_t box_rows) {
+int EncodeMmOperand(CUtensorMap *map, uint64_t ptr, uint64_t inner, uint64_t rows, uint64_t batches, uint32_t box_rows) {
   auto encode = GetEncode();
   if (encode == nullptr) return -10;
   cuuint64_t dims[3] = {inner, rows, batches ? batches : 1};
@@ -498,18 +328,68 @@ int EncodeOperand(CUtensorMap *map, uint64_t ptr, uint64_t inner, uint64_t rows,
   return r == CUDA_SUCCESS ? 0 : -100 - static_cast<int>(r);
 }
 
-}  // namespace
-
-bool MatMulUsesTensorCores(const MmParam &p) {
+bool MmOperandNeedsGather(uint64_t ptr, uint64_t inner, uint64_t slice, uint32_t batches) {
   // the copy engine needs 16-byte aligned bases and row pitches (and slices, for batched operands)
-  const uint64_t a_inner = p.a_mmajor ? p.M : p.K, b_inner = p.b_kmajor ? p.K : p.N;
-  if ((a_inner & 7u) != 0 || (b_inner & 7u) != 0) return false;
-  if ((p.a_ptr & 15u) || (p.b_ptr & 15u)) return false;
-  if (p.a_batches > 1 && (((uint64_t)p.M * p.K) & 7u) != 0) return false;
-  if (p.b_batches > 1 && (((uint64_t)p.N * p.K) & 7u) != 0) return false;
-  if (p.K == 0) return false;
-  return true;
+  return (ptr & 15u) != 0 || (inner & 7u) != 0 || (batches > 1 && (slice & 7u) != 0);
 }
+
+namespace {
+
+struct MmPlan {
+  uint32_t bn, split;   // bn 0: 256 x 256 tiles of CTA pairs; else 128 x bn tiles, K cut into `split` parts
+};
+
+// Estimated clock cycles of a tiling.  The constants are a fit to 34 problem shapes timed in every tiling (1 to 8000 rows);
+// the tiling with the lowest estimate was on average 2 % slower than the fastest one of its shape.
+//  - A CTA alone on its SM spends max(260 + 1.6 bn, bytes / 50) per k-block, two of them together max(that, 2 bytes / 66):
+//    the MMAs of a k-block and what L2 delivers to an SM.
+//  - Loads by the work warps (operands at any even address) cost 1700 per k-block, and hardly overlap between two CTAs.
+//  - A 256 x 256 tile of a pair takes 673 per k-block, or its epilogue, whichever is longer; the last epilogue is exposed.
+double TileCost(const MmParam &p, uint32_t bn, uint32_t split, int sms, bool gather) {
+  const uint32_t kb = (p.K + BK - 1) / BK;
+  const uint64_t batch = static_cast<uint64_t>(p.batch0) * p.batch1, mb = (p.M + BM - 1) / BM;
+  if (bn == 0) {
+    const uint64_t tiles = (mb + 1) / 2 * ((p.N + BN - 1) / BN) * batch, waves = (tiles + sms / 2 - 1) / (sms / 2);
+    return 16700.0 + static_cast<double>(waves) * std::max(kb * 673.0, 12900.0);
+  }
+  const double a_rows = p.M < BM ? p.M : BM, bytes = (a_rows + bn) * 128.0;
+  const uint64_t ctas = mb * ((p.N + bn - 1) / bn) * batch * split;
+  const uint32_t share = (kb + split - 1) / split;
+  double one = std::max(260.0 + 1.6 * bn, bytes / 50.0), two = std::max(one, 2.0 * bytes / 66.0);
+  if (gather) {
+    one = 1700.0;
+    two = 1.8 * one;
+  }
+  const double finish = 4100.0 + 60.0 * bn * (a_rows / BM) / split + (split > 1 ? 3270.0 + 310.0 * split : 0.0);
+  const uint64_t full = ctas / (2 * sms), rest = ctas % (2 * sms);   // two CTAs per SM
+  double t = 5300.0 + static_cast<double>(full) * (share * two + 1.5 * finish);
+  if (rest > static_cast<uint64_t>(sms)) {
+    t += share * two + 1.5 * finish;
+  } else if (rest > 0) {
+    t += share * one + finish;
+  }
+  return t;
+}
+
+MmPlan ChoosePlan(const MmParam &p, int sms, bool gather) {
+  const uint32_t kb = (p.K + BK - 1) / BK;
+  MmPlan best{64, 1};
+  double best_t = TileCost(p, 64, 1, sms, gather);
+  auto consider = [&](uint32_t bn, uint32_t split) {
+    const double t = TileCost(p, bn, split, sms, gather);
+    if (t < best_t) {
+      best_t = t;
+      best = {bn, split};
+    }
+  };
+  for (uint32_t split = 2; split <= 8 && split <= kb; split *= 2) consider(64, split);
+  if (gather) return best;   // (64 columns measured faster than 128 at every size: the loads bound it, not the tile)
+  for (uint32_t split = 1; split <= 8 && (split == 1 || split <= kb); split *= 2) consider(128, split);
+  if (p.M > BM && kb != 0) consider(0, 1);
+  return best;
+}
+
+}  // namespace
 
 int LaunchMatMul(const MmParam &p_in, void *stream) {
   MmParam p = p_in;
@@ -555,43 +435,33 @@ int LaunchMatMul(const MmParam &p_in, void *stream) {
   cudaGetDevice(&dev);
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (!MatMulUsesTensorCores(p)) {
-    const uint64_t total = (uint64_t)p.batch0 * p.batch1 * p.M * ((p.N + 15u) / 16u);
-    const uint64_t blocks = (total + 127) / 128;
-    const uint32_t grid = static_cast<uint32_t>(blocks < (uint64_t)sms * 16 ? blocks : (uint64_t)sms * 16);
-    dvm_b200_mm_simt<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(p);
-    return static_cast<int>(cudaGetLastError());
-  }
   if (p.leave_sms != 0 && static_cast<int>(p.leave_sms) + 32 <= sms) sms -= static_cast<int>(p.leave_sms);
+  const bool gather = MmNeedsGather(p);
+  MmPlan plan = ChoosePlan(p, sms, gather);
+  static const char *const force = getenv("DVM_B200_MM_PLAN");   // "columns,split" (columns 0: CTA pairs)
+  if (force != nullptr) {
+    const uint32_t bn = static_cast<uint32_t>(atoi(force)), split = strchr(force, ',') ? static_cast<uint32_t>(atoi(strchr(force, ',') + 1)) : 1u;
+    const bool pair_ok = bn == 0 && !gather && p.K != 0;
+    if (pair_ok || ((bn == 64 || bn == 128) && (split == 1 || ((split == 2 || split == 4 || split == 8) && split * BK <= p.K)))) plan = {bn, split};
+  }
+  if (plan.bn != 0) return LaunchMmTile(p, plan.bn, plan.split, stream);
   static bool attr_set[64] = {false};
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(dvm_b200_mm_tcgen05, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<1>::kSmemBytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(dvm_b200_mm_tcgen05_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<2>::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(dvm_b200_mm_tcgen05_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_set[dev] = true;
   }
-  // CTA pairs pay off once there are at least two row blocks; a single row block runs unpaired
-  static const int force = getenv("DVM_B200_MM_CTAS") ? atoi(getenv("DVM_B200_MM_CTAS")) : 0;
-  const bool pair = force ? force == 2 : p.M > BM;
   MmMaps maps;
   // fp16 and bf16 are both 2-byte types for the copy engine; the MMA descriptor carries the real format
-  int rc = p.a_mmajor ? EncodeOperand(&maps.a, p.a_ptr, p.M, p.K, p.a_batches, 64)
-                      : EncodeOperand(&maps.a, p.a_ptr, p.K, p.M, p.a_batches, BM);
+  int rc = p.a_mmajor ? EncodeMmOperand(&maps.a, p.a_ptr, p.M, p.K, p.a_batches, 64)
+                      : EncodeMmOperand(&maps.a, p.a_ptr, p.K, p.M, p.a_batches, BM);
   if (rc != 0) return rc;
-  rc = p.b_kmajor ? EncodeOperand(&maps.b, p.b_ptr, p.K, p.N, p.b_batches, pair ? BN / 2 : BN)
-                  : EncodeOperand(&maps.b, p.b_ptr, p.N, p.K, p.b_batches, 64);
+  rc = p.b_kmajor ? EncodeMmOperand(&maps.b, p.b_ptr, p.K, p.N, p.b_batches, BN / 2)
+                  : EncodeMmOperand(&maps.b, p.b_ptr, p.N, p.K, p.b_batches, 64);
   if (rc != 0) return rc;
-  const uint32_t batch = p.batch0 * p.batch1;
-  if (pair) {
-    const uint32_t tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * batch;
-    const uint32_t units = tiles < static_cast<uint32_t>(sms / 2) ? tiles : static_cast<uint32_t>(sms / 2);
-    dvm_b200_mm_tcgen05_pair<<<units * 2, kThreads, Geo<2>::kSmemBytes, static_cast<cudaStream_t>(stream)>>>(p, maps, NextLaunchEpoch());
-  } else {
-    const uint32_t tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * batch;
-    const uint32_t grid = tiles < static_cast<uint32_t>(sms) ? tiles : static_cast<uint32_t>(sms);
-    dvm_b200_mm_tcgen05<<<grid, kThreads, Geo<1>::kSmemBytes, static_cast<cudaStream_t>(stream)>>>(p, maps, NextLaunchEpoch());
-  }
+  const uint32_t tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.batch0 * p.batch1;
+  const uint32_t units = tiles < static_cast<uint32_t>(sms / 2) ? tiles : static_cast<uint32_t>(sms / 2);
+  dvm_b200_mm_tcgen05_pair<<<units * 2, kThreads, kSmemBytes, static_cast<cudaStream_t>(stream)>>>(p, maps, NextLaunchEpoch());
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -600,7 +470,8 @@ unsigned int ReadMatMulStatus() {
   const unsigned int zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_mm_status, sizeof(v)) != cudaSuccess) return 0xffffffffu;
   if (v.first_error != 0) cudaMemcpyToSymbol(g_mm_status, &zero, sizeof(zero), offsetof(WaitStatus, first_error));
-  return v.first_error;
+  const unsigned int tile = ReadMmTileStatus();
+  return v.first_error != 0 ? v.first_error : tile;
 }
 
 }  // namespace dvmb

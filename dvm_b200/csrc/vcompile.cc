@@ -1919,9 +1919,8 @@ std::string DisassembleEpilogue(const MatMulStage &st) {
   std::string o;
   char buf[320];
   snprintf(buf, sizeof(buf),
-           "mmain.sm100(batch=%ux%u, m=%u, n=%u, k=%u, a=%s, b=%s, %s, engine=%s) {\n", P.batch0, P.batch1, P.M, P.N, P.K,
-           P.a_mmajor ? "[k,m]" : "[m,k]", P.b_kmajor ? "[n,k]" : "[k,n]", DTypeName(static_cast<DataType>(P.in_dtype)),
-           MatMulUsesTensorCores(P) ? "tcgen05" : "simt");
+           "mmain.sm100(batch=%ux%u, m=%u, n=%u, k=%u, a=%s, b=%s, %s, engine=tcgen05, loads=%s) {\n", P.batch0, P.batch1, P.M, P.N, P.K,
+           P.a_mmajor ? "[k,m]" : "[m,k]", P.b_kmajor ? "[n,k]" : "[k,n]", DTypeName(static_cast<DataType>(P.in_dtype)), MmNeedsGather(P) ? "simt" : "tma");
   o += buf;
   snprintf(buf, sizeof(buf), "  matmul.%s acc, load(0x%llx), load(0x%llx)%s\n", DTypeName(static_cast<DataType>(P.in_dtype)),
            static_cast<unsigned long long>(P.a_ptr), static_cast<unsigned long long>(P.b_ptr), P.bias_ptr ? ", bias" : "");
