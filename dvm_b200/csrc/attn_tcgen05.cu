@@ -165,7 +165,8 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    // (elect.sync, not `lane == 0`, here and in the MMA warp: see mm_tcgen05.cu)
+    if (elect_one()) {
       mbar_expect_tx(base + kBarQ, 2 * tile_bytes);
       for (uint32_t g = 0; g < 2; ++g)
         for (uint32_t h = 0; h < dhalves; ++h)
@@ -192,29 +193,34 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t fmt = DT == T_BF16 ? 1u : 0u;
       // S = Q K^T: both operands have the head dimension innermost; M = 128, N = 128 keys
       const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((kTileKV >> 3) << 17) | ((kTileQ >> 4) << 24);
       // O += P V: V is stored [key][d] (the contraction axis outermost); N = d
       const uint32_t idesc_o = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 16) | ((P.d >> 3) << 17) | ((kTileQ >> 4) << 24);
-      const uint32_t ksteps_s = P.d / 16;
+      // descriptors of row tile 0 / ring slot 0; everything further is an addition to their address fields
+      const uint64_t dq = make_smem_desc(base + kOffQ, 0, 1024), dp = make_smem_desc(base + kOffP, 0, 1024);
+      const uint64_t dk = make_smem_desc(base + kOffRing, 0, 1024), dv = make_smem_desc(base + kOffRing, kHalfBytes, 1024);
+      constexpr uint64_t kTileStep = kTileBytes >> 4, kHalfStep = kHalfBytes >> 4;
+      const bool two_halves = P.d > 64;
       auto issue_s = [&](uint32_t g, uint32_t kslot) {
-        const uint32_t qa = base + kOffQ + g * kTileBytes, kb = base + kOffRing + kslot * kTileBytes;
-        for (uint32_t kk = 0; kk < ksteps_s; ++kk) {
-          const uint32_t off = (kk >> 2) * kHalfBytes + (kk & 3u) * 32u;
-          umma_f16_cta1(tmem_base + kTmemS + g * 128, make_smem_desc(qa + off, 0, 1024), make_smem_desc(kb + off, 0, 1024), idesc_s,
-                        kk != 0 ? 1u : 0u);
+        const uint64_t a = dq + g * kTileStep, b = dk + kslot * kTileStep;
+        const uint32_t d = tmem_base + kTmemS + g * 128;
+#pragma unroll
+        for (uint32_t kk = 0; kk < 4; ++kk) umma_f16_cta1(d, a + kk * 2, b + kk * 2, idesc_s, kk != 0 ? 1u : 0u);
+        if (two_halves) {
+#pragma unroll
+          for (uint32_t kk = 0; kk < 4; ++kk) umma_f16_cta1(d, a + kHalfStep + kk * 2, b + kHalfStep + kk * 2, idesc_s, 1u);
         }
         umma_commit_cta1(base + kBarSFull + 8 * g);
       };
       auto issue_pv = [&](uint32_t g, uint32_t vslot, bool accumulate) {
-        const uint32_t pa = base + kOffP + g * kTileBytes, vb = base + kOffRing + vslot * kTileBytes;
-        for (uint32_t kk = 0; kk < kTileKV / 16; ++kk) {
-          const uint64_t da = make_smem_desc(pa + (kk >> 2) * kHalfBytes + (kk & 3u) * 32u, 0, 1024);
-          const uint64_t db = make_smem_desc(vb + kk * 2048, kHalfBytes, 1024);
-          umma_f16_cta1(tmem_base + kTmemO + g * 128, da, db, idesc_o, (accumulate || kk != 0) ? 1u : 0u);
-        }
+        const uint64_t a = dp + g * kTileStep, b = dv + vslot * kTileStep;
+        const uint32_t d = tmem_base + kTmemO + g * 128;
+#pragma unroll
+        for (uint32_t kk = 0; kk < kTileKV / 16; ++kk)
+          umma_f16_cta1(d, a + (kk >> 2) * kHalfStep + (kk & 3u) * 2, b + kk * (2048 >> 4), idesc_o, (accumulate || kk != 0) ? 1u : 0u);
         umma_commit_cta1(base + kBarPvDone + 8 * g);
       };
       // ring position of K(j) / V(j) (see the producer) -> slot and phase parity
