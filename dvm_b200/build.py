@@ -21,10 +21,12 @@ SOURCES = [
     "vkernel.cc",
     "partition.cc",
     "stat_fusion.cc",
+    "row_match.cc",
     "comm.cc",
     "runtime.cu",
     "capi.cu",
     "vm_vector.cu",
+    "vm_row.cu",
     "mm_tcgen05.cu",
     "mm_tile.cu",
     "attn_tcgen05.cu",

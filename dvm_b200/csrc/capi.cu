@@ -16,6 +16,7 @@
 #include "graph.h"
 #include "runtime.h"
 #include "vm_launch.h"
+#include "vm_row.h"
 #include "mm_launch.h"
 
 struct dvm_int_array {
@@ -468,7 +469,7 @@ int dvm_rt_memset(void *dst, int value, size_t bytes, void *stream) {
 // Reads (and clears) the status records of the device interpreters: a bounded device wait that expired (the kernel
 // then ran to its end with wrong results) is reported here as an error.  Does not wait for anything.
 int dvm_rt_check_status(void) {
-  const unsigned int sv = dvmb::ReadVectorStatus(), sm = dvmb::ReadMatMulStatus(), sa = dvmb::ReadAttentionStatus();
+  const unsigned int rs = dvmb::ReadRowStatus(), vs = dvmb::ReadVectorStatus(), sv = vs != 0 ? vs : rs, sm = dvmb::ReadMatMulStatus(), sa = dvmb::ReadAttentionStatus();
   if ((sv | sm | sa) != 0) {
     char buf[160];
     snprintf(buf, sizeof(buf), "a bounded device wait expired (vector 0x%08x, matmul 0x%08x, attention 0x%08x)", sv, sm, sa);

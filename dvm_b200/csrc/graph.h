@@ -14,6 +14,7 @@
 #include "../../include/dvm.h"
 #include "isa.h"
 #include "mm_launch.h"
+#include "vm_row.h"
 
 namespace dvm {
 
@@ -139,6 +140,10 @@ struct VectorStage {
   // rebind to an aligned address gets the planned offset back
   uint32_t ring_plan_off[dvmb::kMaxTensors] = {0};
   uint64_t algo_bytes = 0;
+  // a normalisation that a row kernel runs (vm_row.cu) when the bound addresses allow it; the interpreter's program stays
+  // the stage's definition and its fallback
+  dvmb::RowParam row;
+  bool row_ok = false;
 };
 
 // One launch of the tensor-core MatMul with its fused post-ops.
@@ -235,6 +240,9 @@ bool CompileVectorStage(const std::vector<NDObject *> &ops, VectorStage *out, st
 bool CompileEpilogue(const std::vector<NDObject *> &ops, const NDObject *mma_src, MatMulStage *out, std::string *why);
 std::string DisassembleEpilogue(const MatMulStage &st);
 std::string DisassembleStage(const VectorStage &st);
+// row_match.cc: fill st->row when the compiled stage is one of the row kernels' shapes; bind its addresses.
+void MatchRowKernel(VectorStage *st);
+void BindRow(VectorStage *st);
 // Turn the stage's instruction words into the launch program (scalar sections + micro-ops) for the tensor
 // addresses now in the descriptors; called whenever addresses are (re)bound.
 void LowerStage(VectorStage *st);

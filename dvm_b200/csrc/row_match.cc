@@ -1,0 +1,400 @@
+// Recognises the two normalisation shapes that the row kernels (vm_row.cu) run: works on the instruction words and the
+// tensor table that the vector compiler produced, so the graph may be written in any way that compiles to these bodies.
+// What does not match runs on the vector interpreter as before.  No counterpart in the reference, whose kernels run each
+// reduction and each group of element-wise ops as written (src/vm_gpu.cu:1552-1617).
+#include <cstdlib>
+#include <cstring>
+#include <utility>
+#include <vector>
+
+#include "graph.h"
+
+namespace dvm {
+namespace {
+
+using namespace dvmb;
+
+struct Word {
+  uint64_t w;
+  uint32_t opc, sub, kind, idx, rnd, imm;
+  explicit Word(uint64_t v) : w(v), opc(DVMB_OPC(v)), sub(DVMB_SUB(v)), kind(DVMB_OKIND(v)), idx(DVMB_OIDX(v)), rnd(DVMB_RND(v)), imm(DVMB_IMM(v)) {}
+  bool bin(uint32_t b) const { return opc == OP_BIN && sub == b && rnd == RN_NONE; }
+  bool scalar_operand() const { return kind == K_SREG || kind == K_IMM; }
+};
+
+struct Cursor {
+  const std::vector<uint64_t> &code;
+  size_t pc;
+  Word at(size_t i = 0) const { return Word(pc + i < code.size() ? code[pc + i] : 0); }
+  Word next() { return Word(code[pc++]); }
+};
+
+RowScalar ScalarOf(const Word &w, bool recip) {
+  RowScalar s;
+  std::memset(&s, 0, sizeof(s));
+  s.src = w.kind == K_SREG ? 0 : 1;
+  s.idx = static_cast<uint8_t>(w.idx);
+  s.imm = w.imm;
+  s.recip = recip ? 1 : 0;
+  return s;
+}
+
+const RowScalar kAbsent = {static_cast<uint8_t>(kRowNone), 0, 0, 0, 0};
+
+// A store of the accumulator to `tensor` in its own 16-bit or fp32 type, behind the rounding that store repeats anyway.
+bool MatchStore(Cursor &c, const VmParam &P, uint32_t *slot) {
+  uint32_t rnd = RN_NONE;
+  if (c.at().opc == OP_CVT && c.at().sub == V_RND) rnd = c.next().rnd;
+  if (c.at().opc != OP_ST) return false;
+  *slot = c.next().sub;
+  const uint32_t dt = P.tensor[*slot].dtype;
+  return rnd == RN_NONE || (rnd == RN_F16 && dt == T_F16) || (rnd == RN_BF16 && dt == T_BF16);
+}
+
+// The scalar sections as expressions: what every scalar register and every stored value is made of.
+struct Symbolic {
+  enum Op : int { NONE = -1, IN = 0, IMM, PART, UN, BIN };
+  struct Expr {
+    int op, a, b;
+    uint32_t v;   // tensor slot / immediate / partial / operation
+  };
+  std::vector<Expr> e;
+  int acc = NONE, sreg[kNumSRegs];
+  bool ok = true;
+  std::vector<std::pair<uint32_t, int>> stores;   // (tensor slot, value)
+
+  Symbolic() {
+    for (int &r : sreg) r = NONE;
+  }
+  int Make(int op, uint32_t v, int a = NONE, int b = NONE) {
+    if (op == BIN && (v == B_ADD || v == B_MUL) && a > b) std::swap(a, b);
+    for (size_t i = 0; i < e.size(); ++i)
+      if (e[i].op == op && e[i].v == v && e[i].a == a && e[i].b == b) return static_cast<int>(i);
+    e.push_back({op, a, b, v});
+    return static_cast<int>(e.size()) - 1;
+  }
+  int Bin(uint32_t kind, int a, int b) { return a < 0 || b < 0 ? NONE : Make(BIN, kind, a, b); }
+  void Run(const std::vector<uint64_t> &code, size_t pc) {
+    for (;; ++pc) {
+      const Word w(code[pc]);
+      if (w.opc == OP_END) return;
+      int b = NONE;
+      if (w.kind == K_SREG) b = w.idx < static_cast<uint32_t>(kNumSRegs) ? sreg[w.idx] : static_cast<int>(NONE);
+      if (w.kind == K_IMM) b = Make(IMM, w.imm);
+      if (w.kind == K_ACC) b = acc;
+      if (w.kind == K_TENSOR) b = Make(IN, w.idx);
+      switch (w.opc) {
+        case OP_RINIT: break;
+        case OP_RFIN: acc = Make(PART, w.sub & 3u); break;
+        case OP_COPY: acc = b; break;
+        case OP_MOV: sreg[DVMB_DST(w.w)] = acc; break;
+        case OP_ST: stores.emplace_back(w.sub, acc); break;
+        case OP_UN:
+          if (w.rnd != RN_NONE || acc < 0) ok = false; else acc = Make(UN, w.sub, acc);
+          break;
+        case OP_BIN:
+          if (w.rnd != RN_NONE) ok = false;
+          else if (w.sub == B_RSUB) acc = Bin(B_SUB, b, acc);
+          else if (w.sub == B_RDIV_FAST) acc = Bin(B_DIV_FAST, b, acc);
+          else if (w.sub == B_ADD || w.sub == B_SUB || w.sub == B_MUL || w.sub == B_DIV_FAST) acc = Bin(w.sub, acc, b);
+          else ok = false;
+          break;
+        default: ok = false; break;
+      }
+      if (acc < 0 && w.opc != OP_RINIT && w.opc != OP_MOV) ok = false;
+    }
+  }
+  bool IsImm(int i, float *v) const {
+    if (i < 0 || e[i].op != IMM) return false;
+    std::memcpy(v, &e[i].v, 4);
+    return true;
+  }
+  // i = x * imm or x + imm: the immediate, given the other operand
+  bool WithImm(int i, uint32_t kind, int x, float *v) const {
+    if (i < 0 || e[i].op != BIN || e[i].v != kind) return false;
+    if (e[i].a == x) return IsImm(e[i].b, v);
+    return e[i].b == x && IsImm(e[i].a, v);
+  }
+};
+
+struct Matcher {
+  const VectorStage &st;
+  const VmParam &P;
+  RowParam *R;
+
+  Matcher(const VectorStage &s, RowParam *r) : st(s), P(s.param), R(r) {}
+
+  bool AddStream(uint32_t i, uint32_t slot) {
+    RowStream &s = R->stream[i];
+    const TensorDesc &td = P.tensor[slot];
+    for (int j = 0; j < kMaxKept; ++j) s.kstride[j] = td.kstride[j];
+    s.slot = slot;
+    return td.mode != AM_SCALAR;
+  }
+  // same type and the same walk as stream 0
+  bool Like(uint32_t slot, uint32_t slot0, bool same_groups) const {
+    const TensorDesc &a = P.tensor[slot], &b = P.tensor[slot0];
+    if (a.dtype != b.dtype || a.mode == AM_SCALAR) return false;
+    for (int j = 0; j < kMaxEnum; ++j)
+      if (a.estride[j] != b.estride[j] && P.enum_size[j] != 1) return false;
+    for (int j = 0; j < kMaxKept; ++j)
+      if (P.kept_size[j] != 1 && a.kstride[j] != (same_groups ? b.kstride[j] : 0u)) return false;
+    return true;
+  }
+
+  // runs x run_len from the iterated axes of tensor `slot`
+  bool Geometry(uint32_t slot) {
+    const TensorDesc &td = P.tensor[slot];
+    if (P.enum_size[0] != 1 || P.enum_size[1] != 1 || td.estride[kMaxEnum - 1] != 1) return false;
+    R->runs = P.enum_size[kMaxEnum - 2];
+    R->run_len = P.enum_size[kMaxEnum - 1];
+    R->run_stride = R->runs > 1 ? td.estride[kMaxEnum - 2] : 0;
+    R->dtype = td.dtype;
+    R->groups = P.num_groups;
+    for (int j = 0; j < kMaxKept; ++j) R->kept_size[j] = P.kept_size[j];
+    return td.dtype == T_F16 || td.dtype == T_BF16 || td.dtype == T_F32;
+  }
+
+  bool Sections() {
+    R->num_sections = P.num_body + 1;
+    uint32_t n = 0;
+    std::memset(R->scalar_of, 0xff, sizeof(R->scalar_of));
+    auto scalar = [&](uint32_t slot, bool read) {
+      if (P.tensor[slot].mode != AM_SCALAR) return false;
+      if (R->scalar_of[slot] == 0xff) {
+        if (R->n_scalars >= static_cast<uint32_t>(kRowMaxScalars)) return false;
+        R->scalar[R->n_scalars] = P.tensor[slot];
+        R->scalar_of[slot] = static_cast<uint8_t>(R->n_scalars++);
+      }
+      if (read) R->scalar_in |= 1u << R->scalar_of[slot];
+      return true;
+    };
+    for (uint32_t p = 0; p <= P.num_body; ++p) {
+      R->sec[p] = static_cast<uint16_t>(n);
+      for (size_t pc = st.bsec[2 * p];; ++pc) {
+        const Word w(st.bytecode[pc]);
+        if (n >= static_cast<uint32_t>(kRowMaxCode)) return false;
+        if (w.opc == OP_ST && !scalar(w.sub, false)) return false;
+        if ((w.opc == OP_COPY || w.opc == OP_BIN || w.opc == OP_CMP || w.opc == OP_SEL) && w.kind == K_TENSOR && !scalar(w.idx, true)) return false;
+        if (w.opc == OP_RFIN && ((w.sub >> 4) != R_SUM || ((w.sub & 3u) != R->red_slot[0] && (w.sub & 3u) != R->red_slot[1]))) return false;
+        R->code[n++] = w.w;
+        if (w.opc == OP_END) break;
+      }
+    }
+    return true;
+  }
+
+  // The closed form of ROW_STATS_AFFINE's scalar sections (see RowParam::closed).
+  void CloseStats() {
+    Symbolic y;
+    y.Run(st.bytecode, st.bsec[0]);
+    if (R->shift.src != 0 || R->red_slot[0] == kRowNone || R->red_slot[1] == kRowNone) return;
+    const int shift = y.sreg[R->shift.idx];
+    if (!y.ok || shift < 0 || y.e[shift].op != Symbolic::IN) return;
+    const uint32_t shift_slot = y.e[shift].v;
+    if (P.tensor[shift_slot].dtype != R->dtype) return;   // (the kernel writes it into a run's edge lanes: it must be a value of x's type)
+    y.Run(st.bytecode, st.bsec[2]);
+    auto value = [&](const RowScalar &c) { return c.src == 0 ? y.sreg[c.idx] : static_cast<int>(Symbolic::NONE); };
+    const int mean = value(R->chain[0]), den = value(R->chain[1]);
+    if (!y.ok || mean < 0 || den < 0 || !R->chain[1].recip || R->chain[2].recip) return;
+    const int T = y.Make(Symbolic::PART, R->red_slot[0]), Q = y.Make(Symbolic::PART, R->red_slot[1]);
+    // den = sqrt(v + eps), v = (Q - T (T i1)) i2, mean = T i1 + s
+    if (y.e[mean].op != Symbolic::BIN || y.e[mean].v != B_ADD) return;
+    const int ti = y.e[mean].a == shift ? y.e[mean].b : y.e[mean].a;
+    if ((y.e[mean].a != shift && y.e[mean].b != shift) || !y.WithImm(ti, B_MUL, T, &R->i1)) return;
+    if (y.e[den].op != Symbolic::UN || y.e[den].v != U_SQRT) return;
+    const int ve = y.e[den].a;
+    if (y.e[ve].op != Symbolic::BIN || y.e[ve].v != B_ADD) return;
+    const int v = y.IsImm(y.e[ve].a, &R->eps) ? y.e[ve].b : y.e[ve].a;
+    if (!y.WithImm(ve, B_ADD, v, &R->eps)) return;
+    const int dev = y.Bin(B_SUB, Q, y.Bin(B_MUL, T, ti));
+    if (!y.WithImm(v, B_MUL, dev, &R->i2)) return;
+    R->at_gamma = R->at_beta = R->at_mean = R->at_var = kRowNone;
+    auto input = [&](const RowScalar &c, uint32_t *at) {
+      if (c.src == kRowNone) return true;
+      const int i = value(c);
+      if (i < 0 || y.e[i].op != Symbolic::IN) return false;
+      *at = R->scalar_of[y.e[i].v];
+      return true;
+    };
+    if (!input(R->chain[2], &R->at_gamma) || !input(R->chain[3], &R->at_beta)) return;
+    y.Run(st.bytecode, st.bsec[4]);
+    if (!y.ok) return;
+    for (auto &s : y.stores) {
+      uint32_t *at = s.second == mean ? &R->at_mean : (s.second == v ? &R->at_var : nullptr);
+      if (at == nullptr || *at != kRowNone) return;
+      *at = R->scalar_of[s.first];
+    }
+    R->at_shift = R->scalar_of[shift_slot];
+    R->closed = 1;
+  }
+
+  // ... and of ROW_RMS_GATE's.
+  void CloseRms() {
+    Symbolic y;
+    y.Run(st.bytecode, st.bsec[0]);
+    y.Run(st.bytecode, st.bsec[2]);
+    if (!y.ok || R->chain[1].src != 0) return;
+    const int scale = y.sreg[R->chain[1].idx];
+    float one = 0.0f;
+    if (scale < 0 || y.e[scale].op != Symbolic::BIN || y.e[scale].v != B_DIV_FAST || !y.IsImm(y.e[scale].a, &one) || one != 1.0f) return;
+    const int root = y.e[scale].b;
+    if (y.e[root].op != Symbolic::UN || y.e[root].v != U_SQRT) return;
+    const int sum = y.e[root].a;
+    if (y.e[sum].op != Symbolic::BIN || y.e[sum].v != B_ADD) return;
+    const int scaled = y.IsImm(y.e[sum].a, &R->eps) ? y.e[sum].b : y.e[sum].a;
+    if (!y.WithImm(sum, B_ADD, scaled, &R->eps) || !y.WithImm(scaled, B_MUL, y.Make(Symbolic::PART, R->red_slot[0]), &R->i1)) return;
+    y.Run(st.bytecode, st.bsec[4]);
+    R->closed = y.ok && y.stores.empty() ? 1 : 0;
+  }
+
+  bool StatsAffine() {
+    Cursor c{st.bytecode, st.bsec[1]};
+    if (c.at().opc != OP_COPY || c.at().kind != K_TENSOR) return false;
+    const uint32_t x = c.next().idx;
+    R->shift = kAbsent;
+    if (c.at().bin(B_SUB) && c.at().scalar_operand()) R->shift = ScalarOf(c.next(), false);
+    R->red_slot[0] = R->red_slot[1] = kRowNone;
+    if (c.at().opc == OP_RACC && (c.at().sub >> 4) == R_SUM) R->red_slot[0] = c.next().sub & 3u;
+    if (c.at().bin(B_MUL) && c.at().kind == K_ACC) {
+      c.next();
+      if (c.at().opc != OP_RACC || (c.at().sub >> 4) != R_SUM) return false;
+      R->red_slot[1] = c.next().sub & 3u;
+    }
+    if (c.next().opc != OP_END || (R->red_slot[0] == kRowNone && R->red_slot[1] == kRowNone)) return false;
+    Cursor d{st.bytecode, st.bsec[3]};
+    if (d.at().opc != OP_COPY || d.at().kind != K_TENSOR || d.next().idx != x) return false;
+    for (auto &s : R->chain) s = kAbsent;
+    uint32_t stage = 0;   // subtract, multiply, multiply, add: each at most once, in this order
+    for (;;) {
+      const Word w = d.at();
+      if (w.opc != OP_BIN || w.rnd != RN_NONE || !w.scalar_operand()) break;
+      if (w.sub == B_SUB && stage == 0) {
+        R->chain[0] = ScalarOf(w, false);
+        stage = 1;
+      } else if ((w.sub == B_MUL || (w.sub == B_DIV_FAST && w.kind == K_SREG)) && stage <= 2) {
+        const uint32_t at = stage < 2 ? 1 : 2;
+        R->chain[at] = ScalarOf(w, w.sub == B_DIV_FAST);
+        stage = at + 1;
+      } else if (w.sub == B_ADD && stage <= 3) {
+        R->chain[3] = ScalarOf(w, false);
+        stage = 4;
+      } else {
+        return false;
+      }
+      d.next();
+    }
+    uint32_t y = 0;
+    if (!MatchStore(d, P, &y) || d.next().opc != OP_END) return false;
+    if (!Geometry(x) || !Like(y, x, true)) return false;
+    R->form = ROW_STATS_AFFINE;
+    if (!AddStream(0, x) || !AddStream(1, y) || !Sections()) return false;
+    CloseStats();
+    // (outside a run's edges the kernel counts lanes as the shift itself: x's own first element, or nothing subtracted)
+    return R->closed != 0 || R->shift.src == kRowNone;
+  }
+
+  // ((sigmoid(g)) * g) * u -> store (either order of the two products' operands is what the compiler emits)
+  bool Gate(Cursor &c, uint32_t *g, uint32_t *u, uint32_t *y) {
+    if (c.at().opc != OP_COPY || c.at().kind != K_TENSOR) return false;
+    *g = c.next().idx;
+    const Word a = c.at(0), b = c.at(1), e = c.at(2), r = c.at(3), m = c.at(4), n = c.at(5);
+    if (!a.bin(B_MUL) || a.kind != K_IMM || a.imm != 0xbf800000u) return false;
+    if (b.opc != OP_UN || b.sub != U_EXP_FAST || b.rnd != RN_NONE) return false;
+    if (!e.bin(B_ADD) || e.kind != K_IMM || e.imm != 0x3f800000u) return false;
+    if (!r.bin(B_RDIV_FAST) || r.kind != K_IMM || r.imm != 0x3f800000u) return false;
+    if (!m.bin(B_MUL) || m.kind != K_TENSOR || m.idx != *g || !n.bin(B_MUL) || n.kind != K_TENSOR) return false;
+    *u = n.idx;
+    c.pc += 6;
+    return MatchStore(c, P, y);
+  }
+
+  bool RmsGate() {
+    if (P.enum_size[kMaxEnum - 2] != 1) return false;
+    Cursor c{st.bytecode, st.bsec[1]};
+    uint32_t a = 0, b = 0, w = 0, y = 0, g = 0, u = 0, y2 = 0;
+    auto sum = [&](Cursor &q, uint32_t *pa, uint32_t *pb) {
+      if (q.at().opc != OP_COPY || q.at().kind != K_TENSOR) return false;
+      *pa = *pb = q.next().idx;
+      if (q.at().bin(B_ADD) && q.at().kind == K_TENSOR) {
+        *pb = q.next().idx;
+        R->have_b = 1;
+      }
+      return true;
+    };
+    R->have_b = R->have_w = R->have_gate = 0;
+    bool body0_done = false;
+    for (int part = 0; part < 2 && c.at().opc != OP_END; ++part) {
+      const size_t mark = c.pc;
+      if (!body0_done && sum(c, &a, &b) && c.at().bin(B_MUL) && c.at().kind == K_ACC && c.at(1).opc == OP_RACC && (c.at(1).sub >> 4) == R_SUM) {
+        c.next();
+        R->red_slot[0] = c.next().sub & 3u;
+        R->red_slot[1] = kRowNone;
+        body0_done = true;
+        continue;
+      }
+      c.pc = mark;
+      if (R->have_gate || !Gate(c, &g, &u, &y2)) return false;
+      R->have_gate = 1;
+    }
+    if (!body0_done || c.next().opc != OP_END) return false;
+    const uint32_t have_b0 = R->have_b;
+    Cursor d{st.bytecode, st.bsec[3]};
+    uint32_t a1 = 0, b1 = 0;
+    R->have_b = 0;
+    if (!sum(d, &a1, &b1) || a1 != a || b1 != b || R->have_b != have_b0) return false;
+    for (auto &s : R->chain) s = kAbsent;
+    if (!d.at().bin(B_MUL) || !d.at().scalar_operand()) return false;
+    R->chain[1] = ScalarOf(d.next(), false);
+    if (d.at().bin(B_MUL) && d.at().kind == K_TENSOR) {
+      w = d.next().idx;
+      R->have_w = 1;
+    }
+    if (!MatchStore(d, P, &y)) return false;
+    if (d.at().opc != OP_END) {
+      if (R->have_gate || !Gate(d, &g, &u, &y2)) return false;
+      R->have_gate = 1;
+    }
+    if (d.next().opc != OP_END) return false;
+    if (!Geometry(a) || R->runs != 1 || R->dtype == T_F32 || !Like(y, a, true)) return false;
+    R->shift = kAbsent;
+    R->form = ROW_RMS_GATE;
+    if (!AddStream(0, a) || !AddStream(3, y)) return false;
+    if (R->have_b && (!Like(b, a, true) || !AddStream(1, b))) return false;
+    if (R->have_w && (!Like(w, a, false) || !AddStream(2, w))) return false;
+    if (R->have_gate && (!Like(g, a, true) || !Like(u, a, true) || !Like(y2, a, true) || !AddStream(4, g) || !AddStream(5, u) || !AddStream(6, y2))) return false;
+    if (!Sections()) return false;
+    CloseRms();
+    return true;
+  }
+};
+
+}  // namespace
+
+void MatchRowKernel(VectorStage *st) {
+  RowParam &R = st->row;
+  std::memset(&R, 0, sizeof(R));
+  const VmParam &P = st->param;
+  static const bool off = getenv("DVM_B200_NO_ROW") != nullptr;
+  if (off || st->idle || P.mode != VM_GROUP || P.num_body != 2) return;
+  Matcher m(*st, &R);
+  if (m.StatsAffine()) return;
+  std::memset(&R, 0, sizeof(R));
+  if (m.RmsGate()) return;
+  std::memset(&R, 0, sizeof(R));
+}
+
+void BindRow(VectorStage *st) {
+  RowParam &R = st->row;
+  const VmParam &P = st->param;
+  const uint32_t n = R.form == ROW_STATS_AFFINE ? 2u : static_cast<uint32_t>(kRowMaxStreams);
+  for (uint32_t i = 0; i < n; ++i) {
+    const bool used = R.form == ROW_STATS_AFFINE || i == 0 || i == 3 || (i == 1 && R.have_b) || (i == 2 && R.have_w) || (i >= 4 && R.have_gate);
+    R.stream[i].ptr = used ? P.tensor[R.stream[i].slot].ptr : 0;
+  }
+  for (uint32_t s = 0; s < P.n_tensors; ++s)
+    if (R.scalar_of[s] != 0xff) R.scalar[R.scalar_of[s]].ptr = P.tensor[s].ptr;
+  st->row_ok = RowAddressesOk(R);
+}
+
+}  // namespace dvm

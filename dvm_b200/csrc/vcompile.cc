@@ -1290,6 +1290,7 @@ bool CompileVectorStage(const std::vector<NDObject *> &ops, VectorStage *out, st
     std::memset(&out->param, 0, sizeof(out->param));
     Compiler c(ops, out);
     c.Run();
+    MatchRowKernel(out);
     return true;
   } catch (const Fail &f) {
     if (why) *why = f.why;

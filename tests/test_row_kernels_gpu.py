@@ -1,0 +1,98 @@
+"""Row kernels: normalisations over runs of any length and alignment, in every split of a group over CTAs, against float64."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _batchnorm(shape, dtype, offset=0):
+    """Training batch-norm of an NCHW tensor that starts `offset` elements into its buffer; float64 expectation."""
+    from dvm_b200 import workloads as W
+    from dvm_b200.tester import Tester
+    n, c, h, w = shape
+    rng = np.random.default_rng(n + 3 * c + 7 * h + 11 * w)
+    x = (rng.standard_normal(shape) + rng.standard_normal((1, c, 1, 1))).astype(np.float16)
+    g = rng.normal(1, 0.1, (1, c, 1, 1)).astype(np.float32)
+    b = rng.normal(0, 0.1, (1, c, 1, 1)).astype(np.float32)
+    t = Tester("vector")
+    if offset:
+        buf = np.zeros(x.size + offset, np.float16)
+        buf[offset:] = x.reshape(-1)
+        lx = t.view_load(list(shape), [c * h * w, h * w, w, 1], buf, offset)
+    else:
+        lx = t.load(x)
+    stores = [t.store(v) for v in W.batchnorm_train(t, lx, t.load(g), t.load(b), n * h * w)]
+    t.run()
+    got = [t.output(s).astype(np.float64) for s in stores]
+    xd = x.astype(np.float64)
+    m = xd.mean((0, 2, 3), keepdims=True)
+    v = ((xd - m) ** 2).mean((0, 2, 3), keepdims=True)
+    y = (xd - m) / np.sqrt(v + 1e-5) * g + b
+    # fp32 sums over the group in a tree, one rounding of the result to fp16
+    assert np.allclose(got[1], m, rtol=1e-5, atol=1e-5 * float(np.abs(xd).max()))
+    assert np.allclose(got[2], v, rtol=1e-4, atol=1e-6)
+    assert np.all(np.abs(got[0] - y) <= 2.0 ** -10 * np.abs(y) + 1e-3), float(np.abs(got[0] - y).max())
+
+
+# planes of one unit and less, odd planes, runs that end on a unit, groups of one CTA, two, four and eight CTAs
+@pytest.mark.parametrize("shape", [(4, 5, 1, 3), (2, 3, 4, 2), (9, 17, 7, 7), (3, 300, 5, 5), (16, 20, 16, 16), (8, 6, 41, 43),
+                                   (32, 4, 57, 55), (12, 3, 112, 111), (64, 2, 64, 64), (1, 4, 200, 203)])
+def test_batchnorm_planes(shape):
+    _batchnorm(shape, np.float16)
+
+
+@pytest.mark.parametrize("offset", [1, 3, 8])
+def test_batchnorm_input_at_any_address(offset):
+    """(an input whose rows lie unlike the result's relative to 16 bytes goes to the interpreter)"""
+    _batchnorm((6, 5, 9, 9), np.float16, offset)
+
+
+@pytest.mark.parametrize("residual,weight,gate", [(1, 1, 1), (0, 1, 0), (1, 0, 0), (0, 0, 1)])
+@pytest.mark.parametrize("tokens,hidden", [(1, 8), (3, 65), (5, 255), (2, 515), (7, 1024), (130, 1031), (1, 4097), (3, 8185), (600, 700)])
+def test_rmsnorm_rows(tokens, hidden, residual, weight, gate):
+    from dvm_b200.tester import Tester
+    rng = np.random.default_rng(tokens * 31 + hidden)
+    bf = lambda x: Tester.convert_from_bf16(Tester.convert_to_bf16(x.astype(np.float32)))
+    h, r, g, u = (bf(rng.standard_normal((tokens, hidden))) for _ in range(4))
+    w = bf(rng.normal(1, 0.1, (hidden,)))
+    t = Tester("vector")
+    s = t.cast(t.load(h, "bfloat16"), 3)
+    sd = h.astype(np.float64)
+    if residual:
+        s = t.add(s, t.cast(t.load(r, "bfloat16"), 3))
+        sd = sd + r
+    ss = t.sum(t.mul(s, s), (1,), True)
+    y = t.mul(s, t.div(1.0, t.sqrt(t.add(t.mul(ss, 1.0 / hidden), 1e-6))))
+    want = sd / np.sqrt((sd * sd).mean(1, keepdims=True) + 1e-6)
+    if weight:
+        y = t.mul(y, t.cast(t.load(w, "bfloat16"), 3))
+        want = want * w
+    stores, wants = [t.store(t.cast(y, 2))], [want]
+    if gate:
+        gf = t.cast(t.load(g, "bfloat16"), 3)
+        sig = t.div(1.0, t.add(t.exp(t.mul(gf, -1.0)), 1.0))
+        stores.append(t.store(t.cast(t.mul(t.mul(gf, sig), t.cast(t.load(u, "bfloat16"), 3)), 2)))
+        gd = g.astype(np.float64)
+        wants.append(gd / (1 + np.exp(-gd)) * u)
+    t.run()
+    for st, want in zip(stores, wants):
+        got = Tester.convert_from_bf16(t.output(st)).astype(np.float64)
+        # one rounding to bf16 (2^-9), fp32 arithmetic in front of it
+        assert np.all(np.abs(got - want) <= 2.0 ** -8 * np.abs(want) + 1e-5), float(np.abs(got - want).max())
+
+
+def test_scalar_sections_of_any_form_run_as_words():
+    """Statistics whose scalar sections are not the usual closed form (a clamp, several stored scalars)."""
+    from dvm_b200.tester import Tester
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((37, 1500)).astype(np.float32)
+    t = Tester("vector")
+    lx = t.load(x)
+    s1, s2 = t.sum(lx, (1,), True), t.sum(t.mul(lx, lx), (1,), True)
+    a = t.maximum(t.sqrt(t.mul(s2, 1.0 / 1500)), 0.5)
+    stores = [t.store(t.mul(t.sub(lx, t.mul(s1, 1.0 / 1500)), a)), t.store(a), t.store(s1)]
+    t.run()
+    xd = x.astype(np.float64)
+    ad = np.maximum(np.sqrt((xd * xd).mean(1, keepdims=True)), 0.5)
+    for st, want in zip(stores, [(xd - xd.mean(1, keepdims=True)) * ad, ad, xd.sum(1, keepdims=True)]):
+        assert np.allclose(t.output(st), want, rtol=1e-5, atol=1e-4)
