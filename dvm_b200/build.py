@@ -30,6 +30,7 @@ SOURCES = [
     "mm_tcgen05.cu",
     "mm_tile.cu",
     "attn_tcgen05.cu",
+    "attn_decode.cu",
 ]
 
 NVCC_FLAGS = [

@@ -490,6 +490,7 @@ bool AttentionSupported(const AttnParam &p) {
 int LaunchAttention(const AttnParam &p, void *stream) {
   if (!AttentionSupported(p)) return -1;
   if ((p.q_ptr | p.k_ptr | p.v_ptr | p.o_ptr) & 15u) return -2;
+  if (p.sq <= kDecodeMaxRows) return LaunchAttentionDecode(p, stream);   // one MMA of 16 rows holds every query row
   int dev = 0;
   cudaGetDevice(&dev);
   using KernelFn = void (*)(const AttnParam, const AttnMaps, const uint32_t);

@@ -86,6 +86,8 @@ struct AttnParam {
   uint64_t q_ptr, k_ptr, v_ptr, o_ptr;
 };
 int LaunchAttention(const AttnParam &p, void *stream);
+constexpr uint32_t kDecodeMaxRows = 16;
+int LaunchAttentionDecode(const AttnParam &p, void *stream);   // at most kDecodeMaxRows query rows (attn_decode.cu)
 bool AttentionSupported(const AttnParam &p);
 unsigned int ReadAttentionStatus();
 
