@@ -98,6 +98,7 @@ SIGNATURES = {
     "dvm_static_scratch_capacity": (c_size_t, []),
     "dvm_last_jit_us": (ctypes.c_double, [c_void_p]),
     "dvm_object_rank": (c_int, [c_void_p]),
+    "dvm_object_shape": (c_int, [c_void_p, ctypes.POINTER(c_int64), c_int]),
     "dvm_object_dim": (c_int64, [c_void_p, c_int]),
     "dvm_object_dtype": (c_int, [c_void_p]),
     "dvm_dump": (c_char_p, [c_void_p]),

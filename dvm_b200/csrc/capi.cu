@@ -427,6 +427,11 @@ int64_t dvm_object_dim(const dvm_object *o, int i) {
   // (a PadStore reports the shape of its buffer: rows longer by the pad)
   return n->shape.d[i] + (n->kind == dvm::N_STORE && i == n->shape.rank - 1 ? n->pad_size : 0);
 }
+int dvm_object_shape(const dvm_object *o, int64_t *dims, int capacity) {
+  const int rank = dvm_object_rank(o);
+  for (int i = 0; i < rank && i < capacity; ++i) dims[i] = dvm_object_dim(o, i);
+  return rank;
+}
 int dvm_object_dtype(const dvm_object *o) { return reinterpret_cast<const dvm::NDObject *>(o)->dtype; }
 
 const char *dvm_dump(dvm_kernel *k) { return Guard([&]() { return k->kernel.Dump(); }, ""); }

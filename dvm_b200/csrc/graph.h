@@ -196,6 +196,9 @@ class VKernel {
  public:
   VKernel(KernelType type, uint32_t flags) : type_(type), flags_(flags) {}
   void ClearStages();
+  // Everything a plan depends on beside the graph itself: the values of the borrowed shapes and scalars.
+  void Signature(std::vector<int64_t> *out) const;
+  void DropPlans();   // forget the plans kept for other shapes (the graph has changed)
   // stat_fusion.cc: the op list with sums of squared deviations folded into the pass that makes their mean
   std::vector<NDObject *> FuseDeviationSums(const std::vector<NDObject *> &ops);
   void PlanStages(const std::vector<NDObject *> &ops);   // partition.cc: general multi-stage planner
@@ -203,7 +206,8 @@ class VKernel {
 
   NDObject *NewNode(NodeKind kind, DataType dtype);
   void Normalize();
-  size_t Compile();   // build stages for the current shapes; returns workspace bytes
+  size_t Compile();   // stages for the current shapes, built or taken from plans_; returns workspace bytes
+  void CompileFresh();
   void Bind(const RelocEntry *relocs, size_t n, void *workspace);
   int Launch(void *stream);
   int LaunchStage(size_t index, void *stream);   // one launch (or collective) of the plan, for per-stage timing
@@ -224,6 +228,21 @@ class VKernel {
   std::vector<NDObject *> synth_;          // planner-made nodes (clones, workspace temporaries), owned
   std::vector<std::vector<NDObject *>> split_outs_;   // arrays handed out by Kernel::Split (valid for the kernel's life)
   size_t ws_bytes_ = 0;
+  // Plans of the shapes seen last, so that a loop that comes back to a shape (decode steps, the last batch of an epoch)
+  // does not plan it again: at most kMaxPlans of about 10 KB each, the least recently used one goes.  The plan in use is
+  // stages_ / synth_ / ws_bytes_ with signature plan_sig_ (when has_plan_).
+  struct Plan {
+    std::vector<int64_t> sig;
+    std::vector<std::unique_ptr<Stage>> stages;
+    std::vector<NDObject *> synth;
+    size_t ws_bytes = 0;
+    uint64_t used = 0;
+  };
+  static constexpr size_t kMaxPlans = 16;
+  std::vector<Plan> plans_;
+  std::vector<int64_t> sig_, plan_sig_, sig_scratch_;
+  bool has_plan_ = false;
+  uint64_t plan_clock_ = 0;
   int cur_sub_ = 0;                        // sub-kernel that NewNode() tags ops with (SequenceAdd / ParallelAdd advance it)
   void *workspace_ = nullptr;
   bool normalized_ = false;

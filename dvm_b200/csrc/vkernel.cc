@@ -1,7 +1,9 @@
 // VKernel: owns the graph of one dvm::Kernel, runs shape inference, plans the launches and runs them.
 // Counterpart of the reference's VKernel / VKernelS lifecycle (Normalize/CodeGen/CodeGenR/Launch,
 // src/kernel.cc:104-156, 2113-2209) for the sm_100a interpreters.
+#include <algorithm>
 #include <chrono>
+#include <cstddef>
 #include <cstring>
 #include <string>
 
@@ -17,6 +19,7 @@ namespace dvm {
 
 VKernel::~VKernel() {
   ClearStages();
+  DropPlans();
   for (auto n : nodes_) delete n;
   for (void *e : stage_events_)
     if (e) cudaEventDestroy(static_cast<cudaEvent_t>(e));
@@ -28,6 +31,41 @@ void VKernel::ClearStages() {
   stages_.clear();
   for (auto n : synth_) delete n;
   synth_.clear();
+}
+
+void VKernel::DropPlans() {
+  for (auto &p : plans_)
+    for (auto n : p.synth) delete n;
+  plans_.clear();
+  has_plan_ = false;
+}
+
+void VKernel::Signature(std::vector<int64_t> *out) const {
+  out->clear();
+  auto ints = [&](const IntArrayRef *r) {
+    if (r == nullptr) return;
+    out->push_back(static_cast<int64_t>(r->size));
+    for (size_t i = 0; i < r->size && r->data != nullptr; ++i) out->push_back(r->data[i]);
+  };
+  auto scalar = [&](const ScalarRef *r) {
+    if (r == nullptr) return;
+    out->push_back(static_cast<int64_t>(r->type));
+    out->push_back(r->type == kInt64 ? r->i64 : r->type == kFloat16 || r->type == kBFloat16 ? r->f16 : r->i32);   // (fp32: its bits)
+  };
+  for (auto n : nodes_) {
+    if (!n->reduce_all) ints(n->shape_ref);   // (a reduction over every dim makes its own list)
+    ints(n->stride_ref);
+    ints(n->slice_a);
+    ints(n->slice_b);
+    ints(n->slice_c);
+    ints(n->aux_ref);
+    scalar(n->scalar_ref);
+    scalar(n->scalar_ref2);
+    if (n->comm != nullptr) {
+      out->push_back(n->comm->rank);
+      out->push_back(n->comm->size);
+    }
+  }
 }
 
 // Device address of a load/store node: a workspace temporary, a clone of a user's node, or the node itself.
@@ -50,10 +88,15 @@ NDObject *VKernel::NewNode(NodeKind kind, DataType dtype) {
   nodes_.push_back(n);
   normalized_ = false;
   compiled_ = false;
+  DropPlans();
   return n;
 }
 
 void VKernel::Normalize() {
+  Signature(&sig_scratch_);
+  if (normalized_ && sig_scratch_ == sig_) return;   // (inferred, and perhaps planned, for these very values)
+  sig_.swap(sig_scratch_);
+  normalized_ = compiled_ = false;
   // a Store handed to a later op as an operand stands for the value it stores (the reference's sequence kernels read a
   // stage's stored result back in a later stage, tests/ut/test_sequence_fusion.py:170-205)
   for (auto n : nodes_)
@@ -82,12 +125,52 @@ static std::vector<NDObject *> LiveOps(const std::vector<NDObject *> &nodes) {
 
 size_t VKernel::Compile() {
   if (!normalized_) Normalize();
+  if (compiled_) return ws_bytes_;
+  if (has_plan_ && plan_sig_ == sig_) {
+    compiled_ = true;
+    return ws_bytes_;
+  }
+  if (has_plan_) {   // keep the plan of the previous shapes
+    if (plans_.size() >= kMaxPlans) {
+      auto oldest = std::min_element(plans_.begin(), plans_.end(), [](const Plan &a, const Plan &b) { return a.used < b.used; });
+      for (auto n : oldest->synth) delete n;
+      plans_.erase(oldest);
+    }
+    Plan p;
+    p.sig = plan_sig_;
+    p.stages = std::move(stages_);
+    p.synth = std::move(synth_);
+    p.ws_bytes = ws_bytes_;
+    p.used = ++plan_clock_;
+    plans_.push_back(std::move(p));
+    stages_.clear();
+    synth_.clear();
+    has_plan_ = false;
+  }
+  for (size_t i = 0; i < plans_.size(); ++i)
+    if (plans_[i].sig == sig_) {
+      ClearStages();
+      stages_ = std::move(plans_[i].stages);
+      synth_ = std::move(plans_[i].synth);
+      ws_bytes_ = plans_[i].ws_bytes;
+      plans_.erase(plans_.begin() + static_cast<std::ptrdiff_t>(i));
+      plan_sig_ = sig_;
+      has_plan_ = compiled_ = true;
+      return ws_bytes_;
+    }
+  CompileFresh();
+  plan_sig_ = sig_;
+  has_plan_ = true;
+  return ws_bytes_;
+}
+
+void VKernel::CompileFresh() {
   ClearStages();
   ws_bytes_ = 0;
   std::vector<NDObject *> ops = LiveOps(nodes_);
   if (ops.empty()) {
     compiled_ = true;
-    return 0;
+    return;
   }
   bool has_matmul = false, has_empty = false, stacked = false;
   for (auto n : ops) {
@@ -104,19 +187,18 @@ size_t VKernel::Compile() {
       if (CompileVectorStage(folded, &st->vec, &why)) {
         stages_.push_back(std::move(st));
         compiled_ = true;
-        return 0;
+        return;
       }
     }
     auto st = std::make_unique<Stage>();
     if (CompileVectorStage(ops, &st->vec, &why)) {
       stages_.push_back(std::move(st));
       compiled_ = true;
-      return 0;
+      return;
     }
   }
   PlanStages(ops);
   compiled_ = true;
-  return ws_bytes_;
 }
 
 void VKernel::Bind(const RelocEntry *relocs, size_t n, void *workspace) {

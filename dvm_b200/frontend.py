@@ -7,6 +7,7 @@ helpers of the C ABI, like the reference's DevRunner (src/pybind_api.cc:195-271)
 copies host -> device, ``output`` copies device -> host.
 """
 import ctypes
+import weakref
 
 import numpy as np
 
@@ -35,6 +36,8 @@ for _i, _n in enumerate(DataType._names):
     setattr(DataType, _n, DataType(_i))
 
 ITEM_SIZE = [1, 2, 2, 4, 4, 8]
+_MAX_RANK = 16   # room for any shape the library hands out
+_INT64_ARRAYS = [ctypes.c_int64 * max(1, n) for n in range(_MAX_RANK + 1)]
 
 
 def np_dtype_of(dtype):
@@ -60,8 +63,8 @@ class NDObject:
         self._owner = owner  # keeps the kernel alive
 
     def shape(self):
-        lib = _capi.load()
-        return tuple(int(lib.dvm_object_dim(self._h, i)) for i in range(lib.dvm_object_rank(self._h)))
+        dims = (ctypes.c_int64 * _MAX_RANK)()
+        return tuple(dims[:_capi.load().dvm_object_shape(self._h, dims, _MAX_RANK)])
 
     def dtype(self):
         return DataType(_capi.load().dvm_object_dtype(self._h))
@@ -69,10 +72,11 @@ class NDObject:
 
 class IntArrayRef:
     def __init__(self, shape=None):
-        lib = _capi.load()
-        vals = [int(v) for v in (shape or [])]
+        self._lib = _capi.load()
+        vals = tuple(map(int, shape or ()))
         arr = (ctypes.c_int64 * max(1, len(vals)))(*vals)
-        self._h = check_ptr(lib.dvm_int_array_new(arr, len(vals)), "int array")
+        self._h = check_ptr(self._lib.dvm_int_array_new(arr, len(vals)), "int array")
+        self._vals = vals   # what the native array holds: an update to the same values needs no call
 
     def shape(self):
         lib = _capi.load()
@@ -81,9 +85,11 @@ class IntArrayRef:
         return tuple(int(data[i]) for i in range(n))
 
     def update(self, shape):
-        vals = [int(v) for v in shape]
-        arr = (ctypes.c_int64 * max(1, len(vals)))(*vals)
-        _capi.load().dvm_int_array_update(self._h, arr, len(vals))
+        vals = tuple(map(int, shape))
+        if vals != self._vals:
+            self._lib.dvm_int_array_update(self._h, _INT64_ARRAYS[len(vals)](*vals) if len(vals) <= _MAX_RANK else
+                                           (ctypes.c_int64 * len(vals))(*vals), len(vals))
+            self._vals = vals
 
     def __del__(self):
         try:
@@ -425,6 +431,7 @@ class _DevBuf:
 
 class _ExternalBuf:
     """Device memory owned by the caller (e.g. a torch tensor) bound to a load or store."""
+    __slots__ = ("ptr", "nbytes")
 
     def __init__(self, ptr, nbytes):
         self.ptr = int(ptr)
@@ -538,7 +545,12 @@ class PyKernel(Kernel):
         self._run_type = run_type
         self._dev_id = int(dev_id)
         self._loads = []   # [op, dev buffer, host array]
-        self._stores = []  # [op, dev buffer, host array]
+        self._stores = []  # [op, dev buffer, host array, its type, shape of the result]
+        self._by_handle = {}    # op handle -> its record
+        self._preset = {}       # store handle -> (host array, byte offset): set_output()
+        self._load_offset = {}  # load handle -> byte offset of the tensor in its array
+        self._relocs = None     # (array, count, its entries) as the last code generation was given them
+        self._dims = (ctypes.c_int64 * _MAX_RANK)()
         self._ws = None
         self._ws_cb = None
         if run_type == "dev":
@@ -583,12 +595,14 @@ class PyKernel(Kernel):
         check_rc(lib.dvm_kernel_clone(self._k, base._k, m), "clone")
         self._ktype, self._flags = base._ktype, base._flags
         self._loads, self._stores = [], []
+        self._by_handle.clear()
+        self._relocs = None
         for rec, ref in zip(base._loads, load_refs):
             op = self._obj(lib.dvm_clone_map_object(m, rec[0]._h), "clone")
             op._shape_ref = ref
             self._loads.append([op, None, None])
         for rec in base._stores:
-            self._stores.append([self._obj(lib.dvm_clone_map_object(m, rec[0]._h), "clone"), None, None])
+            self._stores.append([self._obj(lib.dvm_clone_map_object(m, rec[0]._h), "clone"), None, None, None, None])
         known = {rec[0]._h: rec[0] for rec in self._loads + self._stores}
         for i, x in enumerate(remap):
             if isinstance(x, NDObject):
@@ -604,7 +618,7 @@ class PyKernel(Kernel):
 
     def store(self, obj, type=None):
         op = Kernel.store(self, obj, type)
-        self._stores.append([op, None, None])
+        self._stores.append([op, None, None, None, None])
         return op
 
     def view_load(self, shape, stride, type):
@@ -614,7 +628,7 @@ class PyKernel(Kernel):
 
     def pad_store(self, obj, pad_size):
         op = Kernel.pad_store(self, obj, pad_size)
-        self._stores.append([op, None, None])
+        self._stores.append([op, None, None, None, None])
         return op
 
     def slice_load(self, shape, start, size, type):
@@ -629,7 +643,7 @@ class PyKernel(Kernel):
 
     def view_store(self, obj, stride, type=None):
         op = Kernel.view_store(self, obj, stride, type)
-        self._stores.append([op, None, None])
+        self._stores.append([op, None, None, None, None])
         return op
 
     def set_output(self, store, array, offset=0):
@@ -639,14 +653,22 @@ class PyKernel(Kernel):
         starts, the counterpart of input()'s offset."""
         rec = self._find(self._stores, store)
         rec[2] = np.ascontiguousarray(array)
-        self._preset = getattr(self, "_preset", {})
         self._preset[store._h] = (rec[2], int(offset) * rec[2].dtype.itemsize)
 
+    def _record(self, op):
+        """The record of a load or store of this kernel, or None."""
+        table = self._by_handle
+        if len(table) != len(self._loads) + len(self._stores):
+            table.clear()
+            for rec in self._loads + self._stores:
+                table[rec[0]._h] = rec
+        return table.get(op._h)
+
     def _find(self, table, op):
-        for rec in table:
-            if rec[0] is op or rec[0]._h == op._h:
-                return rec
-        raise DvmError("object does not belong to this kernel")
+        rec = self._record(op)
+        if rec is None or (len(rec) == 3) != (table is self._loads):   # (a load's record has three fields)
+            raise DvmError("object does not belong to this kernel")
+        return rec
 
     @staticmethod
     def convert_to_bf16(array):
@@ -684,7 +706,6 @@ class PyKernel(Kernel):
                 rec[1].free()
             rec[1] = _DevBuf(max(arr.nbytes, 1))
         rec[2] = arr
-        self._load_offset = getattr(self, "_load_offset", {})
         self._load_offset[obj._h] = int(offset) * arr.dtype.itemsize   # the tensor starts `offset` elements into the array
         if arr.nbytes:
             check_rc(self._lib.dvm_rt_memcpy_h2d(rec[1].ptr, arr.ctypes.data, arr.nbytes, None), "H2D copy")
@@ -692,69 +713,86 @@ class PyKernel(Kernel):
     def bind_device(self, obj, ptr, nbytes):
         """Use caller-owned device memory for a load or store (no counterpart in the reference's Python API, which
         always copies through NumPy; the C++ API takes device pointers through RelocEntry, include/dvm.h:201-206)."""
-        for recs in (self._loads, self._stores):
-            for rec in recs:
-                if rec[0]._h == obj._h:
-                    if rec[1] is not None:
-                        rec[1].free()
-                    rec[1] = _ExternalBuf(ptr, nbytes)
-                    return
-        raise DvmError("bind_device: not a load or store of this kernel")
+        rec = self._record(obj)
+        if rec is None:
+            raise DvmError("bind_device: not a load or store of this kernel")
+        buf = rec[1]
+        if type(buf) is _ExternalBuf:
+            buf.ptr, buf.nbytes = int(ptr), int(nbytes)
+            return
+        if buf is not None:
+            buf.free()
+        rec[1] = _ExternalBuf(ptr, nbytes)
 
-    def codegen(self, pass_names=None):
-        check_rc(self._lib.dvm_normalize(self._k), "normalize")
-        relocs = []
-        for rec in self._stores:
-            op = rec[0]
-            shape = op.shape()
-            dt = np_dtype_of(op.dtype())
-            nbytes = int(np.prod(shape, dtype=np.int64)) * dt.itemsize if len(shape) else dt.itemsize
-            preset, preset_off = getattr(self, "_preset", {}).get(op._h, (None, 0))
-            if preset is not None:
-                rec[2] = preset
-                nbytes = preset.nbytes
-            else:
-                rec[2] = np.empty(shape, dtype=dt)
-            if self._run_type == "dev":
-                if rec[1] is None or rec[1].nbytes < nbytes:
-                    if rec[1] is not None:
-                        rec[1].free()
-                    rec[1] = _DevBuf(max(nbytes, 1))
-                if preset is not None and nbytes:
-                    check_rc(self._lib.dvm_rt_memcpy_h2d(rec[1].ptr, preset.ctypes.data, nbytes, None), "H2D copy")
-                relocs.append((op._h, rec[1].ptr + preset_off))
-            else:
-                relocs.append((op._h, 0x1000 * (len(relocs) + 1)))
-        for rec in self._loads:
-            if self._run_type == "dev":
-                if rec[1] is None:
-                    raise DvmError("load has no input bound; call input() first")
-                relocs.append((rec[0]._h, rec[1].ptr + getattr(self, "_load_offset", {}).get(rec[0]._h, 0)))
-            else:
-                relocs.append((rec[0]._h, 0x1000 * (len(relocs) + 1)))
-        arr = (_capi.Reloc * max(1, len(relocs)))()
-        for i, (h, p) in enumerate(relocs):
-            arr[i].io = h
-            arr[i].addr = p
+    def _ws_callback(self):
+        # (the callback must not keep the kernel alive: a cycle would leave its device memory to the collector)
+        me = weakref.ref(self)
 
         def alloc(size, _user):
-            if self._run_type != "dev":
+            k = me()
+            if k is None or k._run_type != "dev":
                 return 0x100000
-            if self._ws is None or self._ws.nbytes < size:
-                if self._ws is not None:
-                    self._ws.free()
-                self._ws = _DevBuf(size)
-            return self._ws.ptr
+            if k._ws is None or k._ws.nbytes < size:
+                if k._ws is not None:
+                    k._ws.free()
+                k._ws = _DevBuf(size)
+            return k._ws.ptr
 
-        self._ws_cb = _capi.WS_ALLOC_FN(alloc)
-        self._reloc_args = (arr, len(relocs))   # what the last code generation was given (kept for repeat_codegen_launch)
-        check_rc(self._lib.dvm_codegen(self._k, arr, len(relocs), self._ws_cb, None), "codegen")
+        return _capi.WS_ALLOC_FN(alloc)
+
+    def codegen(self, pass_names=None):
+        lib, dev, presets, offsets, dims = self._lib, self._run_type == "dev", self._preset, self._load_offset, self._dims
+        check_rc(lib.dvm_normalize(self._k), "normalize")
+        count = len(self._stores) + len(self._loads)
+        if self._relocs is None or self._relocs[1] != count:
+            arr = (_capi.Reloc * max(1, count))()
+            for i, rec in enumerate(self._stores + self._loads):
+                arr[i].io = rec[0]._h
+            self._relocs = (arr, count, [arr[i] for i in range(count)])
+        arr, _, entries = self._relocs
+        i = 0
+        for rec in self._stores:
+            h = rec[0]._h
+            dt = rec[3]
+            if dt is None:
+                dt = rec[3] = np_dtype_of(rec[0].dtype())
+            shape = rec[4] = dims[:lib.dvm_object_shape(h, dims, _MAX_RANK)]
+            nbytes = dt.itemsize
+            for n in shape:
+                nbytes *= n
+            preset, at = presets.get(h, (None, 0)) if presets else (None, 0)
+            rec[2] = preset   # (without one, output() makes the host array)
+            if preset is not None:
+                nbytes = preset.nbytes
+            if dev:
+                buf = rec[1]
+                if buf is None or buf.nbytes < nbytes:
+                    if buf is not None:
+                        buf.free()
+                    buf = rec[1] = _DevBuf(max(nbytes, 1))
+                if preset is not None and nbytes:
+                    check_rc(lib.dvm_rt_memcpy_h2d(buf.ptr, preset.ctypes.data, nbytes, None), "H2D copy")
+                entries[i].addr = buf.ptr + at
+            else:
+                entries[i].addr = 0x1000 * (i + 1)
+            i += 1
+        for rec in self._loads:
+            if dev:
+                if rec[1] is None:
+                    raise DvmError("load has no input bound; call input() first")
+                entries[i].addr = rec[1].ptr + (offsets.get(rec[0]._h, 0) if offsets else 0)
+            else:
+                entries[i].addr = 0x1000 * (i + 1)
+            i += 1
+        if self._ws_cb is None:
+            self._ws_cb = self._ws_callback()
+        check_rc(lib.dvm_codegen(self._k, arr, count, self._ws_cb, None), "codegen")
 
     def repeat_codegen_launch(self, stream=None):
         """Shape inference + planning + emission + binding + launch once more, with the addresses of the last codegen():
         the three C calls a framework makes when a new shape arrives (dvm_normalize is part of dvm_codegen), without this
         front-end's own bookkeeping around them."""
-        arr, n = self._reloc_args
+        arr, n = self._relocs[:2]
         check_rc(self._lib.dvm_codegen(self._k, arr, n, self._ws_cb, None), "codegen")
         check_rc(self._lib.dvm_launch(self._k, stream), "launch")
 
@@ -772,7 +810,9 @@ class PyKernel(Kernel):
         rec = self._find(self._stores, store)
         host = rec[2]
         if host is None:
-            raise DvmError("output() before codegen()")
+            if rec[4] is None:
+                raise DvmError("output() before codegen()")
+            host = rec[2] = np.empty(rec[4], dtype=rec[3])
         if host.nbytes:
             check_rc(self._lib.dvm_rt_memcpy_d2h(host.ctypes.data, rec[1].ptr, host.nbytes, None), "D2H copy")
             check_rc(self._lib.dvm_rt_sync(None), "synchronize")
@@ -804,6 +844,10 @@ class PyKernel(Kernel):
         check_rc(self._lib.dvm_kernel_reset(self._k, self._ktype, self._flags), "reset")
         self._loads = []
         self._stores = []
+        self._by_handle.clear()
+        self._preset.clear()
+        self._load_offset.clear()
+        self._relocs = None
         self._keep = []
 
     def release_io(self):
@@ -813,10 +857,8 @@ class PyKernel(Kernel):
                 rec[1] = None
 
     def device_ptr(self, op):
-        for rec in self._loads + self._stores:
-            if rec[0]._h == op._h:
-                return rec[1].ptr if rec[1] is not None else None
-        return None
+        rec = self._record(op)
+        return rec[1].ptr if rec is not None and rec[1] is not None else None
 
     def __del__(self):
         try:

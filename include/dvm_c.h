@@ -183,6 +183,8 @@ DVM_C_API double dvm_last_jit_us(const dvm_kernel *k);
 
 /* ---- introspection (NDObjectPy::GetShape/GetDType include/dvm_py.h:28-38; Dump/DumpR/Das/Inspect dvm.h:619-637) ---- */
 DVM_C_API int dvm_object_rank(const dvm_object *o);
+/* the whole shape at once: at most `capacity` dims, returns the rank */
+DVM_C_API int dvm_object_shape(const dvm_object *o, int64_t *dims, int capacity);
 DVM_C_API int64_t dvm_object_dim(const dvm_object *o, int i);
 DVM_C_API int dvm_object_dtype(const dvm_object *o);
 DVM_C_API const char *dvm_dump(dvm_kernel *k);
