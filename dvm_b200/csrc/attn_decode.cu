@@ -17,6 +17,7 @@
 #include <cstdint>
 #include <cstring>
 
+#include "chain.cuh"
 #include "mm_launch.h"
 #include "runtime.h"
 #include "vm_ops.cuh"
@@ -108,6 +109,8 @@ template <uint32_t DT, uint32_t D, bool SCALE_FIRST>
 __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs &A) {
   constexpr uint32_t JK = D / 32, HV = D / 64;   // 16-byte pieces of a key row per thread, 64-element halves of a value row
   extern __shared__ __align__(16) uint8_t smem[];
+  chain_wait();
+  chain_launch();
   Combine<D> &sm = *reinterpret_cast<Combine<D> *>(smem);
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, q4 = lane & 3u, q8 = lane >> 2;
   const uint32_t CL = A.cluster, rank = CL > 1 ? rank_in_cluster() : 0u;
@@ -367,13 +370,14 @@ int LaunchAttentionDecode(const AttnParam &p, void *stream) {
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = p.d == 128 ? sizeof(Combine<128>) : sizeof(Combine<64>);
   cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cl;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = cl > 1 ? 1 : 0;
+  ChainAttribute(&cfg, attr);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, table[p.dtype == T_BF16 ? 0 : 1][p.d == 128 ? 1 : 0][p.scale_first ? 1 : 0], p, a);
   return e != cudaSuccess ? static_cast<int>(e) : static_cast<int>(cudaGetLastError());
 }

@@ -24,6 +24,7 @@
 #include <cstdint>
 #include <cstring>
 
+#include "chain.cuh"
 #include "mm_launch.h"
 #include "sm100_sync.cuh"
 #include "vm_ops.cuh"
@@ -162,6 +163,8 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
   __syncthreads();
   tcgen05_after_sync();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(smem + kTmemSlot);
+  chain_wait();
+  chain_launch();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -511,8 +514,15 @@ int LaunchAttention(const AttnParam &p, void *stream) {
   if (rc == 0) rc = EncodeRows(&maps.v, p.v_ptr, p.d, p.skv, p.batch);
   if (rc != 0) return rc;
   const uint32_t qblocks = (p.sq + kTileQ * kQTilesPerCta - 1) / (kTileQ * kQTilesPerCta);
-  kernel<<<p.batch * qblocks, kThreads, kSmemBytes, static_cast<cudaStream_t>(stream)>>>(p, maps, NextLaunchEpoch());
-  return static_cast<int>(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(p.batch * qblocks, 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  ChainAttribute(&cfg, attr);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p, maps, NextLaunchEpoch());
+  return e != cudaSuccess ? static_cast<int>(e) : static_cast<int>(cudaGetLastError());
 }
 
 unsigned int ReadAttentionStatus() {

@@ -14,6 +14,7 @@
 #include "../../include/dvm.h"
 #include "isa.h"
 #include "mm_launch.h"
+#include "vm_direct.h"
 #include "vm_row.h"
 
 namespace dvm {
@@ -144,6 +145,9 @@ struct VectorStage {
   // the stage's definition and its fallback
   dvmb::RowParam row;
   bool row_ok = false;
+  // ... and a short reduce-free program that the direct kernel runs (vm_direct.cu)
+  dvmb::DirectParam direct;
+  bool direct_ok = false;
 };
 
 // One launch of the tensor-core MatMul with its fused post-ops.
@@ -262,6 +266,9 @@ std::string DisassembleStage(const VectorStage &st);
 // row_match.cc: fill st->row when the compiled stage is one of the row kernels' shapes; bind its addresses.
 void MatchRowKernel(VectorStage *st);
 void BindRow(VectorStage *st);
+// row_match.cc: the same for the direct kernel.
+void MatchDirectKernel(VectorStage *st);
+void BindDirect(VectorStage *st);
 // Turn the stage's instruction words into the launch program (scalar sections + micro-ops) for the tensor
 // addresses now in the descriptors; called whenever addresses are (re)bound.
 void LowerStage(VectorStage *st);

@@ -28,6 +28,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "chain.cuh"
 #include "mm_epilogue.cuh"
 #include "mm_launch.h"
 #include "sm100_sync.cuh"
@@ -128,6 +129,8 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
   cluster_sync_all();   // the peer's barriers are initialised before anything signals them
   tcgen05_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  chain_wait();
+  chain_launch();
 
   // (The two issuing loops run under elect.sync: inside a plain `lane == 0` branch every MMA took about 100 cycles to
   // issue and every TMA load 150-280 - operands moved to uniform registers one by one - and a k-block 560-630 cycles
@@ -461,8 +464,15 @@ int LaunchMatMul(const MmParam &p_in, void *stream) {
   if (rc != 0) return rc;
   const uint32_t tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.batch0 * p.batch1;
   const uint32_t units = tiles < static_cast<uint32_t>(sms / 2) ? tiles : static_cast<uint32_t>(sms / 2);
-  dvm_b200_mm_tcgen05_pair<<<units * 2, kThreads, kSmemBytes, static_cast<cudaStream_t>(stream)>>>(p, maps, NextLaunchEpoch());
-  return static_cast<int>(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(units * 2, 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  ChainAttribute(&cfg, attr);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, dvm_b200_mm_tcgen05_pair, p, maps, NextLaunchEpoch());
+  return e != cudaSuccess ? static_cast<int>(e) : static_cast<int>(cudaGetLastError());
 }
 
 unsigned int ReadMatMulStatus() {

@@ -22,6 +22,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "chain.cuh"
 #include "mm_epilogue.cuh"
 #include "mm_launch.h"
 #include "sm100_sync.cuh"
@@ -161,6 +162,8 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
   __syncthreads();
   tcgen05_after_sync();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(smem + kTmemSlot);
+  chain_wait();
+  chain_launch();
 
   // stage: B [BN x 64] first, then A (its MMA reads 128 rows; the rows past a_rows are whatever follows, and only feed rows
   // of the accumulator that are never read)
@@ -450,13 +453,14 @@ int LaunchMmTile(const MmParam &p, uint32_t bn, uint32_t split, void *stream) {
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = split;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  ChainAttribute(&cfg, attr);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, bn == 64 ? dvm_b200_mm_tile_n64 : dvm_b200_mm_tile_n128, p, maps, a, NextLaunchEpoch());
   return e != cudaSuccess ? static_cast<int>(e) : static_cast<int>(cudaGetLastError());
 }

@@ -371,6 +371,9 @@ struct Matcher {
 
 }  // namespace
 
+// The direct kernel takes launches of up to this many elements (see the note at MatchDirectKernel).
+constexpr uint32_t kDirectMaxElems = 1u << 20;
+
 void MatchRowKernel(VectorStage *st) {
   RowParam &R = st->row;
   std::memset(&R, 0, sizeof(R));
@@ -395,6 +398,75 @@ void BindRow(VectorStage *st) {
   for (uint32_t s = 0; s < P.n_tensors; ++s)
     if (R.scalar_of[s] != 0xff) R.scalar[R.scalar_of[s]].ptr = P.tensor[s].ptr;
   st->row_ok = RowAddressesOk(R);
+}
+
+void MatchDirectKernel(VectorStage *st) {
+  DirectParam &D = st->direct;
+  std::memset(&D, 0, sizeof(D));
+  const VmParam &P = st->param;
+  static const char *const most_env = getenv("DVM_B200_DIRECT_MAX");
+  static const uint32_t most = most_env ? static_cast<uint32_t>(atoi(most_env)) : kDirectMaxElems;
+  if (st->idle || P.mode != VM_FLAT || P.num_body != 1 || P.group_elems > most || P.n_tensors > static_cast<uint32_t>(kDirectTensors)) return;
+  if (Word(st->bytecode[st->bsec[0]]).opc != OP_END || Word(st->bytecode[st->bsec[2]]).opc != OP_END) return;   // no group scalars
+  uint8_t at[kMaxTensors];
+  std::memset(at, 0xff, sizeof(at));
+  auto add = [&](uint32_t slot) {
+    if (at[slot] != 0xff) return true;
+    if (P.tensor[slot].mode != AM_DENSE) return false;
+    at[slot] = static_cast<uint8_t>(D.n_tensors);
+    D.slot[D.n_tensors] = static_cast<uint8_t>(slot);
+    D.dtype[D.n_tensors++] = P.tensor[slot].dtype;
+    return true;
+  };
+  uint32_t stored = 0;
+  for (int pass = 0; pass < 3; ++pass) {   // inputs, results, then the words
+    uint32_t n = 0;
+    for (size_t pc = st->bsec[1];; ++pc) {
+      const Word w(st->bytecode[pc]);
+      uint64_t out = w.w;
+      const bool takes = w.opc == OP_COPY || w.opc == OP_BIN || w.opc == OP_CMP || w.opc == OP_SEL;
+      auto operand_ok = [&](uint32_t kind, uint32_t idx) {
+        if (kind == K_TENSOR) return pass != 0 || add(idx);
+        return kind == K_IMM || kind == K_ACC || (kind == K_TEMP && idx < static_cast<uint32_t>(kDirectTemps));
+      };
+      if (pass == 0) {
+        if (takes && !operand_ok(w.kind, w.idx)) return;
+        if (w.opc == OP_SEL && !operand_ok(w.sub >> 4, w.sub & 15u)) return;
+        if (w.opc == OP_BIN && w.sub == B_POW) return;   // (its code is as long as all the rest of the kernel)
+        if (w.opc == OP_MOV && DVMB_DST(w.w) >= static_cast<uint32_t>(kDirectTemps)) return;
+        if (w.opc == OP_RACC || w.opc == OP_LD) return;
+      } else if (pass == 1) {
+        if (w.opc == OP_ST) {
+          // (a tensor both read and written: its elements are read before the store by the thread that stores them)
+          if (P.tensor[w.sub].mode != AM_DENSE || !add(w.sub)) return;
+          ++stored;
+        }
+      } else {
+        if (n >= static_cast<uint32_t>(kDirectCode)) return;
+        auto renumber = [&](int shift, uint32_t value) { out = (out & ~(0xfull << shift)) | (static_cast<uint64_t>(value) << shift); };
+        if (takes && w.kind == K_TENSOR) renumber(52, at[w.idx]);
+        if (w.opc == OP_SEL && (w.sub >> 4) == K_TENSOR) renumber(40, at[w.sub & 15u]);
+        if (w.opc == OP_ST) out = (out & ~(0xffull << 40)) | (static_cast<uint64_t>(at[w.sub]) << 40);
+        D.code[n++] = out;
+      }
+      if (w.opc == OP_END) break;
+    }
+    if (pass == 0) {
+      D.n_in = D.n_tensors;
+      if (D.n_in > static_cast<uint32_t>(kDirectInputs)) return;
+    }
+  }
+  if (stored != 0) D.elems = P.group_elems;
+}
+
+void BindDirect(VectorStage *st) {
+  DirectParam &D = st->direct;
+  st->direct_ok = true;
+  for (uint32_t i = 0; i < D.n_tensors; ++i) {
+    const TensorDesc &td = st->param.tensor[D.slot[i]];
+    D.ptr[i] = td.ptr;
+    if (!td.vec_ok) st->direct_ok = false;   // (granules of four elements are read and written whole)
+  }
 }
 
 }  // namespace dvm

@@ -1291,6 +1291,7 @@ bool CompileVectorStage(const std::vector<NDObject *> &ops, VectorStage *out, st
     Compiler c(ops, out);
     c.Run();
     MatchRowKernel(out);
+    MatchDirectKernel(out);
     return true;
   } catch (const Fail &f) {
     if (why) *why = f.why;

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "bounded_wait.cuh"
+#include "chain.cuh"
 #include "runtime.h"
 #include "vm_ops.cuh"
 #include "vm_row.h"
@@ -309,6 +310,8 @@ __device__ __forceinline__ void stats_affine_body(const RowParam &P, const uint3
     cluster_arrive();
     cluster_wait();
   }
+  chain_wait();
+  chain_launch();
 
   if (warp == kWorkWarps) {
     // ------------------------------ streaming warp ------------------------------
@@ -568,6 +571,8 @@ __device__ __forceinline__ float rcp_fast(float x) {
 template <uint32_t DT, int K>
 __device__ __forceinline__ void rms_gate_body(const RowParam &P) {
   __shared__ RowShared sm;
+  chain_wait();
+  chain_launch();
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
   const uint32_t tg = P.tg, rows = blockDim.x / tg, row_in_cta = tid / tg, t = tid - row_in_cta * tg;
   const uint32_t g = blockIdx.x * rows + row_in_cta;
@@ -833,8 +838,14 @@ int LaunchRow(const RowParam &p_in, void *stream) {
     using Fn = void (*)(const RowParam);
     const Fn fn = p.dtype == T_F16 ? (per_thread == 1 ? dvm_b200_row_rms_gate_f16_1 : dvm_b200_row_rms_gate_f16_2)
                                    : (per_thread == 1 ? dvm_b200_row_rms_gate_bf16_1 : dvm_b200_row_rms_gate_bf16_2);
-    fn<<<(p.groups + rows - 1) / rows, block, 0, s>>>(p);
-    return static_cast<int>(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3((p.groups + rows - 1) / rows, 1, 1);
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.stream = s;
+    ChainAttribute(&cfg, attr);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, p);
+    return e != cudaSuccess ? static_cast<int>(e) : static_cast<int>(cudaGetLastError());
   }
   uint32_t smem = 0;
   if (!StatsPlan(p.runs * units, p.groups, sms, &p, &smem)) return -7;
@@ -862,13 +873,14 @@ int LaunchRow(const RowParam &p_in, void *stream) {
   cfg.blockDim = dim3(kStatsThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = p.cluster;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.cluster > 1 ? 1 : 0;
+  ChainAttribute(&cfg, attr);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, p, NextLaunchEpoch());
   return e != cudaSuccess ? static_cast<int>(e) : static_cast<int>(cudaGetLastError());
 }

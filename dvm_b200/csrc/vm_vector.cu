@@ -23,6 +23,7 @@
 #include <cstring>
 
 #include "bounded_wait.cuh"
+#include "chain.cuh"
 #include "isa.h"
 #include "vm_launch.h"
 #include "vm_ops.cuh"
@@ -304,6 +305,9 @@ __device__ __forceinline__ void vm_vector_body(const VmParam &P, const uint32_t 
   } else {
     __syncthreads();
   }
+
+  chain_wait();   // (everything above reads parameters and writes shared memory only)
+  chain_launch();
 
   // =============================== producer warp ===============================
   // One warp feeds the ring: it walks the same tile sequence as the consumers, one stage after the other.
@@ -1381,7 +1385,7 @@ int LaunchVector(const VmParam &param, uint32_t grid, uint32_t threads, uint32_t
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem_bytes;
   cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   if (param.cluster > 1) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = param.cluster;
@@ -1441,6 +1445,7 @@ int LaunchVector(const VmParam &param, uint32_t grid, uint32_t threads, uint32_t
     fprintf(stderr, "dvm_b200 launch: grid=%u threads=%u smem=%u cluster=%u resident=%u blocks/SM=%d active clusters=%d\n", grid,
             threads, smem_bytes, param.cluster, param.resident, per_sm, clusters);
   }
+  ChainAttribute(&cfg, attr);
   const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, param, NextLaunchEpoch());
   if (le != cudaSuccess) return static_cast<int>(le);
   return static_cast<int>(cudaGetLastError());

@@ -543,6 +543,7 @@ class PyKernel(Kernel):
         if run_type not in ("dev", "das"):
             raise DvmError("run type '%s' is not available on this backend" % run_type)
         self._run_type = run_type
+        self._launch = self._lib.dvm_launch
         self._dev_id = int(dev_id)
         self._loads = []   # [op, dev buffer, host array]
         self._stores = []  # [op, dev buffer, host array, its type, shape of the result]
@@ -804,7 +805,9 @@ class PyKernel(Kernel):
 
     def launch(self, stream=None):
         """Enqueue without synchronising (no counterpart in the reference's Python API)."""
-        check_rc(self._lib.dvm_launch(self._k, stream), "launch")
+        rc = self._launch(self._k, stream)
+        if rc:
+            check_rc(rc, "launch")
 
     def output(self, store):
         rec = self._find(self._stores, store)
