@@ -24,6 +24,7 @@ SOURCES = [
     "row_match.cc",
     "comm.cc",
     "runtime.cu",
+    "staging.cc",
     "capi.cu",
     "vm_vector.cu",
     "vm_row.cu",

@@ -128,7 +128,7 @@ __device__ __forceinline__ uint32_t pack_pair(uint32_t dtype, float lo, float hi
 
 namespace {
 template <uint32_t DT, bool SCALE_FIRST>
-__device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMaps &maps, const uint32_t epoch) {
+__device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMaps &maps, const LaunchTag epoch) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
@@ -273,10 +273,9 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
           idle = 0;
           unsigned long long t_now;
           asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_now));
-          if (*reinterpret_cast<volatile unsigned int *>(&g_attn_status.abort_epoch) == epoch) break;
+          if (launch_aborted(&g_attn_status, epoch)) break;
           if (idle == 0 && t_now - t_last > kWaitLimitNs) {
-            atomicCAS(&g_attn_status.first_error, 0u, (11u << 24) | (blockIdx.x & 0xffffffu));
-            atomicExch(&g_attn_status.abort_epoch, epoch);
+            record_expiry(&g_attn_status, 11u, epoch);
             break;
           }
         }
@@ -444,7 +443,7 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
 
 #define DVMB_ATTN_KERNEL(NAME, DT, SF)                                                                              \
   __global__ void __launch_bounds__(kThreads, 1) NAME(const __grid_constant__ AttnParam P,                          \
-                                                      const __grid_constant__ AttnMaps maps, const uint32_t epoch) { \
+                                                      const __grid_constant__ AttnMaps maps, const LaunchTag epoch) { \
     attention_body<DT, SF>(P, maps, epoch);                                                                         \
   }
 DVMB_ATTN_KERNEL(dvm_b200_attention_bf16, T_BF16, false)
@@ -496,7 +495,7 @@ int LaunchAttention(const AttnParam &p, void *stream) {
   if (p.sq <= kDecodeMaxRows) return LaunchAttentionDecode(p, stream);   // one MMA of 16 rows holds every query row
   int dev = 0;
   cudaGetDevice(&dev);
-  using KernelFn = void (*)(const AttnParam, const AttnMaps, const uint32_t);
+  using KernelFn = void (*)(const AttnParam, const AttnMaps, const LaunchTag);
   static const KernelFn kernels[4] = {dvm_b200_attention_bf16, dvm_b200_attention_bf16_sf, dvm_b200_attention_f16,
                                       dvm_b200_attention_f16_sf};
   static bool attr_set[64] = {false};

@@ -21,26 +21,45 @@ struct WaitStatus {
 
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;
 
-// Host side: a fresh non-zero epoch for a launch (runtime.cu).
-uint32_t NextLaunchEpoch();
+// What a launch carries for its waits: its epoch, and a word of pinned host memory (null: none could be had) that an expiry
+// sets, so that the host learns without a device copy whether there is a record to read - reading the records cost five
+// copies of 12 us each at every synchronisation.
+struct LaunchTag {
+  uint32_t epoch;
+  uint32_t pad;
+  volatile uint32_t *host_flag;
+};
+// Host side (runtime.cu): a tag with a fresh non-zero epoch; whether any wait may have expired since the flag was lowered.
+LaunchTag NextLaunchEpoch();
+bool ExpiryFlagRaised();
+void LowerExpiryFlag();
+void RaiseExpiryFlag();
 
 #ifdef __CUDACC__
+__device__ __forceinline__ void record_expiry(WaitStatus *st, uint32_t code, const LaunchTag &tag) {
+  atomicCAS(&st->first_error, 0u, (code << 24) | (blockIdx.x & 0xffffffu));
+  atomicExch(&st->abort_epoch, tag.epoch);
+  __threadfence_system();
+  if (tag.host_flag != nullptr) *tag.host_flag = 1u;
+}
+__device__ __forceinline__ bool launch_aborted(WaitStatus *st, const LaunchTag &tag) {
+  return *reinterpret_cast<volatile unsigned int *>(&st->abort_epoch) == tag.epoch;
+}
 // Spins on `try_once()` until it succeeds, the launch has been marked as failed, or `limit_ns` have passed.
 template <typename TryFn>
-__device__ __forceinline__ void bounded_spin(TryFn try_once, uint32_t code, WaitStatus *st, uint32_t epoch,
+__device__ __forceinline__ void bounded_spin(TryFn try_once, uint32_t code, WaitStatus *st, LaunchTag epoch,
                                              unsigned long long limit_ns) {
   for (int i = 0; i < 4096; ++i)
     if (try_once()) return;
   unsigned long long t0, t1;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
   for (;;) {
-    if (*reinterpret_cast<volatile unsigned int *>(&st->abort_epoch) == epoch) return;
+    if (launch_aborted(st, epoch)) return;
     for (int i = 0; i < 1024; ++i)
       if (try_once()) return;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
     if (t1 - t0 > limit_ns) {
-      atomicCAS(&st->first_error, 0u, (code << 24) | (blockIdx.x & 0xffffffu));
-      atomicExch(&st->abort_epoch, epoch);
+      record_expiry(st, code, epoch);
       return;
     }
   }

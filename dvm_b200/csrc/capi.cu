@@ -14,7 +14,9 @@
 #include "../../include/dvm_c.h"
 #include "comm.h"
 #include "graph.h"
+#include "bounded_wait.cuh"
 #include "runtime.h"
+#include "staging.h"
 #include "vm_launch.h"
 #include "vm_row.h"
 #include "mm_launch.h"
@@ -463,10 +465,10 @@ void *dvm_rt_malloc(size_t bytes) {
 }
 int dvm_rt_free(void *p) { return CudaCheck(cudaFree(p), "cudaFree"); }
 int dvm_rt_memcpy_h2d(void *dst, const void *src, size_t bytes, void *stream) {
-  return CudaCheck(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, static_cast<cudaStream_t>(stream)), "H2D copy");
+  return CudaCheck(dvmb::CopyToDevice(dst, src, bytes, static_cast<cudaStream_t>(stream)), "H2D copy");
 }
 int dvm_rt_memcpy_d2h(void *dst, const void *src, size_t bytes, void *stream) {
-  return CudaCheck(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)), "D2H copy");
+  return CudaCheck(dvmb::CopyToHost(dst, src, bytes, static_cast<cudaStream_t>(stream)), "D2H copy");
 }
 int dvm_rt_memset(void *dst, int value, size_t bytes, void *stream) {
   return CudaCheck(cudaMemsetAsync(dst, value, bytes, static_cast<cudaStream_t>(stream)), "memset");
@@ -474,6 +476,8 @@ int dvm_rt_memset(void *dst, int value, size_t bytes, void *stream) {
 // Reads (and clears) the status records of the device interpreters: a bounded device wait that expired (the kernel
 // then ran to its end with wrong results) is reported here as an error.  Does not wait for anything.
 int dvm_rt_check_status(void) {
+  if (!dvmb::ExpiryFlagRaised()) return 0;
+  dvmb::LowerExpiryFlag();   // (before the records are read: an expiry from here on raises it again)
   const unsigned int rs = dvmb::ReadRowStatus(), vs = dvmb::ReadVectorStatus(), sv = vs != 0 ? vs : rs, sm = dvmb::ReadMatMulStatus(), sa = dvmb::ReadAttentionStatus();
   if ((sv | sm | sa) != 0) {
     char buf[160];
@@ -481,6 +485,7 @@ int dvm_rt_check_status(void) {
     g_error = buf;
     return -1;
   }
+  dvmb::RaiseExpiryFlag();   // the record is another device's
   return 0;
 }
 // Waits for the stream, then reports like dvm_rt_check_status().

@@ -92,7 +92,7 @@ __device__ __forceinline__ void copy_out(const MmParam &P, uint32_t slot, uint32
     }
 }
 
-__device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, const uint32_t epoch) {
+__device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, const LaunchTag epoch) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // 1024-byte alignment of the stage area (required by the 128-byte swizzle pattern)
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -297,7 +297,7 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
 }  // namespace
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-  dvm_b200_mm_tcgen05_pair(const __grid_constant__ MmParam P, const __grid_constant__ MmMaps maps, const uint32_t epoch) {
+  dvm_b200_mm_tcgen05_pair(const __grid_constant__ MmParam P, const __grid_constant__ MmMaps maps, const LaunchTag epoch) {
   pair_body(P, maps, epoch);
 }
 

@@ -129,7 +129,7 @@ __device__ __forceinline__ uint32_t cluster_nctarank() {
 }
 
 template <uint32_t BN>
-__device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps, const TileArgs &A, const uint32_t epoch) {
+__device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps, const TileArgs &A, const LaunchTag epoch) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
@@ -398,11 +398,11 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
 
 // (two CTAs per SM: one's loads and MMAs run beside the other's epilogue)
 __global__ void __launch_bounds__(kThreads, 2) dvm_b200_mm_tile_n64(const __grid_constant__ MmParam P, const __grid_constant__ TileMaps maps,
-                                                                    const __grid_constant__ TileArgs A, const uint32_t epoch) {
+                                                                    const __grid_constant__ TileArgs A, const LaunchTag epoch) {
   tile_body<64>(P, maps, A, epoch);
 }
 __global__ void __launch_bounds__(kThreads, 2) dvm_b200_mm_tile_n128(const __grid_constant__ MmParam P, const __grid_constant__ TileMaps maps,
-                                                                     const __grid_constant__ TileArgs A, const uint32_t epoch) {
+                                                                     const __grid_constant__ TileArgs A, const LaunchTag epoch) {
   tile_body<128>(P, maps, A, epoch);
 }
 

@@ -10,11 +10,36 @@
 
 namespace dvmb {
 
-uint32_t NextLaunchEpoch() {
+// One word for the whole process, mapped into every device's address space; null when it could not be had.
+static volatile uint32_t *ExpiryFlag() {
+  static volatile uint32_t *const flag = []() -> volatile uint32_t * {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // (the first launch may happen inside somebody's capture)
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    } else {
+      *static_cast<volatile uint32_t *>(p) = 0;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return static_cast<volatile uint32_t *>(p);
+  }();
+  return flag;
+}
+
+LaunchTag NextLaunchEpoch() {
   static std::atomic<uint32_t> counter{0};
   uint32_t e = counter.fetch_add(1, std::memory_order_relaxed) + 1;
   if (e == 0) e = counter.fetch_add(1, std::memory_order_relaxed) + 1;   // 0 means "no launch has failed yet"
-  return e;
+  return {e, 0u, ExpiryFlag()};
+}
+bool ExpiryFlagRaised() { return ExpiryFlag() == nullptr || *ExpiryFlag() != 0; }
+void LowerExpiryFlag() {
+  if (ExpiryFlag() != nullptr) *ExpiryFlag() = 0;
+}
+void RaiseExpiryFlag() {
+  if (ExpiryFlag() != nullptr) *ExpiryFlag() = 1;
 }
 
 Runtime &Runtime::Get() {

@@ -39,10 +39,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t addr, uint32_t parity) {
 // Bounded wait (bounded_wait.cuh, about two seconds).  On expiry the status record receives (code << 24 | block
 // index) and the launch's epoch; the other waits of the same launch then return from their slow path at once, so the
 // kernel always runs to its end and the host reports the failure instead of the GPU hanging.
-__device__ __noinline__ void mbar_wait_slow(uint32_t addr, uint32_t parity, uint32_t code, WaitStatus *status, uint32_t epoch) {
+__device__ __noinline__ void mbar_wait_slow(uint32_t addr, uint32_t parity, uint32_t code, WaitStatus *status, LaunchTag epoch) {
   bounded_spin([&]() { return mbar_try_wait(addr, parity); }, code, status, epoch, kWaitLimitNs);
 }
-__device__ __forceinline__ void mbar_wait(uint32_t addr, uint32_t parity, uint32_t code, WaitStatus *status, uint32_t epoch) {
+__device__ __forceinline__ void mbar_wait(uint32_t addr, uint32_t parity, uint32_t code, WaitStatus *status, LaunchTag epoch) {
   if (mbar_try_wait(addr, parity)) return;
   mbar_wait_slow(addr, parity, code, status, epoch);
 }

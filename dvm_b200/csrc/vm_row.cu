@@ -264,10 +264,10 @@ __device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
     : "memory");
   return ok != 0;
 }
-__device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, uint32_t code, uint32_t epoch) {
+__device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, uint32_t code, LaunchTag epoch) {
   bounded_spin([&]() { return try_wait(bar, parity); }, code, &g_row_status, epoch, kWaitLimitNs);
 }
-__device__ __forceinline__ void wait_for(uint32_t bar, uint32_t parity, uint32_t code, uint32_t epoch) {
+__device__ __forceinline__ void wait_for(uint32_t bar, uint32_t parity, uint32_t code, LaunchTag epoch) {
   if (!try_wait(bar, parity)) wait_slow(bar, parity, code, epoch);
 }
 __device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes) {
@@ -280,7 +280,7 @@ __device__ __forceinline__ void work_sync() { asm volatile("bar.sync 1, %0;" ::"
 
 // kWhole: every run starts and ends on 16 bytes, so that every unit belongs to its run with all lanes.
 template <uint32_t DT, bool kWhole>
-__device__ __forceinline__ void stats_affine_body(const RowParam &P, const uint32_t epoch) {
+__device__ __forceinline__ void stats_affine_body(const RowParam &P, const LaunchTag epoch) {
   constexpr uint32_t E = kE<DT>, SH = kShift<DT>;
   extern __shared__ __align__(128) uint8_t smem[];
   StatsShared &sm = *reinterpret_cast<StatsShared *>(smem);
@@ -696,7 +696,7 @@ __device__ __forceinline__ void rms_gate_body(const RowParam &P) {
 }  // namespace
 
 #define DVMB_ROW_STATS(NAME, DT, WHOLE)                                                                             \
-  __global__ void __launch_bounds__(kStatsThreads, 2) NAME(const __grid_constant__ RowParam P, const uint32_t epoch) { \
+  __global__ void __launch_bounds__(kStatsThreads, 2) NAME(const __grid_constant__ RowParam P, const LaunchTag epoch) { \
     stats_affine_body<DT, WHOLE>(P, epoch);                                                                           \
   }
 DVMB_ROW_STATS(dvm_b200_row_stats_affine_f16, T_F16, false)
@@ -850,7 +850,7 @@ int LaunchRow(const RowParam &p_in, void *stream) {
   uint32_t smem = 0;
   if (!StatsPlan(p.runs * units, p.groups, sms, &p, &smem)) return -7;
   const bool whole = RunsAligned(p) && ((p.run_len << ElemShift(p)) & 15u) == 0;
-  using Fn = void (*)(const RowParam, const uint32_t);
+  using Fn = void (*)(const RowParam, const LaunchTag);
   static const Fn table[2][3] = {
     {dvm_b200_row_stats_affine_f16, dvm_b200_row_stats_affine_bf16, dvm_b200_row_stats_affine_f32},
     {dvm_b200_row_stats_affine_f16_whole, dvm_b200_row_stats_affine_bf16_whole, dvm_b200_row_stats_affine_f32_whole}};

@@ -61,7 +61,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t addr, uint32_t parity) {
 // (A warp that has to wait sleeps between its polls: polled back to back, the producer warps' waits alone were a fifth of
 // the instructions an issue-bound kernel executed.)
 constexpr uint32_t kPollSleepNs = 200;
-__device__ __noinline__ void mbar_wait_slow(uint32_t addr, uint32_t parity, uint32_t code, uint32_t epoch) {
+__device__ __noinline__ void mbar_wait_slow(uint32_t addr, uint32_t parity, uint32_t code, LaunchTag epoch) {
   bounded_spin(
     [&]() {
       if (mbar_try_wait(addr, parity)) return true;
@@ -70,7 +70,7 @@ __device__ __noinline__ void mbar_wait_slow(uint32_t addr, uint32_t parity, uint
     },
     code, &g_vm_status, epoch, kWaitLimitNs);
 }
-__device__ __forceinline__ void mbar_wait(uint32_t addr, uint32_t parity, uint32_t code, uint32_t epoch) {
+__device__ __forceinline__ void mbar_wait(uint32_t addr, uint32_t parity, uint32_t code, LaunchTag epoch) {
   if (mbar_try_wait(addr, parity)) return;
   mbar_wait_slow(addr, parity, code, epoch);
 }
@@ -99,7 +99,7 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t addr, uint32_t pa
   return ok != 0;
 }
 // Bounded like every other wait of the kernel (status code 3).
-__device__ __noinline__ void mbar_wait_cluster(uint32_t addr, uint32_t parity, uint32_t epoch) {
+__device__ __noinline__ void mbar_wait_cluster(uint32_t addr, uint32_t parity, LaunchTag epoch) {
   bounded_spin([&]() { return mbar_try_wait_cluster(addr, parity); }, 3u, &g_vm_status, epoch, kWaitLimitNs);
 }
 __device__ __forceinline__ float ld_shared_cluster_f32(uint32_t cluster_addr) {
@@ -264,7 +264,7 @@ namespace {
 // kRounds: chunks may hold several rounds (VmParam::rounds > 1).  Only the instantiations with the larger register budget
 // carry the round bookkeeping; the others run one round per chunk and the compiler folds the round loop away.
 template <bool kResident, bool kCoords, bool kRounds, int kModeOnly = 0>
-__device__ __forceinline__ void vm_vector_body(const VmParam &P, const uint32_t epoch) {
+__device__ __forceinline__ void vm_vector_body(const VmParam &P, const LaunchTag epoch) {
   asm volatile(DV_DECLARE);
   asm volatile(DV_LN(DV_SPLATLANE, "va") DV_LN(DV_SPLATLANE, "vb")
                "mov.b32 vp0, %0;\n\tmov.b32 vp1, %0;\n\tmov.b32 vp2, %0;\n\tmov.b32 vp3, %0;" ::"r"(0u));
@@ -1344,7 +1344,7 @@ __device__ __forceinline__ void vm_vector_body(const VmParam &P, const uint32_t 
 // A third budget of 72 registers (five 128-thread CTAs per SM) was measured 50 % slower: its spills sit in the loop.
 #define DVMB_VM_KERNEL(NAME, THREADS, BLOCKS, ...)                                                              \
   __global__ void __launch_bounds__(THREADS, BLOCKS) NAME(const __grid_constant__ VmParam P,                      \
-                                                          const uint32_t epoch) {                                 \
+                                                          const LaunchTag epoch) {                                 \
     vm_vector_body<__VA_ARGS__>(P, epoch);                                                                        \
   }
 // dense layouts (every chunk starts at group offset + element index)
@@ -1454,7 +1454,7 @@ int LaunchVector(const VmParam &param, uint32_t grid, uint32_t threads, uint32_t
 // A launch whose only wait can never succeed: one thread spins on an mbarrier that nothing arrives at, through the same
 // bounded wait as the interpreter, with a caller-chosen limit.  It exists so that a test can watch the expiry path end
 // to end (status recorded, reported by the host, cleared, later launches unaffected) without hanging or faulting the GPU.
-__global__ void dvm_b200_wait_selftest(const uint32_t epoch, const unsigned long long limit_ns) {
+__global__ void dvm_b200_wait_selftest(const LaunchTag epoch, const unsigned long long limit_ns) {
   __shared__ __align__(8) uint64_t bar;
   const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(&bar));
   mbar_init(addr, 1);

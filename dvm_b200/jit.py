@@ -91,8 +91,12 @@ class JitKernel:
                 self._runner.input(slot.target, value)
         if self.dynamic:
             self._runner.codegen(None)
-        self._runner.run()
-        if isinstance(self._results, (list, tuple)):
+        several = isinstance(self._results, (list, tuple))
+        if several and not self._results:
+            self._runner.run()
+        else:
+            self._runner.launch()   # (a result's download waits for it)
+        if several:
             return [self._runner.output(s) for s in self._results]
         return self._runner.output(self._results)
 
