@@ -82,7 +82,7 @@ struct AttnParam {
   uint32_t dtype;           // T_F16 or T_BF16
   uint32_t scale_bits;      // scale in the operand type's register form (fp32 bits)
   uint32_t scale_first;     // 1: the score is rounded to the operand type, scaled, rounded again (the graph's order)
-  uint32_t pad0;
+  uint32_t q_tiles, units;  // set by the launcher: tiles of 128 query rows per unit (1 or 2), units of work
   uint64_t q_ptr, k_ptr, v_ptr, o_ptr;
 };
 int LaunchAttention(const AttnParam &p, void *stream);
