@@ -392,14 +392,14 @@ int dvm_launch_static_scratch(dvm_kernel *k, const dvm_reloc *relocs, size_t rel
     [&]() {
       // the workspace the program compiled for the CURRENT shapes needs (any call that compiles - code generation, a
       // listing, an inspection after a shape update - may have changed it, so it is read here and never cached)
-      const dvm::VKernel *vk = k->kernel.GetImpl();
+      dvm::VKernel *vk = k->kernel.GetImpl();
       if (vk == nullptr || !vk->compiled_) {
         g_error = "dvm_launch_static_scratch needs dvm_pre_codegen() or dvm_codegen() for the current shapes first";
         return -5;
       }
-      if (vk->ws_bytes_ > kStaticScratchBytes) {
+      if (vk->ws_needed_ > kStaticScratchBytes) {
         char buf[160];
-        snprintf(buf, sizeof(buf), "this kernel needs %zu bytes of workspace; the static scratch holds %zu", vk->ws_bytes_,
+        snprintf(buf, sizeof(buf), "this kernel needs %zu bytes of workspace; the static scratch holds %zu", vk->ws_needed_,
                  kStaticScratchBytes);
         g_error = buf;
         return -2;
@@ -416,7 +416,9 @@ int dvm_launch_static_scratch(dvm_kernel *k, const dvm_reloc *relocs, size_t rel
         if (CudaCheck(cudaGetSymbolAddress(&p, g_static_scratch), "cudaGetSymbolAddress(static scratch)") != 0) return -4;
         g_static_scratch_addr[dev] = p;
       }
-      return k->kernel.Launch(reinterpret_cast<const dvm::RelocEntry *>(relocs), reloc_size, g_static_scratch_addr[dev], stream);
+      // (what a plan can do without stays unused: launches that need no workspace do not share this one)
+      vk->Bind(reinterpret_cast<const dvm::RelocEntry *>(relocs), reloc_size, g_static_scratch_addr[dev], vk->ws_needed_);
+      return vk->Launch(stream);
     },
     -1);
 }

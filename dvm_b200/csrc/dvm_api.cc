@@ -773,8 +773,11 @@ void Kernel::CodeGen(const RelocEntry *relocs, size_t reloc_size, WsAllocator *w
   size_t ws = vk->Compile();
   void *workspace = nullptr;
   if (ws > 0) {
-    if (ws_alloc == nullptr) DvmException("this kernel needs a workspace but no WsAllocator was given");
-    workspace = ws_alloc->Alloc(ws);
+    if (ws_alloc != nullptr) {
+      workspace = ws_alloc->Alloc(ws);
+    } else if (vk->ws_needed_ > 0) {
+      DvmException("this kernel needs a workspace but no WsAllocator was given");
+    }
   }
   vk->Bind(relocs, reloc_size, workspace);
 }

@@ -158,6 +158,7 @@ struct MatMulStage {
   std::vector<uint64_t> bytecode;       // the post-fusion program (what Das() prints)
   bool idle = false;
   uint64_t algo_bytes = 0, flops = 0;
+  int64_t a_pack_off = -1, b_pack_off = -1;   // >= 0: workspace for a repacked operand (used when there is a workspace)
 };
 
 // One launch of the fused attention kernel.
@@ -212,7 +213,7 @@ class VKernel {
   void Normalize();
   size_t Compile();   // stages for the current shapes, built or taken from plans_; returns workspace bytes
   void CompileFresh();
-  void Bind(const RelocEntry *relocs, size_t n, void *workspace);
+  void Bind(const RelocEntry *relocs, size_t n, void *workspace, size_t workspace_bytes = ~static_cast<size_t>(0));
   int Launch(void *stream);
   int LaunchStage(size_t index, void *stream);   // one launch (or collective) of the plan, for per-stage timing
   int LaunchPipelined(void *stream);             // a plan with two lanes (see Stage::lane)
@@ -231,15 +232,16 @@ class VKernel {
   std::vector<std::unique_ptr<Stage>> stages_;
   std::vector<NDObject *> synth_;          // planner-made nodes (clones, workspace temporaries), owned
   std::vector<std::vector<NDObject *>> split_outs_;   // arrays handed out by Kernel::Split (valid for the kernel's life)
-  size_t ws_bytes_ = 0;
+  size_t ws_bytes_ = 0;                    // workspace the plan makes use of; without the last part the MatMuls of
+  size_t ws_needed_ = 0;                   // unaligned operands are slower (MmPackBytes), without the first nothing runs
   // Plans of the shapes seen last, so that a loop that comes back to a shape (decode steps, the last batch of an epoch)
   // does not plan it again: at most kMaxPlans of about 10 KB each, the least recently used one goes.  The plan in use is
-  // stages_ / synth_ / ws_bytes_ with signature plan_sig_ (when has_plan_).
+  // stages_ / synth_ / ws_bytes_ / ws_needed_ with signature plan_sig_ (when has_plan_).
   struct Plan {
     std::vector<int64_t> sig;
     std::vector<std::unique_ptr<Stage>> stages;
     std::vector<NDObject *> synth;
-    size_t ws_bytes = 0;
+    size_t ws_bytes = 0, ws_needed = 0;
     uint64_t used = 0;
   };
   static constexpr size_t kMaxPlans = 16;

@@ -260,6 +260,40 @@ __device__ __forceinline__ void pack_strip(uint32_t dtype, const uint32_t (&v)[1
   }
 }
 
+// Eight consecutive 16-bit elements that start `off` elements into the 32 bytes {lo, hi}.
+__device__ __forceinline__ uint4 shift_in(const uint4 &lo, const uint4 &hi, uint32_t off) {
+  const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+  uint32_t a[6], b[5];
+  const bool two = (off & 4u) != 0, one = (off & 2u) != 0;
+  const uint32_t bits = (off & 1u) * 16u;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) a[i] = two ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) b[i] = one ? a[i + 1] : a[i];
+  return make_uint4(__funnelshift_r(b[0], b[1], bits), __funnelshift_r(b[1], b[2], bits), __funnelshift_r(b[2], b[3], bits),
+                    __funnelshift_r(b[3], b[4], bits));
+}
+
+// Rows of 16-bit results at any even address leave as one 16-byte store per aligned unit that lies inside the row and eight
+// single elements: `run` elements (a multiple of 8) whose first lies `ahead` (1 to 8) elements before such a unit hold
+// run / 8 - 1 whole units from element `ahead` on.  (One element per lane took 12 us of the 34 us of a [1024, 5003] result.)
+__device__ __forceinline__ uint32_t elements_ahead(const unsigned short *row) {
+  return 8u - ((uint32_t)(reinterpret_cast<uint64_t>(row) >> 1) & 7u);
+}
+// column of single element i (0 to 7)
+__device__ __forceinline__ uint32_t single_at(uint32_t i, uint32_t ahead, uint32_t run) { return i < ahead ? i : run - 8u + i; }
+// stores a whole unit; `left`: columns of the matrix from its first element on
+__device__ __forceinline__ void store_unit(unsigned short *dst, const uint4 &v, uint32_t left) {
+  if (left >= 8u) {
+    *reinterpret_cast<uint4 *>(dst) = v;
+    return;
+  }
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (uint32_t i = 0; i < 7; ++i)
+    if (i < left) dst[i] = (unsigned short)(w[i >> 1] >> (16u * (i & 1u)));
+}
+
 // Rounding to the operand type and the post-fusion program for one 16-column strip of one row (bias already added).
 // When the whole program is a store in the operand type (plain or gated), the sixteen 16-bit results come back in `pk` and
 // the slot of their tensor is returned: the caller stores them through shared memory, so that rows of any alignment leave

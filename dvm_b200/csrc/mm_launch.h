@@ -36,6 +36,10 @@ struct MmParam {
   uint32_t a_mul0, a_mul1, a_batches;   // batch-slice multipliers and slice count of A
   uint32_t b_mul0, b_mul1, b_batches;
   uint64_t a_ptr, b_ptr, bias_ptr;
+  // Optional: memory of MmPackBytes() bytes each, for a copy of an operand in rows of whole 16-byte units; and the pitch of
+  // such rows in elements, set by the launcher (0: the rows are as long as their contents)
+  uint64_t a_pack, b_pack;
+  uint32_t a_pitch, b_pitch;
   // post-fusion program: instruction words (isa.h Insn) over 16 consecutive columns of one row, ending with
   // OP_END; operand kind K_TENSOR with index `mma_slot` names the rounded product itself
   uint32_t n_tensors;
@@ -59,19 +63,29 @@ struct MmParam {
 int LaunchMatMul(const MmParam &p, void *stream);
 // True when the copy engine cannot address an operand (rows of `inner` 16-bit elements, batch slices of `slice`): base, row
 // pitch or slice not a multiple of 16 bytes.  Its tiles are then loaded by the tile kernel's work warps.
-bool MmOperandNeedsGather(uint64_t ptr, uint64_t inner, uint64_t slice, uint32_t batches);
+bool MmOperandNeedsGather(uint64_t ptr, uint64_t pitch, uint64_t slice, uint32_t batches);
+inline uint32_t MmInnerA(const MmParam &p) { return p.a_mmajor ? p.M : p.K; }
+inline uint32_t MmInnerB(const MmParam &p) { return p.b_kmajor ? p.K : p.N; }
+inline uint32_t MmRowsA(const MmParam &p) { return p.a_mmajor ? p.K : p.M; }
+inline uint32_t MmRowsB(const MmParam &p) { return p.b_kmajor ? p.N : p.K; }
+inline uint32_t MmPitchA(const MmParam &p) { return p.a_pitch != 0 ? p.a_pitch : MmInnerA(p); }
+inline uint32_t MmPitchB(const MmParam &p) { return p.b_pitch != 0 ? p.b_pitch : MmInnerB(p); }
 inline bool MmGatherA(const MmParam &p) {
-  return MmOperandNeedsGather(p.a_ptr, p.a_mmajor ? p.M : p.K, static_cast<uint64_t>(p.M) * p.K, p.a_batches);
+  return MmOperandNeedsGather(p.a_ptr, MmPitchA(p), static_cast<uint64_t>(MmPitchA(p)) * MmRowsA(p), p.a_batches);
 }
 inline bool MmGatherB(const MmParam &p) {
-  return MmOperandNeedsGather(p.b_ptr, p.b_kmajor ? p.K : p.N, static_cast<uint64_t>(p.N) * p.K, p.b_batches);
+  return MmOperandNeedsGather(p.b_ptr, MmPitchB(p), static_cast<uint64_t>(MmPitchB(p)) * MmRowsB(p), p.b_batches);
 }
 inline bool MmNeedsGather(const MmParam &p) { return MmGatherA(p) || MmGatherB(p); }
+// Bytes of memory for repacked operands that make this product faster (0: none; see the rule there).
+void MmPackBytes(const MmParam &p, uint64_t *a_bytes, uint64_t *b_bytes);
+// Copies the operands that the copy engine cannot address into a_pack / b_pack, and makes `p` read them there.
+int LaunchMmPack(MmParam *p, void *stream);
 // The tile kernel (mm_tile.cu): 128 x bn tiles (bn 64 or 128), K cut into `split` (1, 2, 4, 8) parts.
 int LaunchMmTile(const MmParam &p, uint32_t bn, uint32_t split, void *stream);
 unsigned int ReadMmTileStatus();
-// 3-d tensor map over a [batches, rows, inner] 16-bit operand: boxes of box_rows rows of 64 elements, 128-byte swizzle.
-int EncodeMmOperand(CUtensorMap *map, uint64_t ptr, uint64_t inner, uint64_t rows, uint64_t batches, uint32_t box_rows);
+// 3-d tensor map over a [batches, rows, inner] 16-bit operand (`pitch` elements from row to row): boxes of box_rows rows of 64 elements, 128-byte swizzle.
+int EncodeMmOperand(CUtensorMap *map, uint64_t ptr, uint64_t inner, uint64_t pitch, uint64_t rows, uint64_t batches, uint32_t box_rows);
 unsigned int ReadMatMulStatus();
 
 // Fused attention  O[b,h] = softmax(scale * Q[b,h] K[b,h]^T) V[b,h]  (non-causal), bf16 or fp16 operands,

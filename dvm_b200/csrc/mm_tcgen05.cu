@@ -31,6 +31,7 @@
 #include "chain.cuh"
 #include "mm_epilogue.cuh"
 #include "mm_launch.h"
+#include "runtime.h"
 #include "sm100_sync.cuh"
 
 namespace dvmb {
@@ -80,16 +81,29 @@ __device__ __forceinline__ void copy_out(const MmParam &P, uint32_t slot, uint32
     }
     return;
   }
-  // a ragged edge, or rows at any even address: one element per lane
+  // a ragged edge, or rows at any even address
 #pragma unroll 1
-  for (uint32_t row = 0; row < 32 && row0 + row < P.M; ++row)
-#pragma unroll
-    for (uint32_t h = 0; h < 2; ++h) {
-      const uint32_t col = h * 32u + lane;
-      unsigned short v;
-      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(saddr + row * 128u + (((col >> 3) ^ (row & 7u)) << 4) + (col & 7u) * 2u));
-      if (col0 + col < P.N) out[(int64_t)row * t.sm + col] = v;
-    }
+  for (uint32_t j = lane; j < 32u * 7u; j += 32u) {
+    const uint32_t row = j / 7u, u = j - 7u * row;
+    unsigned short *const dst = out + (int64_t)row * t.sm;
+    const uint32_t ahead = elements_ahead(dst), at = ahead + 8u * u, piece = at >> 3;   // (at + 8 <= 64)
+    if (row0 + row >= P.M || col0 + at >= P.N) continue;
+    uint4 lo, hi;
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w) : "r"(saddr + row * 128u + ((piece ^ (row & 7u)) << 4)));
+    hi = lo;
+    if ((ahead & 7u) != 0)
+      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w) : "r"(saddr + row * 128u + (((piece + 1u) ^ (row & 7u)) << 4)));
+    store_unit(dst + at, shift_in(lo, hi, ahead & 7u), P.N - (col0 + at));
+  }
+#pragma unroll 1
+  for (uint32_t j = lane; j < 256u; j += 32u) {
+    const uint32_t row = j >> 3;
+    unsigned short *const dst = out + (int64_t)row * t.sm;
+    const uint32_t col = single_at(j & 7u, elements_ahead(dst), 64u);
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(saddr + row * 128u + (((col >> 3) ^ (row & 7u)) << 4) + (col & 7u) * 2u));
+    if (row0 + row < P.M && col0 + col < P.N) dst[col] = v;
+  }
 }
 
 __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, const LaunchTag epoch) {
@@ -318,11 +332,11 @@ PFN_cuTensorMapEncodeTiled GetEncode() {
 }  // namespace
 
 // 3-d map over a [batches, rows, inner] row-major operand: box = [1, box_rows, 64 elements], 128-byte swizzle
-int EncodeMmOperand(CUtensorMap *map, uint64_t ptr, uint64_t inner, uint64_t rows, uint64_t batches, uint32_t box_rows) {
+int EncodeMmOperand(CUtensorMap *map, uint64_t ptr, uint64_t inner, uint64_t pitch, uint64_t rows, uint64_t batches, uint32_t box_rows) {
   auto encode = GetEncode();
   if (encode == nullptr) return -10;
   cuuint64_t dims[3] = {inner, rows, batches ? batches : 1};
-  cuuint64_t strides[2] = {inner * 2, inner * rows * 2};
+  cuuint64_t strides[2] = {pitch * 2, pitch * rows * 2};
   cuuint32_t box[3] = {64, box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, reinterpret_cast<void *>(ptr), dims, strides, box, estr,
@@ -331,9 +345,9 @@ int EncodeMmOperand(CUtensorMap *map, uint64_t ptr, uint64_t inner, uint64_t row
   return r == CUDA_SUCCESS ? 0 : -100 - static_cast<int>(r);
 }
 
-bool MmOperandNeedsGather(uint64_t ptr, uint64_t inner, uint64_t slice, uint32_t batches) {
+bool MmOperandNeedsGather(uint64_t ptr, uint64_t pitch, uint64_t slice, uint32_t batches) {
   // the copy engine needs 16-byte aligned bases and row pitches (and slices, for batched operands)
-  return (ptr & 15u) != 0 || (inner & 7u) != 0 || (batches > 1 && (slice & 7u) != 0);
+  return (ptr & 15u) != 0 || (pitch & 7u) != 0 || (batches > 1 && (slice & 7u) != 0);
 }
 
 namespace {
@@ -374,15 +388,17 @@ double TileCost(const MmParam &p, uint32_t bn, uint32_t split, int sms, bool gat
   return t;
 }
 
-MmPlan ChoosePlan(const MmParam &p, int sms, bool gather) {
+MmPlan ChoosePlan(const MmParam &p, int sms, bool gather, double *cost = nullptr) {
   const uint32_t kb = (p.K + BK - 1) / BK;
   MmPlan best{64, 1};
   double best_t = TileCost(p, 64, 1, sms, gather);
+  if (cost != nullptr) *cost = best_t;
   auto consider = [&](uint32_t bn, uint32_t split) {
     const double t = TileCost(p, bn, split, sms, gather);
     if (t < best_t) {
       best_t = t;
       best = {bn, split};
+      if (cost != nullptr) *cost = t;
     }
   };
   for (uint32_t split = 2; split <= 8 && split <= kb; split *= 2) consider(64, split);
@@ -393,6 +409,30 @@ MmPlan ChoosePlan(const MmParam &p, int sms, bool gather) {
 }
 
 }  // namespace
+
+// A copy of an operand in rows of whole 16-byte units pays where the tiles read it often: it costs a launch (of which about
+// 700 cycles show beside the product) and a cycle for 2700 bytes read or written; the estimates above say what it saves.
+void MmPackBytes(const MmParam &p, uint64_t *a_bytes, uint64_t *b_bytes) {
+  *a_bytes = *b_bytes = 0;
+  if (p.M == 0 || p.N == 0 || p.K == 0 || p.batch0 * p.batch1 == 0) return;
+  MmParam q = p;   // (addresses are not known yet: what the shapes alone make unaligned)
+  q.a_ptr = q.b_ptr = 0;
+  auto bytes = [](uint64_t inner, uint64_t rows, uint64_t batches) {
+    const uint64_t pieces = (inner + 7) / 8 * rows * batches;
+    return pieces < (1ull << 31) ? pieces * 16 : ~0ull;
+  };
+  const uint64_t a = MmGatherA(q) ? bytes(MmInnerA(p), MmRowsA(p), p.a_batches) : 0;
+  const uint64_t b = MmGatherB(q) ? bytes(MmInnerB(p), MmRowsB(p), p.b_batches) : 0;
+  if ((a | b) == 0 || a == ~0ull || b == ~0ull) return;
+  int sms = Runtime::Get().sm_count_or_default();
+  if (p.leave_sms != 0 && static_cast<int>(p.leave_sms) + 32 <= sms) sms -= static_cast<int>(p.leave_sms);
+  double gathered = 0.0, packed = 0.0;
+  ChoosePlan(p, sms, true, &gathered);
+  ChoosePlan(p, sms, false, &packed);
+  if (packed + 700.0 + 2.0 * static_cast<double>(a + b) / 2700.0 >= gathered) return;
+  *a_bytes = a;
+  *b_bytes = b;
+}
 
 int LaunchMatMul(const MmParam &p_in, void *stream) {
   MmParam p = p_in;
@@ -439,6 +479,10 @@ int LaunchMatMul(const MmParam &p_in, void *stream) {
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (p.leave_sms != 0 && static_cast<int>(p.leave_sms) + 32 <= sms) sms -= static_cast<int>(p.leave_sms);
+  if (MmNeedsGather(p) && (p.a_pack | p.b_pack) != 0) {
+    const int rc = LaunchMmPack(&p, stream);
+    if (rc != 0) return rc;
+  }
   const bool gather = MmNeedsGather(p);
   MmPlan plan = ChoosePlan(p, sms, gather);
   static const char *const force = getenv("DVM_B200_MM_PLAN");   // "columns,split" (columns 0: CTA pairs)
@@ -456,11 +500,9 @@ int LaunchMatMul(const MmParam &p_in, void *stream) {
   }
   MmMaps maps;
   // fp16 and bf16 are both 2-byte types for the copy engine; the MMA descriptor carries the real format
-  int rc = p.a_mmajor ? EncodeMmOperand(&maps.a, p.a_ptr, p.M, p.K, p.a_batches, 64)
-                      : EncodeMmOperand(&maps.a, p.a_ptr, p.K, p.M, p.a_batches, BM);
+  int rc = EncodeMmOperand(&maps.a, p.a_ptr, MmInnerA(p), MmPitchA(p), MmRowsA(p), p.a_batches, p.a_mmajor ? 64 : BM);
   if (rc != 0) return rc;
-  rc = p.b_kmajor ? EncodeMmOperand(&maps.b, p.b_ptr, p.K, p.N, p.b_batches, BN / 2)
-                  : EncodeMmOperand(&maps.b, p.b_ptr, p.N, p.K, p.b_batches, 64);
+  rc = EncodeMmOperand(&maps.b, p.b_ptr, MmInnerB(p), MmPitchB(p), MmRowsB(p), p.b_batches, p.b_kmajor ? BN / 2 : 64);
   if (rc != 0) return rc;
   const uint32_t tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.batch0 * p.batch1;
   const uint32_t units = tiles < static_cast<uint32_t>(sms / 2) ? tiles : static_cast<uint32_t>(sms / 2);

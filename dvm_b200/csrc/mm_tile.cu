@@ -13,7 +13,8 @@
 // What bounds it: a [16, 8192] x [8192, 8192] product is the read of the weight (134 MB, 21 us at the measured copy
 // bandwidth).  In 128 x 256 tiles that was 32 CTAs on 148 SMs; in tiles of 64 columns with K cut in two it is 256 CTAs
 // with 2 x 80 KB of weight in flight per SM.  A product of [1024, 1001] and [1001, 5003] (rows of the second at any even
-// address) took 6.4 ms on CUDA cores, element by element.
+// address) took 6.4 ms on CUDA cores, element by element, 56 us with the work warps as loaders and 26 us with the operand
+// repacked first (dvm_b200_mm_pack below); the loaders remain for what is not worth a copy and for launches without a workspace.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -53,20 +54,6 @@ struct TileArgs {
 };
 
 // ---- operands at any even address ------------------------------------------------------------------------
-// Eight consecutive 16-bit elements that start `off` elements into the 32 bytes {lo, hi}.
-__device__ __forceinline__ uint4 shift_in(const uint4 &lo, const uint4 &hi, uint32_t off) {
-  const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-  uint32_t a[6], b[5];
-  const bool two = (off & 4u) != 0, one = (off & 2u) != 0;
-  const uint32_t bits = (off & 1u) * 16u;
-#pragma unroll
-  for (int i = 0; i < 6; ++i) a[i] = two ? w[i + 2] : w[i];
-#pragma unroll
-  for (int i = 0; i < 5; ++i) b[i] = one ? a[i + 1] : a[i];
-  return make_uint4(__funnelshift_r(b[0], b[1], bits), __funnelshift_r(b[1], b[2], bits), __funnelshift_r(b[2], b[3], bits),
-                    __funnelshift_r(b[3], b[4], bits));
-}
-
 struct Gather {
   const unsigned short *base;   // first element of the batch slice
   uint32_t inner, rows;         // extent of the contiguous axis (= row pitch) and of the other one
@@ -88,9 +75,7 @@ __device__ __forceinline__ void piece_at(const Gather &g, uint32_t i, uint32_t m
     col = mn0 + (i >> 9) * 64u + (i & 7u) * 8u;
   }
 }
-__device__ __forceinline__ void load_piece(const Gather &g, uint32_t i, uint32_t mn0, uint32_t k0, Piece &p) {
-  uint32_t row, col;
-  piece_at(g, i, mn0, k0, row, col);
+__device__ __forceinline__ void load_at(const Gather &g, uint32_t row, uint32_t col, Piece &p) {
   p.lo = p.hi = make_uint4(0, 0, 0, 0);
   p.off = 0;
   p.valid = 0;
@@ -103,7 +88,12 @@ __device__ __forceinline__ void load_piece(const Gather &g, uint32_t i, uint32_t
   p.lo = __ldg(reinterpret_cast<const uint4 *>(a));
   if (p.off + p.valid > 8u) p.hi = __ldg(reinterpret_cast<const uint4 *>(a) + 1);
 }
-__device__ __forceinline__ void store_piece(const Gather &g, uint32_t i, uint32_t box, const Piece &p) {
+__device__ __forceinline__ void load_piece(const Gather &g, uint32_t i, uint32_t mn0, uint32_t k0, Piece &p) {
+  uint32_t row, col;
+  piece_at(g, i, mn0, k0, row, col);
+  load_at(g, row, col, p);
+}
+__device__ __forceinline__ uint4 elements_of(const Piece &p) {
   uint4 v = shift_in(p.lo, p.hi, p.off);
   if (p.valid < 8u) {   // what lies past the row (or outside the matrix) is zero
     uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -111,6 +101,10 @@ __device__ __forceinline__ void store_piece(const Gather &g, uint32_t i, uint32_
     for (uint32_t j = 0; j < 4; ++j) w[j] = 2 * j + 2 <= p.valid ? w[j] : (2 * j + 1 <= p.valid ? (w[j] & 0xffffu) : 0u);
     v = make_uint4(w[0], w[1], w[2], w[3]);
   }
+  return v;
+}
+__device__ __forceinline__ void store_piece(const Gather &g, uint32_t i, uint32_t box, const Piece &p) {
+  const uint4 v = elements_of(p);
   // both forms: rows of 128 bytes, 16-byte piece c of row r at c ^ (r & 7); boxes of the [k][64] form are 8 KB apart
   const uint32_t r = i >> 3, c = i & 7u;
   const uint32_t dst = box + r * 128u + ((c ^ (r & 7u)) << 4);
@@ -383,10 +377,31 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
         }
       }
     } else {
-      // rows at any even address: one element per lane, 32 consecutive columns per warp and store
-      for (uint32_t j = threadIdx.x; j < 16u * (i_end - i_begin); j += kThreads) {
-        const uint32_t i = i_begin + (j >> 4), row = i / kSpr, col = col0 + (i - row * kSpr) * 16u + (j & 15u);
-        if (col < P.N) out[(int64_t)(row0 + row) * t.sm + col] = *reinterpret_cast<const unsigned short *>(staged + 2u * j);
+      // rows at any even address, or strips that start inside one
+      const uint32_t r_begin = i_begin / kSpr, r_count = i_end > i_begin ? (i_end - 1) / kSpr + 1 - r_begin : 0u;
+      constexpr uint32_t kUnits = 2 * kSpr - 1;
+      auto row_of = [&](uint32_t r, unsigned short *&dst, uint32_t &col, uint32_t &run, uint32_t &from) {
+        const uint32_t first = max(i_begin, r * kSpr), last = min(i_end, (r + 1) * kSpr);
+        col = col0 + (first - r * kSpr) * 16u;
+        run = (last - first) * 16u;
+        from = (first - i_begin) * 32u;
+        dst = out + (int64_t)(row0 + r) * t.sm + col;
+      };
+      unsigned short *dst;
+      uint32_t col, run, from;
+      for (uint32_t j = threadIdx.x; j < r_count * kUnits; j += kThreads) {
+        const uint32_t r = j / kUnits, u = j - r * kUnits;
+        row_of(r_begin + r, dst, col, run, from);
+        const uint32_t ahead = elements_ahead(dst), at = ahead + 8u * u;
+        if (at + 8u > run || col + at >= P.N) continue;
+        const uint4 *piece = reinterpret_cast<const uint4 *>(staged + from) + (at >> 3);
+        const uint4 lo = piece[0], hi = (ahead & 7u) != 0 ? piece[1] : lo;
+        store_unit(dst + at, shift_in(lo, hi, ahead & 7u), P.N - (col + at));
+      }
+      for (uint32_t j = threadIdx.x; j < r_count * 8u; j += kThreads) {
+        row_of(r_begin + (j >> 3), dst, col, run, from);
+        const uint32_t at = single_at(j & 7u, elements_ahead(dst), run);
+        if (col + at < P.N) dst[at] = *reinterpret_cast<const unsigned short *>(staged + from + 2u * at);
       }
     }
   }
@@ -404,6 +419,62 @@ __global__ void __launch_bounds__(kThreads, 2) dvm_b200_mm_tile_n64(const __grid
 __global__ void __launch_bounds__(kThreads, 2) dvm_b200_mm_tile_n128(const __grid_constant__ MmParam P, const __grid_constant__ TileMaps maps,
                                                                      const __grid_constant__ TileArgs A, const LaunchTag epoch) {
   tile_body<128>(P, maps, A, epoch);
+}
+
+// Operands of unaligned rows, copied to rows of whole 16-byte units for the copy engine.  Loading them by the work warps of
+// every tile costs 1700 cycles per k-block, seven times its MMAs, and each tile does it again.
+// Bound by memory: one pass, four independent pieces per thread.  [4096, 4095] x [4001, 4095]^T: 886 -> 123 us in all,
+// [2000, 2001] x [2001, 2001] 144 -> 34, [180, 511] x [565, 511]^T 12.7 -> 8.9.
+struct PackJob {
+  const unsigned short *src;
+  uint4 *dst;
+  uint32_t inner, rows;      // rows of all batch slices
+  uint32_t units, blocks;    // 16-byte units per row of the copy; thread blocks of this job
+};
+constexpr uint32_t kPackThreads = 256, kPackPieces = 4;
+
+__global__ void __launch_bounds__(kPackThreads) dvm_b200_mm_pack(const PackJob ja, const PackJob jb) {
+  chain_wait();
+  chain_launch();
+  const bool second = blockIdx.x >= ja.blocks;
+  const PackJob &j = second ? jb : ja;
+  const Gather g{j.src, j.inner, j.rows, true};
+  const uint32_t first = (blockIdx.x - (second ? ja.blocks : 0u)) * (kPackThreads * kPackPieces) + threadIdx.x;
+  Piece p[kPackPieces];
+#pragma unroll
+  for (uint32_t i = 0; i < kPackPieces; ++i) {
+    const uint32_t at = first + i * kPackThreads, row = at / j.units;
+    load_at(g, row, (at - row * j.units) * 8u, p[i]);   // (nothing past the last row)
+  }
+#pragma unroll
+  for (uint32_t i = 0; i < kPackPieces; ++i)
+    if (p[i].valid != 0) j.dst[first + i * kPackThreads] = elements_of(p[i]);
+}
+
+int LaunchMmPack(MmParam *p, void *stream) {
+  PackJob job[2];
+  memset(job, 0, sizeof(job));
+  auto fill = [](PackJob *j, uint64_t *ptr, uint32_t *pitch, uint64_t to, uint32_t inner, uint64_t rows) {
+    j->src = reinterpret_cast<const unsigned short *>(*ptr);
+    j->dst = reinterpret_cast<uint4 *>(to);
+    j->inner = inner;
+    j->rows = static_cast<uint32_t>(rows);
+    j->units = (inner + 7) / 8;
+    j->blocks = static_cast<uint32_t>((rows * j->units + kPackThreads * kPackPieces - 1) / (kPackThreads * kPackPieces));
+    *ptr = to;
+    *pitch = j->units * 8;
+  };
+  if (p->a_pack != 0 && MmGatherA(*p)) fill(&job[0], &p->a_ptr, &p->a_pitch, p->a_pack, MmInnerA(*p), static_cast<uint64_t>(MmRowsA(*p)) * p->a_batches);
+  if (p->b_pack != 0 && MmGatherB(*p)) fill(&job[1], &p->b_ptr, &p->b_pitch, p->b_pack, MmInnerB(*p), static_cast<uint64_t>(MmRowsB(*p)) * p->b_batches);
+  if (job[0].blocks + job[1].blocks == 0) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(job[0].blocks + job[1].blocks, 1, 1);
+  cfg.blockDim = dim3(kPackThreads, 1, 1);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  ChainAttribute(&cfg, attr);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, dvm_b200_mm_pack, job[0], job[1]);
+  return e != cudaSuccess ? static_cast<int>(e) : static_cast<int>(cudaGetLastError());
 }
 
 int LaunchMmTile(const MmParam &p, uint32_t bn, uint32_t split, void *stream) {
@@ -441,9 +512,9 @@ int LaunchMmTile(const MmParam &p, uint32_t bn, uint32_t split, void *stream) {
   memset(&maps, 0, sizeof(maps));
   int rc = 0;
   if (!a.gather_a && kblocks != 0)
-    rc = p.a_mmajor ? EncodeMmOperand(&maps.a, p.a_ptr, p.M, p.K, p.a_batches, 64) : EncodeMmOperand(&maps.a, p.a_ptr, p.K, p.M, p.a_batches, a.a_rows);
+    rc = EncodeMmOperand(&maps.a, p.a_ptr, MmInnerA(p), MmPitchA(p), MmRowsA(p), p.a_batches, p.a_mmajor ? 64 : a.a_rows);
   if (rc == 0 && !a.gather_b && kblocks != 0)
-    rc = p.b_kmajor ? EncodeMmOperand(&maps.b, p.b_ptr, p.K, p.N, p.b_batches, bn) : EncodeMmOperand(&maps.b, p.b_ptr, p.N, p.K, p.b_batches, 64);
+    rc = EncodeMmOperand(&maps.b, p.b_ptr, MmInnerB(p), MmPitchB(p), MmRowsB(p), p.b_batches, p.b_kmajor ? bn : 64);
   if (rc != 0) return rc;
   const uint64_t tiles = static_cast<uint64_t>((p.M + BM - 1) / BM) * ((p.N + bn - 1) / bn) * p.batch0 * p.batch1;
   if (tiles * split >= (1ull << 31)) return -6;

@@ -1076,6 +1076,19 @@ struct Planner {
 void VKernel::PlanStages(const std::vector<NDObject *> &ops) {
   Planner p(this, ops);
   p.Run();
+  ws_needed_ = p.ws_top;
+  for (auto &st : stages_) {
+    if (st->kind != STAGE_MATMUL || st->mm.idle) continue;
+    uint64_t a = 0, b = 0;
+    dvmb::MmPackBytes(st->mm.param, &a, &b);
+    auto place = [&](uint64_t bytes) {
+      const size_t off = p.ws_top;
+      p.ws_top = (p.ws_top + bytes + 255) & ~static_cast<size_t>(255);
+      return bytes != 0 ? static_cast<int64_t>(off) : -1;
+    };
+    st->mm.a_pack_off = place(a);
+    st->mm.b_pack_off = place(b);
+  }
   ws_bytes_ = p.ws_top;
 }
 

@@ -141,6 +141,7 @@ size_t VKernel::Compile() {
     p.stages = std::move(stages_);
     p.synth = std::move(synth_);
     p.ws_bytes = ws_bytes_;
+    p.ws_needed = ws_needed_;
     p.used = ++plan_clock_;
     plans_.push_back(std::move(p));
     stages_.clear();
@@ -153,6 +154,7 @@ size_t VKernel::Compile() {
       stages_ = std::move(plans_[i].stages);
       synth_ = std::move(plans_[i].synth);
       ws_bytes_ = plans_[i].ws_bytes;
+      ws_needed_ = plans_[i].ws_needed;
       plans_.erase(plans_.begin() + static_cast<std::ptrdiff_t>(i));
       plan_sig_ = sig_;
       has_plan_ = compiled_ = true;
@@ -166,7 +168,7 @@ size_t VKernel::Compile() {
 
 void VKernel::CompileFresh() {
   ClearStages();
-  ws_bytes_ = 0;
+  ws_bytes_ = ws_needed_ = 0;
   std::vector<NDObject *> ops = LiveOps(nodes_);
   if (ops.empty()) {
     compiled_ = true;
@@ -201,7 +203,7 @@ void VKernel::CompileFresh() {
   compiled_ = true;
 }
 
-void VKernel::Bind(const RelocEntry *relocs, size_t n, void *workspace) {
+void VKernel::Bind(const RelocEntry *relocs, size_t n, void *workspace, size_t workspace_bytes) {
   workspace_ = workspace;
   for (size_t i = 0; i < n; ++i) relocs[i].io->addr = relocs[i].addr;
   for (auto &stp : stages_) {
@@ -209,6 +211,11 @@ void VKernel::Bind(const RelocEntry *relocs, size_t n, void *workspace) {
       MatMulStage &mm = stp->mm;
       mm.param.a_ptr = reinterpret_cast<uint64_t>(AddrOf(mm.a, workspace));
       mm.param.b_ptr = reinterpret_cast<uint64_t>(AddrOf(mm.b, workspace));
+      auto pack_at = [&](int64_t off) {
+        return workspace != nullptr && off >= 0 && workspace_bytes >= ws_bytes_ ? reinterpret_cast<uint64_t>(workspace) + off : 0ull;
+      };
+      mm.param.a_pack = pack_at(mm.a_pack_off);
+      mm.param.b_pack = pack_at(mm.b_pack_off);
       mm.param.bias_ptr = mm.bias ? reinterpret_cast<uint64_t>(AddrOf(mm.bias, workspace)) : 0;
       for (size_t s = 0; s < mm.slot_obj.size(); ++s)
         if (mm.slot_obj[s]) mm.param.tensor[s].ptr = reinterpret_cast<uint64_t>(AddrOf(mm.slot_obj[s], workspace));

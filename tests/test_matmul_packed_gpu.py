@@ -1,0 +1,34 @@
+"""MatMul operands in rows that do not start on 16 bytes: repacked in the workspace, or loaded as they are without one."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("trans", ["", "a", "b"])
+@pytest.mark.parametrize("batch,m,n,k", [((), 1, 9, 1), ((), 300, 259, 65), ((), 129, 1001, 127), ((3,), 257, 63, 71), ((2, 3), 66, 130, 33),
+                                         ((), 513, 264, 1023), ((5,), 8, 7, 1025)])
+def test_both_paths(batch, m, n, k, trans):
+    from dvm_b200 import _capi
+    from dvm_b200.tester import Tester
+    lib = _capi.load()
+    rng = np.random.default_rng(m + 3 * n + 5 * k)
+    a = rng.standard_normal(batch + (m, k)).astype(np.float16)
+    b = (rng.standard_normal(batch[-1:] + (k, n)) / np.sqrt(k)).astype(np.float16)   # (a leading batch axis is broadcast)
+    t = Tester("mix")
+    la = t.load(np.ascontiguousarray(np.swapaxes(a, -1, -2)) if trans == "a" else a)
+    lb = t.load(np.ascontiguousarray(np.swapaxes(b, -1, -2)) if trans == "b" else b)
+    s = t.store(t.matmul(la, lb, trans == "a", trans == "b"))
+    t.run()
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    # one rounding to fp16 (2^-11 of the result); the fp32 sum of k terms of size 1 / sqrt(k) is off by less than k 2^-24
+    bound = 2.0 ** -11 * np.abs(want) + 2.0 ** -24 * (k + 1.0) + 2.0 ** -25
+    assert np.all(np.abs(t.output(s).astype(np.float64) - want) <= bound)
+    ops = [la, lb, s]
+    relocs = (_capi.Reloc * len(ops))()
+    for i, op in enumerate(ops):
+        relocs[i].io, relocs[i].addr = op._h, t.device_ptr(op)
+    assert lib.dvm_rt_memset(t.device_ptr(s), 0, want.size * 2, None) == 0
+    assert lib.dvm_launch_reloc(t._k, relocs, len(relocs), None, None) == 0, _capi.last_error()   # no workspace
+    assert lib.dvm_rt_sync(None) == 0, _capi.last_error()
+    assert np.all(np.abs(t.output(s).astype(np.float64) - want) <= bound)
