@@ -255,6 +255,15 @@ __device__ __forceinline__ uint64_t add_pair(uint64_t a, uint64_t b) {
 __device__ __forceinline__ float bias_at(const MmParam &P, uint32_t col) {
   return P.bias_ptr != 0 && col < P.N ? load_bias(P, col) : 0.0f;
 }
+// The same in two steps: the stored bits (a load in flight), their value.
+__device__ __forceinline__ uint32_t bias_bits(const MmParam &P, uint32_t col) {
+  if (col >= P.N) return 0;
+  return P.bias_dtype == T_F32 ? __ldg(reinterpret_cast<const uint32_t *>(P.bias_ptr) + col)
+                               : __ldg(reinterpret_cast<const unsigned short *>(P.bias_ptr) + col);
+}
+__device__ __forceinline__ float bias_value(const MmParam &P, uint32_t bits) {
+  return u2f(P.bias_dtype == T_F32 ? bits : widen(P.bias_dtype, (unsigned short)bits));
+}
 // Adds sixteen columns' bias from shared memory (staged as fp32 while the product was being made: read from global memory
 // here, each strip waited for its own loads).
 __device__ __forceinline__ void add_bias_staged(uint32_t saddr, uint32_t (&r)[16]) {
@@ -366,16 +375,20 @@ __device__ __forceinline__ void gate_strip(const uint32_t (&c)[3], uint32_t (&r)
 }
 
 // Rounding to the operand type and the post-fusion program for one 16-column strip of one row (bias already added).
-// When the whole program is a store in the operand type (plain or gated), the sixteen 16-bit results come back in `pk` and
-// the slot of their tensor is returned: the caller stores them through shared memory, so that rows of any alignment leave
-// as contiguous runs.  Any other program is stored from here and 0xffffffff is returned.
-__device__ __forceinline__ uint32_t finish_strip(const MmParam &P, const EpiPos &pos, uint32_t (&r)[16], uint32_t (&pk)[8]) {
-  pack_strip(P.in_dtype, r, pk);   // the product in the operand type
-  if (P.fast_store_slot != 0xffffffffu && P.tensor[P.fast_store_slot].dtype == P.in_dtype) return P.fast_store_slot;
+// EPI_STORE and EPI_GATE leave the sixteen 16-bit results in `pk`: the caller stores them through shared memory, so that rows
+// of any alignment leave as contiguous runs.  The other modes are stored from here.
+// (The mode and the type are template arguments because looking them up in the parameters, strip by strip, took 300 of the
+// 350 cycles of a strip that is only stored.)
+constexpr uint32_t kAnyType = 0xffu;   // the type of P
+template <uint32_t MODE, uint32_t DT>
+__device__ __forceinline__ void finish_strip(const MmParam &P, const EpiPos &pos, uint32_t (&r)[16], uint32_t (&pk)[8]) {
+  const uint32_t dt = DT == kAnyType ? P.in_dtype : DT;
+  pack_strip(dt, r, pk);   // the product in the operand type
+  if (MODE == EPI_STORE) return;
   // back to the 32-bit register form of the rounded product
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    if (P.in_dtype == T_BF16) {
+    if (dt == T_BF16) {
       r[2 * i] = pk[i] << 16;
       r[2 * i + 1] = pk[i] & 0xffff0000u;
     } else {
@@ -384,25 +397,40 @@ __device__ __forceinline__ uint32_t finish_strip(const MmParam &P, const EpiPos 
       r[2 * i + 1] = __float_as_uint(f.y);
     }
   }
-  if (P.gate_slot != 0xffffffffu) {
+  if (MODE == EPI_GATE) {
     gate_strip(P.gate_c, r);
-    pack_strip(P.in_dtype, r, pk);
-    return P.gate_slot;
+    pack_strip(dt, r, pk);
+    return;
   }
-  if (pos.valid == 0) return 0xffffffffu;
-  if (P.fast_store_slot != 0xffffffffu && pos.valid == 16u) {
-    // one store of the product widened to fp32 (a partial product that another launch finishes)
-    const EpiTensor &t = P.tensor[P.fast_store_slot];
+  if (pos.valid == 0) return;
+  if (P.epi_mode == EPI_WIDEN && pos.valid == 16u) {
+    const EpiTensor &t = P.tensor[P.out_slot];
     uint8_t *dst = reinterpret_cast<uint8_t *>(t.ptr) + (epi_offset(t, pos) << 2);
-    if (t.dtype == T_F32 && (reinterpret_cast<uint64_t>(dst) & 15u) == 0) {
+    if ((reinterpret_cast<uint64_t>(dst) & 15u) == 0) {
 #pragma unroll
       for (int g = 0; g < 4; ++g)
         *reinterpret_cast<uint4 *>(dst + 16 * g) = make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
-      return 0xffffffffu;
+      return;
     }
   }
   run_epilogue(P, pos, r);
-  return 0xffffffffu;
+}
+
+template <uint32_t M, uint32_t D>
+struct Mode {
+  static constexpr uint32_t mode = M, dtype = D;
+};
+// Runs f with the mode and the operand type as constants (EPI_WIDEN takes EPI_PROGRAM's form).
+template <typename F>
+__device__ __forceinline__ void with_mode(const MmParam &P, F f) {
+  const bool bf = P.in_dtype == T_BF16;
+  if (P.epi_mode == EPI_STORE) {
+    if (bf) f(Mode<EPI_STORE, T_BF16>()); else f(Mode<EPI_STORE, T_F16>());
+  } else if (P.epi_mode == EPI_GATE) {
+    if (bf) f(Mode<EPI_GATE, T_BF16>()); else f(Mode<EPI_GATE, T_F16>());
+  } else {
+    f(Mode<EPI_PROGRAM, kAnyType>());
+  }
 }
 
 }  // namespace

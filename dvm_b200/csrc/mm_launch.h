@@ -46,17 +46,23 @@ struct MmParam {
   uint32_t mma_slot;
   uint32_t num_temps;
   uint32_t group_m;         // row blocks swept together over all column blocks (L2 reuse of the A panel); set by the launcher
-  uint32_t fast_store_slot; // set by the launcher: the post-fusion program is just "store the product to tensor <slot>" (in the
-                            // operand type or widened to fp32), which the kernel does without interpreting; 0xffffffff otherwise
-  // set by the launcher: the post-fusion program is the gated form  y = x / (c2 + exp(c1 * (x + c0 * x^3)))  of the
-  // rounded product x (tanh-GeLU written through the exponential, c0 = 0.044715, c1 = -2 sqrt(2/pi), c2 = 1), rounded to
-  // the operand type and stored to tensor <gate_slot>: the kernel computes it in registers with the interpreter's own
-  // operations in the interpreter's order (same bits) instead of interpreting eleven words per strip; 0xffffffff otherwise
-  uint32_t gate_slot;
+  // Set by the launcher: what the post-fusion program does (EpiMode), and the tensor it stores to when it is one of the forms
+  // that leave through shared memory in the operand type.  EPI_GATE is  y = x / (c2 + exp(c1 * (x + c0 * x^3)))  of the rounded
+  // product x (tanh-GeLU written through the exponential, c0 = 0.044715, c1 = -2 sqrt(2/pi), c2 = 1), computed in registers with
+  // the interpreter's operations in the interpreter's order instead of eleven interpreted words per strip.
+  uint32_t epi_mode, out_slot;
   uint32_t gate_c[3];
+  uint32_t tma_out;         // set by the launcher: the copy engine can address the result (16-byte base and strides)
   uint32_t leave_sms;       // set by the planner: SMs this launch leaves free (a collective runs beside it); 0 = none
   EpiTensor tensor[kMmMaxEpiTensors];
   uint64_t epilogue[kMmMaxEpilogueWords];
+};
+
+enum EpiMode : uint32_t {
+  EPI_PROGRAM = 0,   // interpreted, strip by strip
+  EPI_WIDEN = 1,     // one store of the product widened to fp32 (a partial product that another launch finishes)
+  EPI_STORE = 2,     // one store of the product in the operand type
+  EPI_GATE = 3,      // the gated form, stored in the operand type
 };
 
 // Enqueue the MatMul.  Returns 0, a cudaError_t (> 0), or a negative code for an unsupported shape.

@@ -63,25 +63,15 @@ constexpr uint32_t kSmemBytes = kSmemHeader + kStages * kStageBytes + kEpiWarps 
 
 struct MmMaps {
   CUtensorMap a, b;
+  CUtensorMap o;   // the result, boxes of 32 rows of 32 columns, 64-byte swizzle (P.tma_out)
 };
 
-// 32 rows of 64 staged columns (128 bytes, 16-byte piece p of row r at p ^ (r & 7)) to the result tensor.
-__device__ __forceinline__ void copy_out(const MmParam &P, uint32_t slot, uint32_t b0, uint32_t b1, uint32_t row0, uint32_t col0,
-                                         uint32_t saddr, uint32_t lane) {
-  const EpiTensor &t = P.tensor[slot];
+// 32 rows of 64 staged columns (128 bytes, 16-byte piece p of row r at p ^ (r & 7)) to a result tensor that the copy engine
+// cannot address.
+__device__ __forceinline__ void copy_out(const MmParam &P, uint32_t b0, uint32_t b1, uint32_t row0, uint32_t col0, uint32_t saddr,
+                                         uint32_t lane) {
+  const EpiTensor &t = P.tensor[P.out_slot];
   unsigned short *const out = reinterpret_cast<unsigned short *>(t.ptr) + ((int64_t)b0 * t.sb0 + (int64_t)b1 * t.sb1 + (int64_t)row0 * t.sm + col0);
-  if (((reinterpret_cast<uint64_t>(out) | (uint64_t)(t.sm * 2)) & 15u) == 0 && col0 + 64u <= P.N) {
-    const uint32_t piece = lane & 7u;
-#pragma unroll
-    for (uint32_t i = 0; i < 8; ++i) {
-      const uint32_t row = 4 * i + (lane >> 3);
-      uint4 q;
-      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "r"(saddr + row * 128u + ((piece ^ (row & 7u)) << 4)));
-      if (row0 + row < P.M) *reinterpret_cast<uint4 *>(out + (int64_t)row * t.sm + piece * 8u) = q;
-    }
-    return;
-  }
-  // a ragged edge, or rows at any even address
 #pragma unroll 1
   for (uint32_t j = lane; j < 32u * 7u; j += 32u) {
     const uint32_t row = j / 7u, u = j - 7u * row;
@@ -228,76 +218,101 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
     const uint32_t ew = warp - 2;
     const uint32_t quarter = warp & 3u;          // TMEM lane quarter this warp may read
     const uint32_t col0 = (ew >> 2) * kEpiCols;  // the columns of the tile this warp drains
-    const uint32_t row_in_tile = quarter * 32 + lane;
     const uint32_t out_saddr = stages + kStages * kStageBytes + ew * kOutBytes;
-    // (the program is one store in the operand type: its results go out through shared memory)
-    uint32_t staged_slot = P.gate_slot;
-    if (staged_slot == 0xffffffffu && P.fast_store_slot != 0xffffffffu && P.tensor[P.fast_store_slot].dtype == P.in_dtype)
-      staged_slot = P.fast_store_slot;
     const uint32_t bias_saddr = base + kBiasOff + ew * (kEpiCols * 4u);
     uint32_t acc = 0, acc_parity = 0;
-    for (uint32_t t = unit; t < num_tiles; t += num_units) {
-      uint32_t bz, mb, nb;
+    // Coordinates and bias of a tile are on their way while the tile before is drained: one after the other, in front of each
+    // tile, they took 2000 cycles of a [4096, 1024] x [1024, 4096] product's 13 000 per tile.
+    uint32_t bz, mb, nb;
+    uint32_t bias[kEpiCols / 32];
+    auto look_up = [&](uint32_t t) {
       tile_coords(t, mblocks, nblocks, P.group_m, bz, mb, nb);
-      if (P.bias_ptr != 0) {
-        __syncwarp();   // (the warp has read the previous tile's)
+      if (P.bias_ptr == 0) return;
 #pragma unroll
-        for (uint32_t c = lane; c < kEpiCols; c += 32) {
-          const float b = bias_at(P, nb * BN + col0 + c);
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_saddr + 4u * c), "f"(b) : "memory");
+      for (uint32_t i = 0; i < kEpiCols / 32; ++i) bias[i] = bias_bits(P, nb * BN + col0 + i * 32 + lane);
+    };
+    if (unit < num_tiles) look_up(unit);
+    with_mode(P, [&](auto mode) {
+      constexpr uint32_t MODE = decltype(mode)::mode, DT = decltype(mode)::dtype;
+      constexpr bool kStaged = MODE != EPI_PROGRAM;
+      const bool tma = kStaged && P.tma_out != 0;
+      for (uint32_t t = unit; t < num_tiles; t += num_units) {
+        if (P.bias_ptr != 0) {
+          __syncwarp();   // (the warp has read the previous tile's)
+#pragma unroll
+          for (uint32_t i = 0; i < kEpiCols / 32; ++i)
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_saddr + 4u * (i * 32 + lane)), "f"(bias_value(P, bias[i])) : "memory");
+          __syncwarp();
         }
-        __syncwarp();
-      }
-      mbar_wait(bar_tfull + 8 * acc, acc_parity, 4, &g_mm_status, epoch);
-      tcgen05_after_sync();
-      EpiPos pos;
-      pos.b0 = bz / P.batch1;
-      pos.b1 = bz - pos.b0 * P.batch1;
-      pos.row = (mb * 2 + rank) * BM + row_in_tile;
-      const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * BN + col0;
-      // (one strip per trip and no unrolling: eight copies of the strip code did not fit the instruction cache and made
-      // the epilogue of a CTA's first tile 4 us longer)
-      uint32_t next[16];
-      tmem_ld_32x32b_x16_nowait(taddr, next);
+        EpiPos pos;
+        pos.b0 = bz / P.batch1;
+        pos.b1 = bz - pos.b0 * P.batch1;
+        const uint32_t first_row = (mb * 2 + rank) * BM + quarter * 32u, first_col = nb * BN + col0;
+        pos.row = first_row + lane;
+        if (t + num_units < num_tiles) look_up(t + num_units);
+        mbar_wait(bar_tfull + 8 * acc, acc_parity, 4, &g_mm_status, epoch);
+        tcgen05_after_sync();
+        const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * BN + col0;
+        // (one strip per trip and no unrolling: eight copies of the strip code did not fit the instruction cache and made
+        // the epilogue of a CTA's first tile 4 us longer)
+        uint32_t next[16];
+        tmem_ld_32x32b_x16_nowait(taddr, next);
 #pragma unroll 1
-      for (uint32_t c = 0; c < kEpiCols; c += 16) {
-        uint32_t r[16], pk[8];
-        tmem_ld_wait16(next);
+        for (uint32_t c = 0; c < kEpiCols; c += 16) {
+          uint32_t r[16], pk[8];
+          tmem_ld_wait16(next);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) r[i] = next[i];
-        if (c + 16 < kEpiCols) tmem_ld_32x32b_x16_nowait(taddr + c + 16, next);   // on its way while this strip is worked on
-        pos.col = nb * BN + col0 + c;
-        uint32_t slot = 0xffffffffu;
-        if (pos.col < P.N) {   // (rows past the matrix take part: their results are not copied out)
-          pos.valid = pos.row < P.M ? min(16u, P.N - pos.col) : 0u;
-          if (P.bias_ptr != 0) add_bias_staged(bias_saddr + c * 4u, r);
-          slot = finish_strip(P, pos, r, pk);
+          for (int i = 0; i < 16; ++i) r[i] = next[i];
+          if (c + 16 < kEpiCols) tmem_ld_32x32b_x16_nowait(taddr + c + 16, next);   // on its way while this strip is worked on
+          pos.col = first_col + c;
+          if (pos.col < P.N) {   // (rows past the matrix take part: their results are not copied out)
+            pos.valid = pos.row < P.M ? min(16u, P.N - pos.col) : 0u;
+            if (P.bias_ptr != 0) add_bias_staged(bias_saddr + c * 4u, r);
+            finish_strip<MODE, DT>(P, pos, r, pk);
+          }
+          if (!kStaged) continue;
+          if (tma) {
+            // two buffers of 32 columns: rows of 64 bytes, 16-byte piece p of row r at p ^ (r / 2 & 3)
+            const uint32_t buf = out_saddr + ((c >> 5) & 1u) * (kOutBytes / 2), row_saddr = buf + lane * 64u, at = (c >> 3) & 2u;
+            if ((c & 16u) == 0) {
+              if (lane == 0) tma_store_wait_read<1>();   // the store before the last one has read this buffer
+              __syncwarp();
+            }
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + ((at ^ ((lane >> 1) & 3u)) << 4)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + (((at + 1u) ^ ((lane >> 1) & 3u)) << 4)), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
+            if ((c & 16u) != 0) {
+              fence_async_shared();
+              __syncwarp();
+              if (lane == 0) {
+                const uint32_t box_col = first_col + (c & ~31u);
+                if (box_col < P.N && first_row < P.M)   // (the tensor map cuts off what lies past the matrix)
+                  tma_store_4d(&maps.o, buf, (int)box_col, (int)first_row, (int)pos.b1, (int)pos.b0);
+                tma_store_commit();
+              }
+            }
+          } else {
+            // row `lane`, 16-byte pieces 2 (c / 16 % 4) and the next, each at piece ^ (row & 7)
+            const uint32_t piece = (c >> 3) & 7u, row_saddr = out_saddr + lane * 128u;
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + ((piece ^ (lane & 7u)) << 4)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + (((piece + 1u) ^ (lane & 7u)) << 4)), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
+            if ((c & 48u) == 48u) {
+              __syncwarp();
+              copy_out(P, pos.b0, pos.b1, first_row, first_col + (c & ~63u), out_saddr, lane);
+              __syncwarp();
+            }
+          }
         }
-        if (staged_slot == 0xffffffffu) continue;
-        // row `lane`, 16-byte pieces 2 (c / 16 % 4) and the next, each at piece ^ (row & 7)
-        if (slot != 0xffffffffu) {
-          const uint32_t piece = (c >> 3) & 7u, row_saddr = out_saddr + lane * 128u;
-          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + ((piece ^ (lane & 7u)) << 4)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
-          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + (((piece + 1u) ^ (lane & 7u)) << 4)), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
-        }
-        if ((c & 48u) == 48u) {
-          __syncwarp();
-          const uint32_t first_col = nb * BN + col0 + (c & ~63u), first_row = (mb * 2 + rank) * BM + quarter * 32u;
-          copy_out(P, staged_slot, pos.b0, pos.b1, first_row, first_col, out_saddr, lane);
-          __syncwarp();
+        tmem_ld_wait16(next);
+        tcgen05_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(bar_tempty + 8 * acc, 0));
+        if (++acc == 2) {
+          acc = 0;
+          acc_parity ^= 1u;
         }
       }
-      tmem_ld_wait16(next);
-      tcgen05_before_sync();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive_cluster(map_to_cta(bar_tempty + 8 * acc, 0));
-      }
-      if (++acc == 2) {
-        acc = 0;
-        acc_parity ^= 1u;
-      }
-    }
+    });
+    if (lane == 0) tma_store_wait_read<0>();   // shared memory stays until the last store has read it
   }
   __syncwarp();
   tcgen05_before_sync();
@@ -332,6 +347,21 @@ PFN_cuTensorMapEncodeTiled GetEncode() {
 }  // namespace
 
 // 3-d map over a [batches, rows, inner] row-major operand: box = [1, box_rows, 64 elements], 128-byte swizzle
+// The result as [batch0, batch1, M, N] for the copy engine, if it can address it.
+static bool EncodeMmResult(CUtensorMap *map, const MmParam &p) {
+  const EpiTensor &t = p.tensor[p.out_slot];
+  auto encode = GetEncode();
+  const int64_t row = t.sm * 2, b1 = p.batch1 > 1 ? t.sb1 * 2 : row * p.M, b0 = p.batch0 > 1 ? t.sb0 * 2 : b1 * p.batch1;
+  if (encode == nullptr || ((t.ptr | row | b1 | b0) & 15) != 0 || row <= 0 || b1 <= 0 || b0 <= 0 || b0 >= (1ll << 40)) return false;
+  cuuint64_t dims[4] = {p.N, p.M, p.batch1, p.batch0};
+  cuuint64_t strides[3] = {static_cast<cuuint64_t>(row), static_cast<cuuint64_t>(b1), static_cast<cuuint64_t>(b0)};
+  cuuint32_t box[4] = {32, 32, 1, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, reinterpret_cast<void *>(t.ptr), dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int EncodeMmOperand(CUtensorMap *map, uint64_t ptr, uint64_t inner, uint64_t pitch, uint64_t rows, uint64_t batches, uint32_t box_rows) {
   auto encode = GetEncode();
   if (encode == nullptr) return -10;
@@ -439,17 +469,20 @@ int LaunchMatMul(const MmParam &p_in, void *stream) {
   static const int group_env = getenv("DVM_B200_MM_GROUP_M") ? atoi(getenv("DVM_B200_MM_GROUP_M")) : 0;
   p.group_m = group_env > 0 ? static_cast<uint32_t>(group_env) : 8u;
   // "copy acc, product; store tensor s; end" with a dense row layout: the kernel stores the product directly
-  p.fast_store_slot = 0xffffffffu;
+  p.epi_mode = EPI_PROGRAM;
+  p.out_slot = 0;
   {
     const uint64_t w0 = p.epilogue[0], w1 = p.epilogue[1], w2 = p.epilogue[2];
     if (DVMB_OPC(w0) == OP_COPY && DVMB_OKIND(w0) == K_TENSOR && DVMB_OIDX(w0) == p.mma_slot && DVMB_OPC(w1) == OP_ST &&
         DVMB_OPC(w2) == OP_END && DVMB_SUB(w1) < p.n_tensors) {
       const EpiTensor &t = p.tensor[DVMB_SUB(w1)];
-      if (t.sn == 1 && (t.dtype == p.in_dtype || t.dtype == T_F32)) p.fast_store_slot = DVMB_SUB(w1);
+      if (t.sn == 1 && (t.dtype == p.in_dtype || t.dtype == T_F32)) {
+        p.epi_mode = t.dtype == p.in_dtype ? EPI_STORE : EPI_WIDEN;
+        p.out_slot = DVMB_SUB(w1);
+      }
     }
   }
   // the gated form x / (c2 + exp(c1 * (x + c0 * x^3))) of the product, rounded to the operand type and stored
-  p.gate_slot = 0xffffffffu;
   {
     static const bool off = getenv("DVM_B200_NO_FUSE") != nullptr;
     const uint64_t *w = p.epilogue;
@@ -465,7 +498,8 @@ int LaunchMatMul(const MmParam &p_in, void *stream) {
         DVMB_RND(w[9]) == rnd_out && DVMB_OPC(w[10]) == OP_ST && DVMB_OPC(w[11]) == OP_END && DVMB_SUB(w[10]) < p.n_tensors) {
       const EpiTensor &t = p.tensor[DVMB_SUB(w[10])];
       if (t.sn == 1 && t.dtype == p.in_dtype) {
-        p.gate_slot = DVMB_SUB(w[10]);
+        p.epi_mode = EPI_GATE;
+        p.out_slot = DVMB_SUB(w[10]);
         p.gate_c[0] = DVMB_IMM(w[3]);
         p.gate_c[1] = DVMB_IMM(w[5]);
         p.gate_c[2] = DVMB_IMM(w[7]);
@@ -499,11 +533,13 @@ int LaunchMatMul(const MmParam &p_in, void *stream) {
     attr_set[dev] = true;
   }
   MmMaps maps;
+  memset(&maps.o, 0, sizeof(maps.o));
   // fp16 and bf16 are both 2-byte types for the copy engine; the MMA descriptor carries the real format
   int rc = EncodeMmOperand(&maps.a, p.a_ptr, MmInnerA(p), MmPitchA(p), MmRowsA(p), p.a_batches, p.a_mmajor ? 64 : BM);
   if (rc != 0) return rc;
   rc = EncodeMmOperand(&maps.b, p.b_ptr, MmInnerB(p), MmPitchB(p), MmRowsB(p), p.b_batches, p.b_kmajor ? BN / 2 : 64);
   if (rc != 0) return rc;
+  p.tma_out = p.epi_mode >= EPI_STORE && EncodeMmResult(&maps.o, p) ? 1u : 0u;
   const uint32_t tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.batch0 * p.batch1;
   const uint32_t units = tiles < static_cast<uint32_t>(sms / 2) ? tiles : static_cast<uint32_t>(sms / 2);
   cudaLaunchConfig_t cfg = {};

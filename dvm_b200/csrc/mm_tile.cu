@@ -317,47 +317,44 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
   constexpr uint32_t kSpr = BN / 16;   // strips per row
   const uint32_t strips = rows * kSpr;
   const uint32_t i_begin = strips * rank / S, i_end = strips * (rank + 1) / S;
-  uint32_t slot = 0xffffffffu;
-  for (uint32_t i = i_begin + threadIdx.x; i < i_end; i += kThreads) {
-    const uint32_t row = i / kSpr, strip = i - row * kSpr;
-    EpiPos pos;
-    pos.b0 = b0;
-    pos.b1 = b1;
-    pos.row = row0 + row;
-    pos.col = col0 + strip * 16u;
-    if (pos.col >= P.N) continue;
-    pos.valid = min(16u, P.N - pos.col);
-    const uint32_t at = ring + row * kPitch + strip * 64u;
-    float v[16];
-    for (uint32_t p = 0; p < S; ++p) {
-      const uint32_t from = map_to_cta(at, p);
+  with_mode(P, [&](auto mode) {
+    for (uint32_t i = i_begin + threadIdx.x; i < i_end; i += kThreads) {
+      const uint32_t row = i / kSpr, strip = i - row * kSpr;
+      EpiPos pos;
+      pos.b0 = b0;
+      pos.b1 = b1;
+      pos.row = row0 + row;
+      pos.col = col0 + strip * 16u;
+      if (pos.col >= P.N) continue;
+      pos.valid = min(16u, P.N - pos.col);
+      const uint32_t at = ring + row * kPitch + strip * 64u;
+      float v[16];
+      for (uint32_t p = 0; p < S; ++p) {
+        const uint32_t from = map_to_cta(at, p);
 #pragma unroll
-      for (uint32_t g = 0; g < 4; ++g) {
-        const float4 q = ld_cluster_v4(from + 16u * g);
-        v[4 * g + 0] = p == 0 ? q.x : v[4 * g + 0] + q.x;
-        v[4 * g + 1] = p == 0 ? q.y : v[4 * g + 1] + q.y;
-        v[4 * g + 2] = p == 0 ? q.z : v[4 * g + 2] + q.z;
-        v[4 * g + 3] = p == 0 ? q.w : v[4 * g + 3] + q.w;
+        for (uint32_t g = 0; g < 4; ++g) {
+          const float4 q = ld_cluster_v4(from + 16u * g);
+          v[4 * g + 0] = p == 0 ? q.x : v[4 * g + 0] + q.x;
+          v[4 * g + 1] = p == 0 ? q.y : v[4 * g + 1] + q.y;
+          v[4 * g + 2] = p == 0 ? q.z : v[4 * g + 2] + q.z;
+          v[4 * g + 3] = p == 0 ? q.w : v[4 * g + 3] + q.w;
+        }
+      }
+      uint32_t r[16], pk[8];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) r[j] = f2u(v[j]);
+      if (P.bias_ptr != 0) add_bias_staged(base + kBiasOff + strip * 64u, r);
+      finish_strip<decltype(mode)::mode, decltype(mode)::dtype>(P, pos, r, pk);
+      if (decltype(mode)::mode != EPI_PROGRAM) {
+        const uint32_t dst = ring + A.out_off + (i - i_begin) * 32u;
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 16u), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
       }
     }
-    uint32_t r[16], pk[8];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) r[j] = f2u(v[j]);
-    if (P.bias_ptr != 0) add_bias_staged(base + kBiasOff + strip * 64u, r);
-    if (finish_strip(P, pos, r, pk) != 0xffffffffu) {
-      const uint32_t dst = ring + A.out_off + (i - i_begin) * 32u;
-      asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
-      asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 16u), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
-    }
-  }
-  if (P.gate_slot != 0xffffffffu) {
-    slot = P.gate_slot;
-  } else if (P.fast_store_slot != 0xffffffffu && P.tensor[P.fast_store_slot].dtype == P.in_dtype) {
-    slot = P.fast_store_slot;
-  }
-  if (slot != 0xffffffffu) {
+  });
+  if (P.epi_mode >= EPI_STORE) {
     __syncthreads();
-    const EpiTensor &t = P.tensor[slot];
+    const EpiTensor &t = P.tensor[P.out_slot];
     unsigned short *out = reinterpret_cast<unsigned short *>(t.ptr) + ((int64_t)b0 * t.sb0 + (int64_t)b1 * t.sb1);
     const uint8_t *staged = smem + kHeader + A.out_off;
     const bool vec = (reinterpret_cast<uint64_t>(out) & 15u) == 0 && (t.sm & 7) == 0;
