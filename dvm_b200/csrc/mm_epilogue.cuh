@@ -255,12 +255,7 @@ __device__ __forceinline__ uint64_t add_pair(uint64_t a, uint64_t b) {
 __device__ __forceinline__ float bias_at(const MmParam &P, uint32_t col) {
   return P.bias_ptr != 0 && col < P.N ? load_bias(P, col) : 0.0f;
 }
-// The same in two steps: the stored bits (a load in flight), their value.
-__device__ __forceinline__ uint32_t bias_bits(const MmParam &P, uint32_t col) {
-  if (col >= P.N) return 0;
-  return P.bias_dtype == T_F32 ? __ldg(reinterpret_cast<const uint32_t *>(P.bias_ptr) + col)
-                               : __ldg(reinterpret_cast<const unsigned short *>(P.bias_ptr) + col);
-}
+// Value of a bias loaded as its stored bits.
 __device__ __forceinline__ float bias_value(const MmParam &P, uint32_t bits) {
   return u2f(P.bias_dtype == T_F32 ? bits : widen(P.bias_dtype, (unsigned short)bits));
 }

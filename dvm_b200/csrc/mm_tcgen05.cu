@@ -228,8 +228,15 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
     auto look_up = [&](uint32_t t) {
       tile_coords(t, mblocks, nblocks, P.group_m, bz, mb, nb);
       if (P.bias_ptr == 0) return;
+      // (columns past the last one are not stored: any bias will do.  No value is selected or converted here, that would wait)
+      const uint32_t col = nb * BN + col0 + lane;
+      if (P.bias_dtype == T_F32) {
 #pragma unroll
-      for (uint32_t i = 0; i < kEpiCols / 32; ++i) bias[i] = bias_bits(P, nb * BN + col0 + i * 32 + lane);
+        for (uint32_t i = 0; i < kEpiCols / 32; ++i) bias[i] = __ldg(reinterpret_cast<const uint32_t *>(P.bias_ptr) + min(col + i * 32, P.N - 1));
+      } else {
+#pragma unroll
+        for (uint32_t i = 0; i < kEpiCols / 32; ++i) bias[i] = __ldg(reinterpret_cast<const unsigned short *>(P.bias_ptr) + min(col + i * 32, P.N - 1));
+      }
     };
     if (unit < num_tiles) look_up(unit);
     with_mode(P, [&](auto mode) {
@@ -253,56 +260,58 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
         mbar_wait(bar_tfull + 8 * acc, acc_parity, 4, &g_mm_status, epoch);
         tcgen05_after_sync();
         const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * BN + col0;
-        // (one strip per trip and no unrolling: eight copies of the strip code did not fit the instruction cache and made
-        // the epilogue of a CTA's first tile 4 us longer)
-        uint32_t next[16];
-        tmem_ld_32x32b_x16_nowait(taddr, next);
+        // (two strips per trip and no more: eight copies of the strip code did not fit the instruction cache and made the
+        // epilogue of a CTA's first tile 4 us longer)
+        uint32_t next[32];
+        tmem_ld_32x32b_x32_nowait(taddr, next);
 #pragma unroll 1
-        for (uint32_t c = 0; c < kEpiCols; c += 16) {
-          uint32_t r[16], pk[8];
-          tmem_ld_wait16(next);
+        for (uint32_t c = 0; c < kEpiCols; c += 32) {
+          uint32_t cur[32];
+          tmem_ld_wait32(next);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) r[i] = next[i];
-          if (c + 16 < kEpiCols) tmem_ld_32x32b_x16_nowait(taddr + c + 16, next);   // on its way while this strip is worked on
-          pos.col = first_col + c;
-          if (pos.col < P.N) {   // (rows past the matrix take part: their results are not copied out)
-            pos.valid = pos.row < P.M ? min(16u, P.N - pos.col) : 0u;
-            if (P.bias_ptr != 0) add_bias_staged(bias_saddr + c * 4u, r);
-            finish_strip<MODE, DT>(P, pos, r, pk);
+          for (int i = 0; i < 32; ++i) cur[i] = next[i];
+          if (c + 32 < kEpiCols) tmem_ld_32x32b_x32_nowait(taddr + c + 32, next);   // on its way while these are worked on
+          // buffers of 32 columns in turn: rows of 64 bytes, 16-byte piece p of row r at p ^ (r / 2 & 3)
+          const uint32_t buf = out_saddr + ((c >> 5) & 1u) * (kOutBytes / 2);
+          if (tma) {
+            if (elect_one()) tma_store_wait_read<1>();   // the store before the last one has read this buffer
+            __syncwarp();
+          }
+#pragma unroll
+          for (uint32_t h = 0; h < 2; ++h) {
+            uint32_t r[16], pk[8];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) r[i] = cur[16 * h + i];
+            pos.col = first_col + c + 16 * h;
+            if (pos.col < P.N) {   // (rows past the matrix take part: their results are not copied out)
+              pos.valid = pos.row < P.M ? min(16u, P.N - pos.col) : 0u;
+              if (P.bias_ptr != 0) add_bias_staged(bias_saddr + (c + 16 * h) * 4u, r);
+              finish_strip<MODE, DT>(P, pos, r, pk);
+            }
+            if (!kStaged) continue;
+            // without TMA: rows of 128 bytes, piece p at p ^ (r & 7)
+            const uint32_t piece = ((c >> 3) & 7u) + 2 * h;
+            const uint32_t row_saddr = tma ? buf + lane * 64u : out_saddr + lane * 128u;
+            const uint32_t at = tma ? 2 * h : piece, turn = tma ? (lane >> 1) & 3u : lane & 7u;
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + ((at ^ turn) << 4)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + (((at + 1u) ^ turn) << 4)), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
           }
           if (!kStaged) continue;
           if (tma) {
-            // two buffers of 32 columns: rows of 64 bytes, 16-byte piece p of row r at p ^ (r / 2 & 3)
-            const uint32_t buf = out_saddr + ((c >> 5) & 1u) * (kOutBytes / 2), row_saddr = buf + lane * 64u, at = (c >> 3) & 2u;
-            if ((c & 16u) == 0) {
-              if (lane == 0) tma_store_wait_read<1>();   // the store before the last one has read this buffer
-              __syncwarp();
+            fence_async_shared();
+            __syncwarp();
+            if (elect_one()) {   // (the same lane each time: the copy engine's groups belong to a thread)
+              if (first_col + c < P.N && first_row < P.M)   // (the tensor map cuts off what lies past the matrix)
+                tma_store_4d(&maps.o, buf, (int)(first_col + c), (int)first_row, (int)pos.b1, (int)pos.b0);
+              tma_store_commit();
             }
-            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + ((at ^ ((lane >> 1) & 3u)) << 4)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
-            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + (((at + 1u) ^ ((lane >> 1) & 3u)) << 4)), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
-            if ((c & 16u) != 0) {
-              fence_async_shared();
-              __syncwarp();
-              if (lane == 0) {
-                const uint32_t box_col = first_col + (c & ~31u);
-                if (box_col < P.N && first_row < P.M)   // (the tensor map cuts off what lies past the matrix)
-                  tma_store_4d(&maps.o, buf, (int)box_col, (int)first_row, (int)pos.b1, (int)pos.b0);
-                tma_store_commit();
-              }
-            }
-          } else {
-            // row `lane`, 16-byte pieces 2 (c / 16 % 4) and the next, each at piece ^ (row & 7)
-            const uint32_t piece = (c >> 3) & 7u, row_saddr = out_saddr + lane * 128u;
-            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + ((piece ^ (lane & 7u)) << 4)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
-            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + (((piece + 1u) ^ (lane & 7u)) << 4)), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
-            if ((c & 48u) == 48u) {
-              __syncwarp();
-              copy_out(P, pos.b0, pos.b1, first_row, first_col + (c & ~63u), out_saddr, lane);
-              __syncwarp();
-            }
+            __syncwarp();
+          } else if ((c & 32u) != 0) {
+            __syncwarp();
+            copy_out(P, pos.b0, pos.b1, first_row, first_col + (c & ~63u), out_saddr, lane);
+            __syncwarp();
           }
         }
-        tmem_ld_wait16(next);
         tcgen05_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(map_to_cta(bar_tempty + 8 * acc, 0));
@@ -312,7 +321,7 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
         }
       }
     });
-    if (lane == 0) tma_store_wait_read<0>();   // shared memory stays until the last store has read it
+    if (elect_one()) tma_store_wait_read<0>();   // shared memory stays until the last store has read it
   }
   __syncwarp();
   tcgen05_before_sync();
