@@ -5,6 +5,7 @@
 #define DVM_B200_MM_EPILOGUE_CUH_
 
 #include "mm_launch.h"
+#include "sm100_sync.cuh"
 #include "vm_ops.cuh"
 
 namespace dvmb {
@@ -379,36 +380,37 @@ template <uint32_t MODE, uint32_t DT>
 __device__ __forceinline__ void finish_strip(const MmParam &P, const EpiPos &pos, uint32_t (&r)[16], uint32_t (&pk)[8]) {
   const uint32_t dt = DT == kAnyType ? P.in_dtype : DT;
   pack_strip(dt, r, pk);   // the product in the operand type
-  if (MODE == EPI_STORE) return;
-  // back to the 32-bit register form of the rounded product
+  if constexpr (MODE != EPI_STORE) {
+    // back to the 32-bit register form of the rounded product
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (dt == T_BF16) {
-      r[2 * i] = pk[i] << 16;
-      r[2 * i + 1] = pk[i] & 0xffff0000u;
+    for (int i = 0; i < 8; ++i) {
+      if (dt == T_BF16) {
+        r[2 * i] = pk[i] << 16;
+        r[2 * i + 1] = pk[i] & 0xffff0000u;
+      } else {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&pk[i]));
+        r[2 * i] = __float_as_uint(f.x);
+        r[2 * i + 1] = __float_as_uint(f.y);
+      }
+    }
+    if constexpr (MODE == EPI_GATE) {
+      gate_strip(P.gate_c, r);
+      pack_strip(dt, r, pk);
     } else {
-      const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&pk[i]));
-      r[2 * i] = __float_as_uint(f.x);
-      r[2 * i + 1] = __float_as_uint(f.y);
-    }
-  }
-  if (MODE == EPI_GATE) {
-    gate_strip(P.gate_c, r);
-    pack_strip(dt, r, pk);
-    return;
-  }
-  if (pos.valid == 0) return;
-  if (P.epi_mode == EPI_WIDEN && pos.valid == 16u) {
-    const EpiTensor &t = P.tensor[P.out_slot];
-    uint8_t *dst = reinterpret_cast<uint8_t *>(t.ptr) + (epi_offset(t, pos) << 2);
-    if ((reinterpret_cast<uint64_t>(dst) & 15u) == 0) {
+      if (pos.valid == 0) return;
+      if (P.epi_mode == EPI_WIDEN && pos.valid == 16u) {
+        const EpiTensor &t = P.tensor[P.out_slot];
+        uint8_t *dst = reinterpret_cast<uint8_t *>(t.ptr) + (epi_offset(t, pos) << 2);
+        if ((reinterpret_cast<uint64_t>(dst) & 15u) == 0) {
 #pragma unroll
-      for (int g = 0; g < 4; ++g)
-        *reinterpret_cast<uint4 *>(dst + 16 * g) = make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
-      return;
+          for (int g = 0; g < 4; ++g)
+            *reinterpret_cast<uint4 *>(dst + 16 * g) = make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+          return;
+        }
+      }
+      run_epilogue(P, pos, r);
     }
   }
-  run_epilogue(P, pos, r);
 }
 
 template <uint32_t M, uint32_t D>
@@ -425,6 +427,106 @@ __device__ __forceinline__ void with_mode(const MmParam &P, F f) {
     if (bf) f(Mode<EPI_GATE, T_BF16>()); else f(Mode<EPI_GATE, T_F16>());
   } else {
     f(Mode<EPI_PROGRAM, kAnyType>());
+  }
+}
+
+// ---- TMEM -> result, by the warp that owns 32 rows of COLS columns --------------------------------------------------
+// Staged modes go through shared memory: two buffers of 32 columns in turn for the copy engine, or 64 (32) columns for stores
+// by the lanes, when it cannot address the result.
+template <uint32_t COLS>
+constexpr uint32_t kDrainBytes = COLS >= 64 ? 4096u : 2048u;
+
+// 32 rows of RUN staged columns, 16-byte piece p of row r at p ^ (r & 7) (64 columns) or p ^ (r / 2 & 3) (32 columns).
+template <uint32_t RUN>
+__device__ __forceinline__ void copy_out(const MmParam &P, uint32_t b0, uint32_t b1, uint32_t row0, uint32_t col0, uint32_t saddr,
+                                         uint32_t lane) {
+  const EpiTensor &t = P.tensor[P.out_slot];
+  unsigned short *const out = reinterpret_cast<unsigned short *>(t.ptr) + ((int64_t)b0 * t.sb0 + (int64_t)b1 * t.sb1 + (int64_t)row0 * t.sm + col0);
+  constexpr uint32_t kUnits = RUN / 8 - 1;
+  auto at_piece = [&](uint32_t row, uint32_t piece) {
+    return saddr + row * (RUN * 2u) + ((piece ^ (RUN == 64 ? row & 7u : (row >> 1) & 3u)) << 4);
+  };
+#pragma unroll 1
+  for (uint32_t j = lane; j < 32u * kUnits; j += 32u) {
+    const uint32_t row = j / kUnits, u = j - kUnits * row;
+    unsigned short *const dst = out + (int64_t)row * t.sm;
+    const uint32_t ahead = elements_ahead(dst), at = ahead + 8u * u, piece = at >> 3;   // (at + 8 <= RUN)
+    if (row0 + row >= P.M || col0 + at >= P.N) continue;
+    uint4 lo, hi;
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w) : "r"(at_piece(row, piece)));
+    hi = lo;
+    if ((ahead & 7u) != 0)
+      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w) : "r"(at_piece(row, piece + 1u)));
+    store_unit(dst + at, shift_in(lo, hi, ahead & 7u), P.N - (col0 + at));
+  }
+#pragma unroll 1
+  for (uint32_t j = lane; j < 256u; j += 32u) {
+    const uint32_t row = j >> 3;
+    unsigned short *const dst = out + (int64_t)row * t.sm;
+    const uint32_t col = single_at(j & 7u, elements_ahead(dst), RUN);
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(at_piece(row, col >> 3) + (col & 7u) * 2u));
+    if (row0 + row < P.M && col0 + col < P.N) dst[col] = v;
+  }
+}
+
+// `taddr`: the accumulator's first column, lanes of this warp; `empty`: no contraction took place, the product is zero.
+// pos.b0 and pos.b1 are set.  (Two strips of 16 columns per trip and no more: eight copies of the strip code did not fit the
+// instruction cache and made the first tile of a CTA 4 us longer.)
+template <uint32_t MODE, uint32_t DT, uint32_t COLS>
+__device__ __forceinline__ void drain(const MmParam &P, const CUtensorMap &out_map, uint32_t taddr, bool empty, EpiPos &pos,
+                                      uint32_t first_row, uint32_t first_col, uint32_t bias_saddr, uint32_t out_saddr, uint32_t lane) {
+  constexpr bool kStaged = MODE != EPI_PROGRAM;
+  constexpr uint32_t kRun = COLS >= 64 ? 64u : 32u;   // columns that copy_out takes at a time
+  const bool tma = kStaged && P.tma_out != 0;
+  pos.row = first_row + lane;
+  uint32_t next[32];
+  tmem_ld_32x32b_x32_nowait(taddr, next);
+#pragma unroll 1
+  for (uint32_t c = 0; c < COLS; c += 32) {
+    uint32_t cur[32];
+    tmem_ld_wait32(next);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) cur[i] = empty ? 0u : next[i];
+    if (c + 32 < COLS) tmem_ld_32x32b_x32_nowait(taddr + c + 32, next);   // on its way while these are worked on
+    const uint32_t buf = out_saddr + (COLS >= 64 ? (c >> 5) & 1u : 0u) * 2048u;
+    if (tma) {
+      if (elect_one()) tma_store_wait_read<COLS >= 64 ? 1 : 0>();   // the last store that used this buffer has read it
+      __syncwarp();
+    }
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+      uint32_t r[16], pk[8];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) r[i] = cur[16 * h + i];
+      pos.col = first_col + c + 16 * h;
+      if (pos.col < P.N) {   // (rows past the matrix take part: their results are not copied out)
+        pos.valid = pos.row < P.M ? min(16u, P.N - pos.col) : 0u;
+        if (P.bias_ptr != 0) add_bias_staged(bias_saddr + (c + 16 * h) * 4u, r);
+        finish_strip<MODE, DT>(P, pos, r, pk);
+      }
+      if (!kStaged) continue;
+      const bool narrow = tma || kRun == 32;   // rows of 64 bytes
+      const uint32_t row_saddr = narrow ? buf + lane * 64u : out_saddr + lane * 128u;
+      const uint32_t at = narrow ? 2 * h : ((c >> 3) & 7u) + 2 * h, turn = narrow ? (lane >> 1) & 3u : lane & 7u;
+      asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + ((at ^ turn) << 4)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+      asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + (((at + 1u) ^ turn) << 4)), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
+    }
+    if (!kStaged) continue;
+    if (tma) {
+      fence_async_shared();
+      __syncwarp();
+      if (elect_one()) {   // (the same lane each time: the copy engine's groups belong to a thread)
+        if (first_col + c < P.N && first_row < P.M)   // (the tensor map cuts off what lies past the matrix)
+          tma_store_4d(&out_map, buf, (int)(first_col + c), (int)first_row, (int)pos.b1, (int)pos.b0);
+        tma_store_commit();
+      }
+      __syncwarp();
+    } else if (kRun == 32 || (c & 32u) != 0) {
+      __syncwarp();
+      copy_out<kRun>(P, pos.b0, pos.b1, first_row, first_col + (c & ~(kRun - 1u)), out_saddr, lane);
+      __syncwarp();
+    }
   }
 }
 

@@ -87,6 +87,9 @@ inline bool MmNeedsGather(const MmParam &p) { return MmGatherA(p) || MmGatherB(p
 void MmPackBytes(const MmParam &p, uint64_t *a_bytes, uint64_t *b_bytes);
 // Copies the operands that the copy engine cannot address into a_pack / b_pack, and makes `p` read them there.
 int LaunchMmPack(MmParam *p, void *stream);
+// Tensor map over the result of a staged mode (EPI_STORE, EPI_GATE): boxes of 32 x 32, 64-byte swizzle; false if the copy
+// engine cannot address it.
+bool EncodeMmResult(CUtensorMap *map, const MmParam &p);
 // The tile kernel (mm_tile.cu): 128 x bn tiles (bn 64 or 128), K cut into `split` (1, 2, 4, 8) parts.
 int LaunchMmTile(const MmParam &p, uint32_t bn, uint32_t split, void *stream);
 unsigned int ReadMmTileStatus();

@@ -58,43 +58,13 @@ constexpr uint32_t kStages = 5;
 // Results of 64 columns at a time, per epilogue warp: 32 rows of 128 bytes.  Stored from the registers of the thread that owns
 // the row, every 16-byte store was a write request of its own, and a tile's epilogue took 14 600 cycles against 5 100 for
 // ten k-blocks of MMAs; worth more than the sixth operand stage that the 32 KB would hold.
-constexpr uint32_t kOutBytes = 32 * 128;
+constexpr uint32_t kOutBytes = kDrainBytes<kEpiCols>;
 constexpr uint32_t kSmemBytes = kSmemHeader + kStages * kStageBytes + kEpiWarps * kOutBytes + 1024;
 
 struct MmMaps {
   CUtensorMap a, b;
   CUtensorMap o;   // the result, boxes of 32 rows of 32 columns, 64-byte swizzle (P.tma_out)
 };
-
-// 32 rows of 64 staged columns (128 bytes, 16-byte piece p of row r at p ^ (r & 7)) to a result tensor that the copy engine
-// cannot address.
-__device__ __forceinline__ void copy_out(const MmParam &P, uint32_t b0, uint32_t b1, uint32_t row0, uint32_t col0, uint32_t saddr,
-                                         uint32_t lane) {
-  const EpiTensor &t = P.tensor[P.out_slot];
-  unsigned short *const out = reinterpret_cast<unsigned short *>(t.ptr) + ((int64_t)b0 * t.sb0 + (int64_t)b1 * t.sb1 + (int64_t)row0 * t.sm + col0);
-#pragma unroll 1
-  for (uint32_t j = lane; j < 32u * 7u; j += 32u) {
-    const uint32_t row = j / 7u, u = j - 7u * row;
-    unsigned short *const dst = out + (int64_t)row * t.sm;
-    const uint32_t ahead = elements_ahead(dst), at = ahead + 8u * u, piece = at >> 3;   // (at + 8 <= 64)
-    if (row0 + row >= P.M || col0 + at >= P.N) continue;
-    uint4 lo, hi;
-    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w) : "r"(saddr + row * 128u + ((piece ^ (row & 7u)) << 4)));
-    hi = lo;
-    if ((ahead & 7u) != 0)
-      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w) : "r"(saddr + row * 128u + (((piece + 1u) ^ (row & 7u)) << 4)));
-    store_unit(dst + at, shift_in(lo, hi, ahead & 7u), P.N - (col0 + at));
-  }
-#pragma unroll 1
-  for (uint32_t j = lane; j < 256u; j += 32u) {
-    const uint32_t row = j >> 3;
-    unsigned short *const dst = out + (int64_t)row * t.sm;
-    const uint32_t col = single_at(j & 7u, elements_ahead(dst), 64u);
-    unsigned short v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(saddr + row * 128u + (((col >> 3) ^ (row & 7u)) << 4) + (col & 7u) * 2u));
-    if (row0 + row < P.M && col0 + col < P.N) dst[col] = v;
-  }
-}
 
 __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, const LaunchTag epoch) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -241,8 +211,6 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
     if (unit < num_tiles) look_up(unit);
     with_mode(P, [&](auto mode) {
       constexpr uint32_t MODE = decltype(mode)::mode, DT = decltype(mode)::dtype;
-      constexpr bool kStaged = MODE != EPI_PROGRAM;
-      const bool tma = kStaged && P.tma_out != 0;
       for (uint32_t t = unit; t < num_tiles; t += num_units) {
         if (P.bias_ptr != 0) {
           __syncwarp();   // (the warp has read the previous tile's)
@@ -260,58 +228,7 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
         mbar_wait(bar_tfull + 8 * acc, acc_parity, 4, &g_mm_status, epoch);
         tcgen05_after_sync();
         const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * BN + col0;
-        // (two strips per trip and no more: eight copies of the strip code did not fit the instruction cache and made the
-        // epilogue of a CTA's first tile 4 us longer)
-        uint32_t next[32];
-        tmem_ld_32x32b_x32_nowait(taddr, next);
-#pragma unroll 1
-        for (uint32_t c = 0; c < kEpiCols; c += 32) {
-          uint32_t cur[32];
-          tmem_ld_wait32(next);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) cur[i] = next[i];
-          if (c + 32 < kEpiCols) tmem_ld_32x32b_x32_nowait(taddr + c + 32, next);   // on its way while these are worked on
-          // buffers of 32 columns in turn: rows of 64 bytes, 16-byte piece p of row r at p ^ (r / 2 & 3)
-          const uint32_t buf = out_saddr + ((c >> 5) & 1u) * (kOutBytes / 2);
-          if (tma) {
-            if (elect_one()) tma_store_wait_read<1>();   // the store before the last one has read this buffer
-            __syncwarp();
-          }
-#pragma unroll
-          for (uint32_t h = 0; h < 2; ++h) {
-            uint32_t r[16], pk[8];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) r[i] = cur[16 * h + i];
-            pos.col = first_col + c + 16 * h;
-            if (pos.col < P.N) {   // (rows past the matrix take part: their results are not copied out)
-              pos.valid = pos.row < P.M ? min(16u, P.N - pos.col) : 0u;
-              if (P.bias_ptr != 0) add_bias_staged(bias_saddr + (c + 16 * h) * 4u, r);
-              finish_strip<MODE, DT>(P, pos, r, pk);
-            }
-            if (!kStaged) continue;
-            // without TMA: rows of 128 bytes, piece p at p ^ (r & 7)
-            const uint32_t piece = ((c >> 3) & 7u) + 2 * h;
-            const uint32_t row_saddr = tma ? buf + lane * 64u : out_saddr + lane * 128u;
-            const uint32_t at = tma ? 2 * h : piece, turn = tma ? (lane >> 1) & 3u : lane & 7u;
-            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + ((at ^ turn) << 4)), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
-            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(row_saddr + (((at + 1u) ^ turn) << 4)), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]) : "memory");
-          }
-          if (!kStaged) continue;
-          if (tma) {
-            fence_async_shared();
-            __syncwarp();
-            if (elect_one()) {   // (the same lane each time: the copy engine's groups belong to a thread)
-              if (first_col + c < P.N && first_row < P.M)   // (the tensor map cuts off what lies past the matrix)
-                tma_store_4d(&maps.o, buf, (int)(first_col + c), (int)first_row, (int)pos.b1, (int)pos.b0);
-              tma_store_commit();
-            }
-            __syncwarp();
-          } else if ((c & 32u) != 0) {
-            __syncwarp();
-            copy_out(P, pos.b0, pos.b1, first_row, first_col + (c & ~63u), out_saddr, lane);
-            __syncwarp();
-          }
-        }
+        drain<MODE, DT, kEpiCols>(P, maps.o, taddr, false, pos, first_row, first_col, bias_saddr, out_saddr, lane);
         tcgen05_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(map_to_cta(bar_tempty + 8 * acc, 0));
@@ -357,7 +274,7 @@ PFN_cuTensorMapEncodeTiled GetEncode() {
 
 // 3-d map over a [batches, rows, inner] row-major operand: box = [1, box_rows, 64 elements], 128-byte swizzle
 // The result as [batch0, batch1, M, N] for the copy engine, if it can address it.
-static bool EncodeMmResult(CUtensorMap *map, const MmParam &p) {
+bool EncodeMmResult(CUtensorMap *map, const MmParam &p) {
   const EpiTensor &t = p.tensor[p.out_slot];
   auto encode = GetEncode();
   const int64_t row = t.sm * 2, b1 = p.batch1 > 1 ? t.sb1 * 2 : row * p.M, b0 = p.batch0 > 1 ? t.sb0 * 2 : b1 * p.batch1;

@@ -8,7 +8,8 @@
 //   warps 2-9  loaders of an operand the copy engine cannot address (16-byte loads from the aligned address below, shifted
 //              into place in registers, written to shared memory in the 128-byte swizzled layout TMA would have written);
 //              then TMEM -> shared memory
-//   all warps  sum over the cluster, bias, rounding, post-fusion program; 16-bit results leave through shared memory
+//   all warps  sum over the cluster, bias, rounding, post-fusion program; 16-bit results leave through shared memory (a CTA that
+//              has its tile to itself drains TMEM by warps 2-9 instead, without the exchange)
 //
 // What bounds it: a [16, 8192] x [8192, 8192] product is the read of the weight (134 MB, 21 us at the measured copy
 // bandwidth).  In 128 x 256 tiles that was 32 CTAs on 148 SMs; in tiles of 64 columns with K cut in two it is 256 CTAs
@@ -44,6 +45,7 @@ constexpr uint32_t kBarFull = 0, kBarEmpty = 128, kBarDone = 256, kTmemSlot = 26
 
 struct TileMaps {
   CUtensorMap a, b;
+  CUtensorMap o;   // the result (P.tma_out)
 };
 
 struct TileArgs {
@@ -271,26 +273,52 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
   }
   __syncwarp();
 
-  // ---- the partial product: TMEM -> shared memory (the stages are free: every MMA has completed) ----
-  constexpr uint32_t kPitch = BN * 4 + 16;   // bytes per row; the 16 keep rows off each other's banks
+  // ---- the product of a CTA alone: TMEM -> result ----
   const uint32_t rows = min(BM, P.M - row0);
+  if (S == 1) {
+    if (warp >= 2) {
+      const uint32_t wt = threadIdx.x - 64u;
+      if (wt < BN && P.bias_ptr != 0) reinterpret_cast<float *>(smem + kBiasOff)[wt] = bias_at(P, col0 + wt);
+      asm volatile("bar.sync 1, %0;" ::"n"(kWorkThreads) : "memory");
+      if (kblocks != 0) mbar_wait(base + kBarDone, 0, 4, &g_mm_tile_status, epoch);
+      tcgen05_after_sync();
+      const uint32_t quarter = warp & 3u, half = (warp - 2) >> 2;
+      if (quarter * 32u < rows) {
+        EpiPos pos;
+        pos.b0 = b0;
+        pos.b1 = b1;
+        with_mode(P, [&](auto mode) {
+          drain<decltype(mode)::mode, decltype(mode)::dtype, BN / 2>(
+            P, maps.o, tmem_base + ((quarter * 32u) << 16) + half * (BN / 2), kblocks == 0, pos, row0 + quarter * 32u, col0 + half * (BN / 2),
+            base + kBiasOff + half * (BN / 2) * 4u, ring + (warp - 2) * kDrainBytes<BN / 2>, lane);   // (the stages are free)
+        });
+        if (elect_one()) tma_store_wait_read<0>();   // shared memory stays until the last store has read it
+      }
+    }
+    __syncwarp();
+    tcgen05_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+      tcgen05_after_sync();
+      tmem_dealloc(tmem_base, BN);
+    }
+    return;
+  }
+
+  // ---- a partial product: TMEM -> shared memory (the stages are free: every MMA has completed) ----
+  constexpr uint32_t kPitch = BN * 4 + 16;   // bytes per row; the 16 keep rows off each other's banks
   if (warp >= 2) {
     const uint32_t wt = threadIdx.x - 64u;
     if (wt < BN && P.bias_ptr != 0) reinterpret_cast<float *>(smem + kBiasOff)[wt] = bias_at(P, col0 + wt);
-    if (kblocks != 0) mbar_wait(base + kBarDone, 0, 4, &g_mm_tile_status, epoch);
+    mbar_wait(base + kBarDone, 0, 4, &g_mm_tile_status, epoch);
     tcgen05_after_sync();
     const uint32_t quarter = warp & 3u, half = (warp - 2) >> 2;
     if (quarter * 32u < rows) {
       const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + half * (BN / 2);
       uint32_t r[BN / 2];
-      if (kblocks != 0) {
 #pragma unroll
-        for (uint32_t c = 0; c < BN / 2; c += 32) tmem_ld_32x32b_x32_nowait(taddr + c, &r[c]);
-        tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (uint32_t c = 0; c < BN / 2; ++c) r[c] = 0;   // an empty contraction
-      }
+      for (uint32_t c = 0; c < BN / 2; c += 32) tmem_ld_32x32b_x32_nowait(taddr + c, &r[c]);
+      tmem_ld_wait();
       const uint32_t row = quarter * 32u + lane;
       const uint32_t dst = ring + row * kPitch + half * (BN / 2) * 4u;
       if (row < rows) {   // (the buffer holds the rows the matrix has)
@@ -303,11 +331,7 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
   }
   __syncwarp();
   tcgen05_before_sync();
-  if (S > 1) {
-    cluster_sync_all();
-  } else {
-    __syncthreads();
-  }
+  cluster_sync_all();
   if (warp == 1) {
     tcgen05_after_sync();
     tmem_dealloc(tmem_base, BN);
@@ -317,6 +341,35 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
   constexpr uint32_t kSpr = BN / 16;   // strips per row
   const uint32_t strips = rows * kSpr;
   const uint32_t i_begin = strips * rank / S, i_end = strips * (rank + 1) / S;
+  // The sum first, 16 bytes per lane and side by side: taken strip by strip, 64 bytes apart, the remote reads were 12 us of
+  // the 37 us of a [128, 8192] x [8192, 8192] product.  It replaces this CTA's own partial (its share is read by no one else),
+  // the four pieces of a strip at p ^ (strip / 2 & 3) so that the strips' readers below do not meet on a bank.
+  for (uint32_t u0 = i_begin * 4u; u0 < i_end * 4u; u0 += 2u * kThreads) {
+    float4 v[2];
+    uint32_t to[2];
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+      const uint32_t u = u0 + h * kThreads + threadIdx.x, row = u / (BN / 4), piece = u - row * (BN / 4);
+      to[h] = 0;
+      if (u < i_end * 4u) {
+        const uint32_t at = ring + row * kPitch;
+        to[h] = at + ((piece & ~3u) + ((piece & 3u) ^ ((piece >> 3) & 3u))) * 16u;
+        v[h] = ld_cluster_v4(map_to_cta(at + piece * 16u, 0));
+        for (uint32_t p = 1; p < S; ++p) {
+          const float4 q = ld_cluster_v4(map_to_cta(at + piece * 16u, p));
+          v[h].x += q.x;
+          v[h].y += q.y;
+          v[h].z += q.z;
+          v[h].w += q.w;
+        }
+      }
+    }
+    __syncwarp();   // (the pieces of a strip belong to lanes of one warp)
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h)
+      if (to[h] != 0) asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(to[h]), "f"(v[h].x), "f"(v[h].y), "f"(v[h].z), "f"(v[h].w) : "memory");
+  }
+  __syncthreads();
   with_mode(P, [&](auto mode) {
     for (uint32_t i = i_begin + threadIdx.x; i < i_end; i += kThreads) {
       const uint32_t row = i / kSpr, strip = i - row * kSpr;
@@ -328,21 +381,12 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
       if (pos.col >= P.N) continue;
       pos.valid = min(16u, P.N - pos.col);
       const uint32_t at = ring + row * kPitch + strip * 64u;
-      float v[16];
-      for (uint32_t p = 0; p < S; ++p) {
-        const uint32_t from = map_to_cta(at, p);
-#pragma unroll
-        for (uint32_t g = 0; g < 4; ++g) {
-          const float4 q = ld_cluster_v4(from + 16u * g);
-          v[4 * g + 0] = p == 0 ? q.x : v[4 * g + 0] + q.x;
-          v[4 * g + 1] = p == 0 ? q.y : v[4 * g + 1] + q.y;
-          v[4 * g + 2] = p == 0 ? q.z : v[4 * g + 2] + q.z;
-          v[4 * g + 3] = p == 0 ? q.w : v[4 * g + 3] + q.w;
-        }
-      }
       uint32_t r[16], pk[8];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) r[j] = f2u(v[j]);
+      for (uint32_t g = 0; g < 4; ++g)
+        asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[4 * g]), "=r"(r[4 * g + 1]), "=r"(r[4 * g + 2]), "=r"(r[4 * g + 3])
+                     : "r"(at + ((g ^ ((strip >> 1) & 3u)) << 4)));
       if (P.bias_ptr != 0) add_bias_staged(base + kBiasOff + strip * 64u, r);
       finish_strip<decltype(mode)::mode, decltype(mode)::dtype>(P, pos, r, pk);
       if (decltype(mode)::mode != EPI_PROGRAM) {
@@ -403,7 +447,7 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
     }
   }
   __syncwarp();
-  if (S > 1) cluster_sync_all();   // no CTA leaves while a peer may still read its partial product
+  cluster_sync_all();   // no CTA leaves while a peer may still read its partial product
 }
 
 }  // namespace
@@ -474,7 +518,8 @@ int LaunchMmPack(MmParam *p, void *stream) {
   return e != cudaSuccess ? static_cast<int>(e) : static_cast<int>(cudaGetLastError());
 }
 
-int LaunchMmTile(const MmParam &p, uint32_t bn, uint32_t split, void *stream) {
+int LaunchMmTile(const MmParam &p_in, uint32_t bn, uint32_t split, void *stream) {
+  MmParam p = p_in;
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -503,7 +548,8 @@ int LaunchMmTile(const MmParam &p, uint32_t bn, uint32_t split, void *stream) {
   if (p.M < BM) a.out_off = (p.M * (bn * 4u + 16u) + 127u) & ~127u;
   const uint32_t strips = m_rows * (bn / 16u), share = (strips + split - 1) / split + 1;
   const uint32_t ring_bytes = stages * a.stage_bytes + over, out_bytes = a.out_off + share * 32u;
-  const uint32_t smem = kHeader + 1024u + (ring_bytes > out_bytes ? ring_bytes : out_bytes);
+  const uint32_t drained = kWorkWarps * (bn == 64 ? kDrainBytes<32> : kDrainBytes<64>), after = split == 1 ? drained : out_bytes;
+  const uint32_t smem = kHeader + 1024u + (ring_bytes > after ? ring_bytes : after);
   if (smem > kBudget) return -5;
   TileMaps maps;
   memset(&maps, 0, sizeof(maps));
@@ -513,6 +559,7 @@ int LaunchMmTile(const MmParam &p, uint32_t bn, uint32_t split, void *stream) {
   if (rc == 0 && !a.gather_b && kblocks != 0)
     rc = EncodeMmOperand(&maps.b, p.b_ptr, MmInnerB(p), MmPitchB(p), MmRowsB(p), p.b_batches, p.b_kmajor ? bn : 64);
   if (rc != 0) return rc;
+  p.tma_out = split == 1 && p.epi_mode >= EPI_STORE && EncodeMmResult(&maps.o, p) ? 1u : 0u;
   const uint64_t tiles = static_cast<uint64_t>((p.M + BM - 1) / BM) * ((p.N + bn - 1) / bn) * p.batch0 * p.batch1;
   if (tiles * split >= (1ull << 31)) return -6;
   cudaLaunchConfig_t cfg;
