@@ -124,6 +124,49 @@ __device__ __forceinline__ uint32_t cluster_nctarank() {
   return r;
 }
 
+// Bytes per row of a partial product in shared memory; the 16 keep rows off each other's banks.
+template <uint32_t BN>
+constexpr uint32_t kPitch = BN * 4 + 16;
+
+// The partial products of strips [i_begin, i_end) of a cluster's tile, added in rank order: 16 bytes per lane and side by side,
+// every remote read of two rounds (one of eight CTAs) in flight before the first is used.  (Taken strip by strip, 64 bytes
+// apart, one after the other, they were 12 us of the 37 us of a [128, 8192] x [8192, 8192] product.)  The sum replaces this
+// CTA's own partial, which no one else reads, the four pieces of a strip at p ^ (strip / 2 & 3) so that the readers of
+// whole strips do not meet on a bank.
+template <uint32_t BN, uint32_t S>
+__device__ __forceinline__ void sum_partials(uint32_t ring, uint32_t i_begin, uint32_t i_end) {
+  constexpr uint32_t kRounds = S == 8 ? 1 : 2;
+  for (uint32_t u0 = i_begin * 4u; u0 < i_end * 4u; u0 += kRounds * kThreads) {
+    float4 v[kRounds][S];
+    uint32_t to[kRounds];
+#pragma unroll
+    for (uint32_t h = 0; h < kRounds; ++h) {
+      const uint32_t u = u0 + h * kThreads + threadIdx.x, row = u / (BN / 4), piece = u - row * (BN / 4);
+      to[h] = 0;
+      if (u < i_end * 4u) {
+        const uint32_t at = ring + row * kPitch<BN>;
+        to[h] = at + ((piece & ~3u) + ((piece & 3u) ^ ((piece >> 3) & 3u))) * 16u;
+#pragma unroll
+        for (uint32_t p = 0; p < S; ++p) v[h][p] = ld_cluster_v4(map_to_cta(at + piece * 16u, p));
+      }
+    }
+    __syncwarp();   // (the pieces of a strip belong to lanes of one warp)
+#pragma unroll
+    for (uint32_t h = 0; h < kRounds; ++h) {
+      if (to[h] == 0) continue;
+      float4 w = v[h][0];
+#pragma unroll
+      for (uint32_t p = 1; p < S; ++p) {
+        w.x += v[h][p].x;
+        w.y += v[h][p].y;
+        w.z += v[h][p].z;
+        w.w += v[h][p].w;
+      }
+      asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(to[h]), "f"(w.x), "f"(w.y), "f"(w.z), "f"(w.w) : "memory");
+    }
+  }
+}
+
 template <uint32_t BN>
 __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps, const TileArgs &A, const LaunchTag epoch) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -142,6 +185,21 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
   const uint32_t row0 = mb * BM, col0 = nb * BN;
   const bool gather = (A.gather_a | A.gather_b) != 0;
 
+  if (mblocks == 1 && !A.gather_b && warp == 2 && elect_one()) {
+    // A weight that each tile reads once comes from memory: its first stages are on their way to L2 while the kernel before
+    // this one still runs (a prefetch reads nothing that could be stale, L2 holds whatever is written to it meanwhile;
+    // [16, 8192] x [8192, 8192] 28.8 -> 27.6 us).  Where several rows of tiles share it, it mostly is in L2, and the
+    // prefetches only delay the loads ([1000, 1000] x [1000, 1000] 9.2 -> 10.0).
+    for (uint32_t kb = kb_begin; kb < min(kb_end, kb_begin + A.stages); ++kb) {
+      const int k = (int)(kb * BK);
+      if (P.b_kmajor) {
+        tma_prefetch_3d(&maps.b, k, (int)col0, (int)zb);
+      } else {
+#pragma unroll
+        for (uint32_t j = 0; j < BN / 64; ++j) tma_prefetch_3d(&maps.b, (int)(col0 + j * 64), k, (int)zb);
+      }
+    }
+  }
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < A.stages; ++s) {
       mbar_init(base + kBarFull + 8 * s, gather ? 1u + kWorkWarps : 1u);
@@ -306,7 +364,6 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
   }
 
   // ---- a partial product: TMEM -> shared memory (the stages are free: every MMA has completed) ----
-  constexpr uint32_t kPitch = BN * 4 + 16;   // bytes per row; the 16 keep rows off each other's banks
   if (warp >= 2) {
     const uint32_t wt = threadIdx.x - 64u;
     if (wt < BN && P.bias_ptr != 0) reinterpret_cast<float *>(smem + kBiasOff)[wt] = bias_at(P, col0 + wt);
@@ -320,7 +377,7 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
       for (uint32_t c = 0; c < BN / 2; c += 32) tmem_ld_32x32b_x32_nowait(taddr + c, &r[c]);
       tmem_ld_wait();
       const uint32_t row = quarter * 32u + lane;
-      const uint32_t dst = ring + row * kPitch + half * (BN / 2) * 4u;
+      const uint32_t dst = ring + row * kPitch<BN> + half * (BN / 2) * 4u;
       if (row < rows) {   // (the buffer holds the rows the matrix has)
 #pragma unroll
         for (uint32_t c = 0; c < BN / 2; c += 4)
@@ -341,33 +398,12 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
   constexpr uint32_t kSpr = BN / 16;   // strips per row
   const uint32_t strips = rows * kSpr;
   const uint32_t i_begin = strips * rank / S, i_end = strips * (rank + 1) / S;
-  // The sum first, 16 bytes per lane and side by side: taken strip by strip, 64 bytes apart, the remote reads were 12 us of
-  // the 37 us of a [128, 8192] x [8192, 8192] product.  It replaces this CTA's own partial (its share is read by no one else),
-  // the four pieces of a strip at p ^ (strip / 2 & 3) so that the strips' readers below do not meet on a bank.
-  for (uint32_t u0 = i_begin * 4u; u0 < i_end * 4u; u0 += 2u * kThreads) {
-    float4 v[2];
-    uint32_t to[2];
-#pragma unroll
-    for (uint32_t h = 0; h < 2; ++h) {
-      const uint32_t u = u0 + h * kThreads + threadIdx.x, row = u / (BN / 4), piece = u - row * (BN / 4);
-      to[h] = 0;
-      if (u < i_end * 4u) {
-        const uint32_t at = ring + row * kPitch;
-        to[h] = at + ((piece & ~3u) + ((piece & 3u) ^ ((piece >> 3) & 3u))) * 16u;
-        v[h] = ld_cluster_v4(map_to_cta(at + piece * 16u, 0));
-        for (uint32_t p = 1; p < S; ++p) {
-          const float4 q = ld_cluster_v4(map_to_cta(at + piece * 16u, p));
-          v[h].x += q.x;
-          v[h].y += q.y;
-          v[h].z += q.z;
-          v[h].w += q.w;
-        }
-      }
-    }
-    __syncwarp();   // (the pieces of a strip belong to lanes of one warp)
-#pragma unroll
-    for (uint32_t h = 0; h < 2; ++h)
-      if (to[h] != 0) asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(to[h]), "f"(v[h].x), "f"(v[h].y), "f"(v[h].z), "f"(v[h].w) : "memory");
+  if (S == 2) {
+    sum_partials<BN, 2>(ring, i_begin, i_end);
+  } else if (S == 4) {
+    sum_partials<BN, 4>(ring, i_begin, i_end);
+  } else {
+    sum_partials<BN, 8>(ring, i_begin, i_end);
   }
   __syncthreads();
   with_mode(P, [&](auto mode) {
@@ -380,7 +416,7 @@ __device__ __forceinline__ void tile_body(const MmParam &P, const TileMaps &maps
       pos.col = col0 + strip * 16u;
       if (pos.col >= P.N) continue;
       pos.valid = min(16u, P.N - pos.col);
-      const uint32_t at = ring + row * kPitch + strip * 64u;
+      const uint32_t at = ring + row * kPitch<BN> + strip * 64u;
       uint32_t r[16], pk[8];
 #pragma unroll
       for (uint32_t g = 0; g < 4; ++g)
