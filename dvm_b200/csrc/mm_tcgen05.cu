@@ -312,32 +312,37 @@ struct MmPlan {
   uint32_t bn, split;   // bn 0: 256 x 256 tiles of CTA pairs; else 128 x bn tiles, K cut into `split` parts
 };
 
-// Estimated clock cycles of a tiling.  The constants are a fit to 34 problem shapes timed in every tiling (1 to 8000 rows);
-// the tiling with the lowest estimate was on average 2 % slower than the fastest one of its shape.
-//  - A CTA alone on its SM spends max(260 + 1.6 bn, bytes / 50) per k-block, two of them together max(that, 2 bytes / 66):
-//    the MMAs of a k-block and what L2 delivers to an SM.
+// Estimated clock cycles (1850 per us) of a tiling.  The constants are a fit to 42 problem shapes (1 to 16384 rows) timed in
+// every tiling; the tiling with the lowest estimate was on average 0.5 % slower than the fastest one of its shape.
+//  - A k-block takes max(210 + 2.9 bn, bytes / 154) on a CTA alone on its SM, and max(that, 2 bytes / 79) two of them
+//    together: the MMAs of a k-block and what L2 delivers to an SM.
 //  - Loads by the work warps (operands at any even address) cost 1700 per k-block, and hardly overlap between two CTAs.
-//  - A 256 x 256 tile of a pair takes 673 per k-block, or its epilogue, whichever is longer; the last epilogue is exposed.
+//  - Draining a column of 128 rows takes 30, with the gated form or a program 52; the sum over a cluster moves all of a tile but
+//    its own share through distributed shared memory.
+//  - A 256 x 256 tile of a pair takes 620 per k-block, or its epilogue, whichever is longer; the last epilogue is exposed.
 double TileCost(const MmParam &p, uint32_t bn, uint32_t split, int sms, bool gather) {
   const uint32_t kb = (p.K + BK - 1) / BK;
   const uint64_t batch = static_cast<uint64_t>(p.batch0) * p.batch1, mb = (p.M + BM - 1) / BM;
+  const bool light = p.epi_mode == EPI_STORE || p.epi_mode == EPI_WIDEN;
   if (bn == 0) {
     const uint64_t tiles = (mb + 1) / 2 * ((p.N + BN - 1) / BN) * batch, waves = (tiles + sms / 2 - 1) / (sms / 2);
-    return 16700.0 + static_cast<double>(waves) * std::max(kb * 673.0, 12900.0);
+    return (light ? 10400.0 : 14200.0) + static_cast<double>(waves) * std::max(kb * 620.0, light ? 5800.0 : 9000.0);
   }
-  const double a_rows = p.M < BM ? p.M : BM, bytes = (a_rows + bn) * 128.0;
+  const double part = (p.M < BM ? p.M : BM) / static_cast<double>(BM), bytes = (part * BM + bn) * 128.0;
   const uint64_t ctas = mb * ((p.N + bn - 1) / bn) * batch * split;
   const uint32_t share = (kb + split - 1) / split;
-  double one = std::max(260.0 + 1.6 * bn, bytes / 50.0), two = std::max(one, 2.0 * bytes / 66.0);
+  double one = std::max(210.0 + 2.9 * bn, bytes / 154.0), two = std::max(one, 2.0 * bytes / 79.0);
   if (gather) {
     one = 1700.0;
     two = 1.8 * one;
   }
-  const double finish = 4100.0 + 60.0 * bn * (a_rows / BM) / split + (split > 1 ? 3270.0 + 310.0 * split : 0.0);
+  const double column = light ? 30.0 : 52.0;
+  double finish = column * bn * part / split;
+  if (split > 1) finish += 2940.0 + 36.0 * bn * part * (split - 1) / split + 144.0 * split;
   const uint64_t full = ctas / (2 * sms), rest = ctas % (2 * sms);   // two CTAs per SM
-  double t = 5300.0 + static_cast<double>(full) * (share * two + 1.5 * finish);
+  double t = 4550.0 + static_cast<double>(full) * (share * two + 1.8 * finish);
   if (rest > static_cast<uint64_t>(sms)) {
-    t += share * two + 1.5 * finish;
+    t += share * two + 1.8 * finish;
   } else if (rest > 0) {
     t += share * one + finish;
   }
