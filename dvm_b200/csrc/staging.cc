@@ -2,10 +2,14 @@
 //
 // What bounds it: a NumPy array is pageable, and the driver's own path for it runs one thread at about 17 GB/s (4 MB up in
 // 242 us, a 64 KB array in 43 us) while the link carries 50 GB/s from pinned memory.  Here the calling thread and up to five
-// workers copy 256 KB chunks into (or out of) pinned memory while the copy engine moves the chunks before (or after): the
-// link and those threads' memcpy (42-55 GB/s together) run at the same time.
+// workers copy into (or out of) pinned memory while the copy engine moves the chunk before (or after): the link and those
+// threads' memcpy (42-55 GB/s together) run at the same time.  4 MB up take 120 us and down 124, of which the link needs 84.
 //
-// The ring (4 MB per device used) is allocated at the first copy that needs it and given back after ten seconds without
+// A transfer costs the calling thread about 10 us (the copy, its event, the look at it), so chunks are 1 MB: with 256 KB ones
+// a call on two 4 MB arrays with a 4 MB result took 463 us, now 337.  The threads share a chunk in parts of 64 KB, so that the
+// first one is ready after 25 us.
+//
+// The ring (8 MB per device used) is allocated at the first copy that needs it and given back after ten seconds without
 // one.  One copy uses it at a time; a copy that finds it taken, one on a capturing stream, a small one, one of pinned memory
 // and any in a forked child goes to cudaMemcpyAsync as it is.
 #include "staging.h"
@@ -16,6 +20,7 @@
 #include <emmintrin.h>
 #endif
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -27,12 +32,17 @@
 namespace dvmb {
 namespace {
 
-constexpr size_t kChunk = 256 * 1024;
-constexpr uint32_t kSlots = 16;
+constexpr size_t kChunk = 1024 * 1024;
+constexpr uint32_t kSlots = 8;
+constexpr size_t kPart = 64 * 1024;      // what one thread copies at a time: a chunk is ready when several have shared it
+constexpr uint32_t kParts = kChunk / kPart;
 constexpr size_t kSmall = 32 * 1024;   // (below this the driver's path is as fast: it sends small copies inside the command)
 constexpr int kMaxDevices = 64;
 constexpr uint32_t kMaxWorkers = 5;
 constexpr auto kIdle = std::chrono::seconds(10);
+// A worker looks for the next copy for this long before it sleeps: copies come in groups (two arguments and a result), and
+// waking a thread takes 50 us and more, half the time of a 4 MB copy.
+constexpr auto kLinger = std::chrono::microseconds(150);
 
 // Into pinned memory past the caches: the copy engine reads lines that sit modified in a core's cache at a quarter of the
 // link's rate (4 MB arrived 470 us after the call, the last byte having been copied after 97).
@@ -75,33 +85,41 @@ struct Pool {
   char *mem = nullptr;
   uint64_t first = 0;                      // number of the copy's first transfer
   uint32_t chunks = 0;
-  std::atomic<uint32_t> next{0}, limit{0}, done{0};
-  std::atomic<uint32_t> filled[kSlots];    // up: chunk + 1 that the slot holds; down: chunk + 1 that has left it
+  uint32_t parts = 0;
+  std::atomic<uint32_t> next{0}, limit{0}, done{0};   // in parts: the next to copy, those that may be copied, those copied
+  std::atomic<uint32_t> copied[kSlots];    // parts copied into (out of) the slot
   std::atomic<uint32_t> inside{0};         // workers in the copy
 
   std::mutex m;
   std::condition_variable wake;
-  uint64_t generation = 0;
+  std::atomic<uint64_t> generation{0};
   bool open = false;
   uint32_t workers = 0;
   bool started = false;
 
   size_t SizeOf(uint32_t c) const { return c + 1 == chunks ? bytes - static_cast<size_t>(c) * kChunk : kChunk; }
   char *SlotOf(uint32_t c) const { return mem + (first + c) % kSlots * kChunk; }
+  uint32_t PartsOf(uint32_t c) const { return c + 1 == chunks ? parts - c * kParts : kParts; }
+  // every part of chunk c has been copied (the chunks before it in its slot have, or it would not have begun)
+  bool Copied(uint32_t c) const {
+    return copied[(first + c) % kSlots].load(std::memory_order_acquire) >= c / kSlots * kParts + PartsOf(c);
+  }
 
-  // Copies one chunk if there is one to copy now.
+  // Copies one part if there is one to copy now.
   bool CopyOne() {
-    uint32_t c = next.load(std::memory_order_relaxed);
+    uint32_t i = next.load(std::memory_order_relaxed);
     do {
-      if (c >= chunks || c >= limit.load(std::memory_order_acquire)) return false;
-    } while (!next.compare_exchange_weak(c, c + 1, std::memory_order_relaxed));
-    char *const h = host + static_cast<size_t>(c) * kChunk;
+      if (i >= parts || i >= limit.load(std::memory_order_acquire)) return false;
+    } while (!next.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
+    const uint32_t c = i / kParts;
+    const size_t at = static_cast<size_t>(i - c * kParts) * kPart, n = std::min(kPart, SizeOf(c) - at);
+    char *const h = host + static_cast<size_t>(c) * kChunk + at;
     if (up) {
-      CopyPastCache(SlotOf(c), h, SizeOf(c));
+      CopyPastCache(SlotOf(c) + at, h, n);
     } else {
-      std::memcpy(h, SlotOf(c), SizeOf(c));
+      std::memcpy(h, SlotOf(c) + at, n);
     }
-    filled[(first + c) % kSlots].store(c + 1, std::memory_order_release);
+    copied[(first + c) % kSlots].fetch_add(1, std::memory_order_release);
     done.fetch_add(1, std::memory_order_release);
     return true;
   }
@@ -111,7 +129,7 @@ struct Pool {
     for (;;) {
       {
         std::unique_lock<std::mutex> lock(m);
-        while (!open || generation == seen) {
+        while (!open || generation.load() == seen) {
           if (!keeper) {
             wake.wait(lock);
           } else if (wake.wait_for(lock, kIdle) == std::cv_status::timeout) {
@@ -120,10 +138,10 @@ struct Pool {
             lock.lock();
           }
         }
-        seen = generation;
+        seen = generation.load();
         inside.fetch_add(1);
       }
-      for (int idle = 0; next.load(std::memory_order_relaxed) < chunks;) {
+      for (int idle = 0; next.load(std::memory_order_relaxed) < parts;) {
         if (CopyOne()) {
           idle = 0;
         } else if (++idle > 200) {
@@ -133,6 +151,8 @@ struct Pool {
         }
       }
       inside.fetch_sub(1);
+      const auto until = std::chrono::steady_clock::now() + kLinger;
+      while (generation.load(std::memory_order_relaxed) == seen && std::chrono::steady_clock::now() < until) std::this_thread::yield();
     }
   }
 
@@ -199,11 +219,12 @@ struct Pool {
     mem = r.mem;
     first = r.issued;
     chunks = static_cast<uint32_t>((bytes + kChunk - 1) / kChunk);
+    parts = static_cast<uint32_t>((bytes + kPart - 1) / kPart);
     next = 0;
     limit = 0;
     done = 0;
-    for (auto &f : filled) f = 0;
-    const bool share = chunks > 1;
+    for (auto &n : copied) n = 0;
+    const bool share = parts > 1;
     if (share && up) Open();
     bool opened = share && up;
     cudaError_t err = cudaSuccess;
@@ -216,17 +237,17 @@ struct Pool {
       return false;
     };
     uint32_t room = 0;   // up: chunks whose slot is free
-    while (err == cudaSuccess && (up ? sent : done.load(std::memory_order_acquire)) < chunks) {
+    while (err == cudaSuccess && (up ? sent < chunks : done.load(std::memory_order_acquire) < parts)) {
       bool moved = false;
       if (up) {
         while (room < chunks && err == cudaSuccess) {
           const uint64_t number = first + room;
           if (number >= kSlots && (number - kSlots >= first + sent || !complete(number - kSlots))) break;
           ++room;
-          limit.store(room, std::memory_order_release);
+          limit.store(room * kParts, std::memory_order_release);
           moved = true;
         }
-        while (sent < chunks && filled[(first + sent) % kSlots].load(std::memory_order_acquire) == sent + 1 && err == cudaSuccess) {
+        while (sent < chunks && Copied(sent) && err == cudaSuccess) {
           err = Send(r, device, sent, stream);
           ++sent;
           moved = true;
@@ -235,7 +256,7 @@ struct Pool {
         while (sent < chunks && err == cudaSuccess) {
           const uint64_t number = first + sent;
           if (sent >= kSlots) {
-            if (filled[number % kSlots].load(std::memory_order_acquire) != sent - kSlots + 1) break;
+            if (!Copied(sent - kSlots)) break;
           } else if (number >= kSlots && !complete(number - kSlots)) {
             break;
           }
@@ -245,10 +266,10 @@ struct Pool {
         }
         while (arrived < sent && err == cudaSuccess && complete(first + arrived)) {
           ++arrived;
-          limit.store(arrived, std::memory_order_release);
+          limit.store(arrived * kParts, std::memory_order_release);
           moved = true;
         }
-        if (share && !opened && arrived > 0) {   // (the workers sleep until the first chunk is there)
+        if (share && !opened && arrived > 0) {   // (the workers rest until the first chunk is there)
           Open();
           opened = true;
         }
@@ -256,7 +277,7 @@ struct Pool {
       if (!CopyOne() && !moved) std::this_thread::yield();
     }
     r.issued = first + sent;
-    next.store(chunks);   // (after an error: nothing more to claim)
+    next.store(parts);   // (after an error: nothing more to claim)
     if (opened) {
       {
         std::lock_guard<std::mutex> lock(m);

@@ -8,7 +8,7 @@ from dvm_b200 import _capi
 
 pytestmark = pytest.mark.gpu
 
-CHUNK, RING = 256 * 1024, 16 * 256 * 1024
+PART, CHUNK, RING = 64 * 1024, 1024 * 1024, 8 * 1024 * 1024
 
 
 def _round_trip(lib, n, seed):
@@ -28,7 +28,7 @@ def _round_trip(lib, n, seed):
     assert lib.dvm_rt_free(d) == 0
 
 
-@pytest.mark.parametrize("n", [1, 32 * 1024 - 1, 32 * 1024, CHUNK - 1, CHUNK, CHUNK + 1, RING - 5, RING, RING + 1, 3 * RING + 12345])
+@pytest.mark.parametrize("n", [1, 32 * 1024 - 1, 32 * 1024, PART - 1, PART, PART + 1, 4 * PART + 3, CHUNK - 1, CHUNK, CHUNK + 1, RING - 5, RING, RING + 1, 3 * RING + 12345])
 def test_sizes(n):
     lib = _capi.load()
     assert lib.dvm_rt_set_device(0) == 0
