@@ -105,12 +105,12 @@ struct Combine {
 
 // (A form for at most eight rows that kept no accumulators for the upper half of the MMA, 168 instead of 233 registers and
 // three CTAs per SM, measured 36 us against 25 on [2, 32] heads of 3999 keys.)
-template <uint32_t DT, uint32_t D, bool SCALE_FIRST>
+// NT: tiles of 16 keys per step.
+template <uint32_t DT, uint32_t D, bool SCALE_FIRST, uint32_t NT>
 __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs &A) {
   constexpr uint32_t JK = D / 32, HV = D / 64;   // 16-byte pieces of a key row per thread, 64-element halves of a value row
+  constexpr uint32_t kStep = NT * kTile;
   extern __shared__ __align__(16) uint8_t smem[];
-  chain_wait();
-  chain_launch();
   Combine<D> &sm = *reinterpret_cast<Combine<D> *>(smem);
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, q4 = lane & 3u, q8 = lane >> 2;
   const uint32_t CL = A.cluster, rank = CL > 1 ? rank_in_cluster() : 0u;
@@ -125,23 +125,31 @@ __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs
     if (ok) asm volatile("ld.global.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
   };
-  uint4 kf[2][JK], vf[4][HV];
+  uint4 kf[NT][2][JK], vf[NT][4][HV];
+  auto key_at = [&](uint32_t base, uint32_t u, uint32_t n) { return base + u * kTile + 8u * n + q8; };
+  auto value_at = [&](uint32_t base, uint32_t u, uint32_t i) { return base + u * kTile + 2u * q4 + (i & 1u) + (i >> 1) * 8u; };
   auto load_k = [&](uint32_t base) {
 #pragma unroll
-    for (uint32_t n = 0; n < 2; ++n) {
-      const uint32_t key = base + 8u * n + q8;
+    for (uint32_t u = 0; u < NT; ++u)
 #pragma unroll
-      for (uint32_t j = 0; j < JK; ++j) kf[n][j] = load16(Kh + (uint64_t)key * D + j * 32u + q4 * 8u, key < k_end);
-    }
+      for (uint32_t n = 0; n < 2; ++n) {
+        const uint32_t key = key_at(base, u, n);
+#pragma unroll
+        for (uint32_t j = 0; j < JK; ++j) kf[u][n][j] = load16(Kh + (uint64_t)key * D + j * 32u + q4 * 8u, key < k_end);
+      }
   };
   auto load_v = [&](uint32_t base) {
 #pragma unroll
-    for (uint32_t i = 0; i < 4; ++i) {
-      const uint32_t key = base + 2u * q4 + (i & 1u) + (i >> 1) * 8u;
+    for (uint32_t u = 0; u < NT; ++u)
 #pragma unroll
-      for (uint32_t h = 0; h < HV; ++h) vf[i][h] = load16(Vh + (uint64_t)key * D + h * 64u + q8 * 8u, key < k_end);
-    }
+      for (uint32_t i = 0; i < 4; ++i) {
+        const uint32_t key = value_at(base, u, i);
+#pragma unroll
+        for (uint32_t h = 0; h < HV; ++h) vf[u][i][h] = load16(Vh + (uint64_t)key * D + h * 64u + q8 * 8u, key < k_end);
+      }
   };
+  chain_wait();
+  chain_launch();
   load_k(k_begin);
   load_v(k_begin);
   uint32_t qf[2 * JK][4];   // A fragments of Q in K's order of elements
@@ -169,37 +177,44 @@ __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs
   for (uint32_t r = 0; r < 2; ++r) m[r] = -CUDART_INF_F, l[r] = 0.0f;
 
 #pragma unroll 1
-  for (uint32_t base = k_begin; base < k_end; base += kTile) {
-    float s[2][2][2];   // [row half][n-tile]
+  for (uint32_t base = k_begin; base < k_end; base += kStep) {
+    float s[NT][2][2][2];   // [tile][row half][n-tile]
 #pragma unroll
-    for (uint32_t n = 0; n < 2; ++n) {
+    for (uint32_t u = 0; u < NT; ++u)
 #pragma unroll
-      for (uint32_t r = 0; r < 2; ++r) s[r][n][0] = s[r][n][1] = 0.0f;
+      for (uint32_t n = 0; n < 2; ++n) {
 #pragma unroll
-      for (uint32_t j = 0; j < 2 * JK; ++j) {
-        const uint4 &k = kf[n][j >> 1];
-        const uint32_t b0 = (j & 1u) ? k.z : k.x, b1 = (j & 1u) ? k.w : k.y;
-        mma16816<DT>(s[0][n], s[1][n], qf[j], b0, b1);
+        for (uint32_t r = 0; r < 2; ++r) s[u][r][n][0] = s[u][r][n][1] = 0.0f;
+#pragma unroll
+        for (uint32_t j = 0; j < 2 * JK; ++j) {
+          const uint4 &k = kf[u][n][j >> 1];
+          const uint32_t b0 = (j & 1u) ? k.z : k.x, b1 = (j & 1u) ? k.w : k.y;
+          mma16816<DT>(s[u][0][n], s[u][1][n], qf[j], b0, b1);
+        }
       }
-    }
-    load_k(base + kTile);   // (past the warp's keys: nothing is read)
-    // columns of this thread: keys base + 2 q4 + {0, 1} and eight further
-    float2 x[2][2];
+    load_k(base + kStep);   // (past the warp's keys: nothing is read)
+    // columns of this thread: keys 2 q4 + {0, 1} of each tile and eight further
+    float2 x[NT][2][2];
 #pragma unroll
-    for (uint32_t n = 0; n < 2; ++n) {
-      const uint32_t key = base + 8u * n + 2u * q4;
+    for (uint32_t u = 0; u < NT; ++u)
 #pragma unroll
-      for (uint32_t r = 0; r < 2; ++r) {
-        x[r][n] = score2<DT, SCALE_FIRST>(s[r][n][0], s[r][n][1], scale, scale2);
-        if (key >= k_end) x[r][n].x = -CUDART_INF_F;
-        if (key + 1u >= k_end) x[r][n].y = -CUDART_INF_F;
+      for (uint32_t n = 0; n < 2; ++n) {
+        const uint32_t key = base + u * kTile + 8u * n + 2u * q4;
+#pragma unroll
+        for (uint32_t r = 0; r < 2; ++r) {
+          x[u][r][n] = score2<DT, SCALE_FIRST>(s[u][r][n][0], s[u][r][n][1], scale, scale2);
+          if (key >= k_end) x[u][r][n].x = -CUDART_INF_F;
+          if (key + 1u >= k_end) x[u][r][n].y = -CUDART_INF_F;
+        }
       }
-    }
     bool raise = false;
     float top[2];
 #pragma unroll
     for (uint32_t r = 0; r < 2; ++r) {
-      top[r] = fmaxf(fmaxf(x[r][0].x, x[r][0].y), fmaxf(x[r][1].x, x[r][1].y));
+      top[r] = fmaxf(fmaxf(x[0][r][0].x, x[0][r][0].y), fmaxf(x[0][r][1].x, x[0][r][1].y));
+#pragma unroll
+      for (uint32_t u = 1; u < NT; ++u)
+        top[r] = fmaxf(top[r], fmaxf(fmaxf(x[u][r][0].x, x[u][r][0].y), fmaxf(x[u][r][1].x, x[u][r][1].y)));
       top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 1));
       top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 2));
       raise |= top[r] > m[r] + 8.0f * kLog2e || m[r] == -CUDART_INF_F;
@@ -220,27 +235,30 @@ __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs
           }
       }
     }
-    uint32_t pf[4] = {0, 0, 0, 0};   // P as the A operand: rows q8 / q8 + 8, keys of n-tile 0 / 1
 #pragma unroll
-    for (uint32_t n = 0; n < 2; ++n)
+    for (uint32_t u = 0; u < NT; ++u) {
+      uint32_t pf[4] = {0, 0, 0, 0};   // P as the A operand: rows q8 / q8 + 8, keys of n-tile 0 / 1
 #pragma unroll
-      for (uint32_t r = 0; r < 2; ++r) {
-        const float p0 = exp2_fast(x[r][n].x - m[r]), p1 = exp2_fast(x[r][n].y - m[r]);
-        l[r] += p0 + p1;
-        pf[2 * n + r] = pack2<DT>(p0, p1);
-      }
+      for (uint32_t n = 0; n < 2; ++n)
 #pragma unroll
-    for (uint32_t h = 0; h < HV; ++h) {
-      const uint32_t a[4] = {vf[0][h].x, vf[0][h].y, vf[0][h].z, vf[0][h].w}, b[4] = {vf[1][h].x, vf[1][h].y, vf[1][h].z, vf[1][h].w};
-      const uint32_t c[4] = {vf[2][h].x, vf[2][h].y, vf[2][h].z, vf[2][h].w}, d[4] = {vf[3][h].x, vf[3][h].y, vf[3][h].z, vf[3][h].w};
+        for (uint32_t r = 0; r < 2; ++r) {
+          const float p0 = exp2_fast(x[u][r][n].x - m[r]), p1 = exp2_fast(x[u][r][n].y - m[r]);
+          l[r] += p0 + p1;
+          pf[2 * n + r] = pack2<DT>(p0, p1);
+        }
 #pragma unroll
-      for (uint32_t t = 0; t < 8; ++t) {
-        const uint32_t sel = (t & 1u) ? 0x7632u : 0x5410u;   // element t of the even and of the odd key
-        const uint32_t b0 = __byte_perm(a[t >> 1], b[t >> 1], sel), b1 = __byte_perm(c[t >> 1], d[t >> 1], sel);
-        mma16816<DT>(o[0][h][t], o[1][h][t], pf, b0, b1);
+      for (uint32_t h = 0; h < HV; ++h) {
+        const uint32_t a[4] = {vf[u][0][h].x, vf[u][0][h].y, vf[u][0][h].z, vf[u][0][h].w}, b[4] = {vf[u][1][h].x, vf[u][1][h].y, vf[u][1][h].z, vf[u][1][h].w};
+        const uint32_t c[4] = {vf[u][2][h].x, vf[u][2][h].y, vf[u][2][h].z, vf[u][2][h].w}, d[4] = {vf[u][3][h].x, vf[u][3][h].y, vf[u][3][h].z, vf[u][3][h].w};
+#pragma unroll
+        for (uint32_t t = 0; t < 8; ++t) {
+          const uint32_t sel = (t & 1u) ? 0x7632u : 0x5410u;   // element t of the even and of the odd key
+          const uint32_t b0 = __byte_perm(a[t >> 1], b[t >> 1], sel), b1 = __byte_perm(c[t >> 1], d[t >> 1], sel);
+          mma16816<DT>(o[0][h][t], o[1][h][t], pf, b0, b1);
+        }
       }
     }
-    load_v(base + kTile);
+    load_v(base + kStep);
   }
 
   // ---- combine: warps of the CTA, then CTAs of the cluster ----
@@ -321,34 +339,37 @@ __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs
 
 }  // namespace
 
-#define DVMB_DECODE(NAME, DT, D, SF)                                                                                                  \
+#define DVMB_DECODE(NAME, DT, D, SF, NT)                                                                                              \
   __global__ void __launch_bounds__(kThreads, D == 128 ? 2 : 3) NAME(const __grid_constant__ AttnParam P, const __grid_constant__ DecodeArgs A) { \
-    decode_body<DT, D, SF>(P, A);                                                                                                     \
+    decode_body<DT, D, SF, NT>(P, A);                                                                                                 \
   }
-DVMB_DECODE(dvm_b200_attention_decode_bf16_d64, T_BF16, 64, false)
-DVMB_DECODE(dvm_b200_attention_decode_bf16_d64_sf, T_BF16, 64, true)
-DVMB_DECODE(dvm_b200_attention_decode_bf16_d128, T_BF16, 128, false)
-DVMB_DECODE(dvm_b200_attention_decode_bf16_d128_sf, T_BF16, 128, true)
-DVMB_DECODE(dvm_b200_attention_decode_f16_d64, T_F16, 64, false)
-DVMB_DECODE(dvm_b200_attention_decode_f16_d64_sf, T_F16, 64, true)
-DVMB_DECODE(dvm_b200_attention_decode_f16_d128, T_F16, 128, false)
-DVMB_DECODE(dvm_b200_attention_decode_f16_d128_sf, T_F16, 128, true)
+#define DVMB_DECODE_TYPE(T, DT)                                           \
+  DVMB_DECODE(dvm_b200_attention_decode_##T##_d64, DT, 64, false, 1)      \
+  DVMB_DECODE(dvm_b200_attention_decode_##T##_d64_sf, DT, 64, true, 1)    \
+  DVMB_DECODE(dvm_b200_attention_decode_##T##_d64x2, DT, 64, false, 2)    \
+  DVMB_DECODE(dvm_b200_attention_decode_##T##_d64x2_sf, DT, 64, true, 2)  \
+  DVMB_DECODE(dvm_b200_attention_decode_##T##_d128, DT, 128, false, 1)    \
+  DVMB_DECODE(dvm_b200_attention_decode_##T##_d128_sf, DT, 128, true, 1)
+DVMB_DECODE_TYPE(bf16, T_BF16)
+DVMB_DECODE_TYPE(f16, T_F16)
+#undef DVMB_DECODE_TYPE
 #undef DVMB_DECODE
 
 int LaunchAttentionDecode(const AttnParam &p, void *stream) {
   using Fn = void (*)(const AttnParam, const DecodeArgs);
 #define DVMB_DECODE_FNS(T) {{dvm_b200_attention_decode_##T##_d64, dvm_b200_attention_decode_##T##_d64_sf}, \
+                            {dvm_b200_attention_decode_##T##_d64x2, dvm_b200_attention_decode_##T##_d64x2_sf}, \
                             {dvm_b200_attention_decode_##T##_d128, dvm_b200_attention_decode_##T##_d128_sf}}
-  static const Fn table[2][2][2] = {DVMB_DECODE_FNS(bf16), DVMB_DECODE_FNS(f16)};
+  static const Fn table[2][3][2] = {DVMB_DECODE_FNS(bf16), DVMB_DECODE_FNS(f16)};
 #undef DVMB_DECODE_FNS
   int dev = 0;
   cudaGetDevice(&dev);
   static bool attr_set[64] = {false};
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
     for (auto &t : table)
-      for (int d = 0; d < 2; ++d)
+      for (int d = 0; d < 3; ++d)
         for (auto fn : t[d]) {
-          cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, d ? sizeof(Combine<128>) : sizeof(Combine<64>));
+          cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, d == 2 ? sizeof(Combine<128>) : sizeof(Combine<64>));
           if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
           if (e != cudaSuccess) return static_cast<int>(e);
         }
@@ -365,6 +386,9 @@ int LaunchAttentionDecode(const AttnParam &p, void *stream) {
   DecodeArgs a;
   a.cluster = cl;
   a.keys_per_warp = (tiles + cl * kWarps - 1) / (cl * kWarps) * kTile;
+  // Keys of 64 elements in steps of 32: what a warp has in flight is one step's keys and values, 8 KB as with 128 elements
+  // ([8, 32] heads of 4217 keys 64 -> 54.6 us).  Two steps of 16 answer sooner where that is all a warp has.
+  const uint32_t form = p.d == 128 ? 2u : (a.keys_per_warp > 32u ? 1u : 0u);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.batch * cl, 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
@@ -378,7 +402,7 @@ int LaunchAttentionDecode(const AttnParam &p, void *stream) {
   cfg.attrs = attr;
   cfg.numAttrs = cl > 1 ? 1 : 0;
   ChainAttribute(&cfg, attr);
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, table[p.dtype == T_BF16 ? 0 : 1][p.d == 128 ? 1 : 0][p.scale_first ? 1 : 0], p, a);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, table[p.dtype == T_BF16 ? 0 : 1][form][p.scale_first ? 1 : 0], p, a);
   return e != cudaSuccess ? static_cast<int>(e) : static_cast<int>(cudaGetLastError());
 }
 
