@@ -62,10 +62,19 @@ constexpr uint32_t kOutBytes = kDrainBytes<kEpiCols>;
 constexpr uint32_t kSmemBytes = kSmemHeader + kStages * kStageBytes + kEpiWarps * kOutBytes + 1024;
 
 struct MmMaps {
-  CUtensorMap a, b;
+  CUtensorMap a, b, b_half;   // b_half: the boxes of a half tile (an operand with the contraction axis innermost)
   CUtensorMap o;   // the result, boxes of 32 rows of 32 columns, 64-byte swizzle (P.tma_out)
 };
 
+// First tile that is worked on in halves: the tiles behind the last complete wave, if as halves they fit one wave.  A wave
+// of six tiles cost a [1024, 1008] x [1008, 5008] product (80 tiles on 74 pairs) 4.7 us of 15.5.
+__host__ __device__ inline uint32_t SplitFrom(uint32_t tiles, uint32_t units) {
+  const uint32_t rest = tiles % units;
+  return rest != 0 && rest * 2 <= units ? tiles - rest : tiles;
+}
+
+// HALVES: there are such tiles.  (A form of its own: the larger one cost a [16384, 512] x [512, 8192] product, which has none, 2 %.)
+template <bool HALVES>
 __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, const LaunchTag epoch) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // 1024-byte alignment of the stage area (required by the 128-byte swizzle pattern)
@@ -81,7 +90,12 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
   const uint32_t unit = blockIdx.x / 2, num_units = gridDim.x / 2;
   const uint32_t mblocks = (P.M + BM * 2 - 1) / (BM * 2), nblocks = (P.N + BN - 1) / BN;
   const uint32_t batch = P.batch0 * P.batch1;
-  const uint32_t num_tiles = mblocks * nblocks * batch;
+  // Work items: tiles, the tiles of an incomplete last wave (from item split_from on) as halves of 128 columns.
+  const uint32_t tiles = mblocks * nblocks * batch, split_from = HALVES ? SplitFrom(tiles, num_units) : tiles;
+  const uint32_t num_items = 2 * tiles - split_from;
+  auto half_of = [&](uint32_t t) { return HALVES && t >= split_from; };
+  auto tile_of = [&](uint32_t t) { return half_of(t) ? split_from + ((t - split_from) >> 1) : t; };
+  auto side_of = [&](uint32_t t) { return half_of(t) ? ((t - split_from) & 1u) * (BN / 2) : 0u; };   // its first column in the tile
   const uint32_t kblocks = (P.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -114,19 +128,20 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
     if (elect_one()) {
       const bool a_m = P.a_mmajor != 0, b_k = P.b_kmajor != 0;
       uint32_t stage = 0, parity = 1;
-      for (uint32_t t = unit; t < num_tiles; t += num_units) {
+      for (uint32_t t = unit; t < num_items; t += num_units) {
         uint32_t bz, mb, nb;
-        tile_coords(t, mblocks, nblocks, P.group_m, bz, mb, nb);
+        tile_coords(tile_of(t), mblocks, nblocks, P.group_m, bz, mb, nb);
+        const bool half = half_of(t);
         const uint32_t b0 = bz / P.batch1, b1 = bz - b0 * P.batch1;
         const int za = (int)(b0 * P.a_mul0 + b1 * P.a_mul1), zb = (int)(b0 * P.b_mul0 + b1 * P.b_mul1);
         const int row0 = (int)((mb * 2 + rank) * BM);
-        const int col0 = (int)(nb * BN + rank * (BN / 2));
+        const int col0 = (int)(nb * BN + side_of(t) + rank * (half ? BN / 4 : BN / 2));
         int k = 0;
         for (uint32_t kb = 0; kb < kblocks; ++kb, k += (int)BK) {
           mbar_wait(bar_empty + 8 * stage, parity, 1, &g_mm_status, epoch);
           const uint32_t sa = stages + stage * kStageBytes, sb = sa + kABytes;
           // the pair's first CTA counts the bytes of both CTAs on its barrier
-          if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 2 * kStageBytes);
+          if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 2 * (kABytes + (half ? kBBytes / 2 : kBBytes)));
           const uint32_t full = map_to_cta(bar_full + 8 * stage, 0);
           if (!a_m) {
             tma_load_3d_pair(sa, &maps.a, full, k, row0, za);
@@ -135,10 +150,11 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
             for (uint32_t j = 0; j < BM / 64; ++j) tma_load_3d_pair(sa + j * (64 * BK * 2), &maps.a, full, row0 + (int)(j * 64), k, za);
           }
           if (b_k) {
-            tma_load_3d_pair(sb, &maps.b, full, k, col0, zb);
+            tma_load_3d_pair(sb, half ? &maps.b_half : &maps.b, full, k, col0, zb);
           } else {
 #pragma unroll
-            for (uint32_t j = 0; j < BN / 2 / 64; ++j) tma_load_3d_pair(sb + j * (64 * BK * 2), &maps.b, full, col0 + (int)(j * 64), k, zb);
+            for (uint32_t j = 0; j < BN / 2 / 64; ++j)
+              if (j == 0 || !half) tma_load_3d_pair(sb + j * (64 * BK * 2), &maps.b, full, col0 + (int)(j * 64), k, zb);
           }
           if (++stage == kStages) {
             stage = 0;
@@ -155,21 +171,22 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
       const uint32_t fmt = P.in_dtype == T_BF16 ? 1u : 0u;
       const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((P.a_mmajor ? 1u : 0u) << 15) |
                              ((P.b_kmajor ? 0u : 1u) << 16) | ((BN >> 3) << 17) | (((BM * 2) >> 4) << 24);
+      const uint32_t idesc_half = idesc - ((BN / 2 >> 3) << 17);
       // (descriptors of stage 0; a stage or a K = 16 step further is an addition to their address fields)
       const uint64_t da0 = P.a_mmajor ? make_smem_desc(stages, 64 * BK * 2, 1024) : make_smem_desc(stages, 0, 1024);
       const uint64_t db0 = P.b_kmajor ? make_smem_desc(stages + kABytes, 0, 1024) : make_smem_desc(stages + kABytes, 64 * BK * 2, 1024);
       const uint64_t step_a = P.a_mmajor ? 2048 >> 4 : 32 >> 4, step_b = P.b_kmajor ? 32 >> 4 : 2048 >> 4;
       uint32_t stage = 0, parity = 0, acc = 0, acc_parity = 1;
-      for (uint32_t t = unit; t < num_tiles; t += num_units) {
+      for (uint32_t t = unit; t < num_items; t += num_units) {
         mbar_wait(bar_tempty + 8 * acc, acc_parity, 2, &g_mm_status, epoch);
         tcgen05_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * BN, desc = half_of(t) ? idesc_half : idesc;
         for (uint32_t kb = 0; kb < kblocks; ++kb) {
           mbar_wait(bar_full + 8 * stage, parity, 3, &g_mm_status, epoch);
           const uint64_t da = da0 + stage * (kStageBytes >> 4), db = db0 + stage * (kStageBytes >> 4);
 #pragma unroll
           for (uint32_t kk = 0; kk < BK / 16; ++kk)
-            umma_f16_pair(d_tmem, da + kk * step_a, db + kk * step_b, idesc, (kb | kk) != 0 ? 1u : 0u);
+            umma_f16_pair(d_tmem, da + kk * step_a, db + kk * step_b, desc, (kb | kk) != 0 ? 1u : 0u);
           umma_commit_pair(bar_empty + 8 * stage, 3);   // the stage is free (in both CTAs) once these MMAs have read it
           if (++stage == kStages) {
             stage = 0;
@@ -187,7 +204,8 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
     // ------------------------------ epilogue warps ------------------------------
     const uint32_t ew = warp - 2;
     const uint32_t quarter = warp & 3u;          // TMEM lane quarter this warp may read
-    const uint32_t col0 = (ew >> 2) * kEpiCols;  // the columns of the tile this warp drains
+    auto cols_of = [&](uint32_t t) { return half_of(t) ? kEpiCols / 2 : kEpiCols; };   // the columns this warp drains
+    auto col0_of = [&](uint32_t t) { return (ew >> 2) * cols_of(t); };                  // ... and their first in the item
     const uint32_t out_saddr = stages + kStages * kStageBytes + ew * kOutBytes;
     const uint32_t bias_saddr = base + kBiasOff + ew * (kEpiCols * 4u);
     uint32_t acc = 0, acc_parity = 0;
@@ -196,10 +214,10 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
     uint32_t bz, mb, nb;
     uint32_t bias[kEpiCols / 32];
     auto look_up = [&](uint32_t t) {
-      tile_coords(t, mblocks, nblocks, P.group_m, bz, mb, nb);
+      tile_coords(tile_of(t), mblocks, nblocks, P.group_m, bz, mb, nb);
       if (P.bias_ptr == 0) return;
       // (columns past the last one are not stored: any bias will do.  No value is selected or converted here, that would wait)
-      const uint32_t col = nb * BN + col0 + lane;
+      const uint32_t col = nb * BN + side_of(t) + col0_of(t) + lane;
       if (P.bias_dtype == T_F32) {
 #pragma unroll
         for (uint32_t i = 0; i < kEpiCols / 32; ++i) bias[i] = __ldg(reinterpret_cast<const uint32_t *>(P.bias_ptr) + min(col + i * 32, P.N - 1));
@@ -208,10 +226,10 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
         for (uint32_t i = 0; i < kEpiCols / 32; ++i) bias[i] = __ldg(reinterpret_cast<const unsigned short *>(P.bias_ptr) + min(col + i * 32, P.N - 1));
       }
     };
-    if (unit < num_tiles) look_up(unit);
+    if (unit < num_items) look_up(unit);
     with_mode(P, [&](auto mode) {
       constexpr uint32_t MODE = decltype(mode)::mode, DT = decltype(mode)::dtype;
-      for (uint32_t t = unit; t < num_tiles; t += num_units) {
+      for (uint32_t t = unit; t < num_items; t += num_units) {
         if (P.bias_ptr != 0) {
           __syncwarp();   // (the warp has read the previous tile's)
 #pragma unroll
@@ -222,13 +240,16 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
         EpiPos pos;
         pos.b0 = bz / P.batch1;
         pos.b1 = bz - pos.b0 * P.batch1;
-        const uint32_t first_row = (mb * 2 + rank) * BM + quarter * 32u, first_col = nb * BN + col0;
+        const uint32_t first_row = (mb * 2 + rank) * BM + quarter * 32u, first_col = nb * BN + side_of(t) + col0_of(t);
         pos.row = first_row + lane;
-        if (t + num_units < num_tiles) look_up(t + num_units);
+        if (t + num_units < num_items) look_up(t + num_units);
         mbar_wait(bar_tfull + 8 * acc, acc_parity, 4, &g_mm_status, epoch);
         tcgen05_after_sync();
-        const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * BN + col0;
-        drain<MODE, DT, kEpiCols>(P, maps.o, taddr, false, pos, first_row, first_col, bias_saddr, out_saddr, lane);
+        const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * BN + col0_of(t);
+        if (half_of(t))   // (columns as a template argument: as a variable they cost every whole tile 6 %)
+          drain<MODE, DT, kEpiCols / 2>(P, maps.o, taddr, false, pos, first_row, first_col, bias_saddr, out_saddr, lane);
+        else
+          drain<MODE, DT, kEpiCols>(P, maps.o, taddr, false, pos, first_row, first_col, bias_saddr, out_saddr, lane);
         tcgen05_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(map_to_cta(bar_tempty + 8 * acc, 0));
@@ -253,7 +274,11 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   dvm_b200_mm_tcgen05_pair(const __grid_constant__ MmParam P, const __grid_constant__ MmMaps maps, const LaunchTag epoch) {
-  pair_body(P, maps, epoch);
+  pair_body<false>(P, maps, epoch);
+}
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+  dvm_b200_mm_tcgen05_pair_halves(const __grid_constant__ MmParam P, const __grid_constant__ MmMaps maps, const LaunchTag epoch) {
+  pair_body<true>(P, maps, epoch);
 }
 
 namespace {
@@ -319,14 +344,17 @@ struct MmPlan {
 //  - Loads by the work warps (operands at any even address) cost 1700 per k-block, and hardly overlap between two CTAs.
 //  - Draining a column of 128 rows takes 30, with the gated form or a program 52; the sum over a cluster moves all of a tile but
 //    its own share through distributed shared memory.
-//  - A 256 x 256 tile of a pair takes 620 per k-block, or its epilogue, whichever is longer; the last epilogue is exposed.
+//  - A 256 x 256 tile of a pair takes 620 per k-block, or its epilogue, whichever is longer, a half tile 0.6 of that; the last
+//    epilogue is exposed.
 double TileCost(const MmParam &p, uint32_t bn, uint32_t split, int sms, bool gather) {
   const uint32_t kb = (p.K + BK - 1) / BK;
   const uint64_t batch = static_cast<uint64_t>(p.batch0) * p.batch1, mb = (p.M + BM - 1) / BM;
   const bool light = p.epi_mode == EPI_STORE || p.epi_mode == EPI_WIDEN;
   if (bn == 0) {
-    const uint64_t tiles = (mb + 1) / 2 * ((p.N + BN - 1) / BN) * batch, waves = (tiles + sms / 2 - 1) / (sms / 2);
-    return (light ? 10400.0 : 14200.0) + static_cast<double>(waves) * std::max(kb * 620.0, light ? 5800.0 : 9000.0);
+    const uint64_t tiles = (mb + 1) / 2 * ((p.N + BN - 1) / BN) * batch, pairs = sms / 2;
+    const double whole = std::max(kb * 620.0, light ? 5800.0 : 9000.0), rest = static_cast<double>(tiles % pairs);
+    const double waves = static_cast<double>(tiles / pairs) + (rest == 0 ? 0.0 : rest * 2 <= pairs && tiles > pairs ? 0.6 : 1.0);
+    return (light ? 10400.0 : 14200.0) + waves * whole;
   }
   const double part = (p.M < BM ? p.M : BM) / static_cast<double>(BM), bytes = (part * BM + bn) * 128.0;
   const uint64_t ctas = mb * ((p.N + bn - 1) / bn) * batch * split;
@@ -459,8 +487,10 @@ int LaunchMatMul(const MmParam &p_in, void *stream) {
   if (plan.bn != 0) return LaunchMmTile(p, plan.bn, plan.split, stream);
   static bool attr_set[64] = {false};
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(dvm_b200_mm_tcgen05_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return static_cast<int>(e);
+    for (auto fn : {dvm_b200_mm_tcgen05_pair, dvm_b200_mm_tcgen05_pair_halves}) {
+      cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+      if (e != cudaSuccess) return static_cast<int>(e);
+    }
     attr_set[dev] = true;
   }
   MmMaps maps;
@@ -470,9 +500,13 @@ int LaunchMatMul(const MmParam &p_in, void *stream) {
   if (rc != 0) return rc;
   rc = EncodeMmOperand(&maps.b, p.b_ptr, MmInnerB(p), MmPitchB(p), MmRowsB(p), p.b_batches, p.b_kmajor ? BN / 2 : 64);
   if (rc != 0) return rc;
+  maps.b_half = maps.b;
+  if (p.b_kmajor) rc = EncodeMmOperand(&maps.b_half, p.b_ptr, MmInnerB(p), MmPitchB(p), MmRowsB(p), p.b_batches, BN / 4);
+  if (rc != 0) return rc;
   p.tma_out = p.epi_mode >= EPI_STORE && EncodeMmResult(&maps.o, p) ? 1u : 0u;
   const uint32_t tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.batch0 * p.batch1;
-  const uint32_t units = tiles < static_cast<uint32_t>(sms / 2) ? tiles : static_cast<uint32_t>(sms / 2);
+  const uint32_t pairs = static_cast<uint32_t>(sms / 2);
+  const uint32_t units = 2 * tiles <= pairs ? 2 * tiles : (tiles < pairs ? tiles : pairs);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   cfg.gridDim = dim3(units * 2, 1, 1);
@@ -480,7 +514,8 @@ int LaunchMatMul(const MmParam &p_in, void *stream) {
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = static_cast<cudaStream_t>(stream);
   ChainAttribute(&cfg, attr);
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, dvm_b200_mm_tcgen05_pair, p, maps, NextLaunchEpoch());
+  const auto kernel = SplitFrom(tiles, units) < tiles ? dvm_b200_mm_tcgen05_pair_halves : dvm_b200_mm_tcgen05_pair;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p, maps, NextLaunchEpoch());
   return e != cudaSuccess ? static_cast<int>(e) : static_cast<int>(cudaGetLastError());
 }
 
