@@ -291,6 +291,7 @@ struct VmParam {
   uint32_t num_sregs;        // scalar registers in use
   uint32_t kept_size[kMaxKept];
   uint32_t enum_size[kMaxEnum];   // right-aligned, unused outer slots are 1
+  uint32_t ring_whole;       // mask of the element counts that end whole 16-byte units of every tensor on the ring
   uint32_t need_coords;      // some tensor uses AM_GRANULE or is staged per segment
   uint32_t body_coords_mask; // BODY sections whose vector stores address a strided tensor through the chunk coordinates
   uint32_t num_body;         // number of BODY sections

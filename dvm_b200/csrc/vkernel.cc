@@ -239,6 +239,7 @@ void VKernel::Bind(const RelocEntry *relocs, size_t n, void *workspace, size_t w
     VectorStage &st = stp->vec;
     dvmb::VmParam &P = st.param;
     uint32_t staged = 0;
+    P.ring_whole = ~0u;
     for (size_t s = 0; s < st.slot_obj.size(); ++s) {
       dvmb::TensorDesc &td = P.tensor[s];
       td.ptr = reinterpret_cast<uint64_t>(AddrOf(st.slot_obj[s], workspace));
@@ -247,7 +248,10 @@ void VKernel::Bind(const RelocEntry *relocs, size_t n, void *workspace, size_t w
       // a tensor planned for bulk staging keeps its ring slot only if its address is 16-byte aligned
       const bool on_ring = td.ring_layout && st.ring_plan_off[s] != dvmb::kNoRing && td.ptr % 16 == 0;
       td.ring_off = on_ring ? st.ring_plan_off[s] : dvmb::kNoRing;
-      if (on_ring) staged |= 1u << s;
+      if (on_ring) {
+        staged |= 1u << s;
+        P.ring_whole &= ~(16u / static_cast<uint32_t>(ItemSize(static_cast<DataType>(td.dtype))) - 1u);
+      }
     }
     for (uint32_t q = 0; q < P.num_body; ++q) P.body_ring_mask[q] = st.body_tensor_mask[q] & staged;
     if (st.row.form != dvmb::ROW_OFF) BindRow(&st);

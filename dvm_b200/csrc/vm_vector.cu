@@ -751,8 +751,9 @@ __device__ __forceinline__ void vm_vector_body(const VmParam &P, const LaunchTag
         for (uint32_t rnd = (kRounds && !pos.gvalid) ? n_rounds : 0u; rnd < n_rounds; ++rnd) {
         pos.in_chunk0 = kRounds ? lane4 + rnd * P.round_elems : lane4;
         pos.chunk_valid = kRounds ? min(chunk_total, (rnd + 1u) * P.round_elems) : chunk_total;
-        // every lane of this thread lies inside the round: the vector fast paths apply
-        const bool full_tile = pos.gvalid && pos.in_chunk0 + 3u * pos.gstep + 4u <= pos.chunk_valid;
+        // every lane of this thread lies inside the round, and inside what the bulk copies delivered of it (whole 16-byte
+        // units: of 1870 16-bit elements 1864, although 1864 to 1867 are four valid ones): the vector fast paths apply
+        const bool full_tile = pos.gvalid && pos.in_chunk0 + 3u * pos.gstep + 4u <= (pos.chunk_valid & P.ring_whole);
         // a thread without a single lane inside the round has nothing to fetch, add or store
         const bool lane_active = pos.gvalid && pos.in_chunk0 < pos.chunk_valid;
         // full rounds run the variant without per-lane tests; a thread with nothing to do starts at the final END
