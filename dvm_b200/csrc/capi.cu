@@ -367,7 +367,6 @@ int dvm_codegen(dvm_kernel *k, const dvm_reloc *relocs, size_t reloc_size, dvm_w
       cb.fn = alloc;
       cb.user = user;
       auto t0 = std::chrono::steady_clock::now();
-      k->kernel.Normalize();
       k->kernel.CodeGen(reinterpret_cast<const dvm::RelocEntry *>(relocs), reloc_size, &cb);
       k->last_jit_us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();
       return 0;

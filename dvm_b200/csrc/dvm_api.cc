@@ -762,14 +762,11 @@ void Kernel::SequenceAdd(KernelType type, uint32_t) {
 void Kernel::Normalize() { Impl(this)->Normalize(); }
 
 size_t Kernel::PreCodeGen() {
-  auto vk = Impl(this);
-  vk->Normalize();
-  return vk->Compile();
+  return Impl(this)->Compile();
 }
 
 void Kernel::CodeGen(const RelocEntry *relocs, size_t reloc_size, WsAllocator *ws_alloc) {
   auto vk = Impl(this);
-  if (!vk->normalized_) vk->Normalize();
   size_t ws = vk->Compile();
   void *workspace = nullptr;
   if (ws > 0) {

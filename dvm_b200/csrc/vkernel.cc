@@ -124,7 +124,9 @@ static std::vector<NDObject *> LiveOps(const std::vector<NDObject *> &nodes) {
 }
 
 size_t VKernel::Compile() {
-  if (!normalized_) Normalize();
+  // (always: the borrowed shapes and scalars are read here, whatever has been inferred from them before, and sig_ names
+  // the values that the plan below is made of)
+  Normalize();
   if (compiled_) return ws_bytes_;
   if (has_plan_ && plan_sig_ == sig_) {
     compiled_ = true;

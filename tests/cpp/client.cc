@@ -106,6 +106,35 @@ int main(int argc, char **argv) {
       return 1;
     }
   }
+  {
+    // borrowed scalars and shapes are re-read at every CodeGen(), with or without a Normalize() in front of it, and a value
+    // that comes back finds the plan that was made for it
+    dvm::Kernel s;
+    s.Reset(dvm::kVector, 0);
+    std::vector<int64_t> some{4, 64};
+    dvm::IntArrayRef some_ref(some);
+    dvm::ScalarRef factor(1.0f);
+    dvm::NDObject *in = s.Load(nullptr, &some_ref, dvm::kFloat32);
+    dvm::NDObject *out = s.Store(nullptr, s.Binary<dvm::kMul>(in, &factor));
+    dvm::RelocEntry io[] = {{in, reinterpret_cast<void *>(0x10000)}, {out, reinterpret_cast<void *>(0x20000)}};
+    auto generated = [&](const char *bits) {
+      s.CodeGen(io, 2, nullptr);
+      return std::strstr(s.Das(), bits) != nullptr;
+    };
+    s.Normalize();
+    factor = 2.0f;   // (behind the Normalize: the plan is made for the new value, and must not be kept as the old one's)
+    const bool late = generated("#0x40000000");
+    factor = 3.0f;
+    const bool changed = generated("#0x40400000");
+    factor = 1.0f;
+    const bool back = generated("#0x3f800000");
+    some[0] = 9;
+    s.CodeGen(io, 2, nullptr);
+    if (!late || !changed || !back || dvm::Kernel::GetShape(out)->data[0] != 9) {
+      std::printf("FAIL: CodeGen with stale borrowed values (%d %d %d)\n", late, changed, back);
+      return 1;
+    }
+  }
 
   std::vector<float> hx(rows * cols), hy(rows * cols), hz(rows * cols), hs(rows);
   for (size_t i = 0; i < hx.size(); ++i) {
