@@ -253,6 +253,7 @@ class VKernel {
   void *workspace_ = nullptr;
   bool normalized_ = false;
   bool compiled_ = false;
+  bool bound_ = false;                     // Bind() has given the plan in use its addresses
   std::string text_;
   std::string name_;
   double last_jit_us_ = 0.0;               // host time of the last Normalize+Compile+Bind

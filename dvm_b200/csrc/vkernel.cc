@@ -94,9 +94,10 @@ NDObject *VKernel::NewNode(NodeKind kind, DataType dtype) {
 
 void VKernel::Normalize() {
   Signature(&sig_scratch_);
-  if (normalized_ && sig_scratch_ == sig_) return;   // (inferred, and perhaps planned, for these very values)
+  compiled_ = false;
+  if (normalized_ && sig_scratch_ == sig_) return;   // (inferred for these very values)
   sig_.swap(sig_scratch_);
-  normalized_ = compiled_ = false;
+  normalized_ = false;
   // a Store handed to a later op as an operand stands for the value it stores (the reference's sequence kernels read a
   // stage's stored result back in a later stage, tests/ut/test_sequence_fusion.py:170-205)
   for (auto n : nodes_)
@@ -127,7 +128,7 @@ size_t VKernel::Compile() {
   // (always: the borrowed shapes and scalars are read here, whatever has been inferred from them before, and sig_ names
   // the values that the plan below is made of)
   Normalize();
-  if (compiled_) return ws_bytes_;
+  bound_ = false;   // (a plan that was kept still holds the addresses of its last launch)
   if (has_plan_ && plan_sig_ == sig_) {
     compiled_ = true;
     return ws_bytes_;
@@ -207,6 +208,7 @@ void VKernel::CompileFresh() {
 
 void VKernel::Bind(const RelocEntry *relocs, size_t n, void *workspace, size_t workspace_bytes) {
   workspace_ = workspace;
+  bound_ = true;
   for (size_t i = 0; i < n; ++i) relocs[i].io->addr = relocs[i].addr;
   for (auto &stp : stages_) {
     if (stp->kind == STAGE_MATMUL) {
@@ -315,8 +317,20 @@ int VKernel::LaunchPipelined(void *stream) {
   return 0;
 }
 
+// A stage whose result has no elements: nothing is launched for it.
+static bool Idle(const Stage &st) {
+  switch (st.kind) {
+    case STAGE_MATMUL: return st.mm.idle;
+    case STAGE_COLLECTIVE: return st.coll.count == 0;
+    case STAGE_ATTENTION: return st.attn.idle;
+    default: return st.vec.idle;
+  }
+}
+
 int VKernel::Launch(void *stream) {
   if (!compiled_) DvmException("Launch before CodeGen");
+  for (auto &st : stages_)
+    if (!bound_ && !Idle(*st)) DvmException("Launch with an unbound tensor address");
   dvmb::Runtime::Get().EnsureInit();
   for (auto &st : stages_)
     if (st->lane != 0) return LaunchPipelined(stream);
@@ -329,12 +343,13 @@ int VKernel::Launch(void *stream) {
 
 int VKernel::LaunchStage(size_t index, void *stream) {
   if (!compiled_ || index >= stages_.size()) DvmException("LaunchStage: no such stage");
+  auto &stp = stages_[index];
+  if (Idle(*stp)) return 0;
+  if (!bound_) DvmException("Launch with an unbound tensor address");
   dvmb::Runtime::Get().EnsureInit();
   {
-    auto &stp = stages_[index];
     if (stp->kind == STAGE_MATMUL) {
       MatMulStage &mm = stp->mm;
-      if (mm.idle) return 0;
       if (mm.param.a_ptr == 0 || mm.param.b_ptr == 0) DvmException("Launch with an unbound tensor address");
       for (size_t s = 0; s < mm.slot_obj.size(); ++s)
         if (mm.slot_obj[s] && mm.param.tensor[s].ptr == 0) DvmException("Launch with an unbound tensor address");
@@ -342,7 +357,6 @@ int VKernel::LaunchStage(size_t index, void *stream) {
     }
     if (stp->kind == STAGE_COLLECTIVE) {
       CollStage &co = stp->coll;
-      if (co.count == 0) return 0;
       if (co.send_ptr == 0 || co.recv_ptr == 0) DvmException("Launch with an unbound tensor address");
       std::string err;
       int rc = dvmb::RunCollective(co.comm, static_cast<dvmb::CollKind>(co.kind), co.reduce_type, co.dtype,
@@ -353,13 +367,11 @@ int VKernel::LaunchStage(size_t index, void *stream) {
     }
     if (stp->kind == STAGE_ATTENTION) {
       AttnStage &at = stp->attn;
-      if (at.idle) return 0;
       if (!at.param.q_ptr || !at.param.k_ptr || !at.param.v_ptr || !at.param.o_ptr)
         DvmException("Launch with an unbound tensor address");
       return dvmb::LaunchAttention(at.param, stream);
     }
     VectorStage &st = stp->vec;
-    if (st.idle) return 0;
     for (size_t s = 0; s < st.slot_obj.size(); ++s)
       if (st.param.tensor[s].ptr == 0) DvmException("Launch with an unbound tensor address");
     if (st.row_ok) return dvmb::LaunchRow(st.row, stream);

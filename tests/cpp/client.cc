@@ -130,6 +130,22 @@ int main(int argc, char **argv) {
     const bool back = generated("#0x3f800000");
     some[0] = 9;
     s.CodeGen(io, 2, nullptr);
+    // a plan that comes back is not launched with the addresses of its last use: they are bound anew, or the launch refused
+    auto refused = [&](const char *why) {
+      try {
+        s.Launch(nullptr);
+      } catch (const std::runtime_error &e) {
+        return std::strstr(e.what(), why) != nullptr;
+      }
+      return false;
+    };
+    s.Normalize();
+    const bool before_codegen = refused("Launch before CodeGen");
+    s.PreCodeGen();
+    if (!before_codegen || !refused("unbound tensor address")) {
+      std::printf("FAIL: launch of a plan without addresses\n");
+      return 1;
+    }
     if (!late || !changed || !back || dvm::Kernel::GetShape(out)->data[0] != 9) {
       std::printf("FAIL: CodeGen with stale borrowed values (%d %d %d)\n", late, changed, back);
       return 1;
