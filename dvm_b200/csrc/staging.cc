@@ -87,6 +87,18 @@ void RingFree(void *p) {
   munmap(p, kRingBytes);
 }
 
+// While one of these lives, the thread's CUDA calls neither fail nor break a stream capture because somebody captures: polling
+// an event counts as unsafe in the default mode, whatever stream the event belongs to and whichever thread captures.
+class RelaxedCapture {
+ public:
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  RelaxedCapture(const RelaxedCapture &) = delete;
+
+ private:
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 struct Ring {
   char *mem = nullptr;
   cudaEvent_t event[kSlots] = {nullptr};   // the last transfer that used the slot
@@ -181,8 +193,7 @@ struct Pool {
   void GiveBack() {
     std::unique_lock<std::mutex> lock(use, std::try_to_lock);
     if (!lock.owns_lock() || std::chrono::steady_clock::now() - last_use < kIdle) return;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // (another thread may be capturing)
-    cudaThreadExchangeStreamCaptureMode(&mode);
+    RelaxedCapture relaxed;
     for (int d = 0; d < kMaxDevices; ++d) {
       Ring &r = ring[d];
       if (r.mem == nullptr || cudaSetDevice(d) != cudaSuccess) continue;
@@ -196,7 +207,6 @@ struct Pool {
       r.issued = 0;
     }
     cudaGetLastError();
-    cudaThreadExchangeStreamCaptureMode(&mode);
   }
 
   bool Prepare(int dev) {
@@ -210,12 +220,10 @@ struct Pool {
     }
     Ring &r = ring[dev];
     if (r.mem != nullptr) return true;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
+    RelaxedCapture relaxed;
     void *p = RingAlloc();
     bool ok = p != nullptr;
     for (cudaEvent_t &e : r.event) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-    cudaThreadExchangeStreamCaptureMode(&mode);
     if (!ok) {
       cudaGetLastError();
       for (cudaEvent_t &e : r.event) {
@@ -236,6 +244,7 @@ struct Pool {
 
   // The copy itself; `use` is held.
   cudaError_t Run(int dev, char *device, cudaStream_t stream) {
+    RelaxedCapture relaxed;
     Ring &r = ring[dev];
     mem = r.mem;
     first = r.issued;

@@ -53,3 +53,43 @@ def test_threads():
     for t in threads:
         t.join()
     assert not errors, errors[0]
+
+
+def test_copies_beside_a_stream_capture():
+    """A thread that copies does not break the capture of another one, and is not broken by it."""
+    import torch
+    import dvm_b200 as dvm
+    lib = _capi.load()
+    assert lib.dvm_rt_set_device(0) == 0
+    x, y = torch.arange(4096.0, device="cuda"), torch.zeros(4096, device="cuda")
+    k = dvm.PyKernel("vector")
+    a = k.load([4096], dvm.float32)
+    s = k.store(k.add(a, 1.0))
+    for op, t in ((a, x), (s, y)):
+        k.bind_device(op, t.data_ptr(), t.numel() * 4)
+    k.codegen()
+    k.launch(torch.cuda.current_stream().cuda_stream)
+    n = 4 * CHUNK + 77
+    src, dst = np.random.default_rng(9).integers(0, 256, n, dtype=np.uint8), np.zeros(n, np.uint8)
+    dev, own = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    rcs = []
+
+    def copy():
+        assert lib.dvm_rt_set_device(0) == 0
+        for _ in range(3):
+            rcs.append(lib.dvm_rt_memcpy_h2d(dev.data_ptr(), src.ctypes.data, n, own.cuda_stream))
+            rcs.append(lib.dvm_rt_memcpy_d2h(dst.ctypes.data, dev.data_ptr(), n, own.cuda_stream))
+
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=stream):   # (the default mode: unsafe calls of any thread are refused)
+        k.launch(stream.cuda_stream)
+        t = threading.Thread(target=copy)
+        t.start()
+        t.join()
+    own.synchronize()
+    assert rcs == [0] * 6 and np.array_equal(src, dst)
+    y.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, x + 1.0)
