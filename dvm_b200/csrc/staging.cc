@@ -357,8 +357,13 @@ cudaError_t Copy(void *device, void *host, size_t bytes, bool up, cudaStream_t s
     cudaGetLastError();
     return plain();
   }
-  int dev = -1;
+  // (the ring and its events are the current device's: a stream of another one cannot record them)
+  int dev = -1, stream_dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return plain();
+  if (cudaStreamGetDevice(stream, &stream_dev) != cudaSuccess || stream_dev != dev) {
+    cudaGetLastError();
+    return plain();
+  }
   Pool &p = Pool::Get();
   if (p.dead.load()) return plain();
   std::unique_lock<std::mutex> lock(p.use, std::try_to_lock);
