@@ -247,6 +247,8 @@ __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs
           }
       }
     }
+    // (while every score of a row has been -inf its maximum is -inf too, and -inf - -inf would be NaN: nothing is subtracted then)
+    const float from[2] = {m[0] == -CUDART_INF_F ? 0.0f : m[0], m[1] == -CUDART_INF_F ? 0.0f : m[1]};
 #pragma unroll
     for (uint32_t u = 0; u < NT; ++u) {
       uint32_t pf[4] = {0, 0, 0, 0};   // P as the A operand: rows q8 / q8 + 8, keys of n-tile 0 / 1
@@ -254,7 +256,7 @@ __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs
       for (uint32_t n = 0; n < 2; ++n)
 #pragma unroll
         for (uint32_t r = 0; r < 2; ++r) {
-          const float p0 = exp2_fast(x[u][r][n].x - m[r]), p1 = exp2_fast(x[u][r][n].y - m[r]);
+          const float p0 = exp2_fast(x[u][r][n].x - from[r]), p1 = exp2_fast(x[u][r][n].y - from[r]);
           l[r] += p0 + p1;
           pf[2 * n + r] = pack2<DT>(p0, p1);
         }

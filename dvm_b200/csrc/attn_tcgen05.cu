@@ -413,7 +413,9 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
             __syncwarp();
           }
           if (turns) turn_wait(my_turn);
-          const uint64_t mneg = f2(-m_used, -m_used), log2e = f2(kLog2e, kLog2e);
+          // (a maximum of -inf - every score so far - is not subtracted: -inf - -inf would be NaN, which l and O keep)
+          const float from = m_used == -CUDART_INF_F ? 0.0f : m_used;
+          const uint64_t mneg = f2(-from, -from), log2e = f2(kLog2e, kLog2e);
 #pragma unroll
           for (int i = 0; i < 64; ++i) {
             const float2 x = unpack2<DT>(pk[i]);
@@ -459,7 +461,8 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
             __syncwarp();
           }
           if (turns) turn_wait(my_turn);
-          const uint64_t mneg = f2(-m_used, -m_used);
+          const float from = m_used == -CUDART_INF_F ? 0.0f : m_used;   // (as above)
+          const uint64_t mneg = f2(-from, -from);
 #pragma unroll
           for (int i = 0; i < 64; ++i) {
             const float2 t = halves(add2(f2(u2f(s[2 * i]), u2f(s[2 * i + 1])), mneg));
