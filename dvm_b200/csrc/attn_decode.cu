@@ -99,6 +99,10 @@ __device__ __forceinline__ float2 score2(float a, float b, float scale, uint32_t
   return x;
 }
 
+// Factor of a partial result whose scores had the maximum `m`, in one of maximum `top`.  A partial without a finite score
+// counts nothing, but is multiplied all the same: its sums are 0, or NaN where a score was NaN, which the result has to show.
+__device__ __forceinline__ float weight_of(float m, float top) { return m == -CUDART_INF_F ? 0.0f : exp2_fast(m - top); }
+
 template <uint32_t D>
 struct Combine {
   float m[kWarps][kRows], l[kWarps][kRows];
@@ -306,7 +310,7 @@ __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs
     for (uint32_t w = 1; w < kWarps; ++w) top = fmaxf(top, sm.m[w][row]);
     float sum = 0.0f;
 #pragma unroll
-    for (uint32_t w = 0; w < kWarps; ++w) sum += sm.m[w][row] == -CUDART_INF_F ? 0.0f : sm.o[w][row][col] * exp2_fast(sm.m[w][row] - top);
+    for (uint32_t w = 0; w < kWarps; ++w) sum += sm.o[w][row][col] * weight_of(sm.m[w][row], top);
     sm.o[0][row][col] = sum;
   }
   __syncthreads();
@@ -315,7 +319,7 @@ __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs
 #pragma unroll
     for (uint32_t w = 1; w < kWarps; ++w) top = fmaxf(top, sm.m[w][tid]);
 #pragma unroll
-    for (uint32_t w = 0; w < kWarps; ++w) sum += sm.m[w][tid] == -CUDART_INF_F ? 0.0f : sm.l[w][tid] * exp2_fast(sm.m[w][tid] - top);
+    for (uint32_t w = 0; w < kWarps; ++w) sum += sm.l[w][tid] * weight_of(sm.m[w][tid], top);
     sm.m[0][tid] = top;
     sm.l[0][tid] = sum;
   }
@@ -336,9 +340,7 @@ __device__ __forceinline__ void decode_body(const AttnParam &P, const DecodeArgs
       for (uint32_t c = 0; c < CL; ++c) top = fmaxf(top, ld_peer(&sm.m[0][row], c));
       a = b = sum = 0.0f;
       for (uint32_t c = 0; c < CL; ++c) {
-        const float mc = ld_peer(&sm.m[0][row], c);
-        if (mc == -CUDART_INF_F) continue;   // (no keys)
-        const float f = exp2_fast(mc - top);
+        const float f = weight_of(ld_peer(&sm.m[0][row], c), top);
         a += ld_peer(&sm.o[0][row][col], c) * f;
         b += ld_peer(&sm.o[0][row][col + 1], c) * f;
         sum += ld_peer(&sm.l[0][row], c) * f;

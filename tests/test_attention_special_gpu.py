@@ -1,4 +1,4 @@
-"""Attention with scores that overflow to -inf: in the first keys of a warp, of a key tile, of all of them."""
+"""Attention with scores that overflow to -inf and with NaN: in the first keys of a warp, of a key tile, of all of them."""
 import numpy as np
 import pytest
 
@@ -46,3 +46,16 @@ def test_scores_of_minus_infinity(sq, skv, d, where, scale_first):
     # a score of size |s| is rounded twice (relative error of p: 2 |s| unit), p and the result once each
     largest = np.where(np.isfinite(s), np.abs(s), 0.0).max()
     assert np.all(np.abs(got[ok] - want[ok]) <= 2.0 ** -11 * (2.0 * largest + 2.0) * float(np.abs(v).max()))
+
+
+@pytest.mark.parametrize("scale_first", [True, False])
+@pytest.mark.parametrize("sq,skv,d", SHAPES)
+@pytest.mark.parametrize("count", [1, 16, 128])
+def test_nan_reaches_the_result(sq, skv, d, count, scale_first):
+    """A NaN score makes its row's sum, and so every element of the row's result, NaN - also where it is all that a warp sees."""
+    rng = np.random.default_rng(sq + skv + d)
+    q, k, v = (rng.standard_normal((2, 1, s, d)).astype(np.float16) for s in (sq, skv, skv))
+    at = skv // 2 // 16 * 16
+    k[1, 0, at:at + count] = np.nan
+    got = _attention(q, k, v, 1.0 / np.sqrt(d), scale_first)
+    assert np.all(np.isnan(got[1])) and not np.any(np.isnan(got[0]))
