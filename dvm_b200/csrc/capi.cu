@@ -561,7 +561,7 @@ int dvm_perf_stages(dvm_kernel *k, int warmup, int reps, void *stream, float *me
       for (int it = 0; it < warmup + reps; ++it) {
         cudaEventRecord(ev[0], s);
         for (size_t i = 0; i < n; ++i) {
-          int rc = vk->LaunchStage(i, stream);
+          int rc = vk->LaunchStage(i, stream, stream);
           if (rc != 0) return rc;
           cudaEventRecord(ev[i + 1], s);
         }

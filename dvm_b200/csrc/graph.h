@@ -215,7 +215,8 @@ class VKernel {
   void CompileFresh();
   void Bind(const RelocEntry *relocs, size_t n, void *workspace, size_t workspace_bytes = ~static_cast<size_t>(0));
   int Launch(void *stream);
-  int LaunchStage(size_t index, void *stream);   // one launch (or collective) of the plan, for per-stage timing
+  int LaunchStage(size_t index, void *stream, void *launch_stream);   // one launch (or collective) of the plan, of Launch(launch_stream)
+  bool MayRepack(void *stream);                  // a launch on this stream may copy operands to the workspace
   int LaunchPipelined(void *stream);             // a plan with two lanes (see Stage::lane)
   void *side_stream_ = nullptr;                  // lane 1; created at the first pipelined launch
   std::vector<void *> stage_events_;             // one event per stage that another lane waits for
@@ -251,6 +252,8 @@ class VKernel {
   uint64_t plan_clock_ = 0;
   int cur_sub_ = 0;                        // sub-kernel that NewNode() tags ops with (SequenceAdd / ParallelAdd advance it)
   void *workspace_ = nullptr;
+  bool repack_owned_ = false;
+  unsigned long long repack_stream_ = 0;   // id of the stream whose launches repack operands (when owned)
   bool normalized_ = false;
   bool compiled_ = false;
   bool bound_ = false;                     // Bind() has given the plan in use its addresses

@@ -298,7 +298,7 @@ int VKernel::LaunchPipelined(void *stream) {
         return static_cast<int>(cudaGetLastError());
     }
     side_used |= st.lane != 0;
-    int err = LaunchStage(i, s);
+    int err = LaunchStage(i, s, stream);
     if (err != 0) return err;
     if (signals[i]) {
       if (stage_events_[i] == nullptr) {
@@ -335,13 +335,32 @@ int VKernel::Launch(void *stream) {
   for (auto &st : stages_)
     if (st->lane != 0) return LaunchPipelined(stream);
   for (size_t i = 0; i < stages_.size(); ++i) {
-    int err = LaunchStage(i, stream);
+    int err = LaunchStage(i, stream, stream);
     if (err != 0) return err;
   }
   return 0;
 }
 
-int VKernel::LaunchStage(size_t index, void *stream) {
+// Launches of one kernel on several streams, bound to other tensors in between, are independent of one another where the plan
+// needs no workspace, and have to stay so although a repacked operand lies in one: the workspace belongs to the first
+// stream that repacks there, launches on any other read the rows as they lie (matmul [1024, 1001]^T [1001, 5003]: 56 instead of
+// 23 us).  Nor does a captured launch repack: its graph may be replayed on any stream, and when the workspace is gone.
+bool VKernel::MayRepack(void *stream) {
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;   // (unlike the handle, the id of a stream that is gone does not come back)
+  if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone || cudaStreamGetId(s, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (!repack_owned_) {
+    repack_owned_ = true;
+    repack_stream_ = id;
+  }
+  return repack_stream_ == id;
+}
+
+int VKernel::LaunchStage(size_t index, void *stream, void *launch_stream) {
   if (!compiled_ || index >= stages_.size()) DvmException("LaunchStage: no such stage");
   auto &stp = stages_[index];
   if (Idle(*stp)) return 0;
@@ -353,6 +372,11 @@ int VKernel::LaunchStage(size_t index, void *stream) {
       if (mm.param.a_ptr == 0 || mm.param.b_ptr == 0) DvmException("Launch with an unbound tensor address");
       for (size_t s = 0; s < mm.slot_obj.size(); ++s)
         if (mm.slot_obj[s] && mm.param.tensor[s].ptr == 0) DvmException("Launch with an unbound tensor address");
+      if ((mm.param.a_pack | mm.param.b_pack) != 0 && !MayRepack(launch_stream)) {
+        dvmb::MmParam as_it_lies = mm.param;
+        as_it_lies.a_pack = as_it_lies.b_pack = 0;
+        return dvmb::LaunchMatMul(as_it_lies, stream);
+      }
       return dvmb::LaunchMatMul(mm.param, stream);
     }
     if (stp->kind == STAGE_COLLECTIVE) {

@@ -32,3 +32,62 @@ def test_both_paths(batch, m, n, k, trans):
     assert lib.dvm_launch_reloc(t._k, relocs, len(relocs), None, None) == 0, _capi.last_error()   # no workspace
     assert lib.dvm_rt_sync(None) == 0, _capi.last_error()
     assert np.all(np.abs(t.output(s).astype(np.float64) - want) <= bound)
+
+
+@pytest.mark.parametrize("trans", [False, True])
+def test_one_kernel_on_two_streams(trans):
+    """Launches on two streams, bound to other tensors in between, do not see each other's operands."""
+    import torch
+    import dvm_b200 as dvm
+    m, n, kk, rounds = 515, 2001, 1001, 12
+    g = torch.Generator(device="cuda").manual_seed(1)
+    k = dvm.PyKernel("mix")
+    la, lb = k.load([kk, m] if trans else [m, kk], dvm.float16), k.load([kk, n], dvm.float16)
+    st = k.store(k.matmul(la, lb, trans, False))
+    sets = []
+    for _ in range(rounds):
+        a, b = (torch.randn(shape, generator=g, device="cuda").half() for shape in ((kk, m) if trans else (m, kk), (kk, n)))
+        sets.append((a, b, torch.zeros((m, n), device="cuda", dtype=torch.float16)))
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for i, tensors in enumerate(sets):
+        for op, t in zip((la, lb, st), tensors):
+            k.bind_device(op, t.data_ptr(), t.numel() * 2)
+        k.codegen()
+        k.launch(streams[i % 2].cuda_stream)
+    torch.cuda.synchronize()
+    for a, b, c in sets:
+        want = (a.double().T if trans else a.double()) @ b.double()
+        # (the bound of test_both_paths, for operands of size 1)
+        bound = 2.0 ** -11 * want.abs() + 2.0 ** -24 * (kk + 1.0) * kk ** 0.5 + 2.0 ** -25
+        assert bool(((c.double() - want).abs() <= bound).all())
+
+
+def test_captured_launch_needs_no_workspace():
+    """The graph of a captured launch is replayed after the kernel, and with it its workspace, is gone."""
+    import gc
+    import torch
+    import dvm_b200 as dvm
+    m, n, kk = 300, 1001, 257
+    a, b = torch.randn((m, kk), device="cuda").half(), torch.randn((kk, n), device="cuda").half()
+    c = torch.zeros((m, n), device="cuda", dtype=torch.float16)
+    k = dvm.PyKernel("mix")
+    la, lb = k.load([m, kk], dvm.float16), k.load([kk, n], dvm.float16)
+    st = k.store(k.matmul(la, lb, False, False))
+    for op, t in ((la, a), (lb, b), (st, c)):
+        k.bind_device(op, t.data_ptr(), t.numel() * 2)
+    k.codegen()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    k.launch(stream.cuda_stream)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        k.launch(stream.cuda_stream)
+    del k, la, lb, st
+    gc.collect()
+    a.copy_(torch.randn((m, kk), device="cuda"))
+    c.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    want = a.double() @ b.double()
+    bound = 2.0 ** -11 * want.abs() + 2.0 ** -24 * (kk + 1.0) * kk ** 0.5 + 2.0 ** -25
+    assert bool(((c.double() - want).abs() <= bound).all())
