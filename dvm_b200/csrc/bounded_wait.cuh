@@ -29,11 +29,12 @@ struct LaunchTag {
   uint32_t pad;
   volatile uint32_t *host_flag;
 };
-// Host side (runtime.cu): a tag with a fresh non-zero epoch; whether any wait may have expired since the flag was lowered.
+// Host side (runtime.cu): a tag with a fresh non-zero epoch; and whether a wait of a launch on the current device may have
+// expired since the last look, which lowers the device's flag.  To be called before the records are read: an expiry writes its
+// record first, so one that comes later raises the flag again, and a flag whose record has been read with others is lowered
+// by the next look.
 LaunchTag NextLaunchEpoch();
-bool ExpiryFlagRaised();
-void LowerExpiryFlag();
-void RaiseExpiryFlag();
+bool TakeExpiryFlag();
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void record_expiry(WaitStatus *st, uint32_t code, const LaunchTag &tag) {

@@ -477,8 +477,7 @@ int dvm_rt_memset(void *dst, int value, size_t bytes, void *stream) {
 // Reads (and clears) the status records of the device interpreters: a bounded device wait that expired (the kernel
 // then ran to its end with wrong results) is reported here as an error.  Does not wait for anything.
 int dvm_rt_check_status(void) {
-  if (!dvmb::ExpiryFlagRaised()) return 0;
-  dvmb::LowerExpiryFlag();   // (before the records are read: an expiry from here on raises it again)
+  if (!dvmb::TakeExpiryFlag()) return 0;
   const unsigned int rs = dvmb::ReadRowStatus(), vs = dvmb::ReadVectorStatus(), sv = vs != 0 ? vs : rs, sm = dvmb::ReadMatMulStatus(), sa = dvmb::ReadAttentionStatus();
   if ((sv | sm | sa) != 0) {
     char buf[160];
@@ -486,7 +485,6 @@ int dvm_rt_check_status(void) {
     g_error = buf;
     return -1;
   }
-  dvmb::RaiseExpiryFlag();   // the record is another device's
   return 0;
 }
 // Waits for the stream, then reports like dvm_rt_check_status().

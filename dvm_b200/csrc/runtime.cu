@@ -10,22 +10,31 @@
 
 namespace dvmb {
 
-// One word for the whole process, mapped into every device's address space; null when it could not be had.
-static volatile uint32_t *ExpiryFlag() {
-  static volatile uint32_t *const flag = []() -> volatile uint32_t * {
+constexpr int kMaxFlagDevices = 64;
+
+// One word per device, mapped into every device's address space; null when they could not be had.
+static volatile uint32_t *ExpiryFlags() {
+  static volatile uint32_t *const flags = []() -> volatile uint32_t * {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // (the first launch may happen inside somebody's capture)
     cudaThreadExchangeStreamCaptureMode(&mode);
     void *p = nullptr;
-    if (cudaHostAlloc(&p, sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+    if (cudaHostAlloc(&p, kMaxFlagDevices * sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
       cudaGetLastError();
       p = nullptr;
     } else {
-      *static_cast<volatile uint32_t *>(p) = 0;
+      for (int i = 0; i < kMaxFlagDevices; ++i) static_cast<volatile uint32_t *>(p)[i] = 0;
     }
     cudaThreadExchangeStreamCaptureMode(&mode);
     return static_cast<volatile uint32_t *>(p);
   }();
-  return flag;
+  return flags;
+}
+// The word of the current device; null: none.
+static volatile uint32_t *ExpiryFlag() {
+  volatile uint32_t *const flags = ExpiryFlags();
+  int dev = -1;
+  if (flags == nullptr || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxFlagDevices) return nullptr;
+  return flags + dev;
 }
 
 LaunchTag NextLaunchEpoch() {
@@ -34,12 +43,12 @@ LaunchTag NextLaunchEpoch() {
   if (e == 0) e = counter.fetch_add(1, std::memory_order_relaxed) + 1;   // 0 means "no launch has failed yet"
   return {e, 0u, ExpiryFlag()};
 }
-bool ExpiryFlagRaised() { return ExpiryFlag() == nullptr || *ExpiryFlag() != 0; }
-void LowerExpiryFlag() {
-  if (ExpiryFlag() != nullptr) *ExpiryFlag() = 0;
-}
-void RaiseExpiryFlag() {
-  if (ExpiryFlag() != nullptr) *ExpiryFlag() = 1;
+bool TakeExpiryFlag() {
+  volatile uint32_t *const flag = ExpiryFlag();
+  if (flag == nullptr) return true;
+  if (*flag == 0) return false;
+  *flag = 0;
+  return true;
 }
 
 Runtime &Runtime::Get() {
