@@ -5,7 +5,9 @@
 //
 // Rules that every kernel launched with ChainAttribute() follows:
 //   - every thread calls chain_wait() before its first access to global memory, and no block leaves without it (a kernel
-//     counts as complete for the one after the next only because it has itself waited);
+//     counts as complete for the one after the next only because it has itself waited); prefetches to L2 may come earlier
+//     (attn_decode.cu, mm_tile.cu): they deliver nothing to the kernel, and L2 sees the writes that follow;
+//   - operands are read by ordinary loads (gload() of vm_ops.cuh), which stay behind the wait, not by non-coherent ones;
 //   - chain_launch() comes after the point from which the block needs nothing that a block of the next kernel could hold.
 #ifndef DVM_B200_CHAIN_CUH_
 #define DVM_B200_CHAIN_CUH_

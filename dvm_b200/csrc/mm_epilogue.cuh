@@ -30,10 +30,10 @@ __device__ __noinline__ void epi_fetch(const EpiTensor &t, const EpiPos &p, uint
     uint32_t s;
     switch (t.dtype) {
       case T_F32:
-      case T_I32: s = __ldg(reinterpret_cast<const uint32_t *>(base) + off); break;
+      case T_I32: s = gload(reinterpret_cast<const uint32_t *>(base) + off); break;
       case T_F16:
-      case T_BF16: s = widen(t.dtype, __ldg(reinterpret_cast<const unsigned short *>(base) + off)); break;
-      default: s = __ldg(base + off); break;
+      case T_BF16: s = widen(t.dtype, gload(reinterpret_cast<const unsigned short *>(base) + off)); break;
+      default: s = gload(base + off); break;
     }
 #pragma unroll
     for (int i = 0; i < kEpiLanes; ++i) out[i] = s;
@@ -44,18 +44,18 @@ __device__ __noinline__ void epi_fetch(const EpiTensor &t, const EpiPos &p, uint
     if (sh == 2) {
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
-        const uint4 r = __ldg(reinterpret_cast<const uint4 *>(base + ((off + 4 * g) << 2)));
+        const uint4 r = gload(reinterpret_cast<const uint4 *>(base + ((off + 4 * g) << 2)));
         out[4 * g] = r.x; out[4 * g + 1] = r.y; out[4 * g + 2] = r.z; out[4 * g + 3] = r.w;
       }
     } else if (sh == 1) {
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
-        const uint4 r = __ldg(reinterpret_cast<const uint4 *>(base + ((off + 8 * g) << 1)));
+        const uint4 r = gload(reinterpret_cast<const uint4 *>(base + ((off + 8 * g) << 1)));
         unpack4(t.dtype, make_uint4(r.x, r.y, 0, 0), &out[8 * g]);
         unpack4(t.dtype, make_uint4(r.z, r.w, 0, 0), &out[8 * g + 4]);
       }
     } else {
-      const uint4 r = __ldg(reinterpret_cast<const uint4 *>(base + off));
+      const uint4 r = gload(reinterpret_cast<const uint4 *>(base + off));
       unpack4(T_BOOL, make_uint4(r.x, 0, 0, 0), &out[0]);
       unpack4(T_BOOL, make_uint4(r.y, 0, 0, 0), &out[4]);
       unpack4(T_BOOL, make_uint4(r.z, 0, 0, 0), &out[8]);
@@ -70,10 +70,10 @@ __device__ __noinline__ void epi_fetch(const EpiTensor &t, const EpiPos &p, uint
       const size_t o = off + (size_t)((int64_t)i * t.sn);
       switch (t.dtype) {
         case T_F32:
-        case T_I32: v = __ldg(reinterpret_cast<const uint32_t *>(base) + o); break;
+        case T_I32: v = gload(reinterpret_cast<const uint32_t *>(base) + o); break;
         case T_F16:
-        case T_BF16: v = widen(t.dtype, __ldg(reinterpret_cast<const unsigned short *>(base) + o)); break;
-        default: v = __ldg(base + o); break;
+        case T_BF16: v = widen(t.dtype, gload(reinterpret_cast<const unsigned short *>(base) + o)); break;
+        default: v = gload(base + o); break;
       }
     }
     out[i] = v;
@@ -208,8 +208,8 @@ __device__ __forceinline__ void run_epilogue(const MmParam &P, const EpiPos &pos
 }
 
 __device__ __forceinline__ float load_bias(const MmParam &P, uint32_t col) {
-  if (P.bias_dtype == T_F32) return __ldg(reinterpret_cast<const float *>(P.bias_ptr) + col);
-  const unsigned short raw = __ldg(reinterpret_cast<const unsigned short *>(P.bias_ptr) + col);
+  if (P.bias_dtype == T_F32) return gload(reinterpret_cast<const float *>(P.bias_ptr) + col);
+  const unsigned short raw = gload(reinterpret_cast<const unsigned short *>(P.bias_ptr) + col);
   if (P.bias_dtype == T_BF16) return __uint_as_float(static_cast<uint32_t>(raw) << 16);
   return __half2float(__ushort_as_half(raw));
 }

@@ -220,10 +220,10 @@ __device__ __forceinline__ void pair_body(const MmParam &P, const MmMaps &maps, 
       const uint32_t col = nb * BN + side_of(t) + col0_of(t) + lane;
       if (P.bias_dtype == T_F32) {
 #pragma unroll
-        for (uint32_t i = 0; i < kEpiCols / 32; ++i) bias[i] = __ldg(reinterpret_cast<const uint32_t *>(P.bias_ptr) + min(col + i * 32, P.N - 1));
+        for (uint32_t i = 0; i < kEpiCols / 32; ++i) bias[i] = gload(reinterpret_cast<const uint32_t *>(P.bias_ptr) + min(col + i * 32, P.N - 1));
       } else {
 #pragma unroll
-        for (uint32_t i = 0; i < kEpiCols / 32; ++i) bias[i] = __ldg(reinterpret_cast<const unsigned short *>(P.bias_ptr) + min(col + i * 32, P.N - 1));
+        for (uint32_t i = 0; i < kEpiCols / 32; ++i) bias[i] = gload(reinterpret_cast<const unsigned short *>(P.bias_ptr) + min(col + i * 32, P.N - 1));
       }
     };
     if (unit < num_items) look_up(unit);

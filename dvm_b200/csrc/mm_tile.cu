@@ -87,8 +87,8 @@ __device__ __forceinline__ void load_at(const Gather &g, uint32_t row, uint32_t 
   const uint64_t a = s & ~15ull;
   p.off = (uint32_t)(s & 15ull) >> 1;
   // (a 16-byte unit that holds at least one element of the row never leaves the row's memory page)
-  p.lo = __ldg(reinterpret_cast<const uint4 *>(a));
-  if (p.off + p.valid > 8u) p.hi = __ldg(reinterpret_cast<const uint4 *>(a) + 1);
+  p.lo = gload(reinterpret_cast<const uint4 *>(a));
+  if (p.off + p.valid > 8u) p.hi = gload(reinterpret_cast<const uint4 *>(a) + 1);
 }
 __device__ __forceinline__ void load_piece(const Gather &g, uint32_t i, uint32_t mn0, uint32_t k0, Piece &p) {
   uint32_t row, col;

@@ -220,13 +220,21 @@ __device__ __forceinline__ uint32_t widen(uint32_t dtype, uint32_t raw) {
   }
 }
 
+// Operands are read by ordinary loads, not by __ldg: a launch may begin while the one before it still writes them (chain.cuh),
+// a non-coherent load is for data that nobody writes as long as the kernel lives, and the compiler may move it to the other
+// side of the wait.
+template <typename T>
+__device__ __forceinline__ T gload(const T *p) {
+  return *p;
+}
+
 __device__ __forceinline__ uint32_t load_elem(uint32_t dtype, const uint8_t *base, uint32_t off) {
   switch (dtype) {
     case T_F32:
-    case T_I32: return __ldg(reinterpret_cast<const uint32_t *>(base) + off);
+    case T_I32: return gload(reinterpret_cast<const uint32_t *>(base) + off);
     case T_F16:
-    case T_BF16: return widen(dtype, __ldg(reinterpret_cast<const unsigned short *>(base) + off));
-    default: return __ldg(base + off);
+    case T_BF16: return widen(dtype, gload(reinterpret_cast<const unsigned short *>(base) + off));
+    default: return gload(base + off);
   }
 }
 
@@ -272,14 +280,14 @@ __device__ __forceinline__ uint4 gload4(uint32_t dtype, const uint8_t *base, uin
   uint4 r = make_uint4(0, 0, 0, 0);
   switch (dtype) {
     case T_F32:
-    case T_I32: r = __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const uint32_t *>(base) + off)); break;
+    case T_I32: r = gload(reinterpret_cast<const uint4 *>(reinterpret_cast<const uint32_t *>(base) + off)); break;
     case T_F16:
     case T_BF16: {
-      uint2 v = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const unsigned short *>(base) + off));
+      uint2 v = gload(reinterpret_cast<const uint2 *>(reinterpret_cast<const unsigned short *>(base) + off));
       r.x = v.x; r.y = v.y;
       break;
     }
-    default: r.x = __ldg(reinterpret_cast<const uint32_t *>(base + off)); break;
+    default: r.x = gload(reinterpret_cast<const uint32_t *>(base + off)); break;
   }
   return r;
 }

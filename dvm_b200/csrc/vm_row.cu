@@ -549,9 +549,9 @@ __device__ __forceinline__ uint4 shifted_unit(const unsigned short *base, int32_
   const uint64_t a = s & ~15ull, b0 = reinterpret_cast<uint64_t>(base), b1 = b0 + 2ull * len;
   const uint32_t off = (uint32_t)(s & 15ull) >> 1;
   uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
-  if (a + 16 > b0 && a < b1) lo = __ldg(reinterpret_cast<const uint4 *>(a));
+  if (a + 16 > b0 && a < b1) lo = gload(reinterpret_cast<const uint4 *>(a));
   if (off == 0) return lo;
-  if (a + 16 < b1) hi = __ldg(reinterpret_cast<const uint4 *>(a) + 1);
+  if (a + 16 < b1) hi = gload(reinterpret_cast<const uint4 *>(a) + 1);
   const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
   uint32_t p[6], q[5];
 #pragma unroll
