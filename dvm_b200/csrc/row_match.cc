@@ -174,7 +174,8 @@ struct Matcher {
       for (size_t pc = st.bsec[2 * p];; ++pc) {
         const Word w(st.bytecode[pc]);
         if (n >= static_cast<uint32_t>(kRowMaxCode)) return false;
-        if (w.opc == OP_ST && !scalar(w.sub, false)) return false;
+        // (only the last section stores: the compiler puts up to four stores there, a fifth stays in front of a body)
+        if (w.opc == OP_ST && (p != P.num_body || !scalar(w.sub, false))) return false;
         if ((w.opc == OP_COPY || w.opc == OP_BIN || w.opc == OP_CMP || w.opc == OP_SEL) && w.kind == K_TENSOR && !scalar(w.idx, true)) return false;
         if (w.opc == OP_RFIN && ((w.sub >> 4) != R_SUM || ((w.sub & 3u) != R->red_slot[0] && (w.sub & 3u) != R->red_slot[1]))) return false;
         R->code[n++] = w.w;

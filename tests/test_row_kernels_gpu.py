@@ -96,3 +96,25 @@ def test_scalar_sections_of_any_form_run_as_words():
     ad = np.maximum(np.sqrt((xd * xd).mean(1, keepdims=True)), 0.5)
     for st, want in zip(stores, [(xd - xd.mean(1, keepdims=True)) * ad, ad, xd.sum(1, keepdims=True)]):
         assert np.allclose(t.output(st), want, rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("stored", [1, 4, 5, 6])
+def test_any_number_of_stored_scalars(stored):
+    """(the compiler moves up to four stores of group scalars behind the last body; the others stay in front of it)"""
+    from dvm_b200.tester import Tester
+    rng = np.random.default_rng(stored)
+    x = rng.standard_normal((37, 1500)).astype(np.float32)
+    t = Tester("vector")
+    lx = t.load(x)
+    s1, s2 = t.sum(lx, (1,), True), t.sum(t.mul(lx, lx), (1,), True)
+    mean, square = t.mul(s1, 1.0 / 1500), t.mul(s2, 1.0 / 1500)
+    root = t.sqrt(t.add(square, 0.25))
+    scalars = [s1, s2, mean, square, root, t.mul(root, 2.0)][:stored]
+    stores = [t.store(t.mul(t.sub(lx, mean), root))] + [t.store(v) for v in scalars]
+    t.run()
+    xd = x.astype(np.float64)
+    d1, d2 = xd.sum(1, keepdims=True), (xd * xd).sum(1, keepdims=True)
+    rd = np.sqrt(d2 / 1500 + 0.25)
+    wants = [(xd - d1 / 1500) * rd, d1, d2, d1 / 1500, d2 / 1500, rd, 2 * rd]
+    for st, want in zip(stores, wants):
+        assert np.allclose(t.output(st), want, rtol=1e-5, atol=1e-4)   # (fp32 sums of 1500 terms of size 1)
