@@ -1796,12 +1796,18 @@ std::string DisassembleStage(const VectorStage &st) {
   using namespace dvmb;
   const VmParam &P = st.param;
   std::string o;
-  char buf[256];
+  char buf[384];
+  const char *kernel = "interpreter";   // what a launch runs, with the addresses bound last; the program is the same
+  if (st.row_ok) {
+    kernel = st.row.form == ROW_RMS_GATE ? "row_rms_gate" : "row_stats_affine";
+  } else if (st.direct_ok) {
+    kernel = "direct";
+  }
   snprintf(buf, sizeof(buf),
            "vmain.sm100(mode=%s, groups=%u, group_elems=%u, tg=%u, groups_per_cta=%u, chunk_elems=%u, rounds=%u, chunks=%u, grid=%u, "
-           "threads=%u, smem=%u, stages=%u x %u B%s, cluster=%u) {\n",
+           "threads=%u, smem=%u, stages=%u x %u B%s, cluster=%u, kernel=%s) {\n",
            P.mode == VM_FLAT ? "flat" : "group", P.num_groups, P.group_elems, P.tg, P.groups_per_cta, P.chunk_elems, P.rounds, P.chunks,
-           st.grid, st.threads, st.smem_bytes, P.num_stages, P.stage_bytes, P.resident ? " resident" : "", P.cluster);
+           st.grid, st.threads, st.smem_bytes, P.num_stages, P.stage_bytes, P.resident ? " resident" : "", P.cluster, kernel);
   o += buf;
   for (uint32_t t = 0; t < P.n_tensors; ++t) {
     const TensorDesc &td = P.tensor[t];
