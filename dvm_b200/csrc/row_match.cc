@@ -357,7 +357,7 @@ struct Matcher {
       R->have_gate = 1;
     }
     if (d.next().opc != OP_END) return false;
-    if (!Geometry(a) || R->runs != 1 || R->dtype == T_F32 || !Like(y, a, true)) return false;
+    if (!Geometry(a) || R->runs != 1 || R->run_len > kRowRmsMaxElems || R->dtype == T_F32 || !Like(y, a, true)) return false;
     R->shift = kAbsent;
     R->form = ROW_RMS_GATE;
     if (!AddStream(0, a) || !AddStream(3, y)) return false;
@@ -382,9 +382,10 @@ void MatchRowKernel(VectorStage *st) {
   static const bool off = getenv("DVM_B200_NO_ROW") != nullptr;
   if (off || st->idle || P.mode != VM_GROUP || P.num_body != 2) return;
   Matcher m(*st, &R);
-  if (m.StatsAffine()) return;
-  std::memset(&R, 0, sizeof(R));
+  // (an RMS norm has the statistics form too, with the sum of squares alone; the kernel of its own is several times as fast)
   if (m.RmsGate()) return;
+  std::memset(&R, 0, sizeof(R));
+  if (m.StatsAffine()) return;
   std::memset(&R, 0, sizeof(R));
 }
 

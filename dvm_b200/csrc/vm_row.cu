@@ -798,6 +798,7 @@ bool StatsPlan(uint32_t units, uint32_t groups, uint32_t sms, RowParam *p, uint3
 }
 
 constexpr uint32_t kRmsMaxUnits = 2 * kMaxRowThreads;
+static_assert(kRowRmsMaxElems == kRmsMaxUnits * 8, "two units of eight elements per thread");
 
 }  // namespace
 

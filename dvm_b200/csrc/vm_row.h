@@ -13,6 +13,7 @@ constexpr int kRowMaxStreams = 7;     // tensors walked element by element
 constexpr int kRowMaxScalars = 8;     // group scalars in memory (inputs and results of the scalar sections)
 constexpr int kRowMaxCode = 96;
 constexpr uint32_t kRowNone = 0xffu;
+constexpr uint32_t kRowRmsMaxElems = 8192;   // longest row of ROW_RMS_GATE: it stays in a CTA's registers
 
 enum RowForm : uint32_t {
   ROW_OFF = 0,

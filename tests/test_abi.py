@@ -378,3 +378,29 @@ def test_a_cloned_kernel_is_the_same_program_with_its_own_shapes():
     copy.input(x2, np.zeros((64, 800), np.float32))
     copy.codegen()
     assert list(s2.shape()) == [64, 1] and list(s.shape()) == [1, 512]
+
+
+def _launched(shape, form, dtype=dvm.bfloat16, dims=(1,)):
+    """The kernel that a launch of a normalisation runs, from its listing."""
+    k = dvm.PyKernel("vector", "das", 0)
+    x = k.load(list(shape), dtype)
+    count = 1.0
+    for d in dims:
+        count *= shape[d]
+    f = x if dtype == dvm.float32 else k.cast(x, dvm.float32)
+    if form == "rms":
+        scaled = k.mul(k.sum(k.mul(f, f), dims, True), 1.0 / count)
+        y = k.mul(f, k.div(1.0, k.sqrt(k.add(scaled, 1e-6))))
+    else:
+        mean = k.mul(k.sum(f, dims, True), 1.0 / count)
+        d = k.sub(f, mean)
+        y = k.div(d, k.sqrt(k.add(k.mul(k.sum(k.mul(d, d), dims, True), 1.0 / count), 1e-5)))
+    k.store(y if dtype == dvm.float32 else k.cast(y, dtype))
+    k.codegen()
+    return k.das().split("kernel=")[1].split(")")[0]
+
+
+@pytest.mark.parametrize("shape", [(1, 64), (37, 1031), (2000, 1024), (5000, 4096)])
+def test_an_rms_norm_runs_as_one(shape):
+    """(a sum of squares and a product with a group scalar is the statistics form as well)"""
+    assert _launched(shape, "rms") == "row_rms_gate"
