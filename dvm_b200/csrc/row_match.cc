@@ -399,7 +399,7 @@ void BindRow(VectorStage *st) {
   }
   for (uint32_t s = 0; s < P.n_tensors; ++s)
     if (R.scalar_of[s] != 0xff) R.scalar[R.scalar_of[s]].ptr = P.tensor[s].ptr;
-  st->row_ok = RowAddressesOk(R);
+  st->row_ok = RowAddressesOk(R) && RowKernelPays(R, P.chunk_elems);
 }
 
 void MatchDirectKernel(VectorStage *st) {

@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 #include <mutex>
@@ -819,7 +820,68 @@ bool RowAddressesOk(const RowParam &p) {
   const uint64_t units = static_cast<uint64_t>(p.runs) * UnitsPerRun(p);
   RowParam plan = {};
   uint32_t smem = 0;
-  return units < (1ull << 20) && StatsPlan(static_cast<uint32_t>(units), p.groups, 148, &plan, &smem);
+  const uint32_t sms = static_cast<uint32_t>(Runtime::Get().sm_count_or_default());
+  return units < (1ull << 20) && StatsPlan(static_cast<uint32_t>(units), p.groups, sms, &plan, &smem);
+}
+
+// Estimates of both kernels in microseconds, a fit to launches of 16 to 400 000 groups of 4 to 200 000 elements timed back to back
+// in either (runs of 1 to 256, aligned and not, fp16 and fp32, closed scalar sections and words).  What decides:
+//  - A statistics CTA takes 1.3 us for a group (2.3 with edges) however short it is, and 6 where the scalar sections run as words;
+//    the interpreter gives short groups a slice of a CTA: [100000, 64] fp16 432 us here and 62 there, [1200, 64] 7.7 and 10.7,
+//    [5000, 512] 23 and 31, [5000, 4096] 29 and 68; as words [5000, 1024] 104 and 37, [5000, 4095] 130 and 279.
+//  - An RMS row of up to 32 units takes a warp about 0.35 ns in all: [400000, 16] bf16 138 us and 37, [400000, 64] 148 and 144.
+//  - RMS rows of more than 512 units leave two CTAs on an SM: from 12 rows per SM on, rows that the interpreter's chunks divide
+//    are faster there ([5000, 6144] 78 and 58, [600, 6144] 9.6 and 10.3), others are not ([5000, 5120] 74 and 154); as
+//    words from 512 units and two rows per SM on ([5000, 8192] 155 and 77).
+bool RowKernelPays(const RowParam &p, uint32_t chunk_elems) {
+  const uint32_t sh = ElemShift(p), sms = static_cast<uint32_t>(Runtime::Get().sm_count_or_default()), units = UnitsPerRun(p);
+  const double groups = p.groups, n = static_cast<double>(p.runs) * p.run_len;
+  const bool closed = p.closed != 0, single = p.runs == 1;
+  const bool even = chunk_elems != 0 && static_cast<uint64_t>(p.runs) * p.run_len % chunk_elems == 0;   // no chunk is partly filled
+  // runs in whole units of 16 bytes, and in whole granules of four elements (what the interpreter loads at a time)
+  const bool whole = RunsAligned(p) && ((p.run_len << sh) & 15u) == 0;
+  uint64_t m = p.stream[0].ptr | (static_cast<uint64_t>(p.run_stride | p.run_len) << sh);
+  for (int j = 0; j < kMaxKept; ++j)
+    if (p.kept_size[j] != 1) m |= static_cast<uint64_t>(p.stream[0].kstride[j]) << sh;
+  const bool granules = (m & ((4u << sh) - 1u)) == 0;
+  double padded = 16.0;   // a short group's slice: a power of two of elements
+  while (padded < n) padded *= 2.0;
+
+  if (p.form == ROW_RMS_GATE) {
+    if (units <= 32u) {
+      const double w = p.have_w != 0, b = p.have_b != 0, g = p.have_gate != 0;
+      const double row = (closed ? 1.5 : 4.4) + groups * 1e-3 * (0.345 + 0.035 * w + 0.015 * b + 0.095 * g + (closed ? 0.0 : 0.65));
+      const double per_elem = 1e-6 * (5.0 + 1.5 * w + 3.3 * b + 6.2 * g) * (granules ? 1.0 : 2.2);
+      return row <= std::max(7.0 + 5.0 * b + 5.0 * g, 5.0 + groups * padded * per_elem);
+    }
+    if (!whole || !even) return true;
+    return closed ? units <= kMaxRowThreads || groups <= 12.0 * sms : units < kMaxRowThreads || groups <= 2.0 * sms;
+  }
+
+  RowParam plan = {};
+  uint32_t smem = 0;
+  if (!StatsPlan(p.runs * units, p.groups, sms, &plan, &smem)) return false;
+  const uint32_t slots = std::max(1u, (smem <= kHalfSm ? 2u : 1u) * sms / plan.cluster);
+  const double rounds = std::ceil(groups / slots);
+  // a single round answers sooner than the interpreter, but for a few rows that its chunks divide, as words
+  if (rounds <= 1.0) return closed || !(single && whole && even && n >= 1024.0 && n <= 8192.0);
+  const double per_group = closed ? std::max(whole ? 1.3 : 2.3, 0.6 + 0.035 * p.runs)
+                                  : (whole ? 6.0 : 7.1) + plan.per_cta * 16.0 * 7e-5 + (plan.cluster > 2 ? 3.0 : 0.0);
+  double base, ns;   // the interpreter: a launch, and every group
+  if (n <= 512.0) {
+    base = granules ? (closed ? 10.0 : 8.5) : (single ? 15.0 : 25.0);
+    ns = padded * 1e-3 * (single ? (granules ? 10.0 : 20.0) : (granules ? 15.0 : 22.0)) * (closed ? 1.0 : 0.8);
+  } else if (single) {
+    base = granules ? (!even && n > 2048.0 ? 12.5 : 4.5) : 11.0;
+    ns = granules ? 3.0 + 3.5 * std::ceil(n / 2048.0) + (even ? 0.0 : 14.0) : 11.0 + 0.0125 * n;
+  } else if (granules) {
+    base = p.run_len >= 512u ? 9.0 : 10.0;
+    ns = p.run_len >= 512u ? 5.0 + n * (p.run_len >= 2048u ? 2.5e-3 : 4.6e-3) : 9.0 + 0.0115 * n + (even ? 0.0 : 10.0);
+  } else {
+    base = 25.0;
+    ns = 30.0 + 0.022 * n;
+  }
+  return 1.3 + rounds * per_group <= base + groups * ns * 1e-3;
 }
 
 int LaunchRow(const RowParam &p_in, void *stream) {

@@ -1,4 +1,6 @@
 """Row kernels: normalisations over runs of any length and alignment, in every split of a group over CTAs, against float64."""
+import os
+
 import numpy as np
 import pytest
 
@@ -11,40 +13,63 @@ def _batchnorm(shape, dtype, offset=0):
     from dvm_b200.tester import Tester
     n, c, h, w = shape
     rng = np.random.default_rng(n + 3 * c + 7 * h + 11 * w)
-    x = (rng.standard_normal(shape) + rng.standard_normal((1, c, 1, 1))).astype(np.float16)
+    raw = (rng.standard_normal(shape) + rng.standard_normal((1, c, 1, 1))).astype(np.float32)
+    x = Tester.convert_to_bf16(raw) if dtype == "bfloat16" else raw.astype(dtype)
     g = rng.normal(1, 0.1, (1, c, 1, 1)).astype(np.float32)
     b = rng.normal(0, 0.1, (1, c, 1, 1)).astype(np.float32)
+    code = {"float16": 1, "bfloat16": 2, "float32": 3}[dtype]
     t = Tester("vector")
     if offset:
-        buf = np.zeros(x.size + offset, np.float16)
+        buf = np.zeros(x.size + offset, x.dtype)
         buf[offset:] = x.reshape(-1)
         lx = t.view_load(list(shape), [c * h * w, h * w, w, 1], buf, offset)
     else:
-        lx = t.load(x)
-    stores = [t.store(v) for v in W.batchnorm_train(t, lx, t.load(g), t.load(b), n * h * w)]
+        lx = t.load(x, dtype)
+    f = lx if code == 3 else t.cast(lx, 3)
+    count = 1.0 / (n * h * w)
+    if code == 3:   # (the sums as they are: deviations are for 16-bit inputs)
+        mean = t.mul(t.sum(f, (0, 2, 3), True), count)
+        var = t.sub(t.mul(t.sum(t.mul(f, f), (0, 2, 3), True), count), t.mul(mean, mean))
+        y = t.add(t.mul(t.mul(t.sub(f, mean), t.div(1.0, t.sqrt(t.add(var, 1e-5)))), t.load(g)), t.load(b))
+        stores = [t.store(v) for v in (y, mean, var)]
+    elif code == 2:
+        mean = t.mul(t.sum(f, (0, 2, 3), True), count)
+        xc = t.sub(f, mean)
+        var = t.mul(t.sum(t.mul(xc, xc), (0, 2, 3), True), count)
+        y = t.add(t.mul(t.div(xc, t.sqrt(t.add(var, 1e-5))), t.load(g)), t.load(b))
+        stores = [t.store(v) for v in (t.cast(y, 2), mean, var)]
+    else:
+        stores = [t.store(v) for v in W.batchnorm_train(t, lx, t.load(g), t.load(b), n * h * w)]
     t.run()
-    got = [t.output(s).astype(np.float64) for s in stores]
-    xd = x.astype(np.float64)
+    if not offset and "DVM_B200_NO_ROW" not in os.environ:
+        assert "kernel=row_stats_affine" in t.das()
+    read = lambda s: Tester.convert_from_bf16(t.output(s)) if s.dtype() == 2 else t.output(s)
+    got = [read(s).astype(np.float64) for s in stores]
+    xd = (Tester.convert_from_bf16(x) if code == 2 else x).astype(np.float64)
     m = xd.mean((0, 2, 3), keepdims=True)
     v = ((xd - m) ** 2).mean((0, 2, 3), keepdims=True)
     y = (xd - m) / np.sqrt(v + 1e-5) * g + b
-    # fp32 sums over the group in a tree, one rounding of the result to fp16
+    # fp32 sums over the group in a tree, one rounding of the result to its type; the plain fp32 sums of squares give the
+    # variance as a difference, off by a few 2^-24 of the mean square
+    square = float((xd * xd).mean((0, 2, 3)).max())
     assert np.allclose(got[1], m, rtol=1e-5, atol=1e-5 * float(np.abs(xd).max()))
-    assert np.allclose(got[2], v, rtol=1e-4, atol=1e-6)
-    assert np.all(np.abs(got[0] - y) <= 2.0 ** -10 * np.abs(y) + 1e-3), float(np.abs(got[0] - y).max())
+    assert np.allclose(got[2], v, rtol=1e-4, atol=1e-6 if code != 3 else 1e-6 + 2.0 ** -20 * square)
+    slack = 1e-3 if code != 3 else 1e-3 + 2.0 ** -21 * square / float((v + 1e-5).min()) * float(np.abs(y).max() + 1.0)
+    assert np.all(np.abs(got[0] - y) <= {1: 2.0 ** -10, 2: 2.0 ** -8, 3: 2.0 ** -20}[code] * np.abs(y) + slack), float(np.abs(got[0] - y).max())
 
 
 # planes of one unit and less, odd planes, runs that end on a unit, groups of one CTA, two, four and eight CTAs
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
 @pytest.mark.parametrize("shape", [(4, 5, 1, 3), (2, 3, 4, 2), (9, 17, 7, 7), (3, 300, 5, 5), (16, 20, 16, 16), (8, 6, 41, 43),
                                    (32, 4, 57, 55), (12, 3, 112, 111), (64, 2, 64, 64), (1, 4, 200, 203)])
-def test_batchnorm_planes(shape):
-    _batchnorm(shape, np.float16)
+def test_batchnorm_planes(shape, dtype):
+    _batchnorm(shape, dtype)
 
 
 @pytest.mark.parametrize("offset", [1, 3, 8])
 def test_batchnorm_input_at_any_address(offset):
     """(an input whose rows lie unlike the result's relative to 16 bytes goes to the interpreter)"""
-    _batchnorm((6, 5, 9, 9), np.float16, offset)
+    _batchnorm((6, 5, 9, 9), "float16", offset)
 
 
 @pytest.mark.parametrize("residual,weight,gate", [(1, 1, 1), (0, 1, 0), (1, 0, 0), (0, 0, 1)])
@@ -118,3 +143,42 @@ def test_any_number_of_stored_scalars(stored):
     wants = [(xd - d1 / 1500) * rd, d1, d2, d1 / 1500, d2 / 1500, rd, 2 * rd]
     for st, want in zip(stores, wants):
         assert np.allclose(t.output(st), want, rtol=1e-5, atol=1e-4)   # (fp32 sums of 1500 terms of size 1)
+
+
+@pytest.mark.parametrize("shape,dims", [((1300, 64), (1,)), ((2500, 63), (1,)), ((2500, 64), (1,)), ((2500, 500), (1,)), ((2500, 512), (1,)),
+                                        ((4, 2100, 3, 3), (0, 2, 3)), ((3, 5100, 2, 2), (0, 2, 3)), ((2, 2100, 5, 5), (0, 2, 3))])
+@pytest.mark.parametrize("dtype,code", [("float16", 1), ("bfloat16", 2)])
+def test_statistics_of_many_groups(shape, dims, dtype, code):
+    """Group counts and lengths on both sides of the line between the row kernel and the interpreter."""
+    from dvm_b200.tester import Tester
+    rng = np.random.default_rng(len(shape) + shape[-1])
+    raw = rng.standard_normal(shape).astype(np.float32)
+    x = raw.astype(np.float16) if code == 1 else Tester.convert_to_bf16(raw)
+    xd = (x if code == 1 else Tester.convert_from_bf16(x)).astype(np.float64)
+    n = float(np.prod([shape[d] for d in dims]))
+    t = Tester("vector")
+    f = t.cast(t.load(x, dtype), 3)
+    d = t.sub(f, t.mul(t.sum(f, dims, True), 1.0 / n))
+    st = t.store(t.cast(t.div(d, t.sqrt(t.add(t.mul(t.sum(t.mul(d, d), dims, True), 1.0 / n), 1e-3))), code))
+    t.run()
+    got = t.output(st)
+    got = (got if code == 1 else Tester.convert_from_bf16(got)).astype(np.float64)
+    m = xd.mean(dims, keepdims=True)
+    want = (xd - m) / np.sqrt(((xd - m) ** 2).mean(dims, keepdims=True) + 1e-3)
+    # one rounding of the result; the fp32 sums (deviations from the group's first element) in front of it
+    assert np.all(np.abs(got - want) <= {1: 2.0 ** -11, 2: 2.0 ** -8}[code] * np.abs(want) + 1e-4), float(np.abs(got - want).max())
+
+
+@pytest.mark.parametrize("rows,cols", [(20000, 16), (30000, 24), (30000, 17), (3000, 64), (2000, 6144), (1300, 4608)])
+def test_rms_norm_of_many_rows(rows, cols):
+    from dvm_b200.tester import Tester
+    rng = np.random.default_rng(cols)
+    x = Tester.convert_to_bf16(rng.standard_normal((rows, cols)).astype(np.float32))
+    t = Tester("vector")
+    f = t.cast(t.load(x, "bfloat16"), 3)
+    st = t.store(t.cast(t.mul(f, t.div(1.0, t.sqrt(t.add(t.mul(t.sum(t.mul(f, f), (1,), True), 1.0 / cols), 1e-6)))), 2))
+    t.run()
+    got = Tester.convert_from_bf16(t.output(st)).astype(np.float64)
+    xd = Tester.convert_from_bf16(x).astype(np.float64)
+    want = xd / np.sqrt((xd * xd).mean(1, keepdims=True) + 1e-6)
+    assert np.all(np.abs(got - want) <= 2.0 ** -8 * np.abs(want) + 1e-5)   # (one rounding to bf16)
