@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "graph.h"
+#include "runtime.h"
 
 namespace dvm {
 namespace {
@@ -372,8 +373,18 @@ struct Matcher {
 
 }  // namespace
 
-// The direct kernel takes launches of up to this many elements (see the note at MatchDirectKernel).
-constexpr uint32_t kDirectMaxElems = 1u << 20;
+// The direct kernel takes launches of up to this many elements: it starts sooner than the interpreter, which is the faster one once
+// it runs.  In us, direct | interpreter, launches of exp(x) * y + 0.5 back to back:
+//  - lengths that the interpreter's chunks divide: fp32 one wave of CTAs, five per SM (524 288: 3.25 | 3.41, 757 760: 3.29 | 4.05,
+//    819 200: 4.80 | 4.10); 16-bit types 2^18 (131 072: 3.15 | 3.12, 262 144: 3.24 | 3.16, 524 288: 3.79 | 3.21, 1 048 576: 6.19 | 3.72);
+//  - other lengths, where the last chunk takes it 3 us and more: 2^20 (bf16 500 000: 3.9 | 7.0, 1 000 000: 6.3 | 7.3).
+uint32_t DirectMaxElems(const VmParam &P) {
+  constexpr uint32_t kRagged = 1u << 20, kWhole16 = 1u << 18, kWaveElems = 5u * 1024u;
+  if (P.chunk_elems == 0 || P.group_elems % P.chunk_elems != 0) return kRagged;
+  bool wide = false;
+  for (uint32_t t = 0; t < P.n_tensors; ++t) wide |= P.tensor[t].dtype == T_F32 || P.tensor[t].dtype == T_I32;
+  return wide ? kWaveElems * static_cast<uint32_t>(Runtime::Get().sm_count_or_default()) : kWhole16;
+}
 
 void MatchRowKernel(VectorStage *st) {
   RowParam &R = st->row;
@@ -407,8 +418,7 @@ void MatchDirectKernel(VectorStage *st) {
   std::memset(&D, 0, sizeof(D));
   const VmParam &P = st->param;
   static const char *const most_env = getenv("DVM_B200_DIRECT_MAX");
-  static const uint32_t most = most_env ? static_cast<uint32_t>(atoi(most_env)) : kDirectMaxElems;
-  if (st->idle || P.mode != VM_FLAT || P.num_body != 1 || P.group_elems > most || P.n_tensors > static_cast<uint32_t>(kDirectTensors)) return;
+  if (st->idle || P.mode != VM_FLAT || P.num_body != 1 || P.group_elems > (most_env ? static_cast<uint32_t>(atoi(most_env)) : DirectMaxElems(P)) || P.n_tensors > static_cast<uint32_t>(kDirectTensors)) return;
   if (Word(st->bytecode[st->bsec[0]]).opc != OP_END || Word(st->bytecode[st->bsec[2]]).opc != OP_END) return;   // no group scalars
   uint8_t at[kMaxTensors];
   std::memset(at, 0xff, sizeof(at));

@@ -424,3 +424,15 @@ def test_an_rms_norm_runs_as_one(shape):
 ])
 def test_rows_go_to_the_faster_kernel(shape, form, dtype, dims, kernel):
     assert _launched(shape, form, dtype, dims) == kernel
+
+
+@pytest.mark.parametrize("n,dtype,kernel", [
+    (16000, dvm.bfloat16, "direct"), (262144, dvm.bfloat16, "direct"), (524288, dvm.bfloat16, "interpreter"), (524287, dvm.bfloat16, "direct"),
+    (524288, dvm.float32, "direct"), (819200, dvm.float32, "interpreter"), (1000001, dvm.float32, "direct"), (1048576, dvm.float32, "interpreter"),
+    (1048577, dvm.float16, "interpreter")])
+def test_short_programs_go_to_the_direct_kernel(n, dtype, kernel):
+    k = dvm.PyKernel("vector", "das", 0)
+    x, y = (k.load([n], dtype) for _ in range(2))
+    k.store(k.add(k.mul(k.exp(x), y), 0.5))
+    k.codegen()
+    assert k.das().split("kernel=")[1].split(")")[0] == kernel
