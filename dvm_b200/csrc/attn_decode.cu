@@ -392,12 +392,17 @@ int LaunchAttentionDecode(const AttnParam &p, void *stream) {
     attr_set[dev] = true;
   }
   const uint32_t sms = static_cast<uint32_t>(Runtime::Get().sm_count_or_default()), tiles = (p.skv + kTile - 1) / kTile;
+  const uint64_t slots = static_cast<uint64_t>(sms) * (p.d == 128 ? 2u : 3u);
   // CTAs per head: as many as run in one wave, while every warp has a step of keys (measured on 4 to 512 heads: a second,
   // partly filled wave costs more than the SMs a single one leaves idle); two where the heads alone fill more than a wave
-  // and their caches are long, which shortens the last one
-  const uint64_t slots = static_cast<uint64_t>(sms) * (p.d == 128 ? 2u : 3u);
+  // and their caches are long, which shortens the last one.
+  //   A first cut costs 1 us (one row of 64) to 4 (16 rows of 128, many heads: results read from one CTA by the other) and pays where
+  // it saves more steps than that: a CTA alone | two, in us, 16 rows of 128: 1 head of 128 keys 5.4 | 6.4, of 256 6.6 | 5.7 (four);
+  // 100 heads of 128 keys 5.5 | 8.5, of 512 9.1 | 11.0; one row: 100 heads of 192 keys 4.1 | 5.3.
+  //   Clusters of sixteen find room for eight at a time: 16 heads of 2048 keys of 128 10.9 us in them, 7.1 in clusters of eight.
+  const uint32_t first_cut = 16u + (4u * p.batch < sms ? 0u : p.sq > 8u ? 24u : p.sq > 4u ? 16u : 8u);   // in steps of 16 keys
   uint32_t cl = 1;
-  while (cl < 16u && p.batch * 2ull * cl <= slots && tiles >= 2u * cl * kWarps * (cl < 8u ? 1u : 2u)) cl *= 2;
+  while (cl < (p.batch <= 8u ? 16u : 8u) && p.batch * 2ull * cl <= slots && tiles >= (cl == 1u ? first_cut : 2u * cl * kWarps * (cl < 8u ? 1u : 2u))) cl *= 2;
   if (p.batch > slots && tiles >= 2u * kWarps * 8u) cl = 2;
   DecodeArgs a;
   a.cluster = cl;
