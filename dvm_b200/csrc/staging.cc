@@ -28,6 +28,8 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <new>
+#include <system_error>
 #include <thread>
 
 namespace dvmb {
@@ -214,10 +216,14 @@ struct Pool {
       started = true;
       cpu_set_t set;
       const int cpus = sched_getaffinity(0, sizeof(set), &set) == 0 ? CPU_COUNT(&set) : 1;
-      workers = cpus < 2 ? 1 : (static_cast<uint32_t>(cpus - 1) < kMaxWorkers ? static_cast<uint32_t>(cpus - 1) : kMaxWorkers);
-      for (uint32_t i = 0; i < workers; ++i) std::thread([this, i] { Worker(i == 0); }).detach();
-      pthread_atfork(nullptr, nullptr, [] { Get().dead = true; });
+      const uint32_t wanted = cpus < 2 ? 1 : std::min(static_cast<uint32_t>(cpus - 1), kMaxWorkers);
+      try {
+        for (; workers < wanted; ++workers) std::thread([this, keeper = workers == 0] { Worker(keeper); }).detach();
+      } catch (const std::system_error &) {   // (as many as the system grants)
+      }
+      pthread_atfork(nullptr, nullptr, [] { Get()->dead = true; });
     }
+    if (workers == 0) return false;   // (nobody would give the ring back)
     Ring &r = ring[dev];
     if (r.mem != nullptr) return true;
     RelaxedCapture relaxed;
@@ -237,9 +243,9 @@ struct Pool {
     return true;
   }
 
-  static Pool &Get() {
-    static Pool *const pool = new Pool();   // (never destroyed: its threads may outlive main)
-    return *pool;
+  static Pool *Get() {
+    static Pool *const pool = new (std::nothrow) Pool();   // (never destroyed: its threads may outlive main)
+    return pool;
   }
 
   // The copy itself; `use` is held.
@@ -364,9 +370,10 @@ cudaError_t Copy(void *device, void *host, size_t bytes, bool up, cudaStream_t s
     cudaGetLastError();
     return plain();
   }
-  Pool &p = Pool::Get();
-  if (p.dead.load()) return plain();
-  std::unique_lock<std::mutex> lock(p.use, std::try_to_lock);
+  Pool *const pool = Pool::Get();
+  if (pool == nullptr || pool->dead.load()) return plain();
+  Pool &p = *pool;
+  std::unique_lock<std::mutex> lock(p.use, std::try_to_lock);   // (nothing here throws: this runs behind a C entry)
   if (!lock.owns_lock() || !p.Prepare(dev)) return plain();
   p.host = static_cast<char *>(host);
   p.bytes = bytes;

@@ -1,4 +1,6 @@
 """Copies between pageable arrays and the device: sizes around the staged path's chunks and ring, several threads at once."""
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -93,3 +95,26 @@ def test_copies_beside_a_stream_capture():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, x + 1.0)
+
+
+def test_system_without_threads():
+    """Where no worker thread can be created the copy takes the driver's path; the caller, behind a C entry, sees no exception."""
+    code = """
+import resource
+import numpy as np
+from dvm_b200 import _capi
+lib = _capi.load()
+n = 40 << 20
+src = np.arange(n, dtype=np.uint8)
+assert lib.dvm_rt_set_device(0) == 0
+d = lib.dvm_rt_malloc(n)
+assert lib.dvm_rt_memcpy_h2d(d, src.ctypes.data, 64, None) == 0 and lib.dvm_rt_sync(None) == 0
+used = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (used + (1 << 20), resource.RLIM_INFINITY))   # (less than a thread's stack)
+rc = lib.dvm_rt_memcpy_h2d(d, src.ctypes.data, n, None)
+resource.setrlimit(resource.RLIMIT_AS, (resource.RLIM_INFINITY, resource.RLIM_INFINITY))
+assert rc in (0, 2), rc   # (the driver may need memory of its own: an error, no abort)
+print("DONE")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "DONE" in r.stdout, (r.returncode, r.stderr[-2000:])
