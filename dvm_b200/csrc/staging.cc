@@ -9,9 +9,12 @@
 // a call on two 4 MB arrays with a 4 MB result took 463 us, now 337.  The threads share a chunk in parts of 64 KB, so that the
 // first one is ready after 25 us.
 //
-// The ring (8 MB per device used, in huge pages) is allocated at the first copy that needs it and given back after ten seconds without
-// one.  One copy uses it at a time; a copy that finds it taken, one on a capturing stream, a small one, one of pinned memory
-// and any in a forked child goes to cudaMemcpyAsync as it is.
+// The ring (8 MB per device used, in huge pages) is set up once the copies of a stretch without a pause of a minute have moved
+// 32 MB by the driver's path, and given back after a minute without one: setting it up takes 2 to 4 ms, and up to 80 where the
+// system has to make room for huge pages - a process that calls once, or now and then, would pay that for nothing
+// (a call on two 4 MB arrays every eleven seconds took 2.8 to 84 ms with a ring set up at once and given back after ten
+// seconds, 1.6 by the driver, 0.64 with a ring that is still there).  One copy uses the ring at a time; a copy that finds it taken, one on a capturing stream, a small one, one
+// of pinned memory and any in a forked child goes to cudaMemcpyAsync as it is.
 #include "staging.h"
 
 #include <pthread.h>
@@ -42,7 +45,8 @@ constexpr uint32_t kParts = kChunk / kPart;
 constexpr size_t kSmall = 32 * 1024;   // (below this the driver's path is as fast: it sends small copies inside the command)
 constexpr int kMaxDevices = 64;
 constexpr uint32_t kMaxWorkers = 5;
-constexpr auto kIdle = std::chrono::seconds(10);
+constexpr auto kIdle = std::chrono::seconds(60);
+constexpr size_t kWorth = 32 * 1024 * 1024;   // (about what the driver's path copies in the time that setting up takes)
 // A worker looks for the next copy for this long before it sleeps: copies come in groups (two arguments and a result), and
 // waking a thread takes 50 us and more, half the time of a 4 MB copy.
 constexpr auto kLinger = std::chrono::microseconds(150);
@@ -105,6 +109,7 @@ struct Ring {
   char *mem = nullptr;
   cudaEvent_t event[kSlots] = {nullptr};   // the last transfer that used the slot
   uint64_t issued = 0;                     // transfers ever issued; number i used slot i % kSlots
+  size_t without = 0;                      // bytes that the copies of this stretch moved without a ring
 };
 
 struct Pool {
@@ -191,7 +196,7 @@ struct Pool {
     }
   }
 
-  // Frees rings that nothing has used for a while.
+  // Frees rings when nothing has been copied for a while.
   void GiveBack() {
     std::unique_lock<std::mutex> lock(use, std::try_to_lock);
     if (!lock.owns_lock() || std::chrono::steady_clock::now() - last_use < kIdle) return;
@@ -207,11 +212,21 @@ struct Pool {
       RingFree(r.mem);
       r.mem = nullptr;
       r.issued = 0;
+      r.without = 0;
     }
     cudaGetLastError();
   }
 
-  bool Prepare(int dev) {
+  // Whether the copy of `n` bytes goes through the ring, which is set up now if it has become worth it; `use` is held.
+  bool Prepare(int dev, size_t n) {
+    Ring &r = ring[dev];
+    const auto now = std::chrono::steady_clock::now(), before = last_use;
+    last_use = now;
+    if (r.mem != nullptr) return true;
+    if (now - before > kIdle) r.without = 0;
+    r.without += n;
+    if (r.without < kWorth) return false;
+    r.without = 0;   // (should the system refuse: again after as many bytes)
     if (!started) {
       started = true;
       cpu_set_t set;
@@ -224,8 +239,6 @@ struct Pool {
       pthread_atfork(nullptr, nullptr, [] { Get()->dead = true; });
     }
     if (workers == 0) return false;   // (nobody would give the ring back)
-    Ring &r = ring[dev];
-    if (r.mem != nullptr) return true;
     RelaxedCapture relaxed;
     void *p = RingAlloc();
     bool ok = p != nullptr;
@@ -374,7 +387,7 @@ cudaError_t Copy(void *device, void *host, size_t bytes, bool up, cudaStream_t s
   if (pool == nullptr || pool->dead.load()) return plain();
   Pool &p = *pool;
   std::unique_lock<std::mutex> lock(p.use, std::try_to_lock);   // (nothing here throws: this runs behind a C entry)
-  if (!lock.owns_lock() || !p.Prepare(dev)) return plain();
+  if (!lock.owns_lock() || !p.Prepare(dev, bytes)) return plain();
   p.host = static_cast<char *>(host);
   p.bytes = bytes;
   p.up = up;

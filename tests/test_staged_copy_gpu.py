@@ -13,6 +13,16 @@ pytestmark = pytest.mark.gpu
 PART, CHUNK, RING = 64 * 1024, 1024 * 1024, 8 * 1024 * 1024
 
 
+@pytest.fixture(autouse=True)
+def ring():
+    """The ring is set up once enough has been copied without it."""
+    lib = _capi.load()
+    assert lib.dvm_rt_set_device(0) == 0
+    src = np.zeros(4 * RING + 1, np.uint8)
+    d = lib.dvm_rt_malloc(src.size)
+    assert lib.dvm_rt_memcpy_h2d(d, src.ctypes.data, src.size, None) == 0 and lib.dvm_rt_sync(None) == 0 and lib.dvm_rt_free(d) == 0
+
+
 def _round_trip(lib, n, seed):
     src = np.random.default_rng(seed).integers(0, 256, n, dtype=np.uint8)
     dst = np.zeros(n + 1, np.uint8)
@@ -114,6 +124,25 @@ resource.setrlimit(resource.RLIMIT_AS, (used + (1 << 20), resource.RLIM_INFINITY
 rc = lib.dvm_rt_memcpy_h2d(d, src.ctypes.data, n, None)
 resource.setrlimit(resource.RLIMIT_AS, (resource.RLIM_INFINITY, resource.RLIM_INFINITY))
 assert rc in (0, 2), rc   # (the driver may need memory of its own: an error, no abort)
+print("DONE")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "DONE" in r.stdout, (r.returncode, r.stderr[-2000:])
+
+
+def test_copies_before_the_ring_is_worth_it():
+    """In a process of its own: arrays copied by the driver's path, then the one that has the ring set up, then through it."""
+    code = """
+import numpy as np
+from dvm_b200 import _capi
+lib = _capi.load()
+assert lib.dvm_rt_set_device(0) == 0
+for i, n in enumerate([40_000, 4_000_001, 9_000_000, 3_000_000, 5_000_000, 64 * 1024, 20_000_003]):
+    src, dst = np.random.default_rng(i).integers(0, 256, n, dtype=np.uint8), np.zeros(n, np.uint8)
+    d = lib.dvm_rt_malloc(n)
+    assert lib.dvm_rt_memcpy_h2d(d, src.ctypes.data, n, None) == 0 and lib.dvm_rt_memcpy_d2h(dst.ctypes.data, d, n, None) == 0
+    assert lib.dvm_rt_sync(None) == 0 and lib.dvm_rt_free(d) == 0
+    assert np.array_equal(src, dst), n
 print("DONE")
 """
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
