@@ -777,8 +777,9 @@ constexpr uint32_t kHalfSm = 112 * 1024, kWholeSm = 226 * 1024;
 // A group of `units` units in at most eight CTAs: the cluster, the buffers of each CTA and their size.  False: it does not fit.
 bool StatsPlan(uint32_t units, uint32_t groups, uint32_t sms, RowParam *p, uint32_t *smem) {
   const uint32_t half = kHalfSm - kStatsHeader - 1024u, whole = kWholeSm - kStatsHeader - 1024u;
-  // two CTAs per SM with two buffers each (the next group on its way while this one is worked on), then with one
-  // (the other CTA's copies overlap), then one CTA with one
+  // The smallest cluster that holds a group with two buffers per CTA, two CTAs per SM (the next group on its way while this one is
+  // worked on), then with one (the other CTA's copies overlap), then one CTA with one.  Layouts are not compared by the CTA slots
+  // that they fill: a [64, 256, 56, 56] batch-norm runs in 33 clusters of eight, 264 of 296 slots.
   uint32_t cl = 1, room = half / 2, buffers = 2;
   auto fits = [&]() { return (static_cast<uint64_t>(units) + cl - 1) / cl * 16u <= room; };
   while (cl < 8u && !fits()) cl *= 2;
@@ -824,7 +825,7 @@ bool RowAddressesOk(const RowParam &p) {
   return units < (1ull << 20) && StatsPlan(static_cast<uint32_t>(units), p.groups, sms, &plan, &smem);
 }
 
-// Estimates of both kernels in microseconds, a fit to launches of 16 to 400 000 groups of 4 to 200 000 elements timed back to back
+// Estimates of both kernels in microseconds, a fit to about 2000 launches of 16 to 400 000 groups of 4 to 200 000 elements timed back to back
 // in either (runs of 1 to 256, aligned and not, fp16 and fp32, closed scalar sections and words).  What decides:
 //  - A statistics CTA takes 1.3 us for a group (2.3 with edges) however short it is, and 6 where the scalar sections run as words;
 //    the interpreter gives short groups a slice of a CTA: [100000, 64] fp16 432 us here and 62 there, [1200, 64] 7.7 and 10.7,

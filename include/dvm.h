@@ -12,9 +12,9 @@
 //   * tensor addresses are borrowed device pointers, may be null while building and are supplied or
 //     replaced through RelocEntry at CodeGen()/Launch();
 //   * strings returned by Dump/DumpR/Das/Inspect stay valid until the next such call on the same Kernel.
-//   * a workspace belongs to one kernel, and to one launch at a time: launches of one kernel may be in flight on several streams,
-//     bound anew in between, only if they are given a workspace each - or none, when PreCodeGen() asks for nothing more than
-//     copies of unaligned MatMul operands (then the launch on the second stream reads the operands as they lie).
+//   * a workspace serves one kernel and one launch in flight.  (The copies of unaligned MatMul operands that a plan may keep there
+//     are made only by launches on the first stream that the kernel runs on, and by none that is captured: a kernel that needs its
+//     workspace for nothing else may be in flight on several streams, bound anew in between.)
 // A Kernel is not re-entrant; different phases may run on different threads one after another.
 #ifndef DVM_B200_DVM_H_
 #define DVM_B200_DVM_H_
