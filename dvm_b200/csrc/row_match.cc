@@ -1,6 +1,6 @@
 // Recognises the two normalisation shapes that the row kernels (vm_row.cu) run: works on the instruction words and the
 // tensor table that the vector compiler produced, so the graph may be written in any way that compiles to these bodies.
-// What does not match runs on the vector interpreter as before.  No counterpart in the reference, whose kernels run each
+// What does not match, scalar sections of another form among it, runs on the vector interpreter.  No counterpart in the reference, whose kernels run each
 // reduction and each group of element-wise ops as written (src/vm_gpu.cu:1552-1617).
 #include <cstdlib>
 #include <cstring>
@@ -30,19 +30,22 @@ struct Cursor {
   Word next() { return Word(code[pc++]); }
 };
 
-RowScalar ScalarOf(const Word &w, bool recip) {
-  RowScalar s;
-  std::memset(&s, 0, sizeof(s));
-  s.src = w.kind == K_SREG ? 0 : 1;
-  s.idx = static_cast<uint8_t>(w.idx);
-  s.imm = w.imm;
-  s.recip = recip ? 1 : 0;
+// Where a body's group scalar comes from: a scalar register, or none of that kind.
+struct BodyScalar {
+  bool present = false, is_register = false, recip = false;   // recip: the body divides by it
+  uint32_t idx = 0;
+};
+
+BodyScalar ScalarOf(const Word &w, bool recip) {
+  BodyScalar s;
+  s.present = true;
+  s.is_register = w.kind == K_SREG;
+  s.idx = w.idx;
+  s.recip = recip;
   return s;
 }
 
-const RowScalar kAbsent = {static_cast<uint8_t>(kRowNone), 0, 0, 0, 0};
-
-// A store of the accumulator to `tensor` in its own 16-bit or fp32 type, behind the rounding that store repeats anyway.
+// A store of the accumulator to `tensor` in its own type, behind the rounding that store repeats anyway.
 bool MatchStore(Cursor &c, const VmParam &P, uint32_t *slot) {
   uint32_t rnd = RN_NONE;
   if (c.at().opc == OP_CVT && c.at().sub == V_RND) rnd = c.next().rnd;
@@ -122,6 +125,8 @@ struct Matcher {
   const VectorStage &st;
   const VmParam &P;
   RowParam *R;
+  BodyScalar shift, chain[4];   // chain: subtract, multiply, multiply, add (ROW_RMS_GATE: chain[1] only)
+  uint32_t red_slot[2] = {kRowNone, kRowNone};   // reduction partials the sums belong to (kRowNone: not taken)
 
   Matcher(const VectorStage &s, RowParam *r) : st(s), P(s.param), R(r) {}
 
@@ -153,133 +158,124 @@ struct Matcher {
     R->dtype = td.dtype;
     R->groups = P.num_groups;
     for (int j = 0; j < kMaxKept; ++j) R->kept_size[j] = P.kept_size[j];
-    return td.dtype == T_F16 || td.dtype == T_BF16 || td.dtype == T_F32;
+    return td.dtype == T_F16 || td.dtype == T_BF16;
   }
 
-  bool Sections() {
-    R->num_sections = P.num_body + 1;
-    uint32_t n = 0;
+  // Enters the tensors that the scalar sections read and store.
+  bool Scalars() {
     std::memset(R->scalar_of, 0xff, sizeof(R->scalar_of));
-    auto scalar = [&](uint32_t slot, bool read) {
+    auto scalar = [&](uint32_t slot) {
       if (P.tensor[slot].mode != AM_SCALAR) return false;
       if (R->scalar_of[slot] == 0xff) {
         if (R->n_scalars >= static_cast<uint32_t>(kRowMaxScalars)) return false;
         R->scalar[R->n_scalars] = P.tensor[slot];
         R->scalar_of[slot] = static_cast<uint8_t>(R->n_scalars++);
       }
-      if (read) R->scalar_in |= 1u << R->scalar_of[slot];
       return true;
     };
-    for (uint32_t p = 0; p <= P.num_body; ++p) {
-      R->sec[p] = static_cast<uint16_t>(n);
+    for (uint32_t p = 0; p <= P.num_body; ++p)
       for (size_t pc = st.bsec[2 * p];; ++pc) {
         const Word w(st.bytecode[pc]);
-        if (n >= static_cast<uint32_t>(kRowMaxCode)) return false;
         // (only the last section stores: the compiler puts up to four stores there, a fifth stays in front of a body)
-        if (w.opc == OP_ST && (p != P.num_body || !scalar(w.sub, false))) return false;
-        if ((w.opc == OP_COPY || w.opc == OP_BIN || w.opc == OP_CMP || w.opc == OP_SEL) && w.kind == K_TENSOR && !scalar(w.idx, true)) return false;
-        if (w.opc == OP_RFIN && ((w.sub >> 4) != R_SUM || ((w.sub & 3u) != R->red_slot[0] && (w.sub & 3u) != R->red_slot[1]))) return false;
-        R->code[n++] = w.w;
+        if (w.opc == OP_ST && (p != P.num_body || !scalar(w.sub))) return false;
+        if ((w.opc == OP_COPY || w.opc == OP_BIN || w.opc == OP_CMP || w.opc == OP_SEL) && w.kind == K_TENSOR && !scalar(w.idx)) return false;
+        if (w.opc == OP_RFIN && ((w.sub >> 4) != R_SUM || ((w.sub & 3u) != red_slot[0] && (w.sub & 3u) != red_slot[1]))) return false;
         if (w.opc == OP_END) break;
       }
-    }
     return true;
   }
 
-  // The closed form of ROW_STATS_AFFINE's scalar sections (see RowParam::closed).
-  void CloseStats() {
+  // The closed form of ROW_STATS_AFFINE's scalar sections (see RowParam).
+  bool CloseStats() {
     Symbolic y;
     y.Run(st.bytecode, st.bsec[0]);
-    if (R->shift.src != 0 || R->red_slot[0] == kRowNone || R->red_slot[1] == kRowNone) return;
-    const int shift = y.sreg[R->shift.idx];
-    if (!y.ok || shift < 0 || y.e[shift].op != Symbolic::IN) return;
-    const uint32_t shift_slot = y.e[shift].v;
-    if (P.tensor[shift_slot].dtype != R->dtype) return;   // (the kernel writes it into a run's edge lanes: it must be a value of x's type)
+    if (!shift.present || !shift.is_register || red_slot[0] == kRowNone || red_slot[1] == kRowNone) return false;
+    const int s = y.sreg[shift.idx];
+    if (!y.ok || s < 0 || y.e[s].op != Symbolic::IN) return false;
+    const uint32_t shift_slot = y.e[s].v;
+    if (P.tensor[shift_slot].dtype != R->dtype) return false;   // (the kernel writes it into a run's edge lanes: it must be a value of x's type)
     y.Run(st.bytecode, st.bsec[2]);
-    auto value = [&](const RowScalar &c) { return c.src == 0 ? y.sreg[c.idx] : static_cast<int>(Symbolic::NONE); };
-    const int mean = value(R->chain[0]), den = value(R->chain[1]);
-    if (!y.ok || mean < 0 || den < 0 || !R->chain[1].recip || R->chain[2].recip) return;
-    const int T = y.Make(Symbolic::PART, R->red_slot[0]), Q = y.Make(Symbolic::PART, R->red_slot[1]);
+    auto value = [&](const BodyScalar &c) { return c.is_register ? y.sreg[c.idx] : static_cast<int>(Symbolic::NONE); };
+    const int mean = value(chain[0]), den = value(chain[1]);
+    if (!y.ok || mean < 0 || den < 0 || !chain[1].recip || chain[2].recip) return false;
+    const int T = y.Make(Symbolic::PART, red_slot[0]), Q = y.Make(Symbolic::PART, red_slot[1]);
     // den = sqrt(v + eps), v = (Q - T (T i1)) i2, mean = T i1 + s
-    if (y.e[mean].op != Symbolic::BIN || y.e[mean].v != B_ADD) return;
-    const int ti = y.e[mean].a == shift ? y.e[mean].b : y.e[mean].a;
-    if ((y.e[mean].a != shift && y.e[mean].b != shift) || !y.WithImm(ti, B_MUL, T, &R->i1)) return;
-    if (y.e[den].op != Symbolic::UN || y.e[den].v != U_SQRT) return;
+    if (y.e[mean].op != Symbolic::BIN || y.e[mean].v != B_ADD) return false;
+    const int ti = y.e[mean].a == s ? y.e[mean].b : y.e[mean].a;
+    if ((y.e[mean].a != s && y.e[mean].b != s) || !y.WithImm(ti, B_MUL, T, &R->i1)) return false;
+    if (y.e[den].op != Symbolic::UN || y.e[den].v != U_SQRT) return false;
     const int ve = y.e[den].a;
-    if (y.e[ve].op != Symbolic::BIN || y.e[ve].v != B_ADD) return;
+    if (y.e[ve].op != Symbolic::BIN || y.e[ve].v != B_ADD) return false;
     const int v = y.IsImm(y.e[ve].a, &R->eps) ? y.e[ve].b : y.e[ve].a;
-    if (!y.WithImm(ve, B_ADD, v, &R->eps)) return;
+    if (!y.WithImm(ve, B_ADD, v, &R->eps)) return false;
     const int dev = y.Bin(B_SUB, Q, y.Bin(B_MUL, T, ti));
-    if (!y.WithImm(v, B_MUL, dev, &R->i2)) return;
+    if (!y.WithImm(v, B_MUL, dev, &R->i2)) return false;
     R->at_gamma = R->at_beta = R->at_mean = R->at_var = kRowNone;
-    auto input = [&](const RowScalar &c, uint32_t *at) {
-      if (c.src == kRowNone) return true;
+    auto input = [&](const BodyScalar &c, uint32_t *at) {
+      if (!c.present) return true;
       const int i = value(c);
       if (i < 0 || y.e[i].op != Symbolic::IN) return false;
       *at = R->scalar_of[y.e[i].v];
       return true;
     };
-    if (!input(R->chain[2], &R->at_gamma) || !input(R->chain[3], &R->at_beta)) return;
+    if (!input(chain[2], &R->at_gamma) || !input(chain[3], &R->at_beta)) return false;
     y.Run(st.bytecode, st.bsec[4]);
-    if (!y.ok) return;
-    for (auto &s : y.stores) {
-      uint32_t *at = s.second == mean ? &R->at_mean : (s.second == v ? &R->at_var : nullptr);
-      if (at == nullptr || *at != kRowNone) return;
-      *at = R->scalar_of[s.first];
+    if (!y.ok) return false;
+    for (auto &stored : y.stores) {
+      uint32_t *at = stored.second == mean ? &R->at_mean : (stored.second == v ? &R->at_var : nullptr);
+      if (at == nullptr || *at != kRowNone) return false;
+      *at = R->scalar_of[stored.first];
     }
     R->at_shift = R->scalar_of[shift_slot];
-    R->closed = 1;
+    return true;
   }
 
   // ... and of ROW_RMS_GATE's.
-  void CloseRms() {
+  bool CloseRms() {
     Symbolic y;
     y.Run(st.bytecode, st.bsec[0]);
     y.Run(st.bytecode, st.bsec[2]);
-    if (!y.ok || R->chain[1].src != 0) return;
-    const int scale = y.sreg[R->chain[1].idx];
+    if (!y.ok || !chain[1].is_register) return false;
+    const int scale = y.sreg[chain[1].idx];
     float one = 0.0f;
-    if (scale < 0 || y.e[scale].op != Symbolic::BIN || y.e[scale].v != B_DIV_FAST || !y.IsImm(y.e[scale].a, &one) || one != 1.0f) return;
+    if (scale < 0 || y.e[scale].op != Symbolic::BIN || y.e[scale].v != B_DIV_FAST || !y.IsImm(y.e[scale].a, &one) || one != 1.0f) return false;
     const int root = y.e[scale].b;
-    if (y.e[root].op != Symbolic::UN || y.e[root].v != U_SQRT) return;
+    if (y.e[root].op != Symbolic::UN || y.e[root].v != U_SQRT) return false;
     const int sum = y.e[root].a;
-    if (y.e[sum].op != Symbolic::BIN || y.e[sum].v != B_ADD) return;
+    if (y.e[sum].op != Symbolic::BIN || y.e[sum].v != B_ADD) return false;
     const int scaled = y.IsImm(y.e[sum].a, &R->eps) ? y.e[sum].b : y.e[sum].a;
-    if (!y.WithImm(sum, B_ADD, scaled, &R->eps) || !y.WithImm(scaled, B_MUL, y.Make(Symbolic::PART, R->red_slot[0]), &R->i1)) return;
+    if (!y.WithImm(sum, B_ADD, scaled, &R->eps) || !y.WithImm(scaled, B_MUL, y.Make(Symbolic::PART, red_slot[0]), &R->i1)) return false;
     y.Run(st.bytecode, st.bsec[4]);
-    R->closed = y.ok && y.stores.empty() ? 1 : 0;
+    return y.ok && y.stores.empty();
   }
 
   bool StatsAffine() {
     Cursor c{st.bytecode, st.bsec[1]};
     if (c.at().opc != OP_COPY || c.at().kind != K_TENSOR) return false;
     const uint32_t x = c.next().idx;
-    R->shift = kAbsent;
-    if (c.at().bin(B_SUB) && c.at().scalar_operand()) R->shift = ScalarOf(c.next(), false);
-    R->red_slot[0] = R->red_slot[1] = kRowNone;
-    if (c.at().opc == OP_RACC && (c.at().sub >> 4) == R_SUM) R->red_slot[0] = c.next().sub & 3u;
+    if (c.at().bin(B_SUB) && c.at().scalar_operand()) shift = ScalarOf(c.next(), false);
+    if (c.at().opc == OP_RACC && (c.at().sub >> 4) == R_SUM) red_slot[0] = c.next().sub & 3u;
     if (c.at().bin(B_MUL) && c.at().kind == K_ACC) {
       c.next();
       if (c.at().opc != OP_RACC || (c.at().sub >> 4) != R_SUM) return false;
-      R->red_slot[1] = c.next().sub & 3u;
+      red_slot[1] = c.next().sub & 3u;
     }
-    if (c.next().opc != OP_END || (R->red_slot[0] == kRowNone && R->red_slot[1] == kRowNone)) return false;
+    if (c.next().opc != OP_END || (red_slot[0] == kRowNone && red_slot[1] == kRowNone)) return false;
     Cursor d{st.bytecode, st.bsec[3]};
     if (d.at().opc != OP_COPY || d.at().kind != K_TENSOR || d.next().idx != x) return false;
-    for (auto &s : R->chain) s = kAbsent;
     uint32_t stage = 0;   // subtract, multiply, multiply, add: each at most once, in this order
     for (;;) {
       const Word w = d.at();
       if (w.opc != OP_BIN || w.rnd != RN_NONE || !w.scalar_operand()) break;
       if (w.sub == B_SUB && stage == 0) {
-        R->chain[0] = ScalarOf(w, false);
+        chain[0] = ScalarOf(w, false);
         stage = 1;
       } else if ((w.sub == B_MUL || (w.sub == B_DIV_FAST && w.kind == K_SREG)) && stage <= 2) {
         const uint32_t at = stage < 2 ? 1 : 2;
-        R->chain[at] = ScalarOf(w, w.sub == B_DIV_FAST);
+        chain[at] = ScalarOf(w, w.sub == B_DIV_FAST);
         stage = at + 1;
       } else if (w.sub == B_ADD && stage <= 3) {
-        R->chain[3] = ScalarOf(w, false);
+        chain[3] = ScalarOf(w, false);
         stage = 4;
       } else {
         return false;
@@ -290,10 +286,7 @@ struct Matcher {
     if (!MatchStore(d, P, &y) || d.next().opc != OP_END) return false;
     if (!Geometry(x) || !Like(y, x, true)) return false;
     R->form = ROW_STATS_AFFINE;
-    if (!AddStream(0, x) || !AddStream(1, y) || !Sections()) return false;
-    CloseStats();
-    // (outside a run's edges the kernel counts lanes as the shift itself: x's own first element, or nothing subtracted)
-    return R->closed != 0 || R->shift.src == kRowNone;
+    return AddStream(0, x) && AddStream(1, y) && Scalars() && CloseStats();
   }
 
   // ((sigmoid(g)) * g) * u -> store (either order of the two products' operands is what the compiler emits)
@@ -330,8 +323,8 @@ struct Matcher {
       const size_t mark = c.pc;
       if (!body0_done && sum(c, &a, &b) && c.at().bin(B_MUL) && c.at().kind == K_ACC && c.at(1).opc == OP_RACC && (c.at(1).sub >> 4) == R_SUM) {
         c.next();
-        R->red_slot[0] = c.next().sub & 3u;
-        R->red_slot[1] = kRowNone;
+        red_slot[0] = c.next().sub & 3u;
+        red_slot[1] = kRowNone;
         body0_done = true;
         continue;
       }
@@ -345,9 +338,8 @@ struct Matcher {
     uint32_t a1 = 0, b1 = 0;
     R->have_b = 0;
     if (!sum(d, &a1, &b1) || a1 != a || b1 != b || R->have_b != have_b0) return false;
-    for (auto &s : R->chain) s = kAbsent;
     if (!d.at().bin(B_MUL) || !d.at().scalar_operand()) return false;
-    R->chain[1] = ScalarOf(d.next(), false);
+    chain[1] = ScalarOf(d.next(), false);
     if (d.at().bin(B_MUL) && d.at().kind == K_TENSOR) {
       w = d.next().idx;
       R->have_w = 1;
@@ -358,16 +350,13 @@ struct Matcher {
       R->have_gate = 1;
     }
     if (d.next().opc != OP_END) return false;
-    if (!Geometry(a) || R->runs != 1 || R->run_len > kRowRmsMaxElems || R->dtype == T_F32 || !Like(y, a, true)) return false;
-    R->shift = kAbsent;
+    if (!Geometry(a) || R->runs != 1 || R->run_len > kRowRmsMaxElems || !Like(y, a, true)) return false;
     R->form = ROW_RMS_GATE;
     if (!AddStream(0, a) || !AddStream(3, y)) return false;
     if (R->have_b && (!Like(b, a, true) || !AddStream(1, b))) return false;
     if (R->have_w && (!Like(w, a, false) || !AddStream(2, w))) return false;
     if (R->have_gate && (!Like(g, a, true) || !Like(u, a, true) || !Like(y2, a, true) || !AddStream(4, g) || !AddStream(5, u) || !AddStream(6, y2))) return false;
-    if (!Sections()) return false;
-    CloseRms();
-    return true;
+    return Scalars() && CloseRms();
   }
 };
 
@@ -392,11 +381,9 @@ void MatchRowKernel(VectorStage *st) {
   const VmParam &P = st->param;
   static const bool off = getenv("DVM_B200_NO_ROW") != nullptr;
   if (off || st->idle || P.mode != VM_GROUP || P.num_body != 2) return;
-  Matcher m(*st, &R);
-  // (an RMS norm has the statistics form too, with the sum of squares alone; the kernel of its own is several times as fast)
-  if (m.RmsGate()) return;
+  if (Matcher(*st, &R).RmsGate()) return;
   std::memset(&R, 0, sizeof(R));
-  if (m.StatsAffine()) return;
+  if (Matcher(*st, &R).StatsAffine()) return;
   std::memset(&R, 0, sizeof(R));
 }
 

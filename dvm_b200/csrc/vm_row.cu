@@ -12,8 +12,8 @@
 //                              memory, always in the same order.
 //   dvm_b200_row_rms_gate      a row per group of 32 to 512 threads, every load of the row in flight before the first use.
 //
-// The scalar sections (means, reciprocal roots, what is stored per group) stay programs: each warp runs the stage's own
-// instruction words on registers of its own.
+// The scalar sections (means, reciprocal roots, what is stored per group) are the usual ones, computed in closed form; stages with
+// others run on the interpreter.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -52,20 +52,15 @@ __device__ __forceinline__ uint4 ld_unit(const uint8_t *p) {
   return v;
 }
 
-// ---- units: 16 bytes at an aligned address, kE<DT> elements ------------------------------------------------
-template <uint32_t DT>
-constexpr uint32_t kE = DT == T_F32 ? 4u : 8u;
-template <uint32_t DT>
-constexpr uint32_t kShift = DT == T_F32 ? 2u : 1u;
+// ---- units: 16 bytes at an aligned address, kE elements of 16 bits -----------------------------------------
+constexpr uint32_t kE = 8;
 
 template <uint32_t DT>
-__device__ __forceinline__ void unpack_unit(const uint4 &q, float (&x)[kE<DT>]) {
+__device__ __forceinline__ void unpack_unit(const uint4 &q, float (&x)[kE]) {
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    if constexpr (DT == T_F32) {
-      x[i] = u2f(w[i]);
-    } else if constexpr (DT == T_BF16) {
+    if constexpr (DT == T_BF16) {
       x[2 * i] = u2f(w[i] << 16);
       x[2 * i + 1] = u2f(w[i] & 0xffff0000u);
     } else {
@@ -76,13 +71,11 @@ __device__ __forceinline__ void unpack_unit(const uint4 &q, float (&x)[kE<DT>]) 
   }
 }
 template <uint32_t DT>
-__device__ __forceinline__ uint4 pack_unit(const float (&x)[kE<DT>]) {
+__device__ __forceinline__ uint4 pack_unit(const float (&x)[kE]) {
   uint32_t w[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    if constexpr (DT == T_F32) {
-      w[i] = f2u(x[i]);
-    } else if constexpr (DT == T_BF16) {
+    if constexpr (DT == T_BF16) {
       w[i] = pack_bf16x2(x[2 * i], x[2 * i + 1]);
     } else {
       const __half2 h = __floats2half2_rn(x[2 * i], x[2 * i + 1]);
@@ -121,17 +114,17 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
   return r;
 }
 template <uint32_t DT>
-__device__ __forceinline__ void unpack_pairs(const uint4 &q, F2 (&x)[kE<DT> / 2]) {
-  float f[kE<DT>];
+__device__ __forceinline__ void unpack_pairs(const uint4 &q, F2 (&x)[kE / 2]) {
+  float f[kE];
   unpack_unit<DT>(q, f);
 #pragma unroll
-  for (uint32_t i = 0; i < kE<DT> / 2; ++i) x[i] = f2(f[2 * i], f[2 * i + 1]);
+  for (uint32_t i = 0; i < kE / 2; ++i) x[i] = f2(f[2 * i], f[2 * i + 1]);
 }
 template <uint32_t DT>
-__device__ __forceinline__ uint4 pack_pairs(const F2 (&x)[kE<DT> / 2]) {
-  float f[kE<DT>];
+__device__ __forceinline__ uint4 pack_pairs(const F2 (&x)[kE / 2]) {
+  float f[kE];
 #pragma unroll
-  for (uint32_t i = 0; i < kE<DT> / 2; ++i) {
+  for (uint32_t i = 0; i < kE / 2; ++i) {
     const float2 h = halves(x[i]);
     f[2 * i] = h.x;
     f[2 * i + 1] = h.y;
@@ -139,31 +132,23 @@ __device__ __forceinline__ uint4 pack_pairs(const F2 (&x)[kE<DT> / 2]) {
   return pack_unit<DT>(f);
 }
 // Zero outside lanes [lo, hi).
-template <uint32_t DT>
-__device__ __forceinline__ void mask_pairs(F2 (&x)[kE<DT> / 2], uint32_t lo, uint32_t hi) {
+__device__ __forceinline__ void mask_pairs(F2 (&x)[kE / 2], uint32_t lo, uint32_t hi) {
 #pragma unroll
-  for (uint32_t i = 0; i < kE<DT> / 2; ++i) {
+  for (uint32_t i = 0; i < kE / 2; ++i) {
     const float2 h = halves(x[i]);
     x[i] = f2(2 * i >= lo && 2 * i < hi ? h.x : 0.0f, 2 * i + 1 >= lo && 2 * i + 1 < hi ? h.y : 0.0f);
   }
 }
 // Lanes [lo, hi) of a unit to memory: whole units as one store, the ends of a run element by element.
-template <uint32_t DT>
 __device__ __forceinline__ void store_unit(uint8_t *p, const uint4 &q, uint32_t lo, uint32_t hi) {
-  if (lo == 0 && hi == kE<DT>) {
+  if (lo == 0 && hi == kE) {
     *reinterpret_cast<uint4 *>(p) = q;
     return;
   }
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-  for (uint32_t i = 0; i < kE<DT>; ++i)
-    if (i >= lo && i < hi) {
-      if constexpr (DT == T_F32) {
-        reinterpret_cast<uint32_t *>(p)[i] = w[i];
-      } else {
-        reinterpret_cast<unsigned short *>(p)[i] = (unsigned short)(w[i >> 1] >> (16u * (i & 1u)));
-      }
-    }
+  for (uint32_t i = 0; i < kE; ++i)
+    if (i >= lo && i < hi) reinterpret_cast<unsigned short *>(p)[i] = (unsigned short)(w[i >> 1] >> (16u * (i & 1u)));
 }
 
 __device__ __forceinline__ void group_coords(const RowParam &P, uint32_t g, uint32_t (&k)[kMaxKept]) {
@@ -178,60 +163,6 @@ __device__ __forceinline__ void group_coords(const RowParam &P, uint32_t g, uint
 __device__ __forceinline__ uint32_t group_offset(const uint32_t (&stride)[kMaxKept], const uint32_t (&k)[kMaxKept]) {
   return k[0] * stride[0] + k[1] * stride[1] + k[2] * stride[2];
 }
-
-// ---- scalar sections ---------------------------------------------------------------------------------------
-// Runs section `section` on the warp's own registers `sr` (shared memory; every lane does the same).  `in`: the group
-// scalars read from memory, fetched at kernel start; `total`: the finished sums by partial.
-__device__ __noinline__ void run_section(const RowParam &P, uint32_t section, volatile uint32_t *sr, const uint32_t *in, const float *total,
-                                         bool storer, const uint32_t (&k)[kMaxKept]) {
-  uint32_t acc[1] = {0};
-  for (uint32_t pc = P.sec[section];; ++pc) {
-    const uint64_t w = P.code[pc];
-    const uint32_t opc = DVMB_OPC(w), sub = DVMB_SUB(w), kind = DVMB_OKIND(w), idx = DVMB_OIDX(w);
-    if (opc == OP_END) break;
-    uint32_t b = DVMB_IMM(w);
-    if (kind == K_SREG) b = sr[idx];
-    if (kind == K_ACC) b = acc[0];
-    if (kind == K_TENSOR && (opc == OP_COPY || opc == OP_BIN || opc == OP_CMP || opc == OP_SEL)) b = in[P.scalar_of[idx]];
-    const SplatOperand bo{b};
-    switch (opc) {
-      case OP_ST:
-        if (storer) {
-          const TensorDesc &td = P.scalar[P.scalar_of[sub]];
-          store_elem(td.dtype, reinterpret_cast<uint8_t *>(td.ptr), group_offset(td.kstride, k), acc[0]);
-        }
-        break;
-      case OP_COPY: acc[0] = b; break;
-      case OP_MOV: sr[DVMB_DST(w)] = acc[0]; break;
-      case OP_UN: apply_un<1>(sub, acc); apply_round<1>(DVMB_RND(w), acc); break;
-      case OP_BIN: apply_bin<1>(sub, acc, bo); apply_round<1>(DVMB_RND(w), acc); break;
-      case OP_CMP: apply_cmp<1>(sub, DVMB_ISINT(w), acc, bo); break;
-      case OP_SEL: {
-        const uint32_t c[1] = {sr[sub & 15u]};
-        apply_sel<1>(DVMB_ISINT(w), DVMB_DST(w) & 1u, acc, bo, c);
-        break;
-      }
-      case OP_CVT: apply_cvt<1>(sub, acc); apply_round<1>(DVMB_RND(w), acc); break;
-      case OP_RFIN: acc[0] = f2u(total[sub & 3u]); break;
-      default: break;   // (a partial needs no reset here)
-    }
-  }
-  __syncwarp();
-}
-
-__device__ __forceinline__ float scalar_value(const RowScalar &s, const volatile uint32_t *sr, float absent) {
-  if (s.src == kRowNone) return absent;
-  float v = u2f(s.src == 0 ? sr[s.idx] : s.imm);
-  if (s.recip) v = fast_div(1.0f, v);
-  return v;
-}
-
-struct RowShared {
-  float part[kMaxWarps];         // sum of each warp
-  float total[kMaxWarps][4];     // finished sums by partial, per row of the CTA
-  uint32_t in[kMaxWarps][kRowMaxScalars];
-  uint32_t sr[kMaxWarps][kNumSRegs];
-};
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -249,9 +180,6 @@ constexpr uint32_t kMaxBuffers = 2;
 struct StatsShared {
   uint64_t full[kMaxBuffers], empty[kMaxBuffers], sums[2];
   float2 sum[2][8 * kWorkWarps];   // every warp's sums of every CTA of the cluster, in turn for one group and the next
-  float total[kWorkWarps][4];
-  uint32_t in[kRowMaxScalars];
-  uint32_t sr[kWorkWarps][kNumSRegs];
 };
 constexpr uint32_t kStatsHeader = (sizeof(StatsShared) + 127u) & ~127u;
 
@@ -282,7 +210,7 @@ __device__ __forceinline__ void work_sync() { asm volatile("bar.sync 1, %0;" ::"
 // kWhole: every run starts and ends on 16 bytes, so that every unit belongs to its run with all lanes.
 template <uint32_t DT, bool kWhole>
 __device__ __forceinline__ void stats_affine_body(const RowParam &P, const LaunchTag epoch) {
-  constexpr uint32_t E = kE<DT>, SH = kShift<DT>;
+  constexpr uint32_t E = kE, SH = 1;
   extern __shared__ __align__(128) uint8_t smem[];
   StatsShared &sm = *reinterpret_cast<StatsShared *>(smem);
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
@@ -359,7 +287,6 @@ __device__ __forceinline__ void stats_affine_body(const RowParam &P, const Launc
     __syncwarp();
   } else {
     // ------------------------------ working warps ------------------------------
-    const bool closed = P.closed != 0;
     const uint32_t n_units = u_end - u_begin;
     const uint32_t r_first = (u_begin + tid) / spr, c_first = u_begin + tid - r_first * spr;
     const uint32_t step_r = kWorkThreads / spr, step_c = kWorkThreads - step_r * spr;
@@ -373,20 +300,13 @@ __device__ __forceinline__ void stats_affine_body(const RowParam &P, const Launc
         const TensorDesc &td = P.scalar[i];
         return load_elem(td.dtype, reinterpret_cast<const uint8_t *>(td.ptr), group_offset(td.kstride, k));
       };
-      if (closed) {
-        if (P.at_shift != kRowNone) shift = u2f(scalar_in(P.at_shift));
-        if (P.at_gamma != kRowNone) gamma = u2f(scalar_in(P.at_gamma));
-        if (P.at_beta != kRowNone) beta = u2f(scalar_in(P.at_beta));
-      } else {
-        work_sync();   // (the previous group's sections have read theirs)
-        if (tid < P.n_scalars && ((P.scalar_in >> tid) & 1u)) sm.in[tid] = scalar_in(tid);
-        work_sync();
-        run_section(P, 0, sm.sr[warp], sm.in, sm.total[warp], false, k);
-      }
+      if (P.at_shift != kRowNone) shift = u2f(scalar_in(P.at_shift));
+      if (P.at_gamma != kRowNone) gamma = u2f(scalar_in(P.at_gamma));
+      if (P.at_beta != kRowNone) beta = u2f(scalar_in(P.at_beta));
       uint8_t *const data = smem + buffer(b);
       wait_for(saddr_of(&sm.full[b]), parity, 2, epoch);
       if (!kWhole) {
-        // Lanes of a run's first and last units that lie outside it take the shift's value (x's own first element, or 0), whose
+        // Lanes of a run's first and last units that lie outside it take the shift's value (x's own first element), whose
         // deviation is zero: the sums then need no masks.
         for (uint32_t i = tid; i < 2u * P.runs; i += kWorkThreads) {
           const uint32_t r = i >> 1, mis = (uint32_t)(reinterpret_cast<uint64_t>(x0) + r * run_step) & 15u;
@@ -396,9 +316,7 @@ __device__ __forceinline__ void stats_affine_body(const RowParam &P, const Launc
             const uint32_t u = r * spr + e / E;
             if (u < u_begin || u >= u_end) continue;
             uint8_t *const at = data + 16u * (u - u_begin);
-            if constexpr (DT == T_F32) {
-              reinterpret_cast<float *>(at)[e % E] = shift;
-            } else if constexpr (DT == T_F16) {
+            if constexpr (DT == T_F16) {
               reinterpret_cast<__half *>(at)[e % E] = __float2half_rn(shift);
             } else {
               reinterpret_cast<unsigned short *>(at)[e % E] = (unsigned short)(f2u(shift) >> 16);
@@ -407,7 +325,7 @@ __device__ __forceinline__ void stats_affine_body(const RowParam &P, const Launc
         }
         work_sync();
       }
-      // sums of d and d * d, in eight (four) partial sums per thread
+      // sums of d and d * d, in eight partial sums per thread
       F2 s1[E / 2], s2[E / 2];
 #pragma unroll
       for (uint32_t i = 0; i < E / 2; ++i) s1[i] = s2[i] = f2(0.0f, 0.0f);
@@ -461,29 +379,11 @@ __device__ __forceinline__ void stats_affine_body(const RowParam &P, const Launc
       }
       turn ^= 1u;
       if (turn == 0) turn_parity ^= 1u;
-      float mean = 0.0f, var = 0.0f, c0, c1, c2, c3;
-      if (closed) {
-        const float ti = __fmul_rn(t.x, P.i1);
-        mean = __fadd_rn(ti, shift);
-        var = __fmul_rn(__fsub_rn(t.y, __fmul_rn(t.x, ti)), P.i2);
-        c0 = mean;
-        c1 = fast_div(1.0f, sqrtf(__fadd_rn(var, P.eps)));
-        c2 = gamma;
-        c3 = beta;
-      } else {
-        if (lane == 0) {
-          if (P.red_slot[0] != kRowNone) sm.total[warp][P.red_slot[0]] = t.x;
-          if (P.red_slot[1] != kRowNone) sm.total[warp][P.red_slot[1]] = t.y;
-        }
-        __syncwarp();
-        run_section(P, 1, sm.sr[warp], sm.in, sm.total[warp], false, k);
-        // (an absent step is an identity that changes no bit: - 0, * 1, + (-0))
-        c0 = scalar_value(P.chain[0], sm.sr[warp], 0.0f);
-        c1 = scalar_value(P.chain[1], sm.sr[warp], 1.0f);
-        c2 = scalar_value(P.chain[2], sm.sr[warp], 1.0f);
-        c3 = scalar_value(P.chain[3], sm.sr[warp], -0.0f);
-      }
-      const F2 m0 = f2(-c0, -c0), m1 = f2(c1, c1), m2 = f2(c2, c2), m3 = f2(c3, c3);
+      const float ti = __fmul_rn(t.x, P.i1);
+      const float mean = __fadd_rn(ti, shift), var = __fmul_rn(__fsub_rn(t.y, __fmul_rn(t.x, ti)), P.i2);
+      const float rstd = fast_div(1.0f, sqrtf(__fadd_rn(var, P.eps)));
+      // (an absent gamma or beta is an identity that changes no bit: * 1, + (-0))
+      const F2 m0 = f2(-mean, -mean), m1 = f2(rstd, rstd), m2 = f2(gamma, gamma), m3 = f2(beta, beta);
       uint8_t *run = y0 + r_first * run_step;   // the run's start in the result, the unit's number in the run
       uint32_t c = c_first;
 #pragma unroll 4
@@ -502,7 +402,7 @@ __device__ __forceinline__ void stats_affine_body(const RowParam &P, const Launc
             *reinterpret_cast<uint4 *>(at) = q;
           } else {
             const int32_t left = (int32_t)(mis + run_bytes) - (int32_t)(16u * c);
-            store_unit<DT>(at, q, c == 0 ? mis >> SH : 0u, left <= 0 ? 0u : min(E, (uint32_t)left >> SH));
+            store_unit(at, q, c == 0 ? mis >> SH : 0u, left <= 0 ? 0u : min(E, (uint32_t)left >> SH));
           }
         }
         run += step_r * run_step;
@@ -520,18 +420,14 @@ __device__ __forceinline__ void stats_affine_body(const RowParam &P, const Launc
         b = 0;
         parity ^= 1u;
       }
-      if (closed) {
-        if (tid == 0 && rank == 0) {
-          auto put = [&](uint32_t i, float f) {
-            if (i == kRowNone) return;
-            const TensorDesc &td = P.scalar[i];
-            store_elem(td.dtype, reinterpret_cast<uint8_t *>(td.ptr), group_offset(td.kstride, k), f2u(f));
-          };
-          put(P.at_mean, mean);
-          put(P.at_var, var);
-        }
-      } else if (warp == 0) {
-        run_section(P, 2, sm.sr[0], sm.in, sm.total[0], lane == 0 && rank == 0, k);
+      if (tid == 0 && rank == 0) {
+        auto put = [&](uint32_t i, float f) {
+          if (i == kRowNone) return;
+          const TensorDesc &td = P.scalar[i];
+          store_elem(td.dtype, reinterpret_cast<uint8_t *>(td.ptr), group_offset(td.kstride, k), f2u(f));
+        };
+        put(P.at_mean, mean);
+        put(P.at_var, var);
       }
     }
     __syncwarp();
@@ -571,7 +467,7 @@ __device__ __forceinline__ float rcp_fast(float x) {
 
 template <uint32_t DT, int K>
 __device__ __forceinline__ void rms_gate_body(const RowParam &P) {
-  __shared__ RowShared sm;
+  __shared__ float part[kMaxWarps];   // sum of each warp
   chain_wait();
   chain_launch();
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
@@ -606,10 +502,6 @@ __device__ __forceinline__ void rms_gate_body(const RowParam &P) {
       if (P.have_w) vw[j] = shifted_unit(reinterpret_cast<const unsigned short *>(P.stream[2].ptr), (int32_t)(8u * c) - (int32_t)(mis >> 1), P.run_len);
     }
   }
-  if (!P.closed && t < P.n_scalars && ((P.scalar_in >> t) & 1u) && live) {
-    const TensorDesc &td = P.scalar[t];
-    sm.in[row_in_cta][t] = load_elem(td.dtype, reinterpret_cast<const uint8_t *>(td.ptr), group_offset(td.kstride, k));
-  }
   // the residual sum, and the sum of its squares
   F2 x[K][4];
   float s = 0.0f;
@@ -624,7 +516,7 @@ __device__ __forceinline__ void rms_gate_body(const RowParam &P) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) x[j][i] = add2(x[j][i], b[i]);
     }
-    if (lo != 0 || hi != 8u) mask_pairs<DT>(x[j], lo, hi);
+    if (lo != 0 || hi != 8u) mask_pairs(x[j], lo, hi);
     F2 q = mul2(x[j][0], x[j][0]);
 #pragma unroll
     for (int i = 1; i < 4; ++i) q = fma2(x[j][i], x[j][i], q);
@@ -633,7 +525,7 @@ __device__ __forceinline__ void rms_gate_body(const RowParam &P) {
   }
   s = warp_sum(s);
   if (tg > 32u) {
-    if (lane == 0) sm.part[warp] = s;
+    if (lane == 0) part[warp] = s;
   }
   // the gated product does not need the row's sum: it fills the time until every warp has delivered its part
   if (P.have_gate) {
@@ -652,26 +544,16 @@ __device__ __forceinline__ void rms_gate_body(const RowParam &P) {
           const float e0 = __fadd_rn(fast_exp(-gg[2 * i]), 1.0f), e1 = __fadd_rn(fast_exp(-gg[2 * i + 1]), 1.0f);
           y[i] = mul2(mul2(f2(rcp_fast(e0), rcp_fast(e1)), f2(gg[2 * i], gg[2 * i + 1])), uu[i]);
         }
-        store_unit<DT>(base_of(6) + (16ull * c - mis), pack_pairs<DT>(y), lo, hi);
+        store_unit(base_of(6) + (16ull * c - mis), pack_pairs<DT>(y), lo, hi);
       }
     }
   }
   if (tg > 32u) {
     __syncthreads();
     const uint32_t nw = tg >> 5;
-    s = warp_sum(lane < nw ? sm.part[row_in_cta * nw + lane] : 0.0f);
+    s = warp_sum(lane < nw ? part[row_in_cta * nw + lane] : 0.0f);
   }
-  float scale;
-  if (P.closed) {
-    scale = fast_div(1.0f, sqrtf(__fadd_rn(__fmul_rn(s, P.i1), P.eps)));
-  } else {
-    __syncthreads();   // (the scalars read at the start are in shared memory)
-    if (lane == 0) sm.total[warp][P.red_slot[0]] = s;
-    __syncwarp();
-    run_section(P, 0, sm.sr[warp], sm.in[row_in_cta], sm.total[warp], false, k);
-    run_section(P, 1, sm.sr[warp], sm.in[row_in_cta], sm.total[warp], false, k);
-    scale = scalar_value(P.chain[1], sm.sr[warp], 1.0f);
-  }
+  const float scale = fast_div(1.0f, sqrtf(__fadd_rn(__fmul_rn(s, P.i1), P.eps)));
   const F2 scale2 = f2(scale, scale);
 #pragma unroll
   for (int j = 0; j < K; ++j) {
@@ -688,10 +570,9 @@ __device__ __forceinline__ void rms_gate_body(const RowParam &P) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) y[i] = mul2(y[i], w[i]);
       }
-      store_unit<DT>(base_of(3) + (16ull * c - mis), pack_pairs<DT>(y), lo, hi);
+      store_unit(base_of(3) + (16ull * c - mis), pack_pairs<DT>(y), lo, hi);
     }
   }
-  if (!P.closed && t < 32u) run_section(P, 2, sm.sr[warp], sm.in[row_in_cta], sm.total[warp], t == 0 && live, k);
 }
 
 }  // namespace
@@ -702,10 +583,8 @@ __device__ __forceinline__ void rms_gate_body(const RowParam &P) {
   }
 DVMB_ROW_STATS(dvm_b200_row_stats_affine_f16, T_F16, false)
 DVMB_ROW_STATS(dvm_b200_row_stats_affine_bf16, T_BF16, false)
-DVMB_ROW_STATS(dvm_b200_row_stats_affine_f32, T_F32, false)
 DVMB_ROW_STATS(dvm_b200_row_stats_affine_f16_whole, T_F16, true)
 DVMB_ROW_STATS(dvm_b200_row_stats_affine_bf16_whole, T_BF16, true)
-DVMB_ROW_STATS(dvm_b200_row_stats_affine_f32_whole, T_F32, true)
 #undef DVMB_ROW_STATS
 #define DVMB_ROW_RMS(NAME, DT, K)                                                                    \
   __global__ void __launch_bounds__(kMaxRowThreads) NAME(const __grid_constant__ RowParam P) { rms_gate_body<DT, K>(P); }
@@ -717,21 +596,17 @@ DVMB_ROW_RMS(dvm_b200_row_rms_gate_bf16_2, T_BF16, 2)
 
 namespace {
 
-uint32_t ElemShift(const RowParam &p) { return p.dtype == T_F32 ? 2u : 1u; }
-
 // Every run starts on 16 bytes.
 bool RunsAligned(const RowParam &p) {
-  const uint32_t sh = ElemShift(p);
-  uint64_t m = p.stream[0].ptr | (static_cast<uint64_t>(p.run_stride) << sh);
+  uint64_t m = p.stream[0].ptr | (static_cast<uint64_t>(p.run_stride) << 1);
   for (int j = 0; j < kMaxKept; ++j)
-    if (p.kept_size[j] != 1) m |= static_cast<uint64_t>(p.stream[0].kstride[j]) << sh;
+    if (p.kept_size[j] != 1) m |= static_cast<uint64_t>(p.stream[0].kstride[j]) << 1;
   return (m & 15u) == 0;
 }
 // 16-byte units a run touches at most: one more where runs may start inside a unit
 uint32_t UnitsPerRun(const RowParam &p) {
-  const uint32_t sh = ElemShift(p);
-  const uint64_t bytes = static_cast<uint64_t>(p.run_len) << sh;
-  return static_cast<uint32_t>(RunsAligned(p) ? (bytes + 15) / 16 : (bytes + 15 + (16u - (1u << sh))) / 16);
+  const uint64_t bytes = static_cast<uint64_t>(p.run_len) << 1;
+  return static_cast<uint32_t>(RunsAligned(p) ? (bytes + 15) / 16 : (bytes + 15 + 14) / 16);
 }
 
 // Clusters of `cl` CTAs that run at a time, as the driver says; asked once per kernel and launch shape.
@@ -806,16 +681,16 @@ static_assert(kRowRmsMaxElems == kRmsMaxUnits * 8, "two units of eight elements 
 
 bool RowAddressesOk(const RowParam &p) {
   if (p.form == ROW_OFF || p.stream[0].ptr == 0) return false;
-  const uint32_t sh = ElemShift(p), n = p.form == ROW_STATS_AFFINE ? 2u : static_cast<uint32_t>(kRowMaxStreams);
+  const uint32_t n = p.form == ROW_STATS_AFFINE ? 2u : static_cast<uint32_t>(kRowMaxStreams);
   for (uint32_t i = 0; i < n; ++i) {
     if (p.form == ROW_RMS_GATE && i == 2) {   // (the row vector is read at any element address)
       if (p.have_w && (p.stream[2].ptr & 1u)) return false;
       continue;
     }
     if (p.form == ROW_RMS_GATE && p.stream[i].ptr == 0) continue;   // an absent stream
-    if (((p.stream[i].ptr ^ p.stream[0].ptr) & 15u) != 0 || (p.stream[i].ptr & ((1u << sh) - 1u)) != 0) return false;
+    if (((p.stream[i].ptr ^ p.stream[0].ptr) & 15u) != 0 || (p.stream[i].ptr & 1u) != 0) return false;
   }
-  if ((static_cast<uint64_t>(p.run_len) << sh) >= (1ull << 30)) return false;   // (32-bit byte counts inside a run)
+  if ((static_cast<uint64_t>(p.run_len) << 1) >= (1ull << 30)) return false;   // (32-bit byte counts inside a run)
   if (p.form == ROW_RMS_GATE && UnitsPerRun(p) > kRmsMaxUnits) return false;   // (a row that does not fit a CTA's registers)
   if (p.form == ROW_RMS_GATE) return true;
   const uint64_t units = static_cast<uint64_t>(p.runs) * UnitsPerRun(p);
@@ -825,38 +700,35 @@ bool RowAddressesOk(const RowParam &p) {
   return units < (1ull << 20) && StatsPlan(static_cast<uint32_t>(units), p.groups, sms, &plan, &smem);
 }
 
-// Estimates of both kernels in microseconds, a fit to about 2000 launches of 16 to 400 000 groups of 4 to 200 000 elements timed back to back
-// in either (runs of 1 to 256, aligned and not, fp16 and fp32, closed scalar sections and words).  What decides:
-//  - A statistics CTA takes 1.3 us for a group (2.3 with edges) however short it is, and 6 where the scalar sections run as words;
-//    the interpreter gives short groups a slice of a CTA: [100000, 64] fp16 432 us here and 62 there, [1200, 64] 7.7 and 10.7,
-//    [5000, 512] 23 and 31, [5000, 4096] 29 and 68; as words [5000, 1024] 104 and 37, [5000, 4095] 130 and 279.
+// Estimates of both kernels in microseconds, a fit to about 1200 launches of 16 to 400 000 groups of 4 to 200 000 elements timed back
+// to back in either (runs of 1 to 256, aligned and not).  What decides:
+//  - A statistics CTA takes 1.3 us for a group (2.3 with edges) however short it is; the interpreter gives short groups a slice of
+//    a CTA: [100000, 64] fp16 432 us here and 62 there, [1200, 64] 7.7 and 10.7, [5000, 512] 23 and 31, [5000, 4096] 29 and 68.
 //  - An RMS row of up to 32 units takes a warp about 0.35 ns in all: [400000, 16] bf16 138 us and 37, [400000, 64] 148 and 144.
 //  - RMS rows of more than 512 units leave two CTAs on an SM: from 12 rows per SM on, rows that the interpreter's chunks divide
-//    are faster there ([5000, 6144] 78 and 58, [600, 6144] 9.6 and 10.3), others are not ([5000, 5120] 74 and 154); as
-//    words from 512 units and two rows per SM on ([5000, 8192] 155 and 77).
+//    are faster there ([5000, 6144] 78 and 58, [600, 6144] 9.6 and 10.3), others are not ([5000, 5120] 74 and 154).
 bool RowKernelPays(const RowParam &p, uint32_t chunk_elems) {
-  const uint32_t sh = ElemShift(p), sms = static_cast<uint32_t>(Runtime::Get().sm_count_or_default()), units = UnitsPerRun(p);
+  const uint32_t sms = static_cast<uint32_t>(Runtime::Get().sm_count_or_default()), units = UnitsPerRun(p);
   const double groups = p.groups, n = static_cast<double>(p.runs) * p.run_len;
-  const bool closed = p.closed != 0, single = p.runs == 1;
+  const bool single = p.runs == 1;
   const bool even = chunk_elems != 0 && static_cast<uint64_t>(p.runs) * p.run_len % chunk_elems == 0;   // no chunk is partly filled
   // runs in whole units of 16 bytes, and in whole granules of four elements (what the interpreter loads at a time)
-  const bool whole = RunsAligned(p) && ((p.run_len << sh) & 15u) == 0;
-  uint64_t m = p.stream[0].ptr | (static_cast<uint64_t>(p.run_stride | p.run_len) << sh);
+  const bool whole = RunsAligned(p) && ((p.run_len << 1) & 15u) == 0;
+  uint64_t m = p.stream[0].ptr | (static_cast<uint64_t>(p.run_stride | p.run_len) << 1);
   for (int j = 0; j < kMaxKept; ++j)
-    if (p.kept_size[j] != 1) m |= static_cast<uint64_t>(p.stream[0].kstride[j]) << sh;
-  const bool granules = (m & ((4u << sh) - 1u)) == 0;
+    if (p.kept_size[j] != 1) m |= static_cast<uint64_t>(p.stream[0].kstride[j]) << 1;
+  const bool granules = (m & 7u) == 0;
   double padded = 16.0;   // a short group's slice: a power of two of elements
   while (padded < n) padded *= 2.0;
 
   if (p.form == ROW_RMS_GATE) {
     if (units <= 32u) {
       const double w = p.have_w != 0, b = p.have_b != 0, g = p.have_gate != 0;
-      const double row = (closed ? 1.5 : 4.4) + groups * 1e-3 * (0.345 + 0.035 * w + 0.015 * b + 0.095 * g + (closed ? 0.0 : 0.65));
+      const double row = 1.5 + groups * 1e-3 * (0.345 + 0.035 * w + 0.015 * b + 0.095 * g);
       const double per_elem = 1e-6 * (5.0 + 1.5 * w + 3.3 * b + 6.2 * g) * (granules ? 1.0 : 2.2);
       return row <= std::max(7.0 + 5.0 * b + 5.0 * g, 5.0 + groups * padded * per_elem);
     }
-    if (!whole || !even) return true;
-    return closed ? units <= kMaxRowThreads || groups <= 12.0 * sms : units < kMaxRowThreads || groups <= 2.0 * sms;
+    return !whole || !even || units <= kMaxRowThreads || groups <= 12.0 * sms;
   }
 
   RowParam plan = {};
@@ -864,14 +736,12 @@ bool RowKernelPays(const RowParam &p, uint32_t chunk_elems) {
   if (!StatsPlan(p.runs * units, p.groups, sms, &plan, &smem)) return false;
   const uint32_t slots = std::max(1u, (smem <= kHalfSm ? 2u : 1u) * sms / plan.cluster);
   const double rounds = std::ceil(groups / slots);
-  // a single round answers sooner than the interpreter, but for a few rows that its chunks divide, as words
-  if (rounds <= 1.0) return closed || !(single && whole && even && n >= 1024.0 && n <= 8192.0);
-  const double per_group = closed ? std::max(whole ? 1.3 : 2.3, 0.6 + 0.035 * p.runs)
-                                  : (whole ? 6.0 : 7.1) + plan.per_cta * 16.0 * 7e-5 + (plan.cluster > 2 ? 3.0 : 0.0);
+  if (rounds <= 1.0) return true;   // (a single round answers sooner than the interpreter)
+  const double per_group = std::max(whole ? 1.3 : 2.3, 0.6 + 0.035 * p.runs);
   double base, ns;   // the interpreter: a launch, and every group
   if (n <= 512.0) {
-    base = granules ? (closed ? 10.0 : 8.5) : (single ? 15.0 : 25.0);
-    ns = padded * 1e-3 * (single ? (granules ? 10.0 : 20.0) : (granules ? 15.0 : 22.0)) * (closed ? 1.0 : 0.8);
+    base = granules ? 10.0 : (single ? 15.0 : 25.0);
+    ns = padded * 1e-3 * (single ? (granules ? 10.0 : 20.0) : (granules ? 15.0 : 22.0));
   } else if (single) {
     base = granules ? (!even && n > 2048.0 ? 12.5 : 4.5) : 11.0;
     ns = granules ? 3.0 + 3.5 * std::ceil(n / 2048.0) + (even ? 0.0 : 14.0) : 11.0 + 0.0125 * n;
@@ -913,11 +783,10 @@ int LaunchRow(const RowParam &p_in, void *stream) {
   }
   uint32_t smem = 0;
   if (!StatsPlan(p.runs * units, p.groups, sms, &p, &smem)) return -7;
-  const bool whole = RunsAligned(p) && ((p.run_len << ElemShift(p)) & 15u) == 0;
+  const bool whole = RunsAligned(p) && ((p.run_len << 1) & 15u) == 0;
   using Fn = void (*)(const RowParam, const LaunchTag);
-  static const Fn table[2][3] = {
-    {dvm_b200_row_stats_affine_f16, dvm_b200_row_stats_affine_bf16, dvm_b200_row_stats_affine_f32},
-    {dvm_b200_row_stats_affine_f16_whole, dvm_b200_row_stats_affine_bf16_whole, dvm_b200_row_stats_affine_f32_whole}};
+  static const Fn table[2][2] = {{dvm_b200_row_stats_affine_f16, dvm_b200_row_stats_affine_bf16},
+                                 {dvm_b200_row_stats_affine_f16_whole, dvm_b200_row_stats_affine_bf16_whole}};
   int dev = 0;
   cudaGetDevice(&dev);
   static bool attr_set[64] = {false};
@@ -929,7 +798,7 @@ int LaunchRow(const RowParam &p_in, void *stream) {
       }
     attr_set[dev] = true;
   }
-  const Fn fn = table[whole ? 1 : 0][p.dtype == T_F16 ? 0 : (p.dtype == T_BF16 ? 1 : 2)];
+  const Fn fn = table[whole ? 1 : 0][p.dtype == T_F16 ? 0 : 1];
   // persistent clusters, as many as are resident at a time
   const uint32_t resident = std::max(1u, ResidentClusters(reinterpret_cast<const void *>(fn), kStatsThreads, smem, p.cluster, sms));
   cudaLaunchConfig_t cfg = {};

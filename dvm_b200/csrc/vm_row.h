@@ -11,7 +11,6 @@ namespace dvmb {
 
 constexpr int kRowMaxStreams = 7;     // tensors walked element by element
 constexpr int kRowMaxScalars = 8;     // group scalars in memory (inputs and results of the scalar sections)
-constexpr int kRowMaxCode = 96;
 constexpr uint32_t kRowNone = 0xffu;
 constexpr uint32_t kRowRmsMaxElems = 8192;   // longest row of ROW_RMS_GATE: it stays in a CTA's registers
 
@@ -23,15 +22,6 @@ enum RowForm : uint32_t {
   ROW_RMS_GATE
 };
 
-// Where a body's group scalar comes from.
-struct RowScalar {
-  uint8_t src;      // kRowNone: absent; 0: scalar register `idx`; 1: imm
-  uint8_t idx;
-  uint8_t recip;    // the body divides by it: multiply by its reciprocal
-  uint8_t pad;
-  uint32_t imm;
-};
-
 struct RowStream {
   uint64_t ptr;
   uint32_t kstride[kMaxKept];   // element strides along the group's coordinates
@@ -40,7 +30,7 @@ struct RowStream {
 
 struct RowParam {
   uint32_t form;
-  uint32_t dtype;               // of every stream
+  uint32_t dtype;               // of every stream (16-bit)
   uint32_t groups, kept_size[kMaxKept];
   uint32_t runs, run_len, run_stride;   // a group is `runs` runs of `run_len` elements, `run_stride` elements apart
   // set by the launcher
@@ -50,22 +40,15 @@ struct RowParam {
   uint32_t tg;                  // ROW_RMS_GATE: threads per row
   // ROW_STATS_AFFINE: streams 0 = x, 1 = result.  ROW_RMS_GATE: a, b, w, result 1, g, u, result 2
   RowStream stream[kRowMaxStreams];
-  uint32_t have_b, have_w, have_gate, gate_gu;
-  RowScalar shift, chain[4];    // chain: subtract, multiply, multiply, add (ROW_RMS_GATE: chain[1] only)
-  // the usual scalar sections in closed form (row_match.cc follows the words symbolically); 0: run the words
+  uint32_t have_b, have_w, have_gate;
+  // the scalar sections in closed form (row_match.cc follows the words symbolically)
   //   ROW_STATS_AFFINE: m = T i1 + s, v = (Q - T (T i1)) i2, x' = ((x - m) / sqrt(v + eps)) * gamma + beta, m and v stored
   //   ROW_RMS_GATE: scale = 1 / sqrt(S i1 + eps)
-  uint32_t closed;
   float i1, i2, eps;
   uint32_t at_shift, at_gamma, at_beta, at_mean, at_var;   // entries of scalar[] (kRowNone: absent)
-  uint32_t red_slot[2];         // reduction partials the sums belong to (kRowNone: not taken)
-  // scalar sections: instruction words of the stage, sections ending with OP_END
-  uint32_t num_sections;        // PRO_0 .. PRO_n
-  uint16_t sec[kMaxPhases + 2];
   TensorDesc scalar[kRowMaxScalars];
   uint8_t scalar_of[kMaxTensors];       // tensor slot -> entry of scalar[]
-  uint32_t n_scalars, scalar_in;        // scalar_in: bit mask of the entries that are read
-  uint64_t code[kRowMaxCode];
+  uint32_t n_scalars;
 };
 static_assert(sizeof(RowParam) <= 4000, "RowParam is a kernel parameter");
 

@@ -420,7 +420,7 @@ def test_an_rms_norm_runs_as_one(shape):
     ((600, 6144), "rms", dvm.bfloat16, (1,), "row_rms_gate"),
     ((5000, 6144), "rms", dvm.bfloat16, (1,), "interpreter"),          # more than 512 units, rows of whole chunks
     ((5000, 5120), "rms", dvm.bfloat16, (1,), "row_rms_gate"),
-    ((5000, 16384), "rms", dvm.float32, (1,), "interpreter"),          # statistics with interpreted scalar sections
+    ((5000, 16384), "rms", dvm.float32, (1,), "interpreter"),          # no deviation sums: scalar sections of another form
 ])
 def test_rows_go_to_the_faster_kernel(shape, form, dtype, dims, kernel):
     assert _launched(shape, form, dtype, dims) == kernel

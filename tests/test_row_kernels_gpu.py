@@ -41,8 +41,8 @@ def _batchnorm(shape, dtype, offset=0):
     else:
         stores = [t.store(v) for v in W.batchnorm_train(t, lx, t.load(g), t.load(b), n * h * w)]
     t.run()
-    if not offset and "DVM_B200_NO_ROW" not in os.environ:
-        assert "kernel=row_stats_affine" in t.das()
+    if not offset and "DVM_B200_NO_ROW" not in os.environ:   # (fp32 inputs have no deviation sums and stay on the interpreter)
+        assert ("kernel=row_stats_affine" in t.das()) == (code != 3)
     read = lambda s: Tester.convert_from_bf16(t.output(s)) if s.dtype() == 2 else t.output(s)
     got = [read(s).astype(np.float64) for s in stores]
     xd = (Tester.convert_from_bf16(x) if code == 2 else x).astype(np.float64)
@@ -182,3 +182,33 @@ def test_rms_norm_of_many_rows(rows, cols):
     xd = Tester.convert_from_bf16(x).astype(np.float64)
     want = xd / np.sqrt((xd * xd).mean(1, keepdims=True) + 1e-6)
     assert np.all(np.abs(got - want) <= 2.0 ** -8 * np.abs(want) + 1e-5)   # (one rounding to bf16)
+
+
+@pytest.mark.parametrize("rows,cols", [(7, 3), (33, 257), (5, 8)])
+def test_other_scalar_sections_run_on_the_interpreter(rows, cols):
+    """A sum alone, two group scalars of different types, an immediate factor and a stored 16-bit mean, the result in place of the
+    input: the statistics kernel faulted on [7, 3] when it interpreted such sections."""
+    import torch
+    import dvm_b200 as dvm
+    g = torch.Generator(device="cuda").manual_seed(5)
+    buf = torch.randn(rows * cols + 8, generator=g, device="cuda").half()
+    gamma, beta = torch.randn(rows, generator=g, device="cuda").half(), torch.randn(rows + 3, generator=g, device="cuda")
+    mean = torch.zeros(rows, device="cuda").half()
+    k = dvm.PyKernel("vector")
+    x, lg, lb = k.load([rows, cols], dvm.float16), k.load([rows, 1], dvm.float16), k.load([rows, 1], dvm.float32)
+    f = k.cast(x, dvm.float32)
+    m = k.mul(k.sum(f, (1,), True), 1.0 / cols)
+    y = k.add(k.mul(k.mul(k.sub(f, m), k.cast(lg, dvm.float32)), 1.5), lb)
+    stores = [k.store(k.cast(y, dvm.float16)), k.store(k.cast(m, dvm.float16))]
+    for op, t, off in ((x, buf, 8), (lg, gamma, 0), (lb, beta, 3), (stores[0], buf, 8), (stores[1], mean, 0)):
+        k.bind_device(op, t.data_ptr() + off * t.element_size(), (t.numel() - off) * t.element_size())
+    k.codegen()
+    assert "kernel=interpreter" in k.das()
+    xd = buf[8:].double().reshape(rows, cols)
+    want_mean = xd.mean(1)
+    want = (xd - want_mean[:, None]) * gamma.double()[:, None] * 1.5 + beta[3:].double()[:, None]
+    k.launch(torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    # one rounding to fp16, fp32 sums in front of it
+    assert bool(((buf[8:].double().reshape(rows, cols) - want).abs() <= 2.0 ** -11 * want.abs() + 1e-5).all())
+    assert bool(((mean.double() - want_mean).abs() <= 2.0 ** -11 * want_mean.abs() + 1e-5).all())
