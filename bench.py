@@ -494,7 +494,7 @@ def measured_sustained():
         return None
 
 
-KERNEL_NAME = {"c1": "dvm_b200_vm_vector_flat", "c2": "dvm_b200_row_stats_affine_f16_whole", "c3": "dvm_b200_row_rms_gate_bf16_2",
+KERNEL_NAME = {"c1": "dvm_b200_vm_vector_flat", "c2": "dvm_b200_vm_vector_nd_r128", "c3": "dvm_b200_row_rms_gate_bf16_2",
                "c4": "dvm_b200_attention_bf16_sf", "c5": "dvm_b200_mm_tcgen05_pair"}
 
 
@@ -769,7 +769,7 @@ def main():
     tensor = name in ("c4", "c5")
     # DRAM bytes per full-size launch from the ncu captures summarised under profiles/ (dram__bytes_read + write; the
     # quarter-size captures of c1, c3, c4, c5 are scaled by 4: their traffic grows with the leading dimension)
-    traffic = {"c1": 4 * (135.2e6 + 36.0e6), "c2": 102.8e6 + 48.5e6, "c3": 4 * (134.3e6 + 11.5e6),
+    traffic = {"c1": 4 * (135.2e6 + 36.0e6), "c2": 195.7e6 + 55.8e6, "c3": 4 * (134.3e6 + 11.5e6),
                "c4": 4 * (100.7e6 + 7.2e6), "c5": 4 * (520.8e6 + 57.4e6)}.get(name)
     if traffic is not None and args.scale != 1.0:
         traffic *= args.scale

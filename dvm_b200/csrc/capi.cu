@@ -478,7 +478,7 @@ int dvm_rt_memset(void *dst, int value, size_t bytes, void *stream) {
 // then ran to its end with wrong results) is reported here as an error.  Does not wait for anything.
 int dvm_rt_check_status(void) {
   if (!dvmb::TakeExpiryFlag()) return 0;
-  const unsigned int rs = dvmb::ReadRowStatus(), vs = dvmb::ReadVectorStatus(), sv = vs != 0 ? vs : rs, sm = dvmb::ReadMatMulStatus(), sa = dvmb::ReadAttentionStatus();
+  const unsigned int sv = dvmb::ReadVectorStatus(), sm = dvmb::ReadMatMulStatus(), sa = dvmb::ReadAttentionStatus();
   if ((sv | sm | sa) != 0) {
     char buf[160];
     snprintf(buf, sizeof(buf), "a bounded device wait expired (vector 0x%08x, matmul 0x%08x, attention 0x%08x)", sv, sm, sa);

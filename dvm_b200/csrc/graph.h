@@ -141,7 +141,7 @@ struct VectorStage {
   // rebind to an aligned address gets the planned offset back
   uint32_t ring_plan_off[dvmb::kMaxTensors] = {0};
   uint64_t algo_bytes = 0;
-  // a normalisation that a row kernel runs (vm_row.cu) when the bound addresses allow it; the interpreter's program stays
+  // an RMS norm that the row kernel runs (vm_row.cu) when the bound addresses allow it; the interpreter's program stays
   // the stage's definition and its fallback
   dvmb::RowParam row;
   bool row_ok = false;
@@ -269,7 +269,7 @@ bool CompileVectorStage(const std::vector<NDObject *> &ops, VectorStage *out, st
 bool CompileEpilogue(const std::vector<NDObject *> &ops, const NDObject *mma_src, MatMulStage *out, std::string *why);
 std::string DisassembleEpilogue(const MatMulStage &st);
 std::string DisassembleStage(const VectorStage &st);
-// row_match.cc: fill st->row when the compiled stage is one of the row kernels' shapes; bind its addresses.
+// row_match.cc: fill st->row when the compiled stage is the row kernel's shape; bind its addresses.
 void MatchRowKernel(VectorStage *st);
 void BindRow(VectorStage *st);
 // row_match.cc: the same for the direct kernel.

@@ -1,6 +1,6 @@
-// Recognises the two normalisation shapes that the row kernels (vm_row.cu) run: works on the instruction words and the
-// tensor table that the vector compiler produced, so the graph may be written in any way that compiles to these bodies.
-// What does not match, scalar sections of another form among it, runs on the vector interpreter.  No counterpart in the reference, whose kernels run each
+// Recognises the RMS norm that the row kernel (vm_row.cu) runs: works on the instruction words and the tensor table that the
+// vector compiler produced, so the graph may be written in any way that compiles to these bodies.  What does not match, scalar
+// sections of another form among it, runs on the vector interpreter.  No counterpart in the reference, whose kernels run each
 // reduction and each group of element-wise ops as written (src/vm_gpu.cu:1552-1617).
 #include <cstdlib>
 #include <cstring>
@@ -20,7 +20,6 @@ struct Word {
   uint32_t opc, sub, kind, idx, rnd, imm;
   explicit Word(uint64_t v) : w(v), opc(DVMB_OPC(v)), sub(DVMB_SUB(v)), kind(DVMB_OKIND(v)), idx(DVMB_OIDX(v)), rnd(DVMB_RND(v)), imm(DVMB_IMM(v)) {}
   bool bin(uint32_t b) const { return opc == OP_BIN && sub == b && rnd == RN_NONE; }
-  bool scalar_operand() const { return kind == K_SREG || kind == K_IMM; }
 };
 
 struct Cursor {
@@ -29,21 +28,6 @@ struct Cursor {
   Word at(size_t i = 0) const { return Word(pc + i < code.size() ? code[pc + i] : 0); }
   Word next() { return Word(code[pc++]); }
 };
-
-// Where a body's group scalar comes from: a scalar register, or none of that kind.
-struct BodyScalar {
-  bool present = false, is_register = false, recip = false;   // recip: the body divides by it
-  uint32_t idx = 0;
-};
-
-BodyScalar ScalarOf(const Word &w, bool recip) {
-  BodyScalar s;
-  s.present = true;
-  s.is_register = w.kind == K_SREG;
-  s.idx = w.idx;
-  s.recip = recip;
-  return s;
-}
 
 // A store of the accumulator to `tensor` in its own type, behind the rounding that store repeats anyway.
 bool MatchStore(Cursor &c, const VmParam &P, uint32_t *slot) {
@@ -89,7 +73,10 @@ struct Symbolic {
       if (w.kind == K_TENSOR) b = Make(IN, w.idx);
       switch (w.opc) {
         case OP_RINIT: break;
-        case OP_RFIN: acc = Make(PART, w.sub & 3u); break;
+        case OP_RFIN:
+          acc = Make(PART, w.sub & 3u);
+          if ((w.sub >> 4) != R_SUM) ok = false;
+          break;
         case OP_COPY: acc = b; break;
         case OP_MOV: sreg[DVMB_DST(w.w)] = acc; break;
         case OP_ST: stores.emplace_back(w.sub, acc); break;
@@ -125,8 +112,7 @@ struct Matcher {
   const VectorStage &st;
   const VmParam &P;
   RowParam *R;
-  BodyScalar shift, chain[4];   // chain: subtract, multiply, multiply, add (ROW_RMS_GATE: chain[1] only)
-  uint32_t red_slot[2] = {kRowNone, kRowNone};   // reduction partials the sums belong to (kRowNone: not taken)
+  uint32_t scale_reg = 0, red_slot = 0;   // the scalar register the body multiplies by; the partial of the sum
 
   Matcher(const VectorStage &s, RowParam *r) : st(s), P(s.param), R(r) {}
 
@@ -148,95 +134,26 @@ struct Matcher {
     return true;
   }
 
-  // runs x run_len from the iterated axes of tensor `slot`
+  // rows from the iterated axes of tensor `slot`
   bool Geometry(uint32_t slot) {
     const TensorDesc &td = P.tensor[slot];
-    if (P.enum_size[0] != 1 || P.enum_size[1] != 1 || td.estride[kMaxEnum - 1] != 1) return false;
-    R->runs = P.enum_size[kMaxEnum - 2];
+    for (int j = 0; j < kMaxEnum - 1; ++j)
+      if (P.enum_size[j] != 1) return false;
+    if (td.estride[kMaxEnum - 1] != 1) return false;
     R->run_len = P.enum_size[kMaxEnum - 1];
-    R->run_stride = R->runs > 1 ? td.estride[kMaxEnum - 2] : 0;
     R->dtype = td.dtype;
     R->groups = P.num_groups;
     for (int j = 0; j < kMaxKept; ++j) R->kept_size[j] = P.kept_size[j];
     return td.dtype == T_F16 || td.dtype == T_BF16;
   }
 
-  // Enters the tensors that the scalar sections read and store.
-  bool Scalars() {
-    std::memset(R->scalar_of, 0xff, sizeof(R->scalar_of));
-    auto scalar = [&](uint32_t slot) {
-      if (P.tensor[slot].mode != AM_SCALAR) return false;
-      if (R->scalar_of[slot] == 0xff) {
-        if (R->n_scalars >= static_cast<uint32_t>(kRowMaxScalars)) return false;
-        R->scalar[R->n_scalars] = P.tensor[slot];
-        R->scalar_of[slot] = static_cast<uint8_t>(R->n_scalars++);
-      }
-      return true;
-    };
-    for (uint32_t p = 0; p <= P.num_body; ++p)
-      for (size_t pc = st.bsec[2 * p];; ++pc) {
-        const Word w(st.bytecode[pc]);
-        // (only the last section stores: the compiler puts up to four stores there, a fifth stays in front of a body)
-        if (w.opc == OP_ST && (p != P.num_body || !scalar(w.sub))) return false;
-        if ((w.opc == OP_COPY || w.opc == OP_BIN || w.opc == OP_CMP || w.opc == OP_SEL) && w.kind == K_TENSOR && !scalar(w.idx)) return false;
-        if (w.opc == OP_RFIN && ((w.sub >> 4) != R_SUM || ((w.sub & 3u) != red_slot[0] && (w.sub & 3u) != red_slot[1]))) return false;
-        if (w.opc == OP_END) break;
-      }
-    return true;
-  }
-
-  // The closed form of ROW_STATS_AFFINE's scalar sections (see RowParam).
-  bool CloseStats() {
-    Symbolic y;
-    y.Run(st.bytecode, st.bsec[0]);
-    if (!shift.present || !shift.is_register || red_slot[0] == kRowNone || red_slot[1] == kRowNone) return false;
-    const int s = y.sreg[shift.idx];
-    if (!y.ok || s < 0 || y.e[s].op != Symbolic::IN) return false;
-    const uint32_t shift_slot = y.e[s].v;
-    if (P.tensor[shift_slot].dtype != R->dtype) return false;   // (the kernel writes it into a run's edge lanes: it must be a value of x's type)
-    y.Run(st.bytecode, st.bsec[2]);
-    auto value = [&](const BodyScalar &c) { return c.is_register ? y.sreg[c.idx] : static_cast<int>(Symbolic::NONE); };
-    const int mean = value(chain[0]), den = value(chain[1]);
-    if (!y.ok || mean < 0 || den < 0 || !chain[1].recip || chain[2].recip) return false;
-    const int T = y.Make(Symbolic::PART, red_slot[0]), Q = y.Make(Symbolic::PART, red_slot[1]);
-    // den = sqrt(v + eps), v = (Q - T (T i1)) i2, mean = T i1 + s
-    if (y.e[mean].op != Symbolic::BIN || y.e[mean].v != B_ADD) return false;
-    const int ti = y.e[mean].a == s ? y.e[mean].b : y.e[mean].a;
-    if ((y.e[mean].a != s && y.e[mean].b != s) || !y.WithImm(ti, B_MUL, T, &R->i1)) return false;
-    if (y.e[den].op != Symbolic::UN || y.e[den].v != U_SQRT) return false;
-    const int ve = y.e[den].a;
-    if (y.e[ve].op != Symbolic::BIN || y.e[ve].v != B_ADD) return false;
-    const int v = y.IsImm(y.e[ve].a, &R->eps) ? y.e[ve].b : y.e[ve].a;
-    if (!y.WithImm(ve, B_ADD, v, &R->eps)) return false;
-    const int dev = y.Bin(B_SUB, Q, y.Bin(B_MUL, T, ti));
-    if (!y.WithImm(v, B_MUL, dev, &R->i2)) return false;
-    R->at_gamma = R->at_beta = R->at_mean = R->at_var = kRowNone;
-    auto input = [&](const BodyScalar &c, uint32_t *at) {
-      if (!c.present) return true;
-      const int i = value(c);
-      if (i < 0 || y.e[i].op != Symbolic::IN) return false;
-      *at = R->scalar_of[y.e[i].v];
-      return true;
-    };
-    if (!input(chain[2], &R->at_gamma) || !input(chain[3], &R->at_beta)) return false;
-    y.Run(st.bytecode, st.bsec[4]);
-    if (!y.ok) return false;
-    for (auto &stored : y.stores) {
-      uint32_t *at = stored.second == mean ? &R->at_mean : (stored.second == v ? &R->at_var : nullptr);
-      if (at == nullptr || *at != kRowNone) return false;
-      *at = R->scalar_of[stored.first];
-    }
-    R->at_shift = R->scalar_of[shift_slot];
-    return true;
-  }
-
-  // ... and of ROW_RMS_GATE's.
+  // The closed form of the scalar sections (see RowParam); nothing of a group is stored.
   bool CloseRms() {
     Symbolic y;
     y.Run(st.bytecode, st.bsec[0]);
     y.Run(st.bytecode, st.bsec[2]);
-    if (!y.ok || !chain[1].is_register) return false;
-    const int scale = y.sreg[chain[1].idx];
+    if (!y.ok || scale_reg >= static_cast<uint32_t>(kNumSRegs)) return false;
+    const int scale = y.sreg[scale_reg];
     float one = 0.0f;
     if (scale < 0 || y.e[scale].op != Symbolic::BIN || y.e[scale].v != B_DIV_FAST || !y.IsImm(y.e[scale].a, &one) || one != 1.0f) return false;
     const int root = y.e[scale].b;
@@ -244,49 +161,9 @@ struct Matcher {
     const int sum = y.e[root].a;
     if (y.e[sum].op != Symbolic::BIN || y.e[sum].v != B_ADD) return false;
     const int scaled = y.IsImm(y.e[sum].a, &R->eps) ? y.e[sum].b : y.e[sum].a;
-    if (!y.WithImm(sum, B_ADD, scaled, &R->eps) || !y.WithImm(scaled, B_MUL, y.Make(Symbolic::PART, red_slot[0]), &R->i1)) return false;
+    if (!y.WithImm(sum, B_ADD, scaled, &R->eps) || !y.WithImm(scaled, B_MUL, y.Make(Symbolic::PART, red_slot), &R->i1)) return false;
     y.Run(st.bytecode, st.bsec[4]);
     return y.ok && y.stores.empty();
-  }
-
-  bool StatsAffine() {
-    Cursor c{st.bytecode, st.bsec[1]};
-    if (c.at().opc != OP_COPY || c.at().kind != K_TENSOR) return false;
-    const uint32_t x = c.next().idx;
-    if (c.at().bin(B_SUB) && c.at().scalar_operand()) shift = ScalarOf(c.next(), false);
-    if (c.at().opc == OP_RACC && (c.at().sub >> 4) == R_SUM) red_slot[0] = c.next().sub & 3u;
-    if (c.at().bin(B_MUL) && c.at().kind == K_ACC) {
-      c.next();
-      if (c.at().opc != OP_RACC || (c.at().sub >> 4) != R_SUM) return false;
-      red_slot[1] = c.next().sub & 3u;
-    }
-    if (c.next().opc != OP_END || (red_slot[0] == kRowNone && red_slot[1] == kRowNone)) return false;
-    Cursor d{st.bytecode, st.bsec[3]};
-    if (d.at().opc != OP_COPY || d.at().kind != K_TENSOR || d.next().idx != x) return false;
-    uint32_t stage = 0;   // subtract, multiply, multiply, add: each at most once, in this order
-    for (;;) {
-      const Word w = d.at();
-      if (w.opc != OP_BIN || w.rnd != RN_NONE || !w.scalar_operand()) break;
-      if (w.sub == B_SUB && stage == 0) {
-        chain[0] = ScalarOf(w, false);
-        stage = 1;
-      } else if ((w.sub == B_MUL || (w.sub == B_DIV_FAST && w.kind == K_SREG)) && stage <= 2) {
-        const uint32_t at = stage < 2 ? 1 : 2;
-        chain[at] = ScalarOf(w, w.sub == B_DIV_FAST);
-        stage = at + 1;
-      } else if (w.sub == B_ADD && stage <= 3) {
-        chain[3] = ScalarOf(w, false);
-        stage = 4;
-      } else {
-        return false;
-      }
-      d.next();
-    }
-    uint32_t y = 0;
-    if (!MatchStore(d, P, &y) || d.next().opc != OP_END) return false;
-    if (!Geometry(x) || !Like(y, x, true)) return false;
-    R->form = ROW_STATS_AFFINE;
-    return AddStream(0, x) && AddStream(1, y) && Scalars() && CloseStats();
   }
 
   // ((sigmoid(g)) * g) * u -> store (either order of the two products' operands is what the compiler emits)
@@ -305,7 +182,6 @@ struct Matcher {
   }
 
   bool RmsGate() {
-    if (P.enum_size[kMaxEnum - 2] != 1) return false;
     Cursor c{st.bytecode, st.bsec[1]};
     uint32_t a = 0, b = 0, w = 0, y = 0, g = 0, u = 0, y2 = 0;
     auto sum = [&](Cursor &q, uint32_t *pa, uint32_t *pb) {
@@ -323,8 +199,7 @@ struct Matcher {
       const size_t mark = c.pc;
       if (!body0_done && sum(c, &a, &b) && c.at().bin(B_MUL) && c.at().kind == K_ACC && c.at(1).opc == OP_RACC && (c.at(1).sub >> 4) == R_SUM) {
         c.next();
-        red_slot[0] = c.next().sub & 3u;
-        red_slot[1] = kRowNone;
+        red_slot = c.next().sub & 3u;
         body0_done = true;
         continue;
       }
@@ -338,8 +213,8 @@ struct Matcher {
     uint32_t a1 = 0, b1 = 0;
     R->have_b = 0;
     if (!sum(d, &a1, &b1) || a1 != a || b1 != b || R->have_b != have_b0) return false;
-    if (!d.at().bin(B_MUL) || !d.at().scalar_operand()) return false;
-    chain[1] = ScalarOf(d.next(), false);
+    if (!d.at().bin(B_MUL) || d.at().kind != K_SREG) return false;
+    scale_reg = d.next().idx;
     if (d.at().bin(B_MUL) && d.at().kind == K_TENSOR) {
       w = d.next().idx;
       R->have_w = 1;
@@ -350,13 +225,13 @@ struct Matcher {
       R->have_gate = 1;
     }
     if (d.next().opc != OP_END) return false;
-    if (!Geometry(a) || R->runs != 1 || R->run_len > kRowRmsMaxElems || !Like(y, a, true)) return false;
+    if (!Geometry(a) || R->run_len > kRowRmsMaxElems || !Like(y, a, true)) return false;
     R->form = ROW_RMS_GATE;
     if (!AddStream(0, a) || !AddStream(3, y)) return false;
     if (R->have_b && (!Like(b, a, true) || !AddStream(1, b))) return false;
     if (R->have_w && (!Like(w, a, false) || !AddStream(2, w))) return false;
     if (R->have_gate && (!Like(g, a, true) || !Like(u, a, true) || !Like(y2, a, true) || !AddStream(4, g) || !AddStream(5, u) || !AddStream(6, y2))) return false;
-    return Scalars() && CloseRms();
+    return CloseRms();
   }
 };
 
@@ -381,22 +256,16 @@ void MatchRowKernel(VectorStage *st) {
   const VmParam &P = st->param;
   static const bool off = getenv("DVM_B200_NO_ROW") != nullptr;
   if (off || st->idle || P.mode != VM_GROUP || P.num_body != 2) return;
-  if (Matcher(*st, &R).RmsGate()) return;
-  std::memset(&R, 0, sizeof(R));
-  if (Matcher(*st, &R).StatsAffine()) return;
-  std::memset(&R, 0, sizeof(R));
+  if (!Matcher(*st, &R).RmsGate()) std::memset(&R, 0, sizeof(R));
 }
 
 void BindRow(VectorStage *st) {
   RowParam &R = st->row;
   const VmParam &P = st->param;
-  const uint32_t n = R.form == ROW_STATS_AFFINE ? 2u : static_cast<uint32_t>(kRowMaxStreams);
-  for (uint32_t i = 0; i < n; ++i) {
-    const bool used = R.form == ROW_STATS_AFFINE || i == 0 || i == 3 || (i == 1 && R.have_b) || (i == 2 && R.have_w) || (i >= 4 && R.have_gate);
+  for (int i = 0; i < kRowMaxStreams; ++i) {
+    const bool used = i == 0 || i == 3 || (i == 1 && R.have_b) || (i == 2 && R.have_w) || (i >= 4 && R.have_gate);
     R.stream[i].ptr = used ? P.tensor[R.stream[i].slot].ptr : 0;
   }
-  for (uint32_t s = 0; s < P.n_tensors; ++s)
-    if (R.scalar_of[s] != 0xff) R.scalar[R.scalar_of[s]].ptr = P.tensor[s].ptr;
   st->row_ok = RowAddressesOk(R) && RowKernelPays(R, P.chunk_elems);
 }
 

@@ -1799,7 +1799,7 @@ std::string DisassembleStage(const VectorStage &st) {
   char buf[384];
   const char *kernel = "interpreter";   // what a launch runs, with the addresses bound last; the program is the same
   if (st.row_ok) {
-    kernel = st.row.form == ROW_RMS_GATE ? "row_rms_gate" : "row_stats_affine";
+    kernel = "row_rms_gate";
   } else if (st.direct_ok) {
     kernel = "direct";
   }

@@ -1,4 +1,4 @@
-"""Row kernels: normalisations over runs of any length and alignment, in every split of a group over CTAs, against float64."""
+"""Normalisations over runs of any length and alignment, on the row kernel and on the interpreter, against float64."""
 import os
 
 import numpy as np
@@ -41,8 +41,7 @@ def _batchnorm(shape, dtype, offset=0):
     else:
         stores = [t.store(v) for v in W.batchnorm_train(t, lx, t.load(g), t.load(b), n * h * w)]
     t.run()
-    if not offset and "DVM_B200_NO_ROW" not in os.environ:   # (fp32 inputs have no deviation sums and stay on the interpreter)
-        assert ("kernel=row_stats_affine" in t.das()) == (code != 3)
+    assert "kernel=row" not in t.das()   # (statistics have no kernel of their own)
     read = lambda s: Tester.convert_from_bf16(t.output(s)) if s.dtype() == 2 else t.output(s)
     got = [read(s).astype(np.float64) for s in stores]
     xd = (Tester.convert_from_bf16(x) if code == 2 else x).astype(np.float64)
@@ -58,7 +57,7 @@ def _batchnorm(shape, dtype, offset=0):
     assert np.all(np.abs(got[0] - y) <= {1: 2.0 ** -10, 2: 2.0 ** -8, 3: 2.0 ** -20}[code] * np.abs(y) + slack), float(np.abs(got[0] - y).max())
 
 
-# planes of one unit and less, odd planes, runs that end on a unit, groups of one CTA, two, four and eight CTAs
+# planes of one 16-byte unit and less, odd planes, runs that end on a unit, short groups and long ones
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
 @pytest.mark.parametrize("shape", [(4, 5, 1, 3), (2, 3, 4, 2), (9, 17, 7, 7), (3, 300, 5, 5), (16, 20, 16, 16), (8, 6, 41, 43),
                                    (32, 4, 57, 55), (12, 3, 112, 111), (64, 2, 64, 64), (1, 4, 200, 203)])
@@ -68,7 +67,6 @@ def test_batchnorm_planes(shape, dtype):
 
 @pytest.mark.parametrize("offset", [1, 3, 8])
 def test_batchnorm_input_at_any_address(offset):
-    """(an input whose rows lie unlike the result's relative to 16 bytes goes to the interpreter)"""
     _batchnorm((6, 5, 9, 9), "float16", offset)
 
 
@@ -149,7 +147,7 @@ def test_any_number_of_stored_scalars(stored):
                                         ((4, 2100, 3, 3), (0, 2, 3)), ((3, 5100, 2, 2), (0, 2, 3)), ((2, 2100, 5, 5), (0, 2, 3))])
 @pytest.mark.parametrize("dtype,code", [("float16", 1), ("bfloat16", 2)])
 def test_statistics_of_many_groups(shape, dims, dtype, code):
-    """Group counts and lengths on both sides of the line between the row kernel and the interpreter."""
+    """Short and long groups, few and many, in whole granules and not."""
     from dvm_b200.tester import Tester
     rng = np.random.default_rng(len(shape) + shape[-1])
     raw = rng.standard_normal(shape).astype(np.float32)
@@ -187,7 +185,7 @@ def test_rms_norm_of_many_rows(rows, cols):
 @pytest.mark.parametrize("rows,cols", [(7, 3), (33, 257), (5, 8)])
 def test_other_scalar_sections_run_on_the_interpreter(rows, cols):
     """A sum alone, two group scalars of different types, an immediate factor and a stored 16-bit mean, the result in place of the
-    input: the statistics kernel faulted on [7, 3] when it interpreted such sections."""
+    input: a kernel of its own for statistics, taken out since, faulted on [7, 3]."""
     import torch
     import dvm_b200 as dvm
     g = torch.Generator(device="cuda").manual_seed(5)
