@@ -1,0 +1,66 @@
+"""The build from a checkout that has nothing built, in a copy of the package; nvcc is a stand-in that hands out the library built here."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+BUILT = os.path.join(ROOT, "dvm_b200", "lib", "libdvm_b200.so")
+USE = """
+import dvm_b200 as dvm
+from dvm_b200 import _capi
+r = dvm.IntArrayRef([1])
+r.update([2, 3])
+assert r.shape() == (2, 3)
+k = dvm.PyKernel("vector", "das")
+x = k.load([4, 64], dvm.float32)
+k.store(k.add(x, x))
+k.codegen()
+assert "Add" in k.das()
+"""
+BUILD = "import __graft_entry__ as g\ng.build()\n"
+
+
+@pytest.fixture
+def tree(tmp_path):
+    """(run, library folder): a copy of the sources with nothing built, and what runs a program in it."""
+    skip = shutil.ignore_patterns("lib", "__pycache__")
+    shutil.copytree(os.path.join(ROOT, "dvm_b200"), tmp_path / "dvm_b200", ignore=skip)
+    shutil.copytree(os.path.join(ROOT, "include"), tmp_path / "include")
+    shutil.copy(os.path.join(ROOT, "__graft_entry__.py"), tmp_path)
+    nvcc = tmp_path / "cuda" / "bin" / "nvcc"
+    nvcc.parent.mkdir(parents=True)
+    nvcc.write_text("#!%s\nimport shutil, sys\nto = sys.argv[sys.argv.index('-o') + 1]\n"
+                    "shutil.copy(%r, to) if '-shared' in sys.argv else open(to, 'w').close()\n" % (sys.executable, BUILT))
+    nvcc.chmod(0o755)
+
+    def run(program, **extra):
+        env = {k: v for k, v in os.environ.items() if k != "PYTHONPATH"}
+        env.update({"CUDA_HOME": str(tmp_path / "cuda")}, **extra)
+        r = subprocess.run([sys.executable, "-c", program], cwd=tmp_path, env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        return r.stdout + r.stderr
+
+    return run, tmp_path / "dvm_b200" / "lib"
+
+
+def test_a_checkout_is_built_and_used_in_one_process(tree):
+    run, _ = tree
+    run(BUILD + USE + "assert hasattr(_capi.calls, 'setup')   # (the extension module, not what stands for it)")
+    run(USE)
+
+
+def test_the_build_imports_nothing_that_it_makes(tree):
+    run, _ = tree
+    run("import sys, dvm_b200.build as b\nassert 'dvm_b200._capi' not in sys.modules\nb.build()\n" + USE)
+
+
+def test_names_of_the_package():
+    import dvm_b200
+    for name in dvm_b200.__all__:
+        assert getattr(dvm_b200, name) is not None and name in dir(dvm_b200)
+    assert dvm_b200.float16 is dvm_b200.frontend.DataType.float16 and dvm_b200.kernel is dvm_b200.jit.kernel
+    with pytest.raises(AttributeError):
+        dvm_b200.no_such_name
