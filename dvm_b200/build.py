@@ -4,6 +4,7 @@ Usage: ``python -m dvm_b200.build [--force]``.  Needs nvcc (CUDA >= 12.8) and g+
 sm_100a without a GPU.  The shared library lands in ``dvm_b200/lib/`` next to the package so that it
 travels with the source tree; nothing is installed outside the tree.
 """
+import ctypes
 import os
 import subprocess
 import sys
@@ -61,6 +62,15 @@ def _newer(src, dst):
     return not os.path.exists(dst) or os.path.getmtime(src) > os.path.getmtime(dst)
 
 
+def _loads(path):
+    """False for a file that the loader refuses: cut short, or of another machine."""
+    try:
+        ctypes.CDLL(path)
+    except OSError:
+        return False
+    return True
+
+
 def _deps_mtime():
     latest = 0.0
     for d in (CSRC, os.path.join(HERE, "..", "include")):
@@ -94,13 +104,17 @@ def build(force=False, verbose=False):
         return r
 
     calls_src = os.path.join(CSRC, "py_calls.cc")
-    if force or _newer(calls_src, CALLS_PATH):   # (the front-end's calls into the C ABI; no CUDA in it)
+    calls_new = CALLS_PATH + ".new"   # (takes its place whole, or not at all)
+    calls_job = force or _newer(calls_src, CALLS_PATH) or not _loads(CALLS_PATH)
+    if calls_job:   # (the front-end's calls into the C ABI; no CUDA in it)
         jobs.append(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall", "-Wno-missing-field-initializers",
-                     "-I" + sysconfig.get_paths()["include"], calls_src, "-o", CALLS_PATH])
+                     "-I" + sysconfig.get_paths()["include"], calls_src, "-o", calls_new])
 
     if jobs:
         with ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
             list(ex.map(run, jobs))
+    if calls_job:
+        os.replace(calls_new, CALLS_PATH)
     if jobs or not os.path.exists(LIB_PATH):
         run([_nvcc(), "-shared", "-o", LIB_PATH] + objs + ["-lcudart", "-ldl"])
     return LIB_PATH

@@ -57,6 +57,18 @@ def test_the_build_imports_nothing_that_it_makes(tree):
     run("import sys, dvm_b200.build as b\nassert 'dvm_b200._capi' not in sys.modules\nb.build()\n" + USE)
 
 
+@pytest.mark.parametrize("content", [b"", b"\x7fELF", b"no library"])
+def test_a_damaged_extension_module_is_built_anew(tree, content):
+    run, lib = tree
+    run(BUILD)
+    (module,) = lib.glob("_calls*")
+    size = module.stat().st_size
+    module.write_bytes(content)
+    run(BUILD + USE)
+    assert module.stat().st_size == size and list(lib.glob("_calls*")) == [module]
+    assert run("import dvm_b200.build as b\nb._nvcc = None\nb.subprocess = None\nb.build()") == ""   # (nothing is left to do)
+
+
 def test_names_of_the_package():
     import dvm_b200
     for name in dvm_b200.__all__:
