@@ -131,20 +131,50 @@ SIGNATURES = {
 _lib = None
 
 
-class _NotBuilt:
-    """Stands for the extension module until the build has made it: classes can be declared, load() tells what is missing."""
+class _GeneralCalls:
+    """Stands for the extension module where it could not be built: the same calls through ctypes."""
+
     class IntArray:
-        pass
+        def _attach(self, handle, values):
+            self._held = tuple(values)   # what the native array holds: an update to the same values needs no call
+
+        def update(self, shape):
+            vals = tuple(map(int, shape))
+            if vals != self._held:
+                load().dvm_int_array_update(self._h, (c_int64 * max(1, len(vals)))(*vals), len(vals))
+                self._held = vals
+
+    class ExternalBuf:
+        """Device memory owned by the caller, bound to a load or store."""
+        __slots__ = ("ptr", "nbytes")
+
+        def __init__(self, ptr, nbytes):
+            self.ptr, self.nbytes = int(ptr), int(nbytes)
+
+        def free(self):
+            self.ptr = None
 
     class KernelCalls:
-        pass
+        def bind_device(self, obj, ptr, nbytes):
+            """Use caller-owned device memory for a load or store."""
+            self._bind_device_any(obj, ptr, nbytes)
 
-    ExternalBuf = None
+        def codegen(self, pass_names=None):
+            """Plan for the current shapes and bind the addresses."""
+            self._codegen_any(pass_names)
+
+        def launch(self, stream=None):
+            """Enqueue without synchronising."""
+            self._launch_any(stream)
+
+    @staticmethod
+    def setup(addresses):
+        pass
 
 
 def _load_calls():
     if not os.path.exists(CALLS_PATH):
-        return _NotBuilt
+        return _GeneralCalls
     loader = importlib.machinery.ExtensionFileLoader("dvm_b200._calls", CALLS_PATH)
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader("dvm_b200._calls", loader))
     loader.exec_module(module)
@@ -159,11 +189,10 @@ def load():
     global _lib
     if _lib is not None:
         return _lib
-    for path in (LIB_PATH, CALLS_PATH):
-        if not os.path.exists(path) or (path == CALLS_PATH and calls is _NotBuilt):
-            raise RuntimeError(
-                "dvm_b200: %s is missing; build it with `python -m dvm_b200.build` "
-                "(there is no fallback implementation)" % path)
+    if not os.path.exists(LIB_PATH):
+        raise RuntimeError(
+            "dvm_b200: %s is missing; build it with `python -m dvm_b200.build` "
+            "(there is no fallback implementation)" % LIB_PATH)
     lib = ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL)
     for name, (restype, argtypes) in SIGNATURES.items():
         fn = getattr(lib, name)

@@ -1,7 +1,7 @@
 """In-tree build of libdvm_b200.so (host JIT + sm_100a device interpreters + C ABI) and of the extension module _calls.
 
 Usage: ``python -m dvm_b200.build [--force]``.  Needs nvcc (CUDA >= 12.8) and g++; cross-compiles for
-sm_100a without a GPU.  The shared library lands in ``dvm_b200/lib/`` next to the package so that it
+sm_100a without a GPU.  _calls also takes Python's C headers; without them the package works through ctypes alone.  The shared library lands in ``dvm_b200/lib/`` next to the package so that it
 travels with the source tree; nothing is installed outside the tree.
 """
 import ctypes
@@ -96,7 +96,10 @@ def build(force=False, verbose=False):
             jobs.append(cmd)
 
     def run(cmd):
-        r = subprocess.run(cmd, capture_output=True, text=True)
+        try:
+            r = subprocess.run(cmd, capture_output=True, text=True)
+        except OSError as e:
+            raise RuntimeError("build failed: %s: %s" % (cmd[0], e))
         if r.returncode != 0:
             raise RuntimeError("build failed: %s\n%s\n%s" % (" ".join(cmd), r.stdout, r.stderr))
         if verbose:
@@ -106,15 +109,23 @@ def build(force=False, verbose=False):
     calls_src = os.path.join(CSRC, "py_calls.cc")
     calls_new = CALLS_PATH + ".new"   # (takes its place whole, or not at all)
     calls_job = force or _newer(calls_src, CALLS_PATH) or not _loads(CALLS_PATH)
-    if calls_job:   # (the front-end's calls into the C ABI; no CUDA in it)
-        jobs.append(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall", "-Wno-missing-field-initializers",
-                     "-I" + sysconfig.get_paths()["include"], calls_src, "-o", calls_new])
 
-    if jobs:
-        with ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
-            list(ex.map(run, jobs))
-    if calls_job:
-        os.replace(calls_new, CALLS_PATH)
+    def build_calls():   # (the front-end's calls into the C ABI; no CUDA in it)
+        try:
+            run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall", "-Wno-missing-field-initializers",
+                 "-I" + sysconfig.get_paths()["include"], calls_src, "-o", calls_new])
+            os.replace(calls_new, CALLS_PATH)
+        except RuntimeError as e:
+            if os.path.exists(CALLS_PATH):   # (one of other sources)
+                os.remove(CALLS_PATH)
+            sys.stderr.write("dvm_b200: without the extension module _calls, which takes Python's C headers, a serving loop's steps go "
+                             "through ctypes: slower, with the same results.  %s\n" % e)
+
+    with ThreadPoolExecutor(max_workers=8) as ex:
+        calls = [ex.submit(build_calls)] if calls_job else []
+        list(ex.map(run, jobs))
+        for f in calls:
+            f.result()
     if jobs or not os.path.exists(LIB_PATH):
         run([_nvcc(), "-shared", "-o", LIB_PATH] + objs + ["-lcudart", "-ldl"])
     return LIB_PATH

@@ -4,7 +4,7 @@
 // over seven tensors spent 14 us of 17 in them.  Here such a call goes straight to the C ABI (include/dvm_c.h), whose functions
 // frontend.py hands over once at import.  Only the plain cases are handled: whatever is special - keyword arguments, buffers that the
 // kernel owns, outputs set by the caller, the first call with a graph, errors - goes to the general method of the same purpose in
-// frontend.py.  Replaces the pybind11 methods of the reference's runner (src/pybind_api.cc:195-271, 1066-1116).
+// frontend.py.  Where this module cannot be built (no C headers of Python) everything goes there (_capi.py).  Replaces the pybind11 methods of the reference's runner (src/pybind_api.cc:195-271, 1066-1116).
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 

@@ -3,6 +3,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 import pytest
 
@@ -67,6 +68,23 @@ def test_a_damaged_extension_module_is_built_anew(tree, content):
     run(BUILD + USE)
     assert module.stat().st_size == size and list(lib.glob("_calls*")) == [module]
     assert run("import dvm_b200.build as b\nb._nvcc = None\nb.subprocess = None\nb.build()") == ""   # (nothing is left to do)
+
+
+def test_without_the_headers_of_python(tree):
+    """The library is made, an extension module of before does not stay, and the general methods do the module's work."""
+    run, lib = tree
+    gxx = lib.parent.parent / "bin" / "g++"
+    gxx.parent.mkdir()
+    gxx.write_text("#!/bin/sh\necho 'fatal error: Python.h: No such file or directory' >&2\nexit 1\n")
+    gxx.chmod(0o755)
+    lib.mkdir()
+    (lib / ("_calls" + sysconfig.get_config_var("EXT_SUFFIX"))).write_bytes(b"of other sources")
+    path = str(gxx.parent) + os.pathsep + os.environ["PATH"]
+    assert "Python.h" in run(BUILD + USE, PATH=path)
+    assert (lib / "libdvm_b200.so").exists() and not list(lib.glob("_calls*"))
+    shutil.copy(os.path.join(ROOT, "tests", "test_calls.py"), lib.parent.parent)
+    run("import pytest, sys\nfrom dvm_b200 import _capi\nassert _capi.calls is _capi._GeneralCalls\n"
+        "sys.exit(pytest.main(['-q', '-p', 'no:cacheprovider', 'test_calls.py']))")
 
 
 def test_names_of_the_package():
