@@ -108,12 +108,12 @@ def build(force=False, verbose=False):
 
     calls_src = os.path.join(CSRC, "py_calls.cc")
     calls_new = CALLS_PATH + ".new"   # (takes its place whole, or not at all)
-    calls_job = force or _newer(calls_src, CALLS_PATH) or not _loads(CALLS_PATH)
+    calls_job = force or _newer(calls_src, CALLS_PATH) or hdr_time > os.path.getmtime(CALLS_PATH) or not _loads(CALLS_PATH)
 
     def build_calls():   # (the front-end's calls into the C ABI; no CUDA in it)
         try:
             run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall", "-Wno-missing-field-initializers",
-                 "-I" + sysconfig.get_paths()["include"], calls_src, "-o", calls_new])
+                 "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(HERE, "..", "include"), calls_src, "-o", calls_new])
             os.replace(calls_new, CALLS_PATH)
         except RuntimeError as e:
             if os.path.exists(CALLS_PATH):   # (one of other sources)

@@ -10,24 +10,37 @@
 
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 #include <vector>
+
+#include "dvm.h"
+#include "dvm_c.h"
 
 namespace {
 
 constexpr int kMaxRank = 16;
 constexpr Py_ssize_t kInline = 16;   // values of an int array kept for comparison
 
-// the C ABI
-int (*g_int_array_update)(void *, const int64_t *, size_t) = nullptr;
-int (*g_normalize)(void *) = nullptr;
-int (*g_object_shape)(void *, int64_t *, int) = nullptr;
-int (*g_object_dtype)(void *) = nullptr;
-int (*g_codegen)(void *, const void *, size_t, void *, void *) = nullptr;
-int (*g_launch)(void *, void *) = nullptr;
+// the C ABI: addresses that frontend.py hands over, of the types that the header gives them
+decltype(&dvm_int_array_update) g_int_array_update = nullptr;
+decltype(&dvm_normalize) g_normalize = nullptr;
+decltype(&dvm_object_shape) g_object_shape = nullptr;
+decltype(&dvm_object_dtype) g_object_dtype = nullptr;
+decltype(&dvm_codegen) g_codegen = nullptr;
+decltype(&dvm_launch) g_launch = nullptr;
 
-struct Reloc {   // dvm_reloc
-  void *io, *addr;
-};
+// Bytes of an element; 0 for a type this file does not know.
+long long ItemSize(int type) {
+  switch (type) {
+    case dvm::kBool: return 1;
+    case dvm::kFloat16:
+    case dvm::kBFloat16: return 2;
+    case dvm::kFloat32:
+    case dvm::kInt32: return 4;
+    case dvm::kInt64: return 8;
+  }
+  return 0;
+}
 
 #define DVM_NAMES(X) X(_by_handle) X(_loads) X(_stores) X(_preset) X(_load_offset) X(_relocs) X(_reloc_addr) X(_ws_addr) X(_on_device) X(_k) X(_h) \
   X(_bind_device_any) X(_codegen_any) X(_launch_any)
@@ -49,7 +62,7 @@ struct Ref {
 // ---- IntArray: the base of IntArrayRef ------------------------------------------------------------------------
 struct IntArray {
   PyObject_HEAD
-  void *handle;
+  dvm_int_array *handle;
   Py_ssize_t n;            // values the native array holds (known up to kInline of them), -1: not known
   int64_t vals[kInline];
 };
@@ -89,7 +102,7 @@ PyObject *IntArrayAttach(PyObject *self, PyObject *const *args, Py_ssize_t nargs
   std::vector<int64_t> many;
   const int64_t *v = nullptr;
   if (PyErr_Occurred() || !Values(args[1], &many, a->vals, &v, &a->n)) return nullptr;
-  a->handle = h;
+  a->handle = static_cast<dvm_int_array *>(h);
   if (a->n > kInline) a->n = -1;
   Py_RETURN_NONE;
 }
@@ -202,7 +215,6 @@ PyObject *BindDevice(PyObject *self, PyObject *const *args, Py_ssize_t nargs, Py
 // codegen() of a graph that has been generated before, all of its tensors in memory of the caller that is large enough.
 // 1: done, 0: not such a case (nothing has been bound), -1: failed
 int CodegenFast(PyObject *self) {
-  static const int kItemSize[] = {1, 2, 2, 4, 4, 8};
   Ref dev(PyObject_GetAttr(self, g_name.s_on_device)), preset(PyObject_GetAttr(self, g_name.s_preset)), offset(PyObject_GetAttr(self, g_name.s_load_offset));
   Ref loads(PyObject_GetAttr(self, g_name.s_loads)), stores(PyObject_GetAttr(self, g_name.s_stores)), relocs(PyObject_GetAttr(self, g_name.s_relocs));
   if (dev.p != Py_True || preset.p == nullptr || offset.p == nullptr || loads.p == nullptr || stores.p == nullptr || relocs.p == nullptr) return 0;
@@ -210,8 +222,9 @@ int CodegenFast(PyObject *self) {
   if (!PyList_Check(loads.p) || !PyList_Check(stores.p) || !PyTuple_Check(relocs.p) || PyTuple_GET_SIZE(relocs.p) < 2) return 0;
   const Py_ssize_t n_stores = PyList_GET_SIZE(stores.p), count = n_stores + PyList_GET_SIZE(loads.p);
   if (PyLong_AsSsize_t(PyTuple_GET_ITEM(relocs.p, 1)) != count) return 0;
-  void *const k = Handle(self, g_name.s_k), *const ws = Handle(self, g_name.s_ws_addr);
-  Reloc *const arr = static_cast<Reloc *>(Handle(self, g_name.s_reloc_addr));
+  dvm_kernel *const k = static_cast<dvm_kernel *>(Handle(self, g_name.s_k));
+  const dvm_ws_alloc_fn ws = reinterpret_cast<dvm_ws_alloc_fn>(Handle(self, g_name.s_ws_addr));
+  dvm_reloc *const arr = static_cast<dvm_reloc *>(Handle(self, g_name.s_reloc_addr));
   if (k == nullptr || ws == nullptr || arr == nullptr) return 0;
   auto record = [&](Py_ssize_t i) { return i < n_stores ? PyList_GET_ITEM(stores.p, i) : PyList_GET_ITEM(loads.p, i - n_stores); };
   for (Py_ssize_t i = 0; i < count; ++i) {
@@ -224,11 +237,11 @@ int CodegenFast(PyObject *self) {
     PyObject *rec = record(i);
     const ExternalBuf *b = reinterpret_cast<ExternalBuf *>(PyList_GET_ITEM(rec, 1));
     if (i < n_stores) {
-      void *h = Handle(PyList_GET_ITEM(rec, 0), g_name.s_h);
+      const dvm_object *h = static_cast<const dvm_object *>(Handle(PyList_GET_ITEM(rec, 0), g_name.s_h));
       int64_t dims[kMaxRank];
-      const int rank = h != nullptr ? g_object_shape(h, dims, kMaxRank) : -1, type = h != nullptr ? g_object_dtype(h) : -1;
-      if (rank < 0 || rank > kMaxRank || type < 0 || type > 5) return 0;
-      long long nbytes = kItemSize[type];
+      const int rank = h != nullptr ? g_object_shape(h, dims, kMaxRank) : -1;
+      long long nbytes = h != nullptr ? ItemSize(g_object_dtype(h)) : 0;
+      if (rank < 0 || rank > kMaxRank || nbytes == 0) return 0;
       Ref shape(PyList_New(rank));
       if (shape.p == nullptr) return -1;
       for (int d = 0; d < rank; ++d) {
@@ -263,7 +276,7 @@ PyObject *Codegen(PyObject *self, PyObject *const *args, Py_ssize_t nargs, PyObj
 
 PyObject *Launch(PyObject *self, PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames) {
   if (kwnames == nullptr && (nargs == 0 || (nargs == 1 && (args[0] == Py_None || PyLong_CheckExact(args[0]))))) {
-    void *const k = Handle(self, g_name.s_k);
+    dvm_kernel *const k = static_cast<dvm_kernel *>(Handle(self, g_name.s_k));
     void *stream = nargs == 1 && args[0] != Py_None ? reinterpret_cast<void *>(static_cast<uintptr_t>(PyLong_AsUnsignedLongLongMask(args[0]))) : nullptr;
     if (k != nullptr && !PyErr_Occurred()) {
       int rc = 0;
@@ -292,14 +305,13 @@ PyTypeObject KernelCallsType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
 // setup(addresses): the C ABI, by name
 PyObject *Setup(PyObject *, PyObject *table) {
-  auto get = [&](const char *name, void **to) {
+  auto get = [&](const char *name, auto *to) {
     PyObject *v = PyDict_Check(table) ? PyDict_GetItemString(table, name) : nullptr;
-    *to = v != nullptr ? PyLong_AsVoidPtr(v) : nullptr;
+    *to = reinterpret_cast<std::remove_pointer_t<decltype(to)>>(v != nullptr ? PyLong_AsVoidPtr(v) : nullptr);
     return *to != nullptr;
   };
-  if (!get("dvm_int_array_update", reinterpret_cast<void **>(&g_int_array_update)) || !get("dvm_normalize", reinterpret_cast<void **>(&g_normalize)) ||
-      !get("dvm_object_shape", reinterpret_cast<void **>(&g_object_shape)) || !get("dvm_object_dtype", reinterpret_cast<void **>(&g_object_dtype)) ||
-      !get("dvm_codegen", reinterpret_cast<void **>(&g_codegen)) || !get("dvm_launch", reinterpret_cast<void **>(&g_launch))) {
+  if (!get("dvm_int_array_update", &g_int_array_update) || !get("dvm_normalize", &g_normalize) || !get("dvm_object_shape", &g_object_shape) ||
+      !get("dvm_object_dtype", &g_object_dtype) || !get("dvm_codegen", &g_codegen) || !get("dvm_launch", &g_launch)) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "setup() wants the addresses of the C ABI");
     return nullptr;
   }

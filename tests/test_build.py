@@ -70,6 +70,25 @@ def test_a_damaged_extension_module_is_built_anew(tree, content):
     assert run("import dvm_b200.build as b\nb._nvcc = None\nb.subprocess = None\nb.build()") == ""   # (nothing is left to do)
 
 
+def test_the_extension_module_follows_the_c_abi(tree):
+    """A change of the C ABI's header builds the module anew, and one that its calls do not fit is an error of the compiler."""
+    run, lib = tree
+    run(BUILD)
+    (module,) = lib.glob("_calls*")
+    header = lib.parent.parent / "include" / "dvm_c.h"
+    at = module.stat().st_mtime
+    os.utime(header, (at + 5, at + 5))
+    os.utime(module, (at, at))
+    run(BUILD + USE)
+    assert module.stat().st_mtime != at
+    text, launch = header.read_text(), "int dvm_launch(dvm_kernel *k, void *stream);"
+    assert launch in text
+    header.write_text(text.replace(launch, "int dvm_launch(dvm_kernel *k, void *stream, int priority);"))
+    at = module.stat().st_mtime
+    os.utime(header, (at + 5, at + 5))
+    assert "too few arguments" in run(BUILD + USE) and not module.exists()
+
+
 def test_without_the_headers_of_python(tree):
     """The library is made, an extension module of before does not stay, and the general methods do the module's work."""
     run, lib = tree
