@@ -67,27 +67,33 @@ struct IntArray {
   int64_t vals[kInline];
 };
 
+// tuple(map(int, shape)): into `few` where they fit, else into `many`.  A list or tuple of plain whole numbers is read in place, as nothing
+// can change it meanwhile; the conversion of anything else may run code of any kind and goes through the iterator.
 bool Values(PyObject *shape, std::vector<int64_t> *many, int64_t *few, const int64_t **out, Py_ssize_t *n) {
-  Ref seq(PySequence_Fast(shape, "an iterable of whole numbers is wanted"));
-  if (seq.p == nullptr) return false;
-  *n = PySequence_Fast_GET_SIZE(seq.p);
-  int64_t *to = few;
-  if (*n > kInline) {
-    many->resize(static_cast<size_t>(*n));
-    to = many->data();
+  const getiterfunc iter = Py_TYPE(shape)->tp_iter;
+  const bool list = PyList_Check(shape) && iter == PyList_Type.tp_iter, tuple = PyTuple_Check(shape) && iter == PyTuple_Type.tp_iter;
+  const Py_ssize_t size = list ? PyList_GET_SIZE(shape) : (tuple ? PyTuple_GET_SIZE(shape) : -1);
+  bool plain = size >= 0 && size <= kInline;
+  for (Py_ssize_t i = 0; plain && i < size; ++i) {
+    PyObject *v = list ? PyList_GET_ITEM(shape, i) : PyTuple_GET_ITEM(shape, i);
+    plain = PyLong_CheckExact(v);
+    if (plain) few[i] = static_cast<int64_t>(PyLong_AsUnsignedLongLongMask(v));   // (what ctypes makes of a number beyond 64 bits)
   }
-  for (Py_ssize_t i = 0; i < *n; ++i) {
-    PyObject *v = PySequence_Fast_GET_ITEM(seq.p, i);
-    if (PyLong_CheckExact(v)) {
-      to[i] = static_cast<int64_t>(PyLong_AsUnsignedLongLongMask(v));   // (what ctypes makes of a number beyond 64 bits)
-    } else {
-      Ref whole(PyNumber_Long(v));
-      if (whole.p == nullptr) return false;
-      to[i] = static_cast<int64_t>(PyLong_AsUnsignedLongLongMask(whole.p));
-    }
-    if (PyErr_Occurred()) return false;
+  *out = few;
+  *n = size;
+  if (plain) return true;
+  Ref it(PyObject_GetIter(shape));
+  if (it.p == nullptr) return false;
+  for (;;) {
+    Ref v(PyIter_Next(it.p));
+    if (v.p == nullptr) break;
+    Ref whole(PyNumber_Long(v.p));
+    if (whole.p == nullptr) return false;
+    many->push_back(static_cast<int64_t>(PyLong_AsUnsignedLongLongMask(whole.p)));
   }
-  *out = to;
+  if (PyErr_Occurred()) return false;
+  *out = many->data();
+  *n = static_cast<Py_ssize_t>(many->size());
   return true;
 }
 
@@ -104,6 +110,7 @@ PyObject *IntArrayAttach(PyObject *self, PyObject *const *args, Py_ssize_t nargs
   if (PyErr_Occurred() || !Values(args[1], &many, a->vals, &v, &a->n)) return nullptr;
   a->handle = static_cast<dvm_int_array *>(h);
   if (a->n > kInline) a->n = -1;
+  if (a->n > 0 && v != a->vals) std::memcpy(a->vals, v, sizeof(int64_t) * static_cast<size_t>(a->n));
   Py_RETURN_NONE;
 }
 

@@ -101,3 +101,31 @@ def test_external_buffers():
     assert b.ptr is None
     with pytest.raises(TypeError):
         _ExternalBuf(None, 1)
+
+
+def test_update_of_a_list_that_changes_while_it_is_read():
+    """An element's __int__ may do anything: what counts is what tuple(map(int, shape)) makes of it."""
+    class Whole:
+        def __init__(self, value, act=None):
+            self.value, self.act = value, act
+
+        def __int__(self):
+            if self.act is not None:
+                self.act()
+            return self.value
+
+    for act, want in ((lambda: vals.clear(), (3,)), (lambda: vals.__setitem__(1, 9), (3, 9, 5)), (lambda: vals.extend(range(60)), (3, 4, 5, *range(60)))):
+        r = dvm.IntArrayRef([1])
+        vals = [Whole(3, act), Whole(4), 5]
+        r.update(vals)
+        assert r.shape() == want
+
+
+def test_update_goes_through_the_iterator_of_a_subclass():
+    class Doubled(tuple):
+        def __iter__(self):
+            return (2 * v for v in tuple.__iter__(self))
+
+    r = dvm.IntArrayRef([1])
+    r.update(Doubled((2, 3)))
+    assert r.shape() == (4, 6)
