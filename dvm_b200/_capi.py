@@ -136,7 +136,7 @@ class _GeneralCalls:
 
     class IntArray:
         def _attach(self, handle, values):
-            self._held = tuple(values)   # what the native array holds: an update to the same values needs no call
+            self._held = tuple(map(int, values))   # what the native array holds: an update to the same values needs no call
 
         def update(self, shape):
             vals = tuple(map(int, shape))

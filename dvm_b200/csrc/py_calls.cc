@@ -97,6 +97,12 @@ bool Values(PyObject *shape, std::vector<int64_t> *many, int64_t *few, const int
   return true;
 }
 
+// What the native array now holds.
+void Hold(IntArray *a, const int64_t *v, Py_ssize_t n) {
+  a->n = n <= kInline ? n : -1;
+  if (n > 0 && n <= kInline) std::memcpy(a->vals, v, sizeof(int64_t) * static_cast<size_t>(n));
+}
+
 // _attach(handle, values): the native array, and what it holds
 PyObject *IntArrayAttach(PyObject *self, PyObject *const *args, Py_ssize_t nargs) {
   IntArray *a = reinterpret_cast<IntArray *>(self);
@@ -105,12 +111,13 @@ PyObject *IntArrayAttach(PyObject *self, PyObject *const *args, Py_ssize_t nargs
     return nullptr;
   }
   void *h = PyLong_AsVoidPtr(args[0]);
+  int64_t few[kInline];
   std::vector<int64_t> many;
   const int64_t *v = nullptr;
-  if (PyErr_Occurred() || !Values(args[1], &many, a->vals, &v, &a->n)) return nullptr;
+  Py_ssize_t n = 0;
+  if (PyErr_Occurred() || !Values(args[1], &many, few, &v, &n)) return nullptr;
   a->handle = static_cast<dvm_int_array *>(h);
-  if (a->n > kInline) a->n = -1;
-  if (a->n > 0 && v != a->vals) std::memcpy(a->vals, v, sizeof(int64_t) * static_cast<size_t>(a->n));
+  Hold(a, v, n);
   Py_RETURN_NONE;
 }
 
@@ -132,8 +139,7 @@ PyObject *IntArrayUpdate(PyObject *self, PyObject *const *args, Py_ssize_t nargs
   if (!Values(args[0], &many, few, &v, &n)) return nullptr;
   if (n == a->n && std::memcmp(v, a->vals, sizeof(int64_t) * static_cast<size_t>(n)) == 0) Py_RETURN_NONE;   // (no call for the same values)
   g_int_array_update(a->handle, v, static_cast<size_t>(n));
-  a->n = n <= kInline ? n : -1;
-  if (n <= kInline) std::memcpy(a->vals, v, sizeof(int64_t) * static_cast<size_t>(n));
+  Hold(a, v, n);
   Py_RETURN_NONE;
 }
 

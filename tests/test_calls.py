@@ -129,3 +129,11 @@ def test_update_goes_through_the_iterator_of_a_subclass():
     r = dvm.IntArrayRef([1])
     r.update(Doubled((2, 3)))
     assert r.shape() == (4, 6)
+
+
+def test_a_failed_attach_leaves_what_the_array_is_known_to_hold():
+    r = dvm.IntArrayRef([7, 8])
+    with pytest.raises(TypeError):
+        r._attach(r._h, [9, None])
+    r.update([9, 8])
+    assert r.shape() == (9, 8)
