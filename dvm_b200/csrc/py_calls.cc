@@ -43,7 +43,7 @@ long long ItemSize(int type) {
 }
 
 #define DVM_NAMES(X) X(_by_handle) X(_loads) X(_stores) X(_preset) X(_load_offset) X(_relocs) X(_reloc_addr) X(_ws_addr) X(_on_device) X(_k) X(_h) \
-  X(_bind_device_any) X(_codegen_any) X(_launch_any)
+  X(_bind_device_any) X(_codegen_any) X(_launch_any) X(_launch_result)
 #define DVM_DECLARE(n) PyObject *s##n;
 struct {
   DVM_NAMES(DVM_DECLARE)
@@ -298,8 +298,7 @@ PyObject *Launch(PyObject *self, PyObject *const *args, Py_ssize_t nargs, PyObje
       Py_END_ALLOW_THREADS
       if (rc == 0) Py_RETURN_NONE;
       Ref code(PyLong_FromLong(rc));
-      PyObject *failed[2] = {Py_None, code.p};
-      return code.p == nullptr ? nullptr : General(self, g_name.s_launch_any, failed, 2, nullptr);
+      return code.p == nullptr ? nullptr : General(self, g_name.s_launch_result, &code.p, 1, nullptr);
     }
     PyErr_Clear();
   }

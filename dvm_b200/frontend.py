@@ -793,9 +793,13 @@ class PyKernel(_capi.calls.KernelCalls, Kernel):
         check_rc(self._lib.dvm_launch(self._k, None), "launch")
         check_rc(self._lib.dvm_rt_sync(None), "synchronize")
 
-    def _launch_any(self, stream=None, rc=None):
+    def _launch_any(self, stream=None):
         """launch(): enqueue without synchronising (no counterpart in the reference's Python API)."""
-        check_rc(self._lib.dvm_launch(self._k, stream) if rc is None else rc, "launch")
+        self._launch_result(self._lib.dvm_launch(self._k, stream))
+
+    @staticmethod
+    def _launch_result(rc):
+        check_rc(rc, "launch")
 
     def output(self, store):
         rec = self._find(self._stores, store)

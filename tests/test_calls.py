@@ -137,3 +137,14 @@ def test_a_failed_attach_leaves_what_the_array_is_known_to_hold():
         r._attach(r._h, [9, None])
     r.update([9, 8])
     assert r.shape() == (9, 8)
+
+
+def test_launch_takes_a_stream_and_nothing_else(monkeypatch):
+    """A second argument was the code of a failed launch, and 0 as one of them meant that nothing was launched and nothing said."""
+    k = dvm.PyKernel("vector", "das")
+    launched = []
+    monkeypatch.setattr(k._lib, "dvm_launch", lambda *a: launched.append(a) or 0)
+    for args, kw in (((0, 0), {}), ((None, 3), {}), ((), {"rc": 0}), ((0,), {"rc": None})):
+        with pytest.raises(TypeError):
+            k.launch(*args, **kw)
+    assert not launched
