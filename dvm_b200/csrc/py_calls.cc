@@ -8,6 +8,7 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <climits>
 #include <cstdint>
 #include <cstring>
 #include <type_traits>
@@ -155,6 +156,14 @@ struct ExternalBuf {
   unsigned long long ptr;
   long long nbytes;
   bool gone;
+
+  void Set(PyObject *address, PyObject *size) {   // of two whole numbers; a size beyond 63 bits is the largest there is
+    int beyond = 0;
+    const long long v = PyLong_AsLongLongAndOverflow(size, &beyond);
+    ptr = PyLong_AsUnsignedLongLongMask(address);
+    nbytes = beyond == 0 ? v : (beyond > 0 ? LLONG_MAX : LLONG_MIN);
+    gone = false;
+  }
 };
 int ExternalInit(PyObject *self, PyObject *args, PyObject *) {
   ExternalBuf *b = reinterpret_cast<ExternalBuf *>(self);
@@ -162,10 +171,8 @@ int ExternalInit(PyObject *self, PyObject *args, PyObject *) {
   if (!PyArg_ParseTuple(args, "OO", &p, &n)) return -1;
   Ref ptr(PyNumber_Long(p)), nbytes(ptr.p != nullptr ? PyNumber_Long(n) : nullptr);
   if (nbytes.p == nullptr) return -1;
-  b->ptr = PyLong_AsUnsignedLongLongMask(ptr.p);
-  b->nbytes = PyLong_AsLongLong(nbytes.p);
-  b->gone = false;
-  return PyErr_Occurred() ? -1 : 0;
+  b->Set(ptr.p, nbytes.p);
+  return 0;
 }
 PyObject *ExternalFree(PyObject *self, PyObject *) {
   reinterpret_cast<ExternalBuf *>(self)->gone = true;
@@ -208,13 +215,7 @@ bool BindFast(PyObject *self, PyObject *const *args) {
   if (PyDict_GET_SIZE(table.p) != PyList_GET_SIZE(loads.p) + PyList_GET_SIZE(stores.p)) return false;
   PyObject *rec = PyDict_GetItemWithError(table.p, h.p);   // (borrowed)
   if (rec == nullptr || !PyList_Check(rec) || PyList_GET_SIZE(rec) < 2 || Py_TYPE(PyList_GET_ITEM(rec, 1)) != &ExternalBufType) return false;
-  const unsigned long long ptr = PyLong_AsUnsignedLongLongMask(args[1]);
-  const long long nbytes = PyLong_AsLongLong(args[2]);
-  if (PyErr_Occurred()) return false;
-  ExternalBuf *b = reinterpret_cast<ExternalBuf *>(PyList_GET_ITEM(rec, 1));
-  b->ptr = ptr;
-  b->nbytes = nbytes;
-  b->gone = false;
+  reinterpret_cast<ExternalBuf *>(PyList_GET_ITEM(rec, 1))->Set(args[1], args[2]);
   return true;
 }
 PyObject *BindDevice(PyObject *self, PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames) {

@@ -148,3 +148,19 @@ def test_launch_takes_a_stream_and_nothing_else(monkeypatch):
         with pytest.raises(TypeError):
             k.launch(*args, **kw)
     assert not launched
+
+
+def test_external_buffers_beyond_63_bits():
+    """A size that no memory has is as good as any that is large enough, and a refused one changes nothing."""
+    k, refs, loads, store = _graph()
+    k.codegen()
+    for big in (2 ** 63, 2 ** 64 - 1, 2 ** 70):
+        k.bind_device(store, 0x9000000, big)
+        k.codegen()
+        assert "0x9000000" in k.das() and k.device_ptr(store) == 0x9000000
+    k.bind_device(store, 0x5000000, -2 ** 70)   # (too small)
+    assert k._stores[0][1].nbytes < 0
+    b = _ExternalBuf(64, 7)
+    with pytest.raises(TypeError):
+        b.__init__(128, None)
+    assert (b.ptr, b.nbytes) == (64, 7)
