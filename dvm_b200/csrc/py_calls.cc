@@ -259,7 +259,7 @@ int CodegenFast(PyObject *self) {
       Ref shape(PyList_New(rank));
       if (shape.p == nullptr) return -1;
       for (int d = 0; d < rank; ++d) {
-        nbytes *= dims[d];
+        if (__builtin_mul_overflow(nbytes, dims[d], &nbytes)) return 0;
         PyObject *v = PyLong_FromLongLong(dims[d]);
         if (v == nullptr) return -1;
         PyList_SET_ITEM(shape.p, d, v);

@@ -164,3 +164,33 @@ def test_external_buffers_beyond_63_bits():
     with pytest.raises(TypeError):
         b.__init__(128, None)
     assert (b.ptr, b.nbytes) == (64, 7)
+
+
+def _fake_memory(monkeypatch):
+    """Device allocations as made-up addresses; their sizes."""
+    import dvm_b200.frontend as F
+    made = []
+
+    class Buf:
+        def __init__(self, nbytes):
+            self.nbytes = nbytes
+            self.ptr = 0x40000000 + 0x1000 * len(made)
+            made.append(nbytes)
+
+        def free(self):
+            self.ptr = None
+
+    monkeypatch.setattr(F, "_DevBuf", Buf)
+    return made
+
+
+def test_a_result_larger_than_any_number_of_64_bits_is_not_taken_for_a_small_one(monkeypatch):
+    made = _fake_memory(monkeypatch)
+    k, refs, loads, store = _graph()
+    k.codegen()
+    refs[0].update([2 ** 57, 64])   # 2 ** 65 bytes
+    try:
+        k.codegen()
+    except dvm.DvmError:
+        pass
+    assert made == [2 ** 65]
