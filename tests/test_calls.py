@@ -174,7 +174,7 @@ def _fake_memory(monkeypatch):
     class Buf:
         def __init__(self, nbytes):
             self.nbytes = nbytes
-            self.ptr = 0x40000000 + 0x1000 * len(made)
+            self.ptr = 0x70000000 + 0x1000 * len(made)
             made.append(nbytes)
 
         def free(self):
@@ -194,3 +194,76 @@ def test_a_result_larger_than_any_number_of_64_bits_is_not_taken_for_a_small_one
     except dvm.DvmError:
         pass
     assert made == [2 ** 65]
+
+
+def test_a_buffer_too_small_for_the_new_shape_is_replaced(monkeypatch):
+    made = _fake_memory(monkeypatch)
+    k, refs, loads, store = _graph()
+    k.codegen()
+    k.bind_device(store, 0x9000000, 8 * 64 * 4)
+    k.codegen()
+    assert not made and "0x9000000" in k.das()
+    refs[0].update([9, 64])
+    k.codegen()
+    assert made == [9 * 64 * 4] and k.device_ptr(store) == 0x70000000 and "0x70000000" in k.das() and "0x9000000" not in k.das()
+    refs[0].update([8, 64])
+    k.codegen()   # (the kernel's own memory: the general method, and large enough)
+    assert len(made) == 1 and "0x70000000" in k.das()
+    k.bind_device(store, 0x9000000, 1 << 16)
+    k.codegen()
+    assert "0x9000000" in k.das() and "0x70000000" not in k.das()
+
+
+def test_a_kernel_that_grows_after_its_first_code_generation():
+    k, refs, loads, store = _graph()
+    k.codegen()
+    ref = dvm.IntArrayRef([8, 64])
+    extra = k.load(ref, dvm.float32)
+    second = k.store(k.mul(extra, loads[0]))
+    with pytest.raises(dvm.DvmError):   # (nothing bound to them yet; without a device no memory either)
+        k.codegen()
+    k.bind_device(extra, 0xa000000, 1 << 16)
+    k.bind_device(second, 0xb000000, 1 << 16)
+    for rows in (8, 5):
+        for r in (refs[0], ref):
+            r.update([rows, 64])
+        k.codegen()
+        plan = k.das()
+        assert "0xa000000" in plan and "0xb000000" in plan and k._stores[1][4] == [rows, 64]
+        k._codegen_any()
+        assert k.das() == plan
+
+
+def test_steps_of_several_threads():
+    """A kernel per thread, all stepping at once: the plans of each are those that it makes alone."""
+    import threading
+
+    def steps(at, rounds):
+        k, refs, loads, store = _graph()
+        plans = []
+        for i in range(rounds):
+            rows = 1 + (i * 7 + at) % 40   # (more shapes than plans are kept)
+            refs[0].update([rows, 64])
+            k.bind_device(loads[0], 0x10000000 * (at + 1) + 0x1000 * i, 1 << 16)
+            k.bind_device(store, 0x20000000 * (at + 1) + 0x1000 * i, 1 << 16)
+            k.codegen()
+            plans.append(k.das())
+        return plans
+
+    alone = [steps(at, 60) for at in range(6)]
+    got, failed = [None] * 6, []
+    start = threading.Barrier(6)
+
+    def work(at):
+        try:
+            start.wait(30)
+            got[at] = steps(at, 60)
+        except Exception as e:
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(at,)) for at in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(60)
+    assert not failed and got == alone
