@@ -184,11 +184,6 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-__device__ __forceinline__ uint64_t mul2f(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 __device__ __forceinline__ uint32_t pack_pair(uint32_t dtype, float lo, float hi) {
   if (dtype == T_BF16) return pack_bf16x2(lo, hi);
   const __half2 h = __floats2half2_rn(lo, hi);
@@ -371,10 +366,23 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
       const uint32_t unit = blockIdx.x + it * gridDim.x, bz = unit / qblocks;
       const uint32_t warp_row0 = (unit - bz * qblocks) * unit_rows + g * kTileQ + tile_row;
       float m_used[2] = {-CUDART_INF_F, -CUDART_INF_F};   // of the lane's two rows, in the log2 domain
-      uint64_t sum[2] = {0, 0};                           // ... their sums over the lane's columns, even and odd ones
+      float sum[2] = {0.0f, 0.0f};                        // ... their sums over the lane's columns
+      // A key tile's exponentials are summed by themselves, even and odd columns: a running sum of all keys takes 16 times as many additions,
+      // and like terms round in the same direction.  Added while the warp would wait for the next scores: behind the second half of P the
+      // same additions cost [8, 32, 2048, 64] 425 us instead of 395.
+      uint64_t part[2] = {0, 0};
+      auto fold = [&]() {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float2 h = halves(part[i]);
+          sum[i] += h.x + h.y;
+          part[i] = 0;
+        }
+      };
       for (uint32_t j = 0; j < nkv; ++j, ++n) {
         const uint32_t sb = tiles == 2 ? g : n & 1u;
         const uint32_t t_s = lanes + sb * 128, t_p = P.d > 64 ? t_s : lanes + kTmemP64 + sb * 64;
+        fold();
         mbar_wait(base + kBarSFull + 8 * sb, (tiles == 2 ? n : n >> 1) & 1u, 8, &g_attn_status, epoch);
         tcgen05_after_sync();
         // The scores, rounded to the operand type and (the graph's order) scaled in that type, two at a time: one conversion packs and
@@ -422,7 +430,7 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
             if (raise[i]) {
               alpha[i] = m_used[i] == -CUDART_INF_F ? 0.0f : fast_exp2(m_used[i] - mx[i]);
               m_used[i] = mx[i];
-              sum[i] = mul2f(sum[i], f2(alpha[i], alpha[i]));
+              sum[i] *= alpha[i];
             }
           if (j != 0) {   // O, behind the P V before and in front of the next one
             mbar_wait(base + kBarPvDone + 8 * g, (n - 1) & 1u, 9, &g_attn_status, epoch);
@@ -451,7 +459,7 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
           for (int i = 0; i < 16; ++i) {
             const float2 v = unpack2<DT>(pk[16 * h + i]), t = halves(fma2(f2(v.x, v.y), c2, mneg[i & 1]));
             const float p0 = fast_exp2(t.x), p1 = fast_exp2(t.y);
-            sum[i & 1] = add2(sum[i & 1], f2(p0, p1));
+            part[i & 1] = add2(part[i & 1], f2(p0, p1));
             p[i] = pack_pair(DT, p0, p1);
           }
           tmem_st_pairs(t_p + 32 * h, p);
@@ -461,6 +469,7 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
           if (lane == 0) mbar_arrive(base + kBarPReady + 16 * sb + 8 * h);
         }
       }
+      fold();
       // ---- result: O / l, rounded to the operand type, 64 columns at a time through shared memory to a TMA store
       // (the next unit's first P V overwrites O; it waits for this warp's next P)
       mbar_wait(base + kBarPvDone + 8 * g, (n - 1) & 1u, 10, &g_attn_status, epoch);
@@ -468,8 +477,7 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
       float inv[2];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const float2 h = halves(sum[i]);
-        float l = h.x + h.y;
+        float l = sum[i];
         l += __shfl_xor_sync(0xffffffffu, l, 1);
         l += __shfl_xor_sync(0xffffffffu, l, 2);
         inv[i] = 1.0f / l;

@@ -35,3 +35,24 @@ def test_rising_maxima(batch, sq, skv, d, scale, scale_first):
     # a score of size |s| is rounded twice (relative error of p: 2 |s| unit), p and the result once each
     bound = 2.0 ** -11 * (2.0 * np.abs(s).max(-1, keepdims=True) + 2.0) * float(np.abs(v).max())
     assert np.all(np.abs(got - want) <= bound), float((np.abs(got - want) - bound).max())
+
+
+# one row tile per CTA and two
+@pytest.mark.parametrize("sq", [128, 149 * 128])
+def test_row_sums_of_many_keys(sq):
+    """2 ** 19 keys, all but the first with the same weight: a running fp32 sum that takes them one by one rounds in the same direction
+    every time, by up to 2 ** 16 / 2 units of 2 ** -24 over the lanes; sums per key tile leave 4096 such additions."""
+    from dvm_b200 import workloads as W
+    from dvm_b200.tester import Tester
+    keys, d = 1 << 19, 64
+    score = np.tile(0.25 + 0.1171875 * np.arange(64), sq // 64)   # of the first key; 0 for the others
+    q, k, v = np.zeros((1, 1, sq, d), np.float16), np.zeros((1, 1, keys, d), np.float16), np.zeros((1, 1, keys, d), np.float16)
+    q[0, 0, :, 0] = 8.0 * score
+    k[0, 0, 0, 0], v[0, 0, 0] = 1.0, 32768.0   # (only the first key has values: the result is 32768 over the row's sum)
+    t = Tester("split")
+    st = t.store(W.attention(t, *[t.load(x) for x in (q, k, v)], 0.125, 1))
+    t.run()
+    want = (32768.0 / (1.0 + (keys - 1) * np.exp(-score)))[None, None, :, None]
+    # the result's rounding, and 4096 additions of half a unit each
+    off = np.abs(t.output(st).astype(np.float64) / want - 1.0)
+    assert np.all(off <= 2.0 ** -11 + 4096 * 2.0 ** -25), float(off.max() * 2.0 ** 11)
