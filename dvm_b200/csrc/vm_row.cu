@@ -26,6 +26,7 @@ namespace {
 
 constexpr uint32_t kMaxRowThreads = 512;
 constexpr uint32_t kMaxWarps = kMaxRowThreads / 32;
+constexpr uint32_t kFewRegisters = 72;   // of a thread in the kernels named _few
 
 // ---- residual RMS norm beside a gated product ----------------------------------------------------------------
 // Eight 16-bit elements that start `mis` elements in front of element 0 of `base` plus 8 c (a vector shared by all rows, read
@@ -178,15 +179,18 @@ __device__ __forceinline__ void rms_gate_body(const RowParam &P) {
 
 // Two units per thread: at most 64 registers, so that an SM holds four CTAs of 256 threads and two of 512 (with 72 it was three and one).
 // In us, with 72 | 64 registers: [16384, 4096] with residual and gate 129 | 122, [9000, 7000] 184 | 127, [5000, 6144] 98 | 67 (82 in the
-// interpreter), [8192, 8192] 177 | 127 (161), a plain norm of [16384, 4096] 81 | 70.
-#define DVMB_ROW_RMS(NAME, DT, K, STREAM)                                                            \
-  __global__ void __launch_bounds__(kMaxRowThreads, K == 2 ? 2 : 1) NAME(const __grid_constant__ RowParam P) { rms_gate_body<DT, K, STREAM>(P); }
-DVMB_ROW_RMS(dvm_b200_row_rms_gate_f16_1, T_F16, 1, false)
-DVMB_ROW_RMS(dvm_b200_row_rms_gate_bf16_1, T_BF16, 1, false)
-DVMB_ROW_RMS(dvm_b200_row_rms_gate_f16_2, T_F16, 2, false)
-DVMB_ROW_RMS(dvm_b200_row_rms_gate_bf16_2, T_BF16, 2, false)
-DVMB_ROW_RMS(dvm_b200_row_rms_gate_f16_2_large, T_F16, 2, true)
-DVMB_ROW_RMS(dvm_b200_row_rms_gate_bf16_2_large, T_BF16, 2, true)
+// interpreter), [8192, 8192] 177 | 127 (161), a plain norm of [16384, 4096] 81 | 70.  _few has 72, for launches that are on the chip at
+// once with those as well.
+#define DVMB_ROW_RMS(NAME, DT, K, STREAM, REGISTERS)                                                 \
+  __global__ void REGISTERS NAME(const __grid_constant__ RowParam P) { rms_gate_body<DT, K, STREAM>(P); }
+DVMB_ROW_RMS(dvm_b200_row_rms_gate_f16_1, T_F16, 1, false, __launch_bounds__(kMaxRowThreads))
+DVMB_ROW_RMS(dvm_b200_row_rms_gate_bf16_1, T_BF16, 1, false, __launch_bounds__(kMaxRowThreads))
+DVMB_ROW_RMS(dvm_b200_row_rms_gate_f16_2, T_F16, 2, false, __launch_bounds__(kMaxRowThreads, 2))
+DVMB_ROW_RMS(dvm_b200_row_rms_gate_bf16_2, T_BF16, 2, false, __launch_bounds__(kMaxRowThreads, 2))
+DVMB_ROW_RMS(dvm_b200_row_rms_gate_f16_2_few, T_F16, 2, false, __maxnreg__(kFewRegisters))
+DVMB_ROW_RMS(dvm_b200_row_rms_gate_bf16_2_few, T_BF16, 2, false, __maxnreg__(kFewRegisters))
+DVMB_ROW_RMS(dvm_b200_row_rms_gate_f16_2_large, T_F16, 2, true, __launch_bounds__(kMaxRowThreads, 2))
+DVMB_ROW_RMS(dvm_b200_row_rms_gate_bf16_2_large, T_BF16, 2, true, __launch_bounds__(kMaxRowThreads, 2))
 #undef DVMB_ROW_RMS
 
 namespace {
@@ -256,12 +260,20 @@ int LaunchRow(const RowParam &p_in, void *stream) {
   const bool large = (2ull * p.groups * p.run_len << (p.have_gate ? 1 : 0)) > (128ull << 20);
   const uint32_t block = tg < 128u ? 128u : tg, rows = block / tg;
   using Fn = void (*)(const RowParam);
-  static const Fn fns[2][3] = {{dvm_b200_row_rms_gate_f16_1, dvm_b200_row_rms_gate_f16_2, dvm_b200_row_rms_gate_f16_2_large},
-                               {dvm_b200_row_rms_gate_bf16_1, dvm_b200_row_rms_gate_bf16_2, dvm_b200_row_rms_gate_bf16_2_large}};
-  const Fn fn = fns[p.dtype == T_F16 ? 0 : 1][per_thread == 1 ? 0 : (large ? 2 : 1)];
+  const uint32_t ctas = (p.groups + rows - 1) / rows;
+  // 72 registers where all CTAs are on the chip at once with those too: in us, with 64 | 72, [148, 5000] 3.40 | 3.28, [148, 8192] 3.95 | 3.87,
+  // [1000, 1024] 3.86 | 3.63, [2000, 1024] 5.00 | 4.53; beyond that 64 ([149, 8192] 4.92 | 6.10, [4000, 1024] 7.48 | 7.80).  Except where only
+  // with 64 the CTAs of the next launch find room beside these of 128 threads: [1060 to 1184, 768] 3.4 to 3.6 | 4.0 to 4.1, [1036, 768] 3.30 |
+  // 3.26, [1200, 768] 4.31 | 4.11 (CTAs of 512 threads show no such step).
+  const uint32_t slots = sms * (65536u / (kFewRegisters * block)), slots64 = sms * (65536u / (64u * block));
+  const bool at_once = ctas <= slots && (block == kMaxRowThreads || 2 * ctas <= slots || 2 * ctas > slots64);
+  static const Fn fns[2][4] = {
+    {dvm_b200_row_rms_gate_f16_1, dvm_b200_row_rms_gate_f16_2, dvm_b200_row_rms_gate_f16_2_few, dvm_b200_row_rms_gate_f16_2_large},
+    {dvm_b200_row_rms_gate_bf16_1, dvm_b200_row_rms_gate_bf16_2, dvm_b200_row_rms_gate_bf16_2_few, dvm_b200_row_rms_gate_bf16_2_large}};
+  const Fn fn = fns[p.dtype == T_F16 ? 0 : 1][per_thread == 1 ? 0 : (large ? 3 : (at_once ? 2 : 1))];
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
-  cfg.gridDim = dim3((p.groups + rows - 1) / rows, 1, 1);
+  cfg.gridDim = dim3(ctas, 1, 1);
   cfg.blockDim = dim3(block, 1, 1);
   cfg.stream = static_cast<cudaStream_t>(stream);
   ChainAttribute(&cfg, attr);

@@ -182,6 +182,27 @@ def test_rms_norm_of_many_rows(rows, cols):
     assert np.all(np.abs(got - want) <= 2.0 ** -8 * np.abs(want) + 1e-5)   # (one rounding to bf16)
 
 
+# both sides of the rule for 64 or 72 registers: launches that are on the chip at once, CTAs of 128 threads that leave room for the next's
+@pytest.mark.parametrize("rows,cols", [(1, 4104), (148, 8192), (149, 8192), (75, 5003), (600, 2048), (1036, 1024), (1038, 520), (1184, 768), (1186, 1017),
+                                       (2072, 900), (2074, 1024)])
+@pytest.mark.parametrize("dtype,code", [("float16", 1), ("bfloat16", 2)])
+def test_rms_norm_with_few_and_many_registers(rows, cols, dtype, code):
+    from dvm_b200.tester import Tester
+    rng = np.random.default_rng(rows + cols)
+    raw = [rng.standard_normal((rows, cols)).astype(np.float32) for _ in range(2)]
+    x, r = (v.astype(np.float16) if code == 1 else Tester.convert_to_bf16(v) for v in raw)
+    t = Tester("vector")
+    f = t.add(t.cast(t.load(x, dtype), 3), t.cast(t.load(r, dtype), 3))
+    st = t.store(t.cast(t.mul(f, t.div(1.0, t.sqrt(t.add(t.mul(t.sum(t.mul(f, f), (1,), True), 1.0 / cols), 1e-6)))), code))
+    t.run()
+    assert "kernel=row_rms_gate" in t.das()
+    wide = lambda v: (v if code == 1 else Tester.convert_from_bf16(v)).astype(np.float64)
+    sd = wide(x) + wide(r)
+    want = sd / np.sqrt((sd * sd).mean(1, keepdims=True) + 1e-6)
+    # one rounding of the result, fp32 arithmetic in front of it
+    assert np.all(np.abs(wide(t.output(st)) - want) <= {1: 2.0 ** -11, 2: 2.0 ** -8}[code] * np.abs(want) + 1e-5)
+
+
 @pytest.mark.parametrize("rows,cols", [(7, 3), (33, 257), (5, 8)])
 def test_other_scalar_sections_run_on_the_interpreter(rows, cols):
     """A sum alone, two group scalars of different types, an immediate factor and a stored 16-bit mean, the result in place of the
