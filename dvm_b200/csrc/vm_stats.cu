@@ -236,7 +236,10 @@ uint32_t UnitsPerRun(const StatsParam &p) {
   return static_cast<uint32_t>(RunsWhole(p) ? bytes / 16 : (bytes + 15 + 14) / 16);
 }
 
-constexpr uint32_t kTileUnits = 3136u;                   // of a CTA, four CTAs on an SM
+// A CTA's tile where four CTAs of 256 threads of 64 registers share an SM: a quarter of its shared memory, less the KB that every CTA takes
+// and the header below
+constexpr uint32_t kTileUnits = (228u * 1024u / 4u - 1024u - 8u * kMaxCluster * (256u / 32u)) / 16u;
+constexpr uint32_t kTilePerThread = (kTileUnits + 255u) / 256u;
 constexpr uint32_t kMaxTileUnits = 200u * 1024u / 16u;   // of a CTA: with the header below what an SM has
 
 }  // namespace
@@ -263,18 +266,23 @@ int LaunchStats(const StatsParam &p_in, void *stream) {
   p.units_per_run = UnitsPerRun(p);
   const uint32_t units = p.units_per_run * p.runs;
   // How a group is cut, from launches with 1 to 8 CTAs per group and 1 to 16 units per thread:
-  //  - tiles of 50 KB, four CTAs on an SM: while some wait for their sums others move data ([64, 256, 56, 56] in tiles of 50, 100, 200 KB:
-  //    45, 49, 55 us); smaller ones where the groups alone leave SMs idle ([16, 48, 55, 55] on 1, 2, 4, 8 CTAs: 8.6, 5.7, 5.3, 5.2);
+  //  - tiles of which four fit an SM (55 KB): while some wait for their sums others move data ([64, 256, 56, 56] in tiles of 49, 98, 196 KB: 45,
+  //    49, 55 us; with a limit of 49 instead of 55 KB [9, 800, 56, 56] 18.9 instead of 14.9, [18, 800, 56, 56] 42.5 and 37.9, [38, 440, 27, 27] 13.0
+  //    and 12.1, but [38, 300, 27, 27] 11.1 and 12.0); smaller ones where the groups alone leave SMs idle ([16, 48, 55, 55] on 1, 2, 4, 8 CTAs:
+  //    8.6, 5.7, 5.3, 5.2);
   //  - 8 units per thread: more threads each pay the setup, fewer leave too few warps ([32, 200, 27, 27] with 4, 8, 16: 8.9, 7.0, 8.1;
   //    [64, 1024, 14, 14] with 6, 8, 14: 15.4, 12.9, 14.1); 4 while every CTA has an SM of its own ([16, 128, 28, 28] with 4, 8: 3.4, 3.6);
-  //    14 where tiles of 50 KB queue for SMs, for four of them to fit the registers ([64, 256, 56, 56] with 8 and 14: 51, 45).
+  //    14 where large tiles queue for SMs, for four of them to fit the registers ([64, 256, 56, 56] with 8 and 14: 51, 45);
+  //  - 320 threads where three of them are what an SM gets at most: three fill the registers ([6, 440, 56, 56] 6.6 us, with 14 units per thread 9.3,
+  //    [8, 300, 56, 56] 8.3 and 9.3, [24, 300, 27, 27] 7.9 and 8.3; with 12 units, where that makes 352 threads and two CTAs, up to a third slower).
   uint32_t cluster = 1;
   while (cluster < kMaxCluster && (units > cluster * kTileUnits || (units > cluster * 2048u && static_cast<uint64_t>(p.groups) * cluster < sms))) cluster *= 2;
   p.cluster = cluster;
   p.per_cta = (units + cluster - 1) / cluster;
   const uint64_t ctas = static_cast<uint64_t>(p.groups) * cluster;
-  const uint32_t most = ctas <= sms ? 4u : (p.per_cta <= 2048u || ctas <= 2u * sms ? 8u : 14u);   // units per thread
+  const uint32_t most = ctas <= sms ? 4u : (p.per_cta <= 2048u || ctas <= 2u * sms ? 8u : kTilePerThread);   // units per thread
   uint32_t threads = (p.per_cta + most - 1) / most;
+  if (p.per_cta > 2048u && p.per_cta <= kTileUnits && ctas > 2u * sms && ctas <= 3u * sms) threads = 320u;
   threads = std::min(kMaxThreads, std::max(64u, (threads + 31u) & ~31u));
   const uint32_t per_thread = (p.per_cta + threads - 1) / threads;
   if (per_thread > kMaxPerThread) return -1;

@@ -83,12 +83,14 @@ def _close(pairs, dtype):
         assert bool(((got - ref).abs() <= 1e-4 * ref.abs() + 2e-5).all()), float((got - ref).abs().max())
 
 
-# one unit and less, planes that start anywhere, 4 / 8 / 14 units a thread and one more, 1 to 8 CTAs a group, tiles of 50 KB and above
+# one unit and less, planes that start anywhere, 4 / 8 / 14 units a thread and one more, 1 to 8 CTAs a group, tiles of 55 KB (3552 units) and
+# above, two to four CTAs on an SM
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 @pytest.mark.parametrize("shape", [(1, 3, 1, 2), (2, 5, 1, 3), (3, 2, 2, 4), (5, 4, 3, 3), (4, 300, 5, 5), (7, 40, 7, 7), (2, 150, 16, 16),
                                    (1, 160, 128, 128), (1, 160, 128, 129), (2, 160, 128, 127), (32, 200, 27, 27), (9, 700, 28, 28),
                                    (16, 48, 55, 55), (4, 16, 112, 113), (64, 256, 14, 56), (3, 310, 130, 129), (8, 3, 255, 257),
-                                   (12, 2, 256, 256), (1, 2, 905, 905)])
+                                   (12, 2, 256, 256), (1, 2, 905, 905), (111, 300, 16, 16), (111, 600, 16, 16), (112, 300, 16, 16),
+                                   (65, 444, 16, 16), (65, 445, 16, 16), (38, 300, 27, 27), (38, 500, 27, 27), (222, 160, 16, 16)])
 def test_planes_of_a_channel(shape, dtype):
     kernel, pairs = _run(shape, (0, 2, 3), dtype, gamma="float32", beta="float32")
     assert kernel == "stats_affine"
