@@ -15,7 +15,9 @@ def test_rising_maxima(batch, sq, skv, d, scale, scale_first):
     from dvm_b200 import workloads as W
     from dvm_b200.tester import Tester
     rng = np.random.default_rng(batch + sq + skv + d)
-    q, k, v = (rng.standard_normal((batch, 1, s, d)).astype(np.float16) for s in (sq, skv, skv))
+    # whole numbers and a scale of 1 / 8: every score is exact in fp16, before and after the scale
+    q, k = (rng.integers(-1, 2, (batch, 1, s, d)).astype(np.float16) for s in (sq, skv))
+    v = rng.standard_normal((batch, 1, skv, d)).astype(np.float16)
     # rows 5 of every 16 see scores that grow by more than 8 from key tile to key tile
     q[:, :, 5::16, 0] = np.float16(8.0 * (1.0 if scale >= 0 else -1.0))
     k[:, :, :, 0] = (np.arange(skv) // 64 * 9.0).astype(np.float16)
@@ -32,8 +34,9 @@ def test_rising_maxima(batch, sq, skv, d, scale, scale_first):
     s = q.astype(np.float64) @ np.swapaxes(k.astype(np.float64), -1, -2) * scale
     p = np.exp(s - s.max(-1, keepdims=True))
     want = p @ v.astype(np.float64) / p.sum(-1, keepdims=True)
-    # a score of size |s| is rounded twice (relative error of p: 2 |s| unit), p and the result once each
-    bound = 2.0 ** -11 * (2.0 * np.abs(s).max(-1, keepdims=True) + 2.0) * float(np.abs(v).max())
+    # every p is rounded once (below 2 ** -14 to a multiple of 2 ** -24; the largest of a row is at least 1) and the result once
+    l, size = p.sum(-1, keepdims=True), np.abs(v.astype(np.float64))
+    bound = 2.0 ** -11 * (p @ size / l + np.abs(want)) * 1.01 + 2.0 ** -25 * size.sum(-2, keepdims=True) / l + 2.0 ** -25
     assert np.all(np.abs(got - want) <= bound), float((np.abs(got - want) - bound).max())
 
 
