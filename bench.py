@@ -496,6 +496,8 @@ def measured_sustained():
 
 KERNEL_NAME = {"c1": "dvm_b200_vm_vector_flat", "c2": "dvm_b200_stats_affine_f16_whole_16", "c3": "dvm_b200_row_rms_gate_bf16_2_large",
                "c4": "dvm_b200_attention_bf16", "c5": "dvm_b200_mm_tcgen05_pair"}
+# ... and of another part of the workload, whose size decides which instantiation of the kernel runs
+KERNEL_FAMILY = dict(KERNEL_NAME, c2="dvm_b200_stats_affine_f16_*", c3="dvm_b200_row_rms_gate_bf16_*", c5="dvm_b200_mm_*")
 
 
 def device_summary(name, reps=30):
@@ -767,10 +769,10 @@ def main():
     kernel_us = ms / args.steps * 1e3 / max(1, wl.launches_per_step)
     achieved = work / (ms / args.steps * 1e-3) / unit_scale(name)
     tensor = name in ("c4", "c5")
-    # DRAM bytes per full-size launch from the ncu captures summarised under profiles/ (dram__bytes_read + write; the
-    # quarter-size captures of c1, c3, c4, c5 are scaled by 4: their traffic grows with the leading dimension)
-    traffic = {"c1": 4 * (135.2e6 + 36.0e6), "c2": 195.7e6 + 55.8e6, "c3": 4 * (134.3e6 + 11.5e6),
-               "c4": 4 * (100.7e6 + 7.2e6), "c5": 4 * (520.8e6 + 57.4e6)}.get(name)
+    # DRAM bytes per full-size launch from the ncu captures summarised under profiles/ (dram__bytes_read + write): c2 at full size, c1, c4
+    # and c5 at a quarter and c3 at 9011 of its 16384 rows, where the full size's kernel runs; their traffic grows with the leading dimension
+    traffic = {"c1": 4 * (135.1e6 + 34.2e6), "c2": 102.8e6 + 54.2e6, "c3": (295.3e6 + 109.8e6) * 16384 / 9011,
+               "c4": 4 * (100.8e6 + 8.3e6), "c5": 4 * (523.3e6 + 57.5e6)}.get(name)
     if traffic is not None and args.scale != 1.0:
         traffic *= args.scale
     line = {
@@ -780,7 +782,7 @@ def main():
         "config": config_of(name, algorithmic_bytes_per_step_per_gpu=nbytes, scale=args.scale),
         "roofline": {"bound": "tensor" if tensor else "hbm", "achieved": achieved, "peak": peak, "unit": unit_of(name),
                      "frac": achieved / peak, "traffic": traffic, "traffic_source": "ncu capture (profiles/), bytes per launch",
-                     "peak_source": peak_src, "kernel": KERNEL_NAME[name],
+                     "peak_source": peak_src, "kernel": (KERNEL_NAME if args.scale == 1.0 else KERNEL_FAMILY)[name],
                      "kernel_us": kernel_us, "us_per_launch": {"min": lo, "mean": mean, "max": hi,
                                                                "how": "one event pair per launch (includes the launch latency)"},
                      "frac_of_nominal": achieved / (2250.0 if tensor else 8000.0)},

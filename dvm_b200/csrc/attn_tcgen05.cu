@@ -16,9 +16,10 @@
 //               O / l through shared memory and a TMA store
 // What bounds it: the chain of a row tile, about 3450 cycles per 128 keys where both tiles' MMAs take 2064 and their exponentials 2048:
 // wait 100, scores out of TMEM and rounded 340, maximum 260, exponentials 560 and 900 (the other tile's run meanwhile), the slowest
-// warp and the issuer 400, the rest of P V and the next scores 900.  On [8, 32, 2048, 128] the power cap comes first: 475 us in short
-// runs (495 with P in shared memory and eight softmax warps of 32 rows), 555 among other work (559); with little else on the chip
-// [1, 4, 4096, 128] 41 us (53), [1, 8, 1024, 128] 14.4 (17.0), with d = 64 [8, 32, 2048, 64] 408-424 (474).
+// warp and the issuer 400, the rest of P V and the next scores 900.  On [8, 32, 2048, 128] the power cap comes first: 482 us in short
+// runs (490 with P in shared memory and eight softmax warps of 32 rows, on the same GPU), 557 to 570 among other work (563); with little
+// else on the chip [1, 4, 4096, 128] 41 us (54), [1, 8, 1024, 128] 13.5 (16.8), with d = 64 [8, 32, 2048, 64] 394 (490).
+// 640 threads leave 96 registers each; 12 bytes a thread are spilled, read twice per unit and not per key tile.
 //  - P stays in TMEM: as a tile in shared memory it cost a write and a read of 32 KB per MMA of 512 cycles, which alone fill the 128
 //    bytes a cycle.  With d = 128 it lies over the scores it came from, so the next scores follow P V; a place of its own and one
 //    score buffer for both tiles had every tile wait for the other's scores (547 us with an issuer warp for each, 470-480 with one).
@@ -332,7 +333,9 @@ __device__ __forceinline__ void attention_body(const AttnParam &P, const AttnMap
         wait_kv(v_pos(u, j));
         if (tiles == 2) {
           // The row tiles take turns: while the softmax of one runs, the tensor core has P V and the next scores of the other.
-          // With d = 128 the scores overwrite P: MMAs of one shape run in the order of their issue.
+          // With d = 128 the scores overwrite P, which P V reads: the two MMAs run one after the other because one thread issues them
+          // and they have the same shape and kind.  PTX promises that order for MMAs on one accumulator; that it holds for the tensor
+          // core's queue as a whole is an assumption, one that published attention kernels with P over S make as well.
           for (uint32_t g = 0; g < 2; ++g) {
             issue_pv(g, g, n & 1u, v_pos(u, j), j != 0);
             if (more) issue_s(g, g, u1, j1);

@@ -106,6 +106,12 @@ def test_without_the_headers_of_python(tree):
         "sys.exit(pytest.main(['-q', '-p', 'no:cacheprovider', 'test_calls.py']))")
 
 
+def test_graphs_of_others_load_nothing_of_this_library():
+    """workloads builds its graphs on whatever kernel object it is given (the benchmark's reference arm gives it the reference's)."""
+    code = "import dvm_b200.workloads\nassert not [l for l in open('/proc/self/maps') if 'dvm_b200/lib' in l]"
+    assert subprocess.run([sys.executable, "-c", code], cwd=ROOT).returncode == 0
+
+
 def test_names_of_the_package():
     import dvm_b200
     for name in dvm_b200.__all__:
