@@ -1408,9 +1408,11 @@ int LaunchVector(const VmParam &param, uint32_t grid, uint32_t threads, uint32_t
   }
   // (the 160-thread CTAs run four per SM and need the 96-register build for that)
   static const bool no_r128 = getenv("DVM_B200_NO_R128") != nullptr;
-  const bool r128 = !param.resident && threads > 160 && threads <= 256 && !no_r128;
+  // ... but for 160 consumers without a producer warp (nothing staged), whose chunks may hold several rounds: only r128 walks those
+  const bool looped = param.rounds > 1 || param.cluster > 1;
+  const bool r128 = !param.resident && (threads > 160 || looped) && threads <= 256 && !no_r128;
   if (r128) kernel = param.need_coords ? dvm_b200_vm_vector_nd_r128 : dvm_b200_vm_vector_r128;
-  if ((param.rounds > 1 || param.cluster > 1) && !r128 && !param.resident) return -4;   // (the compiler only plans rounds and clusters for these kernels)
+  if (looped && !r128 && !param.resident) return -4;   // (the compiler only plans rounds and clusters for these kernels)
   if (param.cluster > 1) {
     // A persistent grid of clusters must be resident as a whole: a cluster that has to wait for another one to leave
     // would start its share of the groups only then.  The driver knows how many clusters of this shape fit (fewer than

@@ -206,3 +206,25 @@ def test_element_any(mask, shape):
     b = t.store(t.element_any(t.abs(t.load(a))))
     t.run()
     assert t.output(b)[0] == mask
+
+
+@pytest.mark.parametrize("rows,cols", [(2, 4097), (75, 5003), (300, 4999), (3, 5119), (75, 5121), (5, 10001)])
+@pytest.mark.parametrize("code", [1, 3])
+def test_rows_that_cannot_be_staged(rows, cols, code):
+    """Odd widths: no tensor is staged and no warp feeds a ring, so 4097 to 5119 elements take 160 threads, in chunks of two rounds."""
+    from dvm_b200.tester import Tester
+    rng = np.random.default_rng(cols)
+    x = rng.standard_normal((rows, cols)).astype(np.float16 if code == 1 else np.float32)
+    t = Tester("vector")
+    f = t.load(x)
+    if code == 1:
+        f = t.cast(f, 3)
+    m = t.max(f, (1,), True)
+    e = t.exp(t.sub(f, m))
+    stores = [t.store(t.sum(f, (1,), True)), t.store(t.div(e, t.sum(e, (1,), True)))]
+    t.run()
+    xd = x.astype(np.float64)
+    ed = np.exp(xd - xd.max(1, keepdims=True))
+    # fp32 trees of 16 lanes a thread; 2 ulp of the division and the exponential's 1e-6
+    assert np.allclose(t.output(stores[0]), xd.sum(1, keepdims=True), rtol=1e-5, atol=1e-3)
+    assert np.allclose(t.output(stores[1]), ed / ed.sum(1, keepdims=True), rtol=1e-5, atol=1e-9)
